@@ -48,10 +48,50 @@ size_t blob_stride(const PackSrc& s) {
 
 __device__ __forceinline__ int clampi(int x, int lo, int hi) { return x < lo ? lo : (x > hi ? hi : x); }
 
+// Exclusive prefix of one value per thread over a CTA of kPackThreads, plus the
+// CTA total.
+constexpr int kPackThreads = 512;
+
+__device__ __forceinline__ int pack_exclusive_scan(int v, int* warp_sums, int& total) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int inc = v;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, inc, off);
+        if (lane >= off) inc += o;
+    }
+    if (lane == 31) warp_sums[warp] = inc;
+    __syncthreads();
+    int base = 0, sum = 0;
+#pragma unroll
+    for (int w = 0; w < kPackThreads / 32; ++w) {
+        const int x = warp_sums[w];
+        base += w < warp ? x : 0;
+        sum += x;
+    }
+    __syncthreads();
+    total = sum;
+    return base + inc - v;
+}
+
 // One CTA per problem.  Converts the reference collision_context buffers into
-// the packed blob (see prrtc_device.cuh).  Dynamic shared memory: Q ints.
-__global__ void pack_kernel(PackSrc s, unsigned char* blobs, size_t stride, int cap) {
-    extern __shared__ int s_dense[];
+// the packed blob (see prrtc_device.cuh).
+//
+// Bound by the latency of its dependent loads, not by bytes (a few KB per
+// problem), so every table goes in one pass with one row per thread (rows of
+// different tables on different warps, their loads in flight together), the
+// dense-block test reads its pairs with a warp per coarse pair from operands
+// already in shared memory, and the item lists are written at offsets from a
+// scan.  One problem, cold caches: 25.5 -> 9.5 us (arm, tabletop scene) and
+// 55.8 -> 15.6 us (dual arm, large scene) against the tables one after the
+// other, one thread per coarse pair walking its 64 pairs and one thread writing
+// the lists (16 warps: the dual arm's 131 coarse pairs take 9 rounds).  512
+// problems at once: 23.3 -> 21.0 us.
+__global__ void __launch_bounds__(kPackThreads) pack_kernel(PackSrc s, unsigned char* blobs, size_t stride, int cap) {
+    __shared__ int warp_sums[kPackThreads / 32];
+    __shared__ int4 t_blk[kPackThreads];   // (a0, na, b0, nb) of a tile of coarse pairs; na = 0: not a block
+    __shared__ int t_r0[kPackThreads];
+    __shared__ int t_dense[kPackThreads];
     const int b = blockIdx.x, tid = threadIdx.x, T = blockDim.x;
     unsigned char* blob = blobs + (size_t)b * stride;
     BlobHeader* h = reinterpret_cast<BlobHeader*>(blob);
@@ -65,7 +105,7 @@ __global__ void pack_kernel(PackSrc s, unsigned char* blobs, size_t stride, int 
     const float* wc = s.wc + (s.wc_cnt ? (size_t)b * s.wc_max * 7 : 0);
     const float* wbx = s.wb + (s.wb_cnt ? (size_t)b * s.wb_max * 15 : 0);
     const float* wh = s.wh + (s.wh_cnt ? (size_t)b * s.wh_max * 6 : 0);
-    const int* sp = s.sp + (s.sp_cnt ? (size_t)b * s.sp_max * 2 : 0);
+    const int* __restrict__ sp = s.sp + (s.sp_cnt ? (size_t)b * s.sp_max * 2 : 0);
     const int J = s.J, S = s.S, K = s.K, Q = s.Q;
     const BlobLayout L = blob_layout(J, S, K, Q, s.sp_max, s.ws_max, s.wc_max, s.wb_max, s.wh_max);
 
@@ -76,139 +116,176 @@ __global__ void pack_kernel(PackSrc s, unsigned char* blobs, size_t stride, int 
     bool gated = enabled && coarse_ok && (s.mode == 2 || (s.mode == 3 && J <= 16));
 
     JointRec* jr = reinterpret_cast<JointRec*>(blob + L.o_joint);
-    for (int j = tid; j < J; j += T)
-        jr[j] = make_joint_rec(j, s.ptf, s.twists, s.parent, s.act, s.mmul, s.moff, s.mact, s.dim);
     float4* sph = reinterpret_cast<float4*>(blob + L.o_sph);
     int* sfr = reinterpret_cast<int*>(blob + L.o_sfr);
-    for (int i = tid; i < S; i += T) {
-        sph[i] = make_float4(s.sloc[i * 3], s.sloc[i * 3 + 1], s.sloc[i * 3 + 2], s.srad[i]);
-        const int li = s.sli[i];
-        int f = (li >= 0 && li < J) ? (s.topo_inv ? s.topo_inv[li] : li) : -1;
-        sfr[i] = (f >= 0 && f < J) ? f : -1;
-    }
     float4* grp = reinterpret_cast<float4*>(blob + L.o_grp);
-    for (int k = tid; k < K; k += T) {
-        grp[2 * k] = make_float4(s.cloc[k * 3], s.cloc[k * 3 + 1], s.cloc[k * 3 + 2], s.crad[k]);
-        const int li = s.cli[k];
-        int f = (li >= 0 && li < J) ? (s.topo_inv ? s.topo_inv[li] : li) : -1;
-        if (f >= J) f = -1;
-        const int s0 = s.foff ? clampi(s.foff[k], 0, S) : 0;
-        const int s1 = s.foff ? clampi(s.foff[k + 1], 0, S) : 0;
-        grp[2 * k + 1] = make_float4(__int_as_float(f), __int_as_float(s0), __int_as_float(s1), 0.0f);
-    }
-    // world primitives, pre-conditioned for the FMA-form tests (prrtc_device.cuh)
     float4* o_ws = reinterpret_cast<float4*>(blob + L.o_ws);
-    for (int i = tid; i < Ns; i += T) {
-        const float x = ws[i * 4], y = ws[i * 4 + 1], z = ws[i * 4 + 2], r = ws[i * 4 + 3];
-        o_ws[2 * i] = make_float4(-2.0f * x, -2.0f * y, -2.0f * z, -2.0f * r);
-        o_ws[2 * i + 1] = make_float4(x, y, z, fmaf(x, x, fmaf(y, y, fmaf(z, z, -r * r))));
-    }
     float4* o_wc = reinterpret_cast<float4*>(blob + L.o_wc);
-    for (int i = tid; i < Nc; i += T) {
-        const float* c = &wc[i * 7];
-        const float dx = c[3] - c[0], dy = c[4] - c[1], dz = c[5] - c[2];
-        const float l2 = dx * dx + dy * dy + dz * dz;
-        const float il2 = l2 > 0.0f ? 1.0f / l2 : 0.0f;
-        const float px = dx * il2, py = dy * il2, pz = dz * il2;
-        o_wc[3 * i] = make_float4(c[0], c[1], c[2], c[6]);
-        o_wc[3 * i + 1] = make_float4(px, py, pz, -(px * c[0] + py * c[1] + pz * c[2]));
-        o_wc[3 * i + 2] = make_float4(dx, dy, dz, 0.0f);
-    }
     float4* o_wb = reinterpret_cast<float4*>(blob + L.o_wb);
-    for (int i = tid; i < Nb; i += T) {
-        const float* c = &wbx[i * 15];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const float ax = c[3 + 3 * k], ay = c[4 + 3 * k], az = c[5 + 3 * k];
-            const float off = -(ax * c[0] + ay * c[1] + az * c[2]);
-            o_wb[4 * i + k] = make_float4(ax * kBoxInv, ay * kBoxInv, az * kBoxInv, off * kBoxInv);
-        }
-        o_wb[4 * i + 3] = make_float4(c[12] * kBoxInv, c[13] * kBoxInv, c[14] * kBoxInv, 0.0f);
-    }
     float4* o_wh = reinterpret_cast<float4*>(blob + L.o_wh);
-    for (int i = tid; i < Nh; i += T) {
-        const float* c = &wh[i * 6];
-        o_wh[i] = make_float4(c[0], c[1], c[2], -(c[0] * c[3] + c[1] * c[4] + c[2] * c[5]));
-    }
     int2* cp = reinterpret_cast<int2*>(blob + L.o_cpair);
-    for (int q = tid; q < Q; q += T) cp[q] = make_int2(s.cpairs[2 * q], s.cpairs[2 * q + 1]);
-    // dense-block detection: coarse pair q's range is the row-major product of
-    // its two groups' fine ranges
-    for (int q = tid; q < Q; q += T) {
-        int dense = 0;
-        if (coarse_ok && s.cranges) {
-            const int ci = s.cpairs[2 * q], cj = s.cpairs[2 * q + 1];
-            const int r0 = s.cranges[2 * q], r1 = s.cranges[2 * q + 1];
-            if (ci >= 0 && cj >= 0 && ci < K && cj < K && r0 >= 0 && r1 <= P && r0 <= r1) {
-                const int a0 = clampi(s.foff[ci], 0, S), a1 = clampi(s.foff[ci + 1], 0, S);
-                const int b0 = clampi(s.foff[cj], 0, S), b1 = clampi(s.foff[cj + 1], 0, S);
-                const int na = a1 - a0, nb = b1 - b0;
-                if (na > 0 && nb > 0 && nb <= 0xffff && r1 - r0 == na * nb) {
-                    dense = 1;
-                    for (int m = 0; m < na * nb && dense; ++m) {
-                        const int pi = sp[2 * (r0 + m)], pj = sp[2 * (r0 + m) + 1];
-                        if (pi != a0 + m / nb || pj != b0 + m % nb) dense = 0;
-                    }
-                }
+    // rows of every table in one index space, each table starting at a multiple
+    // of 32 so that a warp holds rows of one table
+    const int e0 = (J + 31) & ~31, e1 = e0 + ((S + 31) & ~31), e2 = e1 + ((K + 31) & ~31), e3 = e2 + ((Ns + 31) & ~31),
+              e4 = e3 + ((Nc + 31) & ~31), e5 = e4 + ((Nb + 31) & ~31), e6 = e5 + ((Nh + 31) & ~31), e7 = e6 + Q;
+    for (int r = tid; r < e7; r += T) {
+        if (r < e0) {
+            if (r < J) jr[r] = make_joint_rec(r, s.ptf, s.twists, s.parent, s.act, s.mmul, s.moff, s.mact, s.dim);
+        } else if (r < e1) {
+            const int i = r - e0;
+            if (i < S) {
+                sph[i] = make_float4(s.sloc[i * 3], s.sloc[i * 3 + 1], s.sloc[i * 3 + 2], s.srad[i]);
+                const int li = s.sli[i];
+                int f = (li >= 0 && li < J) ? (s.topo_inv ? s.topo_inv[li] : li) : -1;
+                sfr[i] = (f >= 0 && f < J) ? f : -1;
             }
-        }
-        s_dense[q] = dense;
-    }
-    __syncthreads();
-    if (tid == 0) {
-        int4* sch = reinterpret_cast<int4*>(blob + L.o_sch);
-        int n_sch = 0;
-        if (gated) {
-            for (int k = 0; k < K; ++k) {
-                const int s0 = clampi(s.foff[k], 0, S), s1 = clampi(s.foff[k + 1], 0, S);
-                for (int a = s0; a < s1 && n_sch < L.sch_cap; a += kSphChunk)
-                    sch[n_sch++] = make_int4(a, min(kSphChunk, s1 - a), k, 0);
+        } else if (r < e2) {
+            const int k = r - e1;
+            if (k < K) {
+                grp[2 * k] = make_float4(s.cloc[k * 3], s.cloc[k * 3 + 1], s.cloc[k * 3 + 2], s.crad[k]);
+                const int li = s.cli[k];
+                int f = (li >= 0 && li < J) ? (s.topo_inv ? s.topo_inv[li] : li) : -1;
+                if (f >= J) f = -1;
+                const int s0 = s.foff ? clampi(s.foff[k], 0, S) : 0;
+                const int s1 = s.foff ? clampi(s.foff[k + 1], 0, S) : 0;
+                grp[2 * k + 1] = make_float4(__int_as_float(f), __int_as_float(s0), __int_as_float(s1), 0.0f);
+            }
+        } else if (r < e3) {  // world primitives, pre-conditioned for the FMA-form tests (prrtc_device.cuh)
+            const int i = r - e2;
+            if (i < Ns) {
+                const float x = ws[i * 4], y = ws[i * 4 + 1], z = ws[i * 4 + 2], rad = ws[i * 4 + 3];
+                o_ws[2 * i] = make_float4(-2.0f * x, -2.0f * y, -2.0f * z, -2.0f * rad);
+                o_ws[2 * i + 1] = make_float4(x, y, z, fmaf(x, x, fmaf(y, y, fmaf(z, z, -rad * rad))));
+            }
+        } else if (r < e4) {
+            const int i = r - e3;
+            if (i < Nc) {
+                const float* c = &wc[i * 7];
+                const float dx = c[3] - c[0], dy = c[4] - c[1], dz = c[5] - c[2];
+                const float l2 = dx * dx + dy * dy + dz * dz;
+                const float il2 = l2 > 0.0f ? 1.0f / l2 : 0.0f;
+                const float px = dx * il2, py = dy * il2, pz = dz * il2;
+                o_wc[3 * i] = make_float4(c[0], c[1], c[2], c[6]);
+                o_wc[3 * i + 1] = make_float4(px, py, pz, -(px * c[0] + py * c[1] + pz * c[2]));
+                o_wc[3 * i + 2] = make_float4(dx, dy, dz, 0.0f);
+            }
+        } else if (r < e5) {
+            const int i = r - e4;
+            if (i < Nb) {
+                const float* c = &wbx[i * 15];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const float ax = c[3 + 3 * k], ay = c[4 + 3 * k], az = c[5 + 3 * k];
+                    const float off = -(ax * c[0] + ay * c[1] + az * c[2]);
+                    o_wb[4 * i + k] = make_float4(ax * kBoxInv, ay * kBoxInv, az * kBoxInv, off * kBoxInv);
+                }
+                o_wb[4 * i + 3] = make_float4(c[12] * kBoxInv, c[13] * kBoxInv, c[14] * kBoxInv, 0.0f);
+            }
+        } else if (r < e6) {
+            const int i = r - e5;
+            if (i < Nh) {
+                const float* c = &wh[i * 6];
+                o_wh[i] = make_float4(c[0], c[1], c[2], -(c[0] * c[3] + c[1] * c[4] + c[2] * c[5]));
             }
         } else {
-            for (int a = 0; a < S && n_sch < L.sch_cap; a += kSphChunk)
-                sch[n_sch++] = make_int4(a, min(kSphChunk, S - a), -1, 0);
+            const int q = r - e6;
+            cp[q] = make_int2(s.cpairs[2 * q], s.cpairs[2 * q + 1]);
         }
-        int4* item = reinterpret_cast<int4*>(blob + L.o_item);
-        int n_items = 0;
-        bool use_ranges = gated;
-        if (!gated && coarse_ok && s.cranges && Q > 0) {
-            // flat checker: reuse the range decomposition when the ranges tile [0, P)
-            int cursor = 0;
-            use_ranges = true;
-            for (int q = 0; q < Q; ++q) {
-                if (s.cranges[2 * q] != cursor) { use_ranges = false; break; }
-                cursor = s.cranges[2 * q + 1];
+    }
+    // sphere chunks of at most kSphChunk: per group (gated; K <= kMaxLinks), else of the whole list
+    int4* sch = reinterpret_cast<int4*>(blob + L.o_sch);
+    int n_sch = 0;
+    if (gated) {
+        int s0 = 0, s1 = 0;
+        if (tid < K) {
+            s0 = clampi(s.foff[tid], 0, S);
+            s1 = clampi(s.foff[tid + 1], 0, S);
+        }
+        int at = pack_exclusive_scan(s1 > s0 ? cdiv(s1 - s0, kSphChunk) : 0, warp_sums, n_sch);
+        for (int a = s0; a < s1 && at < L.sch_cap; a += kSphChunk) sch[at++] = make_int4(a, min(kSphChunk, s1 - a), tid, 0);
+        n_sch = min(n_sch, L.sch_cap);
+    } else {
+        n_sch = min(cdiv(S, kSphChunk), L.sch_cap);
+        for (int i = tid; i < n_sch; i += T) sch[i] = make_int4(i * kSphChunk, min(kSphChunk, S - i * kSphChunk), -1, 0);
+    }
+    // self-pair items: the range decomposition of the coarse pairs, which a flat
+    // checker reuses when the ranges tile [0, P)
+    int4* item = reinterpret_cast<int4*>(blob + L.o_item);
+    bool use_ranges = gated;
+    if (!gated && coarse_ok && s.cranges && Q > 0) {
+        int bad = 0;
+        for (int q = tid; q < Q; q += T) bad |= s.cranges[2 * q] != (q > 0 ? s.cranges[2 * q - 1] : 0);
+        use_ranges = __syncthreads_or(bad) == 0 && s.cranges[2 * Q - 1] == P;
+    }
+    int n_items = 0;
+    bool overflow = false;
+    if (use_ranges) {
+        const int warp = tid >> 5, lane = tid & 31;
+        for (int q0 = 0; q0 < Q && !overflow; q0 += T) {
+            const int q = q0 + tid, nq = min(T, Q - q0);
+            int r0 = 0, r1 = 0, a0 = 0, na = 0, b0 = 0, nb = 0;
+            bool cand = false;
+            if (q < Q) {
+                const int x0 = s.cranges ? s.cranges[2 * q] : 0, x1 = s.cranges ? s.cranges[2 * q + 1] : 0;
+                r0 = clampi(x0, 0, P);
+                r1 = clampi(x1, 0, P);
+                const int ci = s.cpairs[2 * q], cj = s.cpairs[2 * q + 1];
+                if (coarse_ok && s.cranges && ci >= 0 && cj >= 0 && ci < K && cj < K && x0 >= 0 && x1 <= P && x0 <= x1) {
+                    a0 = clampi(s.foff[ci], 0, S);
+                    na = clampi(s.foff[ci + 1], 0, S) - a0;
+                    b0 = clampi(s.foff[cj], 0, S);
+                    nb = clampi(s.foff[cj + 1], 0, S) - b0;
+                    cand = na > 0 && nb > 0 && nb <= 0xffff && x1 - x0 == na * nb;
+                }
+                t_blk[tid] = make_int4(a0, cand ? na : 0, b0, nb);
+                t_r0[tid] = x0;
             }
-            if (cursor != P) use_ranges = false;
-        }
-        bool overflow = false;
-        if (use_ranges) {
-            for (int q = 0; q < Q && !overflow; ++q) {
+            __syncthreads();
+            // dense-block detection: the range is the row-major product of the pair's two groups
+            // (two loads per lane cover a block of 8 x 8; unrolled, so that the loads of four pairs are in flight)
+#pragma unroll 4
+            for (int k = warp; k < nq; k += kPackThreads / 32) {
+                const int4 blk = t_blk[k];
+                const int* src = sp + 2 * (size_t)t_r0[k];
+                const int total = blk.y * blk.w;
+                bool ok = total > 0;
+                if (lane < total) {
+                    const int pi = __ldg(src + 2 * lane), pj = __ldg(src + 2 * lane + 1);
+                    ok = pi == blk.x + lane / blk.w && pj == blk.z + lane % blk.w;
+                }
+                for (int m = lane + 32; m < total; m += 32) {
+                    const int pi = __ldg(src + 2 * m), pj = __ldg(src + 2 * m + 1);
+                    ok = ok && pi == blk.x + m / blk.w && pj == blk.z + m % blk.w;
+                }
+                ok = __all_sync(0xffffffffu, ok);
+                if (lane == 0) t_dense[k] = ok ? 1 : 0;
+            }
+            __syncthreads();
+            const bool dense = q < Q && t_dense[tid];
+            const int n = q < Q ? (dense ? cdiv(na, kSphChunk) : cdiv(r1 > r0 ? r1 - r0 : 0, kPairChunk)) : 0;
+            int tile_total;
+            int at = n_items + pack_exclusive_scan(n, warp_sums, tile_total);
+            n_items += tile_total;
+            overflow = n_items > L.item_cap;  // uniform
+            if (!overflow && q < Q) {
                 const int gate = gated ? q : -1;
-                const int r0 = clampi(s.cranges[2 * q], 0, P), r1 = clampi(s.cranges[2 * q + 1], 0, P);
-                if (s_dense[q]) {
-                    const int ci = s.cpairs[2 * q], cj = s.cpairs[2 * q + 1];
-                    const int a0 = clampi(s.foff[ci], 0, S), a1 = clampi(s.foff[ci + 1], 0, S);
-                    const int b0 = clampi(s.foff[cj], 0, S), b1 = clampi(s.foff[cj + 1], 0, S);
-                    for (int a = a0; a < a1; a += kSphChunk) {
-                        if (n_items >= L.item_cap) { overflow = true; break; }
-                        item[n_items++] = make_int4(a, b0, (min(kSphChunk, a1 - a) << 16) | (b1 - b0), gate);
-                    }
+                if (dense) {
+                    for (int a = a0; a < a0 + na; a += kSphChunk)
+                        item[at++] = make_int4(a, b0, (min(kSphChunk, a0 + na - a) << 16) | nb, gate);
                 } else {
-                    for (int p = r0; p < r1; p += kPairChunk) {
-                        if (n_items >= L.item_cap) { overflow = true; break; }
-                        item[n_items++] = make_int4(p, -1, min(kPairChunk, r1 - p), gate);
-                    }
+                    for (int p = r0; p < r1; p += kPairChunk) item[at++] = make_int4(p, -1, min(kPairChunk, r1 - p), gate);
                 }
             }
         }
-        if (!use_ranges || overflow) {
-            n_items = 0;
-            for (int p = 0; p < P; p += kPairChunk) item[n_items++] = make_int4(p, -1, min(kPairChunk, P - p), -1);
-            if (overflow) {  // fall back to the flat sweep; verdicts are identical
-                gated = false;
-            }
-        }
+    }
+    if (!use_ranges || overflow) {
+        n_items = cdiv(P, kPairChunk);
+        __syncthreads();  // an overflowing list's writes come first
+        for (int i = tid; i < n_items; i += T)
+            item[i] = make_int4(i * kPairChunk, -1, min(kPairChunk, P - i * kPairChunk), -1);
+        if (overflow) gated = false;  // fall back to the flat sweep; verdicts are identical
+    }
+    if (tid == 0) {
         BlobHeader hd;
         hd.J = J; hd.dim = s.dim; hd.S = S; hd.S_pad = odd_pad(S);
         hd.K = K; hd.Q = Q; hd.Ns = Ns; hd.Nc = Nc;
@@ -227,8 +304,7 @@ __global__ void pack_kernel(PackSrc s, unsigned char* blobs, size_t stride, int 
 
 cudaError_t launch_pack(const PackSrc& s, int batch, unsigned char* blobs, size_t stride, cudaStream_t st) {
     if (batch <= 0) return cudaSuccess;
-    const size_t smem = (size_t)std::max(s.Q, 1) * sizeof(int);
-    pack_kernel<<<batch, 256, smem, st>>>(s, blobs, stride, (int)stride);
+    pack_kernel<<<batch, kPackThreads, 0, st>>>(s, blobs, stride, (int)stride);
     return cudaGetLastError();
 }
 
