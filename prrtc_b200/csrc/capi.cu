@@ -12,6 +12,7 @@
 
 #include "../../include/prrtc_b200.h"
 #include "kernels.h"
+#include "prrtc_cull.cuh"
 #include "prrtc_device.cuh"
 
 using namespace prrtc;
@@ -108,7 +109,7 @@ static bool cloud_ok(const prrtc_point_cloud_t* c) {
 }
 
 static Tuned tuned(const prrtc_tuning_t* t) {
-    Tuned o{0.0f, 128, 16, 0, nullptr, nullptr, 1, 0, 0, {nullptr, nullptr}};
+    Tuned o{0.0f, 0, 16, 0, nullptr, nullptr, 1, 0, 0, {nullptr, nullptr}};
     if (t) {
         if (t->edge_resolution > 0.0f) o.edge_res = t->edge_resolution;
         if (t->threads_per_explorer == 32 || t->threads_per_explorer == 64 || t->threads_per_explorer == 128 ||
@@ -136,6 +137,8 @@ static void fill_launch(PlanLaunch& L, const prrtc_outputs_t* out, const prrtc_a
     L.connection = out->connection_info; L.solved = out->solved_flag; L.ktime = out->kernel_time_ms;
     L.E = a->num_new_samples; L.N = a->max_nodes; L.dim = a->dim;
     L.J = s.J; L.S = s.S; L.K = s.K; L.Q = s.Q;
+    L.n_obs = s.ws_max + s.wc_max + s.wb_max + s.wh_max;
+    L.cull = s.foff && cull_shape_ok(s.J, s.K, L.n_obs, s.mode == 1 ? s.margin : 0.0f) ? 1 : 0;
     L.max_iter = a->max_iterations; L.balance_mode = a->balance_mode; L.dd = a->dynamic_domain ? 1 : 0;
     L.granularity = a->granularity; L.step = a->step_size; L.tree_ratio = a->tree_ratio;
     L.dd_alpha = a->dd_alpha; L.dd_radius = a->dd_radius; L.dd_min_radius = a->dd_min_radius;

@@ -65,11 +65,14 @@ struct PlanLaunch {
     int32_t* queue;                    // [3]: head, error, tail-join ticket
     // shape
     int B, E, N, dim, J, S, K, Q;
+    int n_obs;                         // most world primitives of a problem
+    int cull;                          // the shapes allow the culled edge check (prrtc_cull.cuh)
+    int cw_general;                    // pass size of the general checker for its scenes that are not culled (set by launch_plan)
     // attributes
     int max_iter, balance_mode, dd, granularity;
     float step, tree_ratio, dd_alpha, dd_radius, dd_min_radius, edge_res;
     // tuning
-    int threads, cw, resident;
+    int threads, cw, resident;         // threads 0: chosen by launch_plan
     int persistent;
     int tail_join;                     // persistent form: idle CTAs join running problems as extra explorers
     int wait_polls;                    // polls of the scene-staging wait before it gives up (0: default, <0: none)

@@ -31,6 +31,7 @@
 #include <mutex>
 
 #include "kernels.h"
+#include "prrtc_cull.cuh"
 #include "prrtc_device.cuh"
 
 namespace prrtc {
@@ -38,6 +39,7 @@ namespace prrtc {
 #ifndef PRRTC_EXPLORE_MINBLOCKS
 #define PRRTC_EXPLORE_MINBLOCKS 2  // resident 256-thread explorer CTAs per SM the register allocation must allow
 #endif
+constexpr int kWideThreads = 512;  // explorer size of the wide form (one CTA per SM)
 
 // ============================================================================ pack
 
@@ -92,6 +94,8 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(PackSrc s, unsigned 
     __shared__ int4 t_blk[kPackThreads];   // (a0, na, b0, nb) of a tile of coarse pairs; na = 0: not a block
     __shared__ int t_r0[kPackThreads];
     __shared__ int t_dense[kPackThreads];
+    __shared__ unsigned s_scale;  // bits of the largest coordinate size (L1) of a world primitive
+    __shared__ int s_cull;
     const int b = blockIdx.x, tid = threadIdx.x, T = blockDim.x;
     unsigned char* blob = blobs + (size_t)b * stride;
     BlobHeader* h = reinterpret_cast<BlobHeader*>(blob);
@@ -114,6 +118,12 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(PackSrc s, unsigned 
         J > 0 && J <= kMaxJoints && S > 0 && (Ns > 0 || Nc > 0 || Nb > 0 || Nh > 0 || P > 0 || s.has_cloud);
     const bool coarse_ok = K > 0 && K <= kMaxLinks && s.foff != nullptr;
     bool gated = enabled && coarse_ok && (s.mode == 2 || (s.mode == 3 && J <= 16));
+    if (tid == 0) {
+        s_scale = 0u;
+        s_cull = enabled && coarse_ok && J <= 32 && !(s.mode == 1 && !(s.margin >= 0.0f)) && s.foff[0] == 0 && s.foff[K] == S;
+    }
+    __syncthreads();
+    auto note_size = [&](float l1) { atomicMax(&s_scale, __float_as_uint(l1) & 0x7fffffffu); };  // NaN orders above all
 
     JointRec* jr = reinterpret_cast<JointRec*>(blob + L.o_joint);
     float4* sph = reinterpret_cast<float4*>(blob + L.o_sph);
@@ -154,6 +164,7 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(PackSrc s, unsigned 
             const int i = r - e2;
             if (i < Ns) {
                 const float x = ws[i * 4], y = ws[i * 4 + 1], z = ws[i * 4 + 2], rad = ws[i * 4 + 3];
+                note_size(fabsf(x) + fabsf(y) + fabsf(z) + fabsf(rad));
                 o_ws[2 * i] = make_float4(-2.0f * x, -2.0f * y, -2.0f * z, -2.0f * rad);
                 o_ws[2 * i + 1] = make_float4(x, y, z, fmaf(x, x, fmaf(y, y, fmaf(z, z, -rad * rad))));
             }
@@ -162,6 +173,7 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(PackSrc s, unsigned 
             if (i < Nc) {
                 const float* c = &wc[i * 7];
                 const float dx = c[3] - c[0], dy = c[4] - c[1], dz = c[5] - c[2];
+                note_size(fabsf(c[0]) + fabsf(c[1]) + fabsf(c[2]) + fabsf(dx) + fabsf(dy) + fabsf(dz) + fabsf(c[6]));
                 const float l2 = dx * dx + dy * dy + dz * dz;
                 const float il2 = l2 > 0.0f ? 1.0f / l2 : 0.0f;
                 const float px = dx * il2, py = dy * il2, pz = dz * il2;
@@ -179,18 +191,64 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(PackSrc s, unsigned 
                     const float off = -(ax * c[0] + ay * c[1] + az * c[2]);
                     o_wb[4 * i + k] = make_float4(ax * kBoxInv, ay * kBoxInv, az * kBoxInv, off * kBoxInv);
                 }
-                o_wb[4 * i + 3] = make_float4(c[12] * kBoxInv, c[13] * kBoxInv, c[14] * kBoxInv, 0.0f);
+                // distances along the axes bound distances only for orthonormal axes (or shorter ones)
+                bool ok = true;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const float* u = c + 3 + 3 * k;
+                    const float* v = c + 3 + 3 * ((k + 1) % 3);
+                    ok = ok && u[0] * u[0] + u[1] * u[1] + u[2] * u[2] <= 1.0002f &&
+                         fabsf(u[0] * v[0] + u[1] * v[1] + u[2] * v[2]) <= 1e-4f;
+                }
+                note_size(fabsf(c[0]) + fabsf(c[1]) + fabsf(c[2]) + fabsf(c[12]) + fabsf(c[13]) + fabsf(c[14]));
+                o_wb[4 * i + 3] = make_float4(c[12] * kBoxInv, c[13] * kBoxInv, c[14] * kBoxInv, ok ? 0.0f : 1.0f);
             }
         } else if (r < e6) {
             const int i = r - e5;
             if (i < Nh) {
                 const float* c = &wh[i * 6];
                 o_wh[i] = make_float4(c[0], c[1], c[2], -(c[0] * c[3] + c[1] * c[4] + c[2] * c[5]));
+                note_size(fabsf(c[3]) + fabsf(c[4]) + fabsf(c[5]));
+                if (!(c[0] * c[0] + c[1] * c[1] + c[2] * c[2] <= 1.0002f)) atomicAnd(&s_cull, 0);
             }
         } else {
             const int q = r - e6;
             cp[q] = make_int2(s.cpairs[2 * q], s.cpairs[2 * q + 1]);
         }
+    }
+    // cull spheres (prrtc_cull.cuh): a link's reach about its coarse centre plus
+    // the scene's share of the pad, 8 lanes per link; infinite when the reach is
+    // not finite, too large or a radius is negative, so that nothing is culled
+    __syncthreads();  // s_scale
+    if (coarse_ok) {
+        const int k = tid >> 3, l8 = tid & 7;
+        const bool mine = k < K;
+        float reach = 0.0f;
+        bool ok = true, own = true;
+        if (mine) {
+            const int f0 = s.foff[k], f1 = s.foff[k + 1];
+            own = f0 >= 0 && f1 >= f0 && f1 <= S && s.cli[k] >= 0 && s.cli[k] < J;
+            const float cx = s.cloc[3 * k], cy = s.cloc[3 * k + 1], cz = s.cloc[3 * k + 2];
+            reach = fabsf(s.crad[k]);
+            for (int i = clampi(f0, 0, S) + l8; i < clampi(f1, 0, S); i += 8) {
+                const float dx = s.sloc[3 * i] - cx, dy = s.sloc[3 * i + 1] - cy, dz = s.sloc[3 * i + 2] - cz;
+                const float x = sqrtf(dx * dx + dy * dy + dz * dz) + s.srad[i];
+                ok = ok && s.srad[i] >= 0.0f && x <= kCullReachMax;
+                own = own && s.sli[i] == s.cli[k];
+                reach = fmaxf(reach, x);
+            }
+            if (s.topo_inv && own) own = s.topo_inv[s.cli[k]] >= 0 && s.topo_inv[s.cli[k]] < J;
+        }
+#pragma unroll
+        for (int off = 4; off > 0; off >>= 1) reach = fmaxf(reach, __shfl_xor_sync(0xffffffffu, reach, off));
+        const unsigned all_ok = __ballot_sync(0xffffffffu, ok) >> (tid & 24) & 0xffu;
+        if (mine && l8 == 0) {
+            const float pad = kCullPad * (1.0f + __uint_as_float(s_scale));
+            const float r = reach * 1.00001f + pad;
+            reinterpret_cast<float*>(grp + 2 * k + 1)[3] =
+                all_ok == 0xffu && reach <= kCullReachMax && r < 1e6f ? r : INFINITY;
+        }
+        if (mine && !own) atomicAnd(&s_cull, 0);
     }
     // sphere chunks of at most kSphChunk: per group (gated; K <= kMaxLinks), else of the whole list
     int4* sch = reinterpret_cast<int4*>(blob + L.o_sch);
@@ -268,7 +326,8 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(PackSrc s, unsigned 
             n_items += tile_total;
             overflow = n_items > L.item_cap;  // uniform
             if (!overflow && q < Q) {
-                const int gate = gated ? q : -1;
+                // gate of a gated checker; a flat checker's block keeps its coarse pair as -2 - q
+                const int gate = gated ? q : (dense ? -2 - q : -1);
                 if (dense) {
                     for (int a = a0; a < a0 + na; a += kSphChunk)
                         item[at++] = make_int4(a, b0, (min(kSphChunk, a0 + na - a) << 16) | nb, gate);
@@ -285,6 +344,7 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(PackSrc s, unsigned 
             item[i] = make_int4(i * kPairChunk, -1, min(kPairChunk, P - i * kPairChunk), -1);
         if (overflow) gated = false;  // fall back to the flat sweep; verdicts are identical
     }
+    __syncthreads();  // s_cull
     if (tid == 0) {
         BlobHeader hd;
         hd.J = J; hd.dim = s.dim; hd.S = S; hd.S_pad = odd_pad(S);
@@ -297,7 +357,8 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(PackSrc s, unsigned 
         hd.o_joint = L.o_joint; hd.o_sph = L.o_sph; hd.o_sfr = L.o_sfr; hd.o_grp = L.o_grp;
         hd.o_sch = L.o_sch; hd.o_ws = L.o_ws; hd.o_wc = L.o_wc; hd.o_wb = L.o_wb;
         hd.o_wh = L.o_wh; hd.o_item = L.o_item; hd.o_cpair = L.o_cpair; hd.used_bytes = L.bytes;
-        hd.P = P; hd.cap_bytes = cap; hd.error = overflow ? kBlobItemOverflow : 0; hd.pad0 = 0;
+        hd.P = P; hd.cap_bytes = cap; hd.error = overflow ? kBlobItemOverflow : 0;
+        hd.cull = s_cull && !overflow ? 1 : 0;
         *h = hd;
     }
 }
@@ -312,37 +373,47 @@ cudaError_t launch_pack(const PackSrc& s, int batch, unsigned char* blobs, size_
 
 // ============================================================================ nearest neighbour
 
-// Group-wide argmin of the squared distance from q (shared memory) over nodes
-// [0, n) of the SoA tree (row stride N).  dsq = d0*d0, then fma(dd, dd, dsq) in
-// dimension order -- bit-identical to the reference's `dsq += diff*diff`
-// (prrtc_planner.cu:845-849) under nvcc's default contraction.  Result:
-// red_d[0], red_i[0] (INT_MAX when no valid node).
-template <class G>
-__device__ void group_nearest(const G& grp, const float* __restrict__ tree, int N, int dim, int n, const float* q,
-                              float* red_d, int* red_i) {
-    const int tid = grp.rank(), T = grp.size();
+// Argmin of the squared distance from q (shared memory) over nodes [0, n) of the
+// SoA tree (row stride N), by the whole CTA.  dsq = d0*d0, then fma(dd, dd, dsq)
+// in dimension order -- bit-identical to the reference's `dsq += diff*diff`
+// (prrtc_planner.cu:845-849) under nvcc's default contraction (the chain starts
+// from +0, which leaves d0*d0 as it is).  Valid in warp 0: the node (INT_MAX when
+// there is none) in the low word, the bits of its squared distance in the high
+// one; ties go to the lowest index, NaN slots never win.
+//
+// A scan of the usual small tree (hundreds of nodes) is one round trip to L2
+// and a reduction, so the loads of 8 dimensions go out together, a warp reduces
+// with two integer minima (a non-negative float orders like its bits) instead
+// of ten shuffles, and warp 0 alone reduces over the warps, without a second
+// barrier.  Out of line: the extend and the connect step share the code.
+static __device__ __noinline__ unsigned long long group_nearest(const float* __restrict__ tree, int N, int dim, int n,
+                                                                const float* q, unsigned* red_d, int* red_i) {
+    const int tid = threadIdx.x, T = blockDim.x;
     float best = INFINITY;
     int bi = INT_MAX;
-    float qr[kDimMax];
-#pragma unroll
-    for (int d = 0; d < kDimMax; ++d) qr[d] = d < dim ? q[d] : 0.0f;
     if ((N & 3) == 0 && (reinterpret_cast<uintptr_t>(tree) & 15) == 0) {
         const int n4 = (n + 3) >> 2;
         const float4* t4 = reinterpret_cast<const float4*>(tree);
         const size_t row4 = (size_t)(N >> 2);
         for (int g = tid; g < n4; g += T) {
-            float4 v = __ldcg(t4 + g);
-            float dx = __fsub_rn(v.x, qr[0]), dy = __fsub_rn(v.y, qr[0]), dz = __fsub_rn(v.z, qr[0]),
-                  dw = __fsub_rn(v.w, qr[0]);
-            float ax = __fmul_rn(dx, dx), ay = __fmul_rn(dy, dy), az = __fmul_rn(dz, dz), aw = __fmul_rn(dw, dw);
+            float ax = 0.0f, ay = 0.0f, az = 0.0f, aw = 0.0f;
+            for (int d0 = 0; d0 < dim; d0 += 8) {
+                float4 v[8];
+                float qr[8];
 #pragma unroll
-            for (int d = 1; d < kDimMax; ++d) {
-                if (d < dim) {
-                    v = __ldcg(t4 + d * row4 + g);
-                    dx = __fsub_rn(v.x, qr[d]); dy = __fsub_rn(v.y, qr[d]);
-                    dz = __fsub_rn(v.z, qr[d]); dw = __fsub_rn(v.w, qr[d]);
-                    ax = __fmaf_rn(dx, dx, ax); ay = __fmaf_rn(dy, dy, ay);
-                    az = __fmaf_rn(dz, dz, az); aw = __fmaf_rn(dw, dw, aw);
+                for (int k = 0; k < 8; ++k) {
+                    const int d = min(d0 + k, dim - 1);
+                    v[k] = __ldcg(t4 + d * row4 + g);
+                    qr[k] = q[d];
+                }
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    if (d0 + k < dim) {
+                        const float dx = __fsub_rn(v[k].x, qr[k]), dy = __fsub_rn(v[k].y, qr[k]);
+                        const float dz = __fsub_rn(v[k].z, qr[k]), dw = __fsub_rn(v[k].w, qr[k]);
+                        ax = __fmaf_rn(dx, dx, ax); ay = __fmaf_rn(dy, dy, ay);
+                        az = __fmaf_rn(dz, dz, az); aw = __fmaf_rn(dw, dw, aw);
+                    }
                 }
             }
             const int i0 = g << 2;
@@ -353,36 +424,27 @@ __device__ void group_nearest(const G& grp, const float* __restrict__ tree, int 
         }
     } else {
         for (int i = tid; i < n; i += T) {
-            float dd = __fsub_rn(__ldcg(tree + i), qr[0]);
-            float acc = __fmul_rn(dd, dd);
-            for (int d = 1; d < dim; ++d) {
-                dd = __fsub_rn(__ldcg(tree + (size_t)d * N + i), qr[d]);
+            float acc = 0.0f;
+            for (int d = 0; d < dim; ++d) {
+                const float dd = __fsub_rn(__ldcg(tree + (size_t)d * N + i), q[d]);
                 acc = __fmaf_rn(dd, dd, acc);
             }
             if (acc < best) { best = acc; bi = i; }
         }
     }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        const float od = __shfl_xor_sync(0xffffffffu, best, off);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
-        if (od < best || (od == best && oi < bi)) { best = od; bi = oi; }
-    }
-    const int warp = tid >> 5, lane = tid & 31, nwarp = (T + 31) >> 5;
-    if (lane == 0) { red_d[warp] = best; red_i[warp] = bi; }
-    grp.sync();
+    const int warp = tid >> 5, lane = tid & 31, nwarp = T >> 5;
+    unsigned key = __float_as_uint(best);
+    unsigned m = __reduce_min_sync(0xffffffffu, key);
+    unsigned i = __reduce_min_sync(0xffffffffu, key == m ? (unsigned)bi : (unsigned)INT_MAX);
+    if (lane == 0) { red_d[warp] = m; red_i[warp] = (int)i; }
+    __syncthreads();
     if (warp == 0) {
-        best = lane < nwarp ? red_d[lane] : INFINITY;
+        key = lane < nwarp ? red_d[lane] : 0x7f800000u;
         bi = lane < nwarp ? red_i[lane] : INT_MAX;
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const float od = __shfl_xor_sync(0xffffffffu, best, off);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
-            if (od < best || (od == best && oi < bi)) { best = od; bi = oi; }
-        }
-        if (lane == 0) { red_d[0] = best; red_i[0] = bi; }
+        m = __reduce_min_sync(0xffffffffu, key);
+        i = __reduce_min_sync(0xffffffffu, key == m ? (unsigned)bi : (unsigned)INT_MAX);
     }
-    grp.sync();
+    return (unsigned long long)m << 32 | i;
 }
 
 // ============================================================================ explorer
@@ -420,12 +482,14 @@ __device__ __forceinline__ Prob prob_ptrs(const PlanLaunch& L, int b) {
 }
 
 struct ExplorerSmem {
-    float sample[kDimMax], base[kDimMax], cand[kDimMax], delta[kDimMax], curr[kDimMax], vec[kDimMax];
-    float red_d[32];
+    float sample[2][kDimMax];  // this iteration's and the next one's
+    float base[kDimMax], cand[kDimMax], delta[kDimMax], curr[kDimMax], vec[kDimMax];
+    unsigned red_d[32];
     int red_i[32];
     int order[16];
     int halton[kDimMax];
     int stop, t, n_t, n_o, nn, skip, new_idx, n_ext, ext_parent, ext_idx, G1, G2, vamp, cnn, abort_;
+    int pre, pre_solved, pre_a, pre_b;  // solved flag and tree sizes read ahead for the next iteration
     int slot, problem, join_e;
 };
 
@@ -453,8 +517,8 @@ __device__ int tail_join_pick(const PlanLaunch& L, int* e_out) {
 // verdict (any waypoint in collision) does not depend on the order.
 // The waypoints are computed inside the checker's FK step (no staging pass).
 template <class Grp>
-__device__ bool group_edge_collides(const Grp& grp, const Scene& sc, const CcBufs& B, const float* base,
-                                    const float* delta, int G, int CW, int& par) {
+__device__ __forceinline__ bool group_edge_collides(const Grp& grp, const Scene& sc, const CcBufs& B, const float* base,
+                                                    const float* delta, int G, int CW, int& par) {
     if (B.stats && grp.rank() == 0) atomicAdd(&B.stats[kStatEdges], 1ull);
     const int nchunk = (G + CW - 1) / CW;
     for (int c = 0; c < nchunk; ++c) {
@@ -465,80 +529,188 @@ __device__ bool group_edge_collides(const Grp& grp, const Scene& sc, const CcBuf
     return false;
 }
 
+// Edge checker of the general form: any robot and coarse model.
+struct GeneralEdges {
+    CcBufs B;
+    Scene sc;
+    int CW;
+    int par;
+    __device__ __forceinline__ void reset() {
+        if (threadIdx.x == 0) B.hit[0] = B.hit[1] = 0u;  // the checker's two result words
+        par = 0;
+    }
+    template <class Grp>
+    __device__ __forceinline__ bool collides(const Grp& grp, const float* base, const float* delta, int G) {
+        return group_edge_collides(grp, sc, B, base, delta, G, CW, par);
+    }
+};
+
+// A scene that the culled check does not take (BlobHeader::cull not set: groups
+// that do not cover the spheres on their own frames, ...), in the culled
+// kernel: the general checker in the same shared memory, CW waypoints at a
+// time.  Out of line, so that its registers and code stay off the main path.
+static __device__ __noinline__ bool general_edge_collides(const unsigned char* blob, const int2* pairs, const PcView* pc,
+                                                   unsigned char* smem, unsigned long long* stats, const float* base,
+                                                   const float* delta, int G, int CW) {
+    Scene sc = scene_view(blob);
+    sc.pairs = pairs;
+    sc.pc = *pc;
+    CcBufs B = cc_bufs(smem, sc.h->J, sc.h->S, sc.h->K, sc.h->Q, CW);
+    B.stats = stats;
+    __syncthreads();
+    if (threadIdx.x == 0) B.hit[0] = B.hit[1] = 0u;
+    __syncthreads();
+    int par = 0;
+    const bool r = group_edge_collides(CtaGroup{}, sc, B, base, delta, G, CW, par);
+    __syncthreads();
+    return r;
+}
+
+// Edge checker of the culled form (prrtc_cull.cuh).  One out-of-line copy
+// serves the extend and the connect step: less code to fetch, and the
+// explorer's own registers are saved around the call.  The buffers are
+// addressed from the dynamic shared memory itself, so that their accesses stay
+// shared-memory instructions.  Returns the answer in bit 0 and the next `par` in
+// bit 1.
+struct CulledEdges {  // in shared memory
+    const int2* pairs;
+    PcView pc;
+    unsigned long long* stats;
+    int blob_cap, J, K, n_obs, CW, CW_general;
+};
+
+static __device__ __noinline__ int culled_edge_collides(const CulledEdges* a, const float* base, const float* delta, int G,
+                                                 int par) {
+    extern __shared__ __align__(128) unsigned char dsm[];
+    Scene sc = scene_view(dsm);
+    if (!sc.h->cull) {
+        if (!sc.h->enabled) {
+            __syncthreads();  // as a check does: the caller rewrites what the last one read
+            return par << 1;
+        }
+        return (general_edge_collides(dsm, a->pairs, &a->pc, dsm + a->blob_cap, a->stats, base, delta, G, a->CW_general)
+                    ? 1 : 0) | par << 1;
+    }
+    CullBufs B = cull_bufs(dsm + a->blob_cap, a->J, a->K, a->n_obs, a->CW, true);
+    B.stats = a->stats;
+    sc.pairs = a->pairs;
+    sc.pc = a->pc;
+    if (B.stats && threadIdx.x == 0) atomicAdd(&B.stats[kStatEdges], 1ull);
+    const int nchunk = (G + a->CW - 1) / a->CW;
+    for (int c = 0; c < nchunk; ++c) {
+        const int nw = (G - c + nchunk - 1) / nchunk;
+        const EdgeSrc e{base, delta, G, nchunk, c};
+        if (cull_check<true>(CtaGroup{}, sc, B, nw, a->CW, par, &e) != 0u) return 1 | par << 1;
+    }
+    return par << 1;
+}
+
+struct CulledEdgesRef {
+    const CulledEdges* a;
+    uint32_t* hit;
+    int par;
+    __device__ __forceinline__ void reset() {
+        if (threadIdx.x < 6) hit[threadIdx.x] = 0u;
+        par = 0;
+    }
+    template <class Grp>
+    __device__ __forceinline__ bool collides(const Grp&, const float* base, const float* delta, int G) {
+        const int r = culled_edge_collides(a, base, delta, G, par);
+        par = r >> 1;
+        return (r & 1) != 0;
+    }
+};
+
 __device__ __forceinline__ void stamp_end(const Prob& P) {
     atomicCAS(&P.ts[1], 0ull, globaltimer());
 }
 
 // One explorer (problem P, index e of E) until the problem terminates or the
 // explorer exits.  All threads of the group call it.
-template <class Grp>
-__device__ void run_explorer(const Grp& grp, const PlanLaunch& L, const Prob& P, const Scene& sc, const CcBufs& B,
-                             ExplorerSmem& X, int e) {
+template <class Grp, class Edges>
+__device__ __forceinline__ void run_explorer(const Grp& grp, const PlanLaunch& L, const Prob& P, Edges& edges,
+                                             ExplorerSmem& X, int e) {
     const int tid = grp.rank();
     const int dim = L.dim, N = L.N;
     if (tid == 0) {
         prime_order(e, X.order);
         for (int d = 0; d < kDimMax; ++d) X.halton[d] = 1;
         X.vamp = 0;
-        B.hit[0] = B.hit[1] = 0u;  // the checker's two result words
+        X.pre = 0;
     }
+    edges.reset();
     grp.sync();
-    int par = 0;  // which hit word the next checker call uses (same in every thread)
+    // The next iteration's sample depends on the explorer alone, so another warp
+    // than the one that waits for the problem's state draws it meanwhile.
+    const int sampler = grp.size() > 32 ? 32 : 0;
+    auto draw = [&](int lane, float* out) {  // halton_sample, one dimension per lane
+        if (lane < dim) {
+            const float val = halton_next(X.order[lane & 15], X.halton[lane]);
+            out[lane] = __fmaf_rn(val, __fsub_rn(L.hi[lane], L.lo[lane]), L.lo[lane]);
+        }
+    };
+    if (tid >= sampler && tid < sampler + 32) draw(tid - sampler, X.sample[1]);
     int local_iter = 0;
     // The per-iteration scalar work runs on warp 0 with one lane per dimension
-    // (Halton digits, extend, connect vector); lane 0 does the rest.  Every lane
-    // repeats lane 0's arithmetic for its own dimension, so results are the
-    // same bits as a sequential loop.
+    // (extend, connect vector); lane 0 does the rest.  Every lane repeats lane
+    // 0's arithmetic for its own dimension, so results are the same bits as a
+    // sequential loop.
     while (true) {
         ++local_iter;
-        if (tid < 32) {
-            const int lane = tid;
-            int stop = 0, sa = 0, sb = 0;
-            if (lane == 0) {
+        const float* sample = X.sample[local_iter & 1];
+        if (tid == 0) {
+            int sv, sa, sb;
+            if (X.pre) {  // read with the last extension's node (one round trip for all)
+                sv = X.pre_solved;
+                sa = X.pre_a;
+                sb = X.pre_b;
+            } else {
                 // the three loads go out together: one round trip, not three
-                const int sv = ld_volatile(P.solved);
+                sv = ld_volatile(P.solved);
                 sa = ld_volatile(&P.sizes[0]);
                 sb = ld_volatile(&P.sizes[1]);
-                stop = sv != 0;
-                if (!stop && local_iter > L.max_iter) {
-                    if (atomicCAS(P.solved, 0, -1) == 0) stamp_end(P);
-                    atomicMax(P.iter_count, local_iter);
-                    stop = 1;
-                }
             }
-            stop = __shfl_sync(0xffffffffu, stop, 0);
+            int stop = sv != 0;
+            if (!stop && local_iter > L.max_iter) {
+                if (atomicCAS(P.solved, 0, -1) == 0) stamp_end(P);
+                atomicMax(P.iter_count, local_iter);
+                stop = 1;
+            }
             if (!stop) {
-                if (lane < dim) {  // halton_sample, one dimension per lane
-                    const float val = halton_next(X.order[lane & 15], X.halton[lane]);
-                    X.sample[lane] = __fmaf_rn(val, __fsub_rn(L.hi[lane], L.lo[lane]), L.lo[lane]);
-                }
-                if (lane == 0) {
-                    const int t = choose_tree(L.balance_mode, local_iter, e % L.E, L.E, sa, sb, L.tree_ratio, X.vamp);
-                    X.t = t;
-                    X.n_t = min(t == 0 ? sa : sb, P.cap);
-                }
+                const int t = choose_tree(L.balance_mode, local_iter, e % L.E, L.E, sa, sb, L.tree_ratio, X.vamp);
+                X.t = t;
+                X.n_t = min(t == 0 ? sa : sb, P.cap);
             }
-            if (lane == 0) X.stop = stop;
+            X.stop = stop;
         }
+        if (tid >= sampler && tid < sampler + 32) draw(tid - sampler, X.sample[(local_iter + 1) & 1]);
         grp.sync();
         if (X.stop) break;
         const int t = X.t, o = 1 - t;
-        group_nearest(grp, P.tree[t], N, dim, X.n_t, X.sample, X.red_d, X.red_i);
+        unsigned long long nearest = group_nearest(P.tree[t], N, dim, X.n_t, sample, X.red_d, X.red_i);
         if (tid < 32) {
             const int lane = tid;
-            const int nn = X.red_i[0];
+            const int nn = (int)(unsigned)nearest;
             int skip = nn == INT_MAX;
             if (!skip) {
-                // radius and node loads issued together (one round trip)
+                // radius and node loads issued together (one round trip), and
+                // the state that the next iteration starts from if this one
+                // inserts nothing
                 const float rad = L.dd ? __ldcg(&P.radii[t][nn]) : 0.0f;
                 const float bv = lane < dim ? __ldcg(&P.tree[t][(size_t)lane * N + nn]) : 0.0f;
-                const float nd = __fsqrt_rn(X.red_d[0]);
+                if (lane == 0) {
+                    X.pre_solved = ld_volatile(P.solved);
+                    X.pre_a = ld_volatile(&P.sizes[0]);
+                    X.pre_b = ld_volatile(&P.sizes[1]);
+                    X.pre = 1;
+                }
+                const float nd = __fsqrt_rn(__uint_as_float((unsigned)(nearest >> 32)));
                 skip = L.dd && (rad < nd);
                 if (!skip) {
                     const float scl = nd > 1e-8f ? fminf(1.0f, __fdiv_rn(L.step, nd)) : 1.0f;
                     if (lane < dim) {
                         X.base[lane] = bv;
-                        const float c = __fmaf_rn(__fsub_rn(X.sample[lane], bv), scl, bv);
+                        const float c = __fmaf_rn(__fsub_rn(sample[lane], bv), scl, bv);
                         X.cand[lane] = c;
                         X.delta[lane] = __fsub_rn(c, bv);
                     }
@@ -554,7 +726,7 @@ __device__ void run_explorer(const Grp& grp, const PlanLaunch& L, const Prob& P,
         }
         grp.sync();
         if (X.skip) continue;
-        if (group_edge_collides(grp, sc, B, X.base, X.delta, X.G1, L.cw, par)) {
+        if (edges.collides(grp, X.base, X.delta, X.G1)) {
             if (tid == 0 && L.dd) radius_shrink(P.radii[t], X.nn, L.dd_alpha, L.dd_radius, L.dd_min_radius, &L.queue[1]);
             continue;
         }
@@ -575,21 +747,21 @@ __device__ void run_explorer(const Grp& grp, const PlanLaunch& L, const Prob& P,
                 X.new_idx = idx;
             }
             X.n_o = min(so, P.cap);
+            X.pre = 0;  // the sizes change: read again
         }
         grp.sync();
         if (X.new_idx < 0) break;
         if (tid < dim) __stcg(&P.tree[t][(size_t)tid * N + X.new_idx], X.cand[tid]);
         if (tid == 0) atomicAdd(&P.completed[t], 1);
         if (L.dd && tid == (grp.size() > 32 ? 32 : 0)) radius_grow(P.radii[t], X.nn, L.dd_alpha, &L.queue[1]);
-        // connect (prrtc_planner.cu:949-1043); group_nearest's first barrier
-        // follows the scan, so X.cand / X.n_o written above are visible
-        group_nearest(grp, P.tree[o], N, dim, X.n_o, X.cand, X.red_d, X.red_i);
+        // connect (prrtc_planner.cu:949-1043)
+        nearest = group_nearest(P.tree[o], N, dim, X.n_o, X.cand, X.red_d, X.red_i);
         if (tid < 32) {
             const int lane = tid;
-            const int cnn = X.red_i[0];
+            const int cnn = (int)(unsigned)nearest;
             int n_ext = 0;
             if (cnn != INT_MAX) {
-                const float cd = __fsqrt_rn(X.red_d[0]);
+                const float cd = __fsqrt_rn(__uint_as_float((unsigned)(nearest >> 32)));
                 if (L.step > 1e-8f && cd > 1e-8f) n_ext = (int)ceilf(__fdiv_rn(cd, L.step));
                 if (lane < dim) {
                     const float c = X.cand[lane];
@@ -616,7 +788,7 @@ __device__ void run_explorer(const Grp& grp, const PlanLaunch& L, const Prob& P,
         const int n_ext = X.n_ext;
         for (int ext = 0; ext < n_ext && !failed; ++ext) {
             if (X.abort_) { failed = true; break; }
-            if (group_edge_collides(grp, sc, B, X.curr, X.vec, X.G2, L.cw, par)) { failed = true; break; }
+            if (edges.collides(grp, X.curr, X.vec, X.G2)) { failed = true; break; }
             if (tid < 32) {
                 const int lane = tid;
                 int eidx = 0;
@@ -664,21 +836,33 @@ __device__ void run_explorer(const Grp& grp, const PlanLaunch& L, const Prob& P,
 }
 
 // Plain form: grid = E explorers of problem blockIdx.y.  Persistent form: CTAs
-// pop (problem, explorer) slots until the queue is empty.
-__global__ void __launch_bounds__(256, PRRTC_EXPLORE_MINBLOCKS) explore_kernel(PlanLaunch L) {
+// pop (problem, explorer) slots until the queue is empty.  CULL: edges by the
+// culled check, the scene always staged (launch_plan's rule).
+//
+// Bound by the latency of an explorer's chain (sample, nearest node, edge
+// passes of link frames -> bounds -> touching primitives -> fine tests), not by
+// arithmetic or memory: a lone CTA of 256 threads issues 0.18 instructions per
+// cycle and scheduler, its warps waiting for fixed-latency results and shared
+// memory.  So an explorer gets 128 registers per thread (80 and three CTAs per
+// SM measured 8-12% slower per plan, no faster per batch), and more threads
+// where SMs are idle (launch_plan).  Against the general
+// checker, kernel times: 152 -> 95 us (16 spheres, 128 explorers), 2.50 -> 1.60
+// ms (512 uneven problems, E = 2), 4.74 -> 2.57 ms (200 tabletop problems, E =
+// 1), 34.1 -> 5.6 ms (61 dual-arm problems, E = 1).
+template <bool CULL, int THREADS, int MINBLOCKS>
+__global__ void __launch_bounds__(THREADS, MINBLOCKS) explore_kernel(PlanLaunch L) {
     extern __shared__ __align__(128) unsigned char dsm[];
     __shared__ ExplorerSmem X;
+    __shared__ CulledEdges C;
     __shared__ __align__(8) uint64_t mbar;
     const int tid = threadIdx.x;
-    const bool staged = L.blob_cap > 0;
+    const bool staged = CULL || L.blob_cap > 0;
     unsigned char* blob_sm = dsm;
-    CcBufs B = cc_bufs(dsm + (staged ? L.blob_cap : 0), L.J, L.S, L.K, L.Q, L.cw);
-    B.stats = L.stats;
+    unsigned char* bufs = dsm + (staged ? L.blob_cap : 0);
     if (tid == 0) mbar_init(&mbar);
     __syncthreads();
     uint32_t phase = 0;
     int cur = -1;
-    Scene sc;
     const int total = L.persistent ? L.B * L.E : 1;
     for (int iter = 0;; ++iter) {
         int b, e;
@@ -719,17 +903,28 @@ __global__ void __launch_bounds__(256, PRRTC_EXPLORE_MINBLOCKS) explore_kernel(P
                 if (!stage_blob(blob_sm, gblob, min(bytes, L.blob_cap), &mbar, phase, &L.queue[1], 1,
                                 L.wait_polls == 0 ? kWaitLimit : max(L.wait_polls, 0)))
                     break;
-                sc = scene_view(blob_sm);
-            } else {
-                sc = scene_view(gblob);
             }
-            sc.pairs = reinterpret_cast<const int2*>(L.pairs) + (size_t)b * L.pairs_stride;
-            sc.pc = L.pc;
             cur = b;
         }
+        const int2* pairs = reinterpret_cast<const int2*>(L.pairs) + (size_t)b * L.pairs_stride;
         const Prob P = prob_ptrs(L, b);
         if (L.persistent && tid == 0) atomicCAS(&P.ts[0], 0ull, globaltimer());
-        run_explorer(CtaGroup{}, L, P, sc, B, X, e);
+        if constexpr (CULL) {
+            if (tid == 0) C = CulledEdges{pairs, L.pc, L.stats, L.blob_cap, L.J, L.K, L.n_obs, L.cw, L.cw_general};
+            CulledEdgesRef edges;
+            edges.a = &C;
+            edges.hit = reinterpret_cast<uint32_t*>(bufs);  // first in the buffers
+            run_explorer(CtaGroup{}, L, P, edges, X, e);
+        } else {
+            GeneralEdges edges;
+            edges.B = cc_bufs(bufs, L.J, L.S, L.K, L.Q, L.cw);
+            edges.B.stats = L.stats;
+            edges.sc = scene_view(staged ? blob_sm : gblob);
+            edges.sc.pairs = pairs;
+            edges.sc.pc = L.pc;
+            edges.CW = L.cw;
+            run_explorer(CtaGroup{}, L, P, edges, X, e);
+        }
     }
 }
 
@@ -866,7 +1061,7 @@ struct ExploreAttrs {
     size_t static_smem = 0;
 };
 constexpr int kMaxCachedDevices = 256;
-static ExploreAttrs g_explore_attr[kMaxCachedDevices];
+static ExploreAttrs g_explore_attr[kMaxCachedDevices][3];  // [device][general, culled, culled wide]
 static std::mutex g_explore_attr_mutex;
 
 // An optional timing event on the stream; inside a stream capture it becomes an
@@ -892,14 +1087,49 @@ cudaError_t launch_plan(PlanLaunch& L, cudaStream_t st) {
     init_kernel<<<L.B, 128, 0, st>>>(L, L.persistent ? 0 : 1);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
 
-    const size_t cc = (size_t)cc_smem_bytes(L.J, L.S, L.K, L.Q, L.cw);
     const size_t max_smem = device_max_smem();
-    const size_t static_smem = sizeof(ExplorerSmem) + 64;
-    size_t dyn = cc + (size_t)L.blob_cap;
-    if (dyn + static_smem > max_smem) {  // scene too large to stage: read it from global memory
-        L.blob_cap = 0;
-        dyn = cc;
+    const size_t static_smem = sizeof(ExplorerSmem) + sizeof(CulledEdges) + 64;
+    size_t dyn = 0;
+    // The culled form with 64 waypoints per pass, or as many (32, 16, 8) as
+    // leave room for its CTAs: a pass costs mostly the latency of its phases,
+    // so fewer passes win (batches of 300 tabletop problems, E = 2: 2.49 -> 2.20
+    // ms against 16 per pass; 61 dual-arm problems, E = 1: 7.3 -> 5.2 ms).
+    // Wide form: a batch of at most two explorers per SM leaves most of the GPU
+    // idle at the sizes it asks for, so each explorer gets 512 threads, one CTA
+    // per SM (200 tabletop problems, E = 1: 3.97 -> 3.74 ms against 256 threads; 61
+    // dual-arm problems: 6.7 -> 5.1 ms; at E = 2 x 512 problems it loses, 4.4
+    // -> 4.7 ms).
+    const bool wide = L.persistent && (long long)L.B * L.E <= 2ll * device_sm_count();
+    bool cull = false;
+    if (L.cull) {
+        const size_t room = max_smem / (wide ? 1 : 2) - (wide ? 0 : 1024);
+        for (int cw = 64; cw >= 8 && !cull; cw /= 2) {
+            // the buffers also hold the general checker's, for a scene that is not culled
+            size_t need = (size_t)cull_smem_bytes(L.J, L.K, L.n_obs, cw, true);
+            need = std::max(need, (size_t)cc_smem_bytes(L.J, L.S, L.K, L.Q, 8));
+            if (need + (size_t)L.blob_cap + static_smem > (cw > 8 ? room : max_smem)) continue;
+            cull = true;
+            L.cw = cw;
+            L.cw_general = 8;
+            while (L.cw_general < cw && (size_t)cc_smem_bytes(L.J, L.S, L.K, L.Q, 2 * L.cw_general) <= need)
+                L.cw_general *= 2;
+            dyn = need + (size_t)L.blob_cap;
+        }
     }
+    if (!cull) {
+        const size_t cc = (size_t)cc_smem_bytes(L.J, L.S, L.K, L.Q, L.cw);
+        dyn = cc + (size_t)L.blob_cap;
+        if (dyn + static_smem > max_smem) {  // scene too large to stage: read it from global memory
+            L.blob_cap = 0;
+            dyn = cc;
+        }
+    }
+    if (cull && wide) L.threads = kWideThreads;
+    else if (L.threads == 0) L.threads = cull ? 256 : 128;
+    const int form = !cull ? 0 : (L.threads > 256 ? 2 : 1);
+    void (*const kern)(PlanLaunch) = form == 0   ? explore_kernel<false, 256, PRRTC_EXPLORE_MINBLOCKS>
+                                     : form == 1 ? explore_kernel<true, 256, PRRTC_EXPLORE_MINBLOCKS>
+                                                 : explore_kernel<true, kWideThreads, 1>;
     // ctas_per_sm > 0: the smallest shared-memory carve-out that holds that many
     // CTAs, so the rest of the SM's unified L1 / shared memory is L1 (the
     // explorers read trees, radii and unstaged scene data through it); measured
@@ -915,13 +1145,13 @@ cudaError_t launch_plan(PlanLaunch& L, cudaStream_t st) {
         const unsigned long long ctx = current_context_key();
         std::lock_guard<std::mutex> lock(g_explore_attr_mutex);
         ExploreAttrs dflt;
-        ExploreAttrs& c = (dev >= 0 && dev < kMaxCachedDevices) ? g_explore_attr[dev] : dflt;
+        ExploreAttrs& c = (dev >= 0 && dev < kMaxCachedDevices) ? g_explore_attr[dev][form] : dflt;
         if (!ctx || c.ctx != ctx) {
             c = ExploreAttrs{};
             c.ctx = ctx;
         }
         if ((int)dyn > c.max_dyn) {
-            if ((e = cudaFuncSetAttribute(explore_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn)) !=
+            if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn)) !=
                 cudaSuccess)
                 return e;
             c.max_dyn = (int)dyn;
@@ -934,7 +1164,7 @@ cudaError_t launch_plan(PlanLaunch& L, cudaStream_t st) {
                         cudaSuccess ||
                     (e = cudaDeviceGetAttribute(&c.reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev)) !=
                         cudaSuccess ||
-                    (e = cudaFuncGetAttributes(&fa, explore_kernel)) != cudaSuccess)
+                    (e = cudaFuncGetAttributes(&fa, kern)) != cudaSuccess)
                     return e;
                 c.static_smem = fa.sharedSizeBytes;
                 c.have_smem = true;
@@ -943,7 +1173,7 @@ cudaError_t launch_plan(PlanLaunch& L, cudaStream_t st) {
             carve = c.sm_smem > 0 ? (int)std::min<size_t>(100, (100 * need + c.sm_smem - 1) / (size_t)c.sm_smem) : -1;
         }
         if (carve != c.carve) {
-            if ((e = cudaFuncSetAttribute(explore_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, carve)) !=
+            if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, carve)) !=
                 cudaSuccess)
                 return e;
             c.carve = carve;
@@ -951,7 +1181,7 @@ cudaError_t launch_plan(PlanLaunch& L, cudaStream_t st) {
     }
     if (L.persistent) {
         int per_sm = 0;
-        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, explore_kernel, L.threads, dyn)) !=
+        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, L.threads, dyn)) !=
             cudaSuccess)
             return e;
         per_sm = std::max(per_sm, 1);
@@ -963,10 +1193,10 @@ cudaError_t launch_plan(PlanLaunch& L, cudaStream_t st) {
         // piling extra explorers onto a few problems
         grid = std::min<long long>(grid, (long long)L.B * L.E);
         if ((e = record_event(L.explore_events[0], st)) != cudaSuccess) return e;
-        explore_kernel<<<(unsigned)std::max<long long>(grid, 1), L.threads, dyn, st>>>(L);
+        kern<<<(unsigned)std::max<long long>(grid, 1), L.threads, dyn, st>>>(L);
     } else {
         if ((e = record_event(L.explore_events[0], st)) != cudaSuccess) return e;
-        explore_kernel<<<dim3(L.E, L.B), L.threads, dyn, st>>>(L);
+        kern<<<dim3(L.E, L.B), L.threads, dyn, st>>>(L);
     }
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if ((e = record_event(L.explore_events[1], st)) != cudaSuccess) return e;

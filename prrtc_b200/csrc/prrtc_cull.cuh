@@ -1,0 +1,483 @@
+// prrtc_cull.cuh -- the culled collision check: the verdicts of cc_chunk
+// (prrtc_device.cuh), bit for bit, from a small part of its pair tests.
+//
+// Every link has a cull sphere (pack kernel): the centre of its coarse sphere
+// and a radius that encloses its fine spheres and the coarse sphere with a pad.
+// A primitive whose distance from the cull sphere is positive cannot pass any
+// fine test of that link, so only the links, waypoints and primitives that
+// touch are tested, with the same arithmetic as cc_chunk's.  The pad covers the
+// rounding of the fine tests: the largest error of the expanded sphere test,
+// |c|^2 - r^2 + |o|^2 - r_o^2 - 2 (c.o + r r_o), is below 1.1e-6 M^2 for
+// M = |c| + |o| + radii, and a gap of d metres beyond the cull sphere leaves
+// |c_f - o|^2 - (r_f + r_o)^2 >= d^2, so d = 2e-3 M (4e-6 M^2) suffices; the
+// other tests are first order in the distance and need 1e-6 M.  Comparisons are
+// written so that NaN and infinities count as touching.
+//
+// For the waypoints of an edge a first level bounds each link's cull spheres
+// over the whole pass by one sphere (centre of the middle waypoint) and lists
+// the primitives that it touches; the waypoints then test that list only.
+//
+// Fine work is a shared-memory list of (link, waypoint, mask of primitives) and
+// one of (self item, waypoint); 8 lanes take an entry, a sphere per lane, and
+// place their sphere centres from the link frames as they need them (no pass
+// over all spheres, no centre buffer).
+#pragma once
+
+#include "prrtc_device.cuh"
+
+namespace prrtc {
+
+constexpr int kCullLinkList = 256;  // primitives listed per link of an edge; more: all of them are tested
+
+// Shared-memory buffers of a culled check of CW waypoints.
+struct CullBufs {
+    float* q;          // [CW][kDimMax] (configurations; unused for edges)
+    float* pose;       // [CW][J][12]
+    float4* cctr;      // [K][CW] coarse sphere centres, .w = radius + inflation
+    float4* swept;     // [K] (edges) bound of the link's cull spheres over the pass
+    uint32_t* dirty;   // [CW][2] links whose coarse sphere touches the world (gated)
+    int2* wlist;       // [wcap] (group of 32 << 12 | link << 6 | waypoint, mask of primitives in the group)
+    int* slist;        // [scap] self item << 6 | waypoint
+    int4* ncand;       // [K] (edges) primitives listed for a link: ends of the spheres, capsules, boxes, all; .w -1: too many
+    uint16_t* cand;    // [K][ccap] (edges)
+    uint32_t* hit;     // [6]: result words, world and self list lengths, alternating between calls
+    int wcap, scap, ccap;
+    unsigned long long* stats;
+};
+
+__host__ __device__ inline int cull_link_list(int n_obs) { return n_obs < kCullLinkList ? (n_obs + 7) & ~7 : kCullLinkList; }
+// List capacities: room for every second link of every waypoint; a pass that
+// needs more tests without lists.
+__host__ __device__ inline int cull_wcap(int K, int CW) { return (K * CW / 2 + 63) & ~31; }
+__host__ __device__ inline int cull_scap(int CW) { return 12 * CW; }
+
+__host__ __device__ inline int cull_smem_bytes(int J, int K, int n_obs, int CW, bool edge) {
+    int b = edge ? 0 : CW * kDimMax * 4;
+    b += CW * J * 48 + K * CW * 16 + K * 32 + CW * 8;
+    b += cull_wcap(K, CW) * 8 + cull_scap(CW) * 4 + 32;
+    if (edge) b += align16(K * cull_link_list(n_obs) * 2);
+    return b;
+}
+
+__device__ __forceinline__ CullBufs cull_bufs(unsigned char* p, int J, int K, int n_obs, int CW, bool edge) {
+    CullBufs b;
+    b.wcap = cull_wcap(K, CW);
+    b.scap = cull_scap(CW);
+    b.ccap = cull_link_list(n_obs);
+    b.hit = reinterpret_cast<uint32_t*>(p);    p += 32;
+    b.q = reinterpret_cast<float*>(p);         p += edge ? 0 : CW * kDimMax * 4;
+    b.pose = reinterpret_cast<float*>(p);      p += CW * J * 48;
+    b.cctr = reinterpret_cast<float4*>(p);     p += K * CW * 16;
+    b.swept = reinterpret_cast<float4*>(p);    p += K * 16;
+    b.ncand = reinterpret_cast<int4*>(p);      p += K * 16;
+    b.dirty = reinterpret_cast<uint32_t*>(p);  p += CW * 8;
+    b.wlist = reinterpret_cast<int2*>(p);      p += b.wcap * 8;
+    b.slist = reinterpret_cast<int*>(p);       p += b.scap * 4;
+    b.cand = reinterpret_cast<uint16_t*>(p);
+    b.stats = nullptr;
+    return b;
+}
+
+// Whether a launch can use the culled check at all (the scene's own flag,
+// BlobHeader::cull, decides per problem).
+inline bool cull_shape_ok(int J, int K, int n_obs, float inflate) {
+    return J >= 1 && J <= 32 && K >= 1 && K <= kMaxLinks && n_obs < 65536 && inflate >= 0.0f;
+}
+
+// True when a sphere at distance sqrt(d2) with radius sum b certainly does not
+// touch (false for NaN, and for a distance so large that it may be an overflow).
+__device__ __forceinline__ bool cull_far(float d2, float b) { return d2 > b * b && d2 < 1e30f; }
+
+// Whether one primitive of each type may touch the sphere (c, R).
+__device__ __forceinline__ bool cull_sphere(const Scene& sc, int o, float4 c, float R) {
+    const float4 O = sc.ws[2 * o];  // (-2 centre, -2 radius)
+    const float dx = fmaf(0.5f, O.x, c.x), dy = fmaf(0.5f, O.y, c.y), dz = fmaf(0.5f, O.z, c.z);
+    return !cull_far(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), fmaf(0.5f, fabsf(O.w), R));
+}
+__device__ __forceinline__ bool cull_capsule(const Scene& sc, int o, float4 c, float R) {
+    const float4 p1 = sc.wc[3 * o], dp = sc.wc[3 * o + 1], d = sc.wc[3 * o + 2];
+    const float t = __saturatef(fmaf(dp.x, c.x, fmaf(dp.y, c.y, fmaf(dp.z, c.z, dp.w))));
+    const float ex = fmaf(-t, d.x, c.x - p1.x), ey = fmaf(-t, d.y, c.y - p1.y), ez = fmaf(-t, d.z, c.z - p1.z);
+    return !cull_far(fmaf(ex, ex, fmaf(ey, ey, ez * ez)), R + fabsf(p1.w));
+}
+__device__ __forceinline__ bool cull_box(const Scene& sc, int o, float4 c, float R) {
+    const float4 cc[1] = {c};
+    const float4 hl = sc.wb[4 * o + 3];
+    float v[1];
+    h_box<1>(v, cc, sc.wb[4 * o], sc.wb[4 * o + 1], sc.wb[4 * o + 2], hl);
+    return !(v[0] > (R * kBoxInv) * (R * kBoxInv)) || hl.w != 0.0f;
+}
+__device__ __forceinline__ bool cull_halfspace(const Scene& sc, int o, float4 c, float R) {
+    const float4 cc[1] = {c};
+    float v[1];
+    h_halfspace<1>(v, cc, sc.wh[o]);
+    return !(v[0] > R);
+}
+
+// The exact test of primitive o (combined index) against one sphere: the
+// arithmetic of obstacles_vs_spheres.
+__device__ __forceinline__ bool prim_hits(const Scene& sc, const BlobHeader& h, int o, float4 c) {
+    const float4 cc[1] = {c};
+    float v[1];
+    if (o < h.Ns) {
+        h_sphere<1>(v, cc, sc.ws[2 * o], sc.ws[2 * o + 1].w);
+        return v[0] <= -sphere_A(c);
+    }
+    o -= h.Ns;
+    if (o < h.Nc) {
+        h_capsule<1>(v, cc, sc.wc[3 * o], sc.wc[3 * o + 1], sc.wc[3 * o + 2]);
+        return v[0] <= 0.0f;
+    }
+    o -= h.Nc;
+    if (o < h.Nb) {
+        h_box<1>(v, cc, sc.wb[4 * o], sc.wb[4 * o + 1], sc.wb[4 * o + 2], sc.wb[4 * o + 3]);
+        return v[0] <= (c.w * kBoxInv) * (c.w * kBoxInv);
+    }
+    h_halfspace<1>(v, cc, sc.wh[o - h.Nb]);
+    return v[0] <= c.w;
+}
+
+__device__ __forceinline__ int prim_flops(const BlobHeader& h, int o) {
+    return o < h.Ns ? kFlopSphere : (o < h.Ns + h.Nc ? kFlopCapsule : (o < h.Ns + h.Nc + h.Nb ? kFlopBox : kFlopHalfspace));
+}
+
+// One point in the frame of joint f at waypoint w (three 16-byte loads).
+__device__ __forceinline__ float4 pose_point(const float* pose, int J, int w, int f, float4 l) {
+    const float4* p = reinterpret_cast<const float4*>(pose + (w * J + f) * 12);
+    const float4 p0 = p[0], p1 = p[1], p2 = p[2];
+    const float F[12] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w, p2.x, p2.y, p2.z, p2.w};
+    return xform_point(F, l);
+}
+
+// Centre of fine sphere s at waypoint w (the arithmetic of cc_centres).
+__device__ __forceinline__ float4 fine_centre(const Scene& sc, const float* pose, int J, int w, int s, float inflate) {
+    const int f = sc.sfr[s];
+    if (f < 0) return absent_sphere();
+    float4 l = sc.sph[s];
+    l.w += inflate;
+    return pose_point(pose, J, w, f, l);
+}
+
+// Padded cull radius of a link whose coarse centre is c (grp record .w: reach
+// of its spheres and the scene's share of the pad).
+__device__ __forceinline__ float cull_radius(float reach, float inflate, float4 c) {
+    return reach + inflate + kCullPad * (fabsf(c.x) + fabsf(c.y) + fabsf(c.z));
+}
+
+// Whether self item ii needs its fine test at waypoint w: the gate of a gated
+// checker (as cc_chunk), or whether the cull spheres of its block's links touch.
+// Items of no coarse pair always do.
+__device__ __forceinline__ bool cull_self_touch(const Scene& sc, const CullBufs& B, int CW, int4 item, int w, float inflate) {
+    const int q = item.w >= 0 ? item.w : -2 - item.w;
+    if (q < 0) return true;
+    const int2 cp = sc.cpair[q];
+    if (cp.x < 0 || cp.y < 0 || cp.x >= sc.h->K || cp.y >= sc.h->K) return false;
+    const float4 a = B.cctr[cp.x * CW + w], b = B.cctr[cp.y * CW + w];
+    const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
+    const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+    if (item.w >= 0) {
+        const float t = a.w + b.w - inflate;
+        return d2 <= t * t;
+    }
+    return !cull_far(d2, cull_radius(sc.grp[2 * cp.x + 1].w, inflate, a) + cull_radius(sc.grp[2 * cp.y + 1].w, inflate, b));
+}
+
+// Fine test of self item ii at waypoint w by 8 consecutive lanes (l8 = 0..7 of
+// `mask`) together: a sphere of the first group per lane.
+__device__ __forceinline__ bool cull_self_item(const Scene& sc, const CullBufs& B, int CW, int ii, int w, int l8,
+                                               unsigned mask, float inflate, unsigned& flops) {
+    const BlobHeader& h = *sc.h;
+    const int J = h.J, S = h.S;
+    const int4 item = sc.item[ii];
+    bool hit = false;
+    if (item.y >= 0) {  // block: spheres [a0, a0+na) x [b0, b0+nb)
+        const int na = item.z >> 16, nb = item.z & 0xffff;
+        const float half = 0.5f * inflate;
+        float4 a[1] = {l8 < na ? fine_centre(sc, B.pose, J, w, item.x + l8, inflate) : absent_sphere()};
+        // no sphere of the first group near the second link's cull sphere: nothing can touch
+        const int lb = sc.cpair[item.w >= 0 ? item.w : -2 - item.w].y;
+        const float4 cb = B.cctr[lb * CW + w];
+        const float ex = a[0].x - cb.x, ey = a[0].y - cb.y, ez = a[0].z - cb.z;
+        const bool near = l8 < na && !cull_far(fmaf(ex, ex, fmaf(ey, ey, ez * ez)),
+                                               a[0].w + cull_radius(sc.grp[2 * lb + 1].w, inflate, cb) +
+                                                   kCullPad * (fabsf(a[0].x) + fabsf(a[0].y) + fabsf(a[0].z)));
+        if (!__any_sync(mask, near)) return false;
+        a[0].w -= half;
+        const float thr = -sphere_A(a[0]);
+        for (int b0 = 0; b0 < nb; b0 += 8) {
+            float4 b = b0 + l8 < nb ? fine_centre(sc, B.pose, J, w, item.y + b0 + l8, inflate) : absent_sphere();
+            b.w -= half;
+            const float4 O = make_float4(-2.0f * b.x, -2.0f * b.y, -2.0f * b.z, -2.0f * b.w);
+            const float A = sphere_A(b);
+#pragma unroll
+            for (int m = 0; m < 8; ++m) {
+                const float4 Om = make_float4(__shfl_sync(mask, O.x, m, 8), __shfl_sync(mask, O.y, m, 8),
+                                              __shfl_sync(mask, O.z, m, 8), __shfl_sync(mask, O.w, m, 8));
+                float v[1];
+                h_sphere<1>(v, a, Om, __shfl_sync(mask, A, m, 8));
+                hit |= v[0] <= thr;
+            }
+        }
+        flops += l8 < na ? nb * kFlopPair + 2 * kFlopXform : 0;
+    } else {  // explicit pairs [p0, p0+count) of the pair list (global memory)
+        const int p1 = min(item.x + item.z, h.P);
+        for (int p = item.x + l8; p < p1; p += 8) {
+            const int2 pr = __ldg(&sc.pairs[p]);
+            if (pr.x < 0 || pr.y < 0 || pr.x >= S || pr.y >= S) continue;
+            const float4 a = fine_centre(sc, B.pose, J, w, pr.x, inflate), b = fine_centre(sc, B.pose, J, w, pr.y, inflate);
+            const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
+            const float t = a.w + b.w - inflate;
+            hit |= fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= t * t;
+            flops += kFlopPairExplicit + 2 * kFlopXform;
+        }
+    }
+    return hit;
+}
+
+// Fine test of link k at waypoint w against every primitive, sphere lane l8 of 8
+// (a pass whose world list ran over).  Out of line: the code is rarely needed.
+static __device__ __noinline__ bool cull_link_all(const unsigned char* blob, const float* pose, int k, int w, int l8) {
+    const Scene sc = scene_view(blob);
+    const BlobHeader& h = *sc.h;
+    const float4 gr = sc.grp[2 * k + 1];
+    const int s1 = __float_as_int(gr.z);
+    bool hit = false;
+    for (int s = __float_as_int(gr.y) + l8; s < s1; s += 8) {
+        const float4 c = fine_centre(sc, pose, h.J, w, s, __int_as_float(h.inflate_bits));
+#pragma unroll 1
+        for (int o = 0; o < h.Ns + h.Nc + h.Nb + h.Nh; ++o) hit |= prim_hits(sc, h, o, c);
+    }
+    return hit;
+}
+
+// One type's primitives of a link's bound (a warp, a primitive per lane):
+// appends those that touch to the link's list and returns its new length.
+template <class Touch>
+__device__ __forceinline__ int cull_append(int count, int base, int n, int cap, uint16_t* list, int lane, Touch touch) {
+#pragma unroll 1
+    for (int o0 = 0; o0 < count; o0 += 32) {
+        const int o = o0 + lane;
+        const bool t = o < count && touch(o);
+        const unsigned b = __ballot_sync(0xffffffffu, t);
+        const int at = n + __popc(b & ((1u << lane) - 1u));
+        if (t && at < cap) list[at] = (uint16_t)(base + o);
+        n += __popc(b);
+    }
+    return n;
+}
+
+// Collision check of nw (<= CW <= 64) waypoints of `edge` (EDGE: the answer is
+// whether any collides) or of the configurations in B.q (nw <= 32: bit w of the
+// answer).  Called by every thread of the CTA with the same `par`, which the call
+// flips: the result words and list lengths alternate between calls, so that a
+// call clears the next call's after its first barrier.  All must be zero and
+// `par` 0 before the first call.  The scene must have BlobHeader::cull set.
+template <bool EDGE, class G>
+__device__ __forceinline__ uint32_t cull_check(const G& g, const Scene& sc, const CullBufs& B, int nw, int CW, int& par,
+                                               const EdgeSrc* edge) {
+    const BlobHeader& h = *sc.h;
+    const int tid = g.rank(), T = g.size(), lane = tid & 31, warp = tid >> 5, n_warps = T >> 5;
+    const int J = h.J, S = h.S, K = h.K;
+    const int Ns = h.Ns, Nc = h.Nc, Nb = h.Nb, Nh = h.Nh;
+    const bool gated = h.gated != 0;
+    const float inflate = __int_as_float(h.inflate_bits);
+    uint32_t* hw = B.hit + par;
+    volatile uint32_t* vhit = hw;
+    int* nwl = reinterpret_cast<int*>(B.hit + 2 + par);
+    int* nsl = reinterpret_cast<int*>(B.hit + 4 + par);
+    par ^= 1;
+    unsigned flops = 0;
+
+    // 1. link frames (as cc_chunk) and coarse centres
+    if (gated)
+        for (int i = tid; i < 2 * nw; i += T) B.dirty[i] = 0u;
+    fk_segments(sc, B.q, B.pose, EDGE ? edge : nullptr, nw, J, tid, T, [&](int w, int j, int SEG) {
+        for (int k = j; k < K; k += SEG) {
+            float4 l = sc.grp[2 * k];
+            l.w += inflate;
+            B.cctr[k * CW + w] = pose_point(B.pose, J, w, __float_as_int(sc.grp[2 * k + 1].x), l);
+        }
+    });
+    g.sync();
+    if (tid == 0) {  // the next call's words (every thread has read them by now)
+        B.hit[par] = 0u;
+        B.hit[2 + par] = B.hit[4 + par] = 0u;
+    }
+    // 2. edges: one bound per link over the pass, and the primitives it touches (a warp per link)
+    if constexpr (EDGE) {
+        for (int k = warp; k < K; k += n_warps) {
+            const float4 m = B.cctr[k * CW + (nw >> 1)];
+            unsigned far2 = 0u;  // bits of the largest squared distance (NaN orders above infinity)
+            for (int w = lane; w < nw; w += 32) {
+                const float4 c = B.cctr[k * CW + w];
+                const float dx = c.x - m.x, dy = c.y - m.y, dz = c.z - m.z;
+                far2 = max(far2, __float_as_uint(fmaf(dx, dx, fmaf(dy, dy, dz * dz))) & 0x7fffffffu);
+            }
+            const float d = __fsqrt_ru(__uint_as_float(__reduce_max_sync(0xffffffffu, far2)));
+            const float R = cull_radius(sc.grp[2 * k + 1].w, inflate, m) + (1.0f + 2.0f * kCullPad) * d;
+            uint16_t* list = B.cand + k * B.ccap;
+            int4 n;
+            n.x = cull_append(Ns, 0, 0, B.ccap, list, lane, [&](int o) { return cull_sphere(sc, o, m, R); });
+            n.y = cull_append(Nc, Ns, n.x, B.ccap, list, lane, [&](int o) { return cull_capsule(sc, o, m, R); });
+            n.z = cull_append(Nb, Ns + Nc, n.y, B.ccap, list, lane, [&](int o) { return cull_box(sc, o, m, R); });
+            n.w = cull_append(Nh, Ns + Nc + Nb, n.z, B.ccap, list, lane, [&](int o) { return cull_halfspace(sc, o, m, R); });
+            if (lane == 0) {
+                B.swept[k] = make_float4(m.x, m.y, m.z, R);
+                B.ncand[k] = n.w <= B.ccap ? n : make_int4(0, 0, 0, -1);
+                if (B.stats) flops += Ns * kFlopSphere + Nc * kFlopCapsule + Nb * kFlopBox + Nh * kFlopHalfspace;
+            }
+        }
+        g.sync();
+    }
+    // 3. touching (link, waypoint) primitives and self items: a warp per link or item, a waypoint per lane
+    const int wide = (nw + 31) >> 5;
+    for (int u = warp; u < K * wide + h.n_items; u += n_warps) {
+        if (u < K * wide) {
+            const int k = wide == 1 ? u : u >> 1, w = (wide == 1 ? 0 : (u & 1) << 5) + lane;
+            int4 n = make_int4(Ns, Ns + Nc, Ns + Nc + Nb, Ns + Nc + Nb + Nh);
+            const uint16_t* list = nullptr;  // the link's list, or every primitive
+            if constexpr (EDGE) {
+                const int4 m = B.ncand[k];
+                if (m.w >= 0) {
+                    n = m;
+                    list = B.cand + k * B.ccap;
+                }
+            }
+            auto at_index = [&](int i) { return EDGE && list ? (int)list[i] : i; };
+            if (w >= nw) continue;
+            const float4 c = B.cctr[k * CW + w];
+            const float R = cull_radius(sc.grp[2 * k + 1].w, inflate, c);
+            bool dirty = false;
+            for (int i0 = 0; i0 < n.w; i0 += 32) {
+                const int i1 = min(n.w, i0 + 32);
+                unsigned bits = 0u;
+                int i = i0;
+#pragma unroll 1
+                for (; i < min(n.x, i1); ++i) bits |= (unsigned)cull_sphere(sc, at_index(i), c, R) << (i - i0);
+#pragma unroll 1
+                for (; i < min(n.y, i1); ++i) bits |= (unsigned)cull_capsule(sc, at_index(i) - Ns, c, R) << (i - i0);
+#pragma unroll 1
+                for (; i < min(n.z, i1); ++i) bits |= (unsigned)cull_box(sc, at_index(i) - Ns - Nc, c, R) << (i - i0);
+#pragma unroll 1
+                for (; i < i1; ++i) bits |= (unsigned)cull_halfspace(sc, at_index(i) - Ns - Nc - Nb, c, R) << (i - i0);
+                if (!bits) continue;
+                if (gated)
+                    for (unsigned rest = bits; rest && !dirty; rest &= rest - 1u)
+                        dirty = prim_hits(sc, h, at_index(i0 + __ffs(rest) - 1), c);
+                const int at = atomicAdd(nwl, 1);
+                if (at < B.wcap) B.wlist[at] = make_int2((i0 >> 5) << 12 | k << 6 | w, (int)bits);
+            }
+            if (dirty) atomicOr(&B.dirty[2 * w + (k >> 5)], 1u << (k & 31));
+            if (B.stats)
+                flops += n.x * kFlopSphere + (n.y - n.x) * kFlopCapsule + (n.z - n.y) * kFlopBox + (n.w - n.z) * kFlopHalfspace;
+        } else {
+            const int ii = u - K * wide;
+            const int4 item = sc.item[ii];
+            if constexpr (EDGE) {  // links whose bounds are apart: no waypoint touches
+                const int q = item.w >= 0 ? item.w : -2 - item.w;
+                if (q >= 0) {
+                    const int2 cp = sc.cpair[q];
+                    if (cp.x < 0 || cp.y < 0 || cp.x >= K || cp.y >= K) continue;
+                    const float4 a = B.swept[cp.x], b = B.swept[cp.y];
+                    const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
+                    if (cull_far(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), a.w + b.w)) continue;
+                }
+            }
+            for (int w = lane; w < nw; w += 32) {
+                flops += kFlopPairExplicit;
+                if (!cull_self_touch(sc, B, CW, item, w, inflate)) continue;
+                const int at = atomicAdd(nsl, 1);
+                if (at < B.scap) B.slist[at] = ii << 6 | w;
+            }
+        }
+    }
+    g.sync();
+    // 4. fine tests, 8 lanes per entry.  A list that ran over is not used: every
+    // (link, waypoint) with every primitive, or every (item, waypoint), is an
+    // entry then.  Nothing here may depend on *vhit without a vote of the 8
+    // lanes: it changes under other warps, and lanes that disagreed would wait
+    // for one another.
+    const bool wfull = *nwl > B.wcap, sfull = *nsl > B.scap;
+    const int Lw = wfull ? K * nw : *nwl, Ls = sfull ? h.n_items * nw : *nsl;
+    const bool cloud = sc.pc.n > 0;
+    if (Lw + Ls > 0 || cloud) {
+        const int l8 = tid & 7;
+        const unsigned mask = 0xffu << (lane & 24);
+        for (int it = tid >> 3; it < Lw + Ls; it += T >> 3) {
+            bool hit = false;
+            int w;
+            const uint32_t seen = __shfl_sync(mask, (uint32_t)*vhit, 0, 8);
+            if (it < Lw) {
+                int2 e = make_int2(0, 0);
+                int k;
+                if (wfull) {
+                    k = it / nw;
+                    w = it - k * nw;
+                } else {
+                    e = B.wlist[it];
+                    k = (e.x >> 6) & 63;
+                    w = e.x & 63;
+                }
+                if (EDGE ? (seen != 0u) : ((seen >> w) & 1u)) continue;
+                if (gated && !(B.dirty[2 * w + (k >> 5)] & (1u << (k & 31)))) continue;
+                if (wfull) {
+                    if (cull_link_all(reinterpret_cast<const unsigned char*>(sc.h), B.pose, k, w, l8))
+                        atomicOr(hw, 1u << (w & 31));
+                    continue;
+                }
+                const float4 gr = sc.grp[2 * k + 1];
+                const int i0 = (e.x >> 12) << 5;
+                const uint16_t* list = nullptr;
+                if constexpr (EDGE) list = B.ncand[k].w >= 0 ? B.cand + k * B.ccap + i0 : nullptr;
+                const int s1 = __float_as_int(gr.z);
+#pragma unroll 1
+                for (int s = __float_as_int(gr.y) + l8; s < s1; s += 8) {
+                    const float4 c = fine_centre(sc, B.pose, J, w, s, inflate);
+#pragma unroll 1
+                    for (unsigned rest = (unsigned)e.y; rest; rest &= rest - 1u) {
+                        const int i = __ffs(rest) - 1;
+                        const int o = EDGE && list ? (int)list[i] : i0 + i;
+                        hit |= prim_hits(sc, h, o, c);
+                        if (B.stats) flops += prim_flops(h, o);
+                    }
+                    flops += kFlopXform;
+                }
+            } else {
+                int ii;
+                if (sfull) {
+                    ii = (it - Lw) / nw;
+                    w = (it - Lw) - ii * nw;
+                } else {
+                    const int e = B.slist[it - Lw];
+                    ii = e >> 6;
+                    w = e & 63;
+                }
+                if (EDGE ? (seen != 0u) : ((seen >> w) & 1u)) continue;
+                if (sfull && !cull_self_touch(sc, B, CW, sc.item[ii], w, inflate)) continue;
+                hit = cull_self_item(sc, B, CW, ii, w, l8, mask, inflate, flops);
+            }
+            if (hit) atomicOr(hw, 1u << (w & 31));
+        }
+        if (cloud) {
+            unsigned long long f = 0;
+            for (int it = tid; it < S * nw; it += T) {
+                const int s = it / nw, w = it - s * nw;
+                if (EDGE ? (*vhit != 0u) : ((*vhit >> w) & 1u)) continue;
+                if (pc_sphere_hits(sc.pc, fine_centre(sc, B.pose, J, w, s, inflate), false, f)) atomicOr(hw, 1u << (w & 31));
+            }
+            flops += (unsigned)f;
+        }
+    }
+    if (B.stats) {
+        if (tid == 0) {
+            flops += (unsigned)(nw * (J * (kFlopJointLocal + kFlopJointChain) + K * kFlopXform));
+            atomicAdd(&B.stats[kStatConfigs], (unsigned long long)nw);
+        }
+        if (flops) atomicAdd(&B.stats[kStatFlops], (unsigned long long)flops);
+    }
+    if (Lw + Ls == 0 && !cloud) return *vhit;  // no entry, so no write of the word: no barrier
+    g.sync();
+    return *vhit;
+}
+
+}  // namespace prrtc

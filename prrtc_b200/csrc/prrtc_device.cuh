@@ -34,6 +34,8 @@ constexpr int kObsChunk = 32;    // world primitives per work item
 #endif
 constexpr int kSphChunk = PRRTC_SPH_CHUNK;  // fine spheres held in registers per work item
 constexpr int kPairChunk = 32;   // explicit self pairs per work item
+constexpr float kCullPad = 2.0e-3f;  // pad of the cull spheres per metre of coordinate size (prrtc_cull.cuh)
+constexpr float kCullReachMax = 4.0f;  // a link reaching further (or not finite) is never culled
 constexpr float kFar = 1.0e18f;  // centre of a sphere that can never collide
 // Box records are stored scaled by 1/kBoxScale (a power of two, so the scaling
 // is exact): the checker's relu(|l| - h) becomes a saturating add, exact for
@@ -63,7 +65,8 @@ struct BlobHeader {
     int32_t o_joint, o_sph, o_sfr, o_grp;
     int32_t o_sch, o_ws, o_wc, o_wb;
     int32_t o_wh, o_item, o_cpair, used_bytes;
-    int32_t P, cap_bytes, error, pad0;
+    int32_t P, cap_bytes, error;
+    int32_t cull;  // the groups cover every sphere on their own frames: prrtc_cull.cuh applies
 };
 static_assert(sizeof(BlobHeader) == 128, "header must stay 128 bytes");
 // Bits of BlobHeader::error: the pack kernel's self-pair item list overflowed
@@ -124,11 +127,11 @@ struct Scene {  // typed view of a blob (shared or global memory)
     const JointRec* joints;
     const float4* sph;
     const int* sfr;
-    const float4* grp;   // [K][2]: (c, r) then int4 bits (frame, s0, s1, 0)
+    const float4* grp;   // [K][2]: (c, r) then int bits (frame, s0, s1) and the cull sphere's radius
     const int4* sch;
     const float4* ws;    // [Ns][2]: (-2x,-2y,-2z,-2r), (x,y,z, x^2+y^2+z^2-r^2)
     const float4* wc;    // [Nc][3]: (p1, r), (d/|d|^2, -p1.d/|d|^2), (d, 0)   with d = p2 - p1
-    const float4* wb;    // [Nb][4]: (a1, -a1.c), (a2, -a2.c), (a3, -a3.c), (h1, h2, h3, 0)
+    const float4* wb;    // [Nb][4]: (a1, -a1.c), (a2, -a2.c), (a3, -a3.c), (h1, h2, h3, axes not orthonormal)
     const float4* wh;    // [Nh]:    (n, -n.p)
     const int4* item;
     const int2* cpair;
@@ -426,10 +429,10 @@ __device__ inline void joint_local(const JointRec& jr, float v, float* out) {
         const float wx = jr.tw.x * v, wy = jr.tw.y * v, wz = jr.tw.z * v;
         const float th2 = fmaf(wx, wx, fmaf(wy, wy, wz * wz));
         const float th = sqrtf(th2);
+        float s, c;  // one call for both kinds: its code is large
+        sincosf(kind == 1 ? v : th, &s, &c);
         float A, B, Cc;
         if (kind == 1) {  // unit axis: th = |v|, R = I + sin(v) K + (1-cos(v)) K^2 with K from the axis
-            float s, c;
-            sincosf(v, &s, &c);
             const float ax = jr.tw.x, ay = jr.tw.y, az = jr.tw.z;
             const float oc = 1.0f - c;
             E[0] = fmaf(oc, ax * ax - 1.0f, 1.0f); E[1] = fmaf(oc, ax * ay, -s * az); E[2] = fmaf(oc, ax * az, s * ay);
@@ -442,8 +445,6 @@ __device__ inline void joint_local(const JointRec& jr, float v, float* out) {
                 B = 0.5f - th2 * (1.0f / 24.0f);
                 Cc = (1.0f / 6.0f) - th2 * (1.0f / 120.0f);
             } else {
-                float s, c;
-                sincosf(th, &s, &c);
                 A = s / th;
                 B = (1.0f - c) / th2;
                 Cc = (th - s) / (th2 * th);
@@ -842,17 +843,65 @@ struct EdgeSrc {
     int G, nchunk, c;
 };
 
-__device__ __forceinline__ float cc_q(const CcBufs& B, const EdgeSrc* e, int w, int d) {
-    if (!e) return B.q[w * kDimMax + d];
+__device__ __forceinline__ float cc_q(const float* q, const EdgeSrc* e, int w, int d) {
+    if (!e) return q[w * kDimMax + d];
     const float t = __fdiv_rn((float)(e->c + w * e->nchunk + 1), (float)e->G);
     return __fmaf_rn(t, e->delta[d], e->base[d]);
 }
 
 // joint_value of waypoint w
-__device__ __forceinline__ float cc_joint_value(const JointRec& jr, const CcBufs& B, const EdgeSrc* e, int w) {
-    if (jr.idx.z >= 0) return fmaf(jr.tv.w, cc_q(B, e, w, jr.idx.z), jr.tw.w);
-    if (jr.idx.y >= 0) return cc_q(B, e, w, jr.idx.y);
+__device__ __forceinline__ float cc_joint_value(const JointRec& jr, const float* q, const EdgeSrc* e, int w) {
+    if (jr.idx.z >= 0) return fmaf(jr.tv.w, cc_q(q, e, w, jr.idx.z), jr.tw.w);
+    if (jr.idx.y >= 0) return cc_q(q, e, w, jr.idx.y);
     return 0.0f;
+}
+
+// Link frames of nw waypoints for robots of up to 32 joints, in registers: a
+// warp segment of SEG lanes per waypoint, lane j computes joint j's local
+// transform, then pointer jumping composes the chain -- each round
+// T_j = T_anc(j) o T_j, anc(j) = anc(anc(j)), ancestors read with shuffles -- in
+// ceil(log2 J) rounds with no barrier.  Parents precede their children (pack
+// order).  The frames go to pose[w][j][12] (three 16-byte stores per lane, which
+// spread over the banks); then after(w, j, SEG) runs on the segment's lanes,
+// which may read that waypoint's frames.
+template <class After>
+__device__ __forceinline__ void fk_segments(const Scene& sc, const float* q, float* pose, const EdgeSrc* edge, int nw,
+                                            int J, int tid, int T, After after) {
+    const int SEG = J <= 8 ? 8 : (J <= 16 ? 16 : 32);
+    const int per_warp = 32 / SEG, n_warps = T >> 5, warp = tid >> 5, lane = tid & 31;
+    const int sub = lane / SEG, j = lane - sub * SEG;
+    const int rounds = J <= 1 ? 0 : 32 - __clz(J - 1);
+    for (int w0 = warp * per_warp; w0 < nw; w0 += n_warps * per_warp) {
+        const int w = w0 + sub;
+        const bool act = j < J && w < nw;
+        float X[12] = {1.0f, 0.0f, 0.0f, 0.0f, 1.0f, 0.0f, 0.0f, 0.0f, 1.0f, 0.0f, 0.0f, 0.0f};
+        int a = -1;
+        if (act) {
+            const JointRec& jr = sc.joints[j];
+            joint_local(jr, cc_joint_value(jr, q, edge, w), X);
+            const int p = jr.idx.x;
+            a = (p >= 0 && p < j) ? p : -1;
+        }
+        for (int r = 0; r < rounds; ++r) {
+            const int src = lane - j + max(a, 0);
+            float Y[12];
+#pragma unroll
+            for (int i = 0; i < 12; ++i) Y[i] = __shfl_sync(0xffffffffu, X[i], src);
+            const int aa = __shfl_sync(0xffffffffu, a, src);
+            if (a >= 0) {
+                compose(Y, X, X);
+                a = aa;
+            }
+        }
+        if (act) {
+            float4* P = reinterpret_cast<float4*>(pose + (w * J + j) * 12);
+            P[0] = make_float4(X[0], X[1], X[2], X[3]);
+            P[1] = make_float4(X[4], X[5], X[6], X[7]);
+            P[2] = make_float4(X[8], X[9], X[10], X[11]);
+        }
+        __syncwarp();
+        if (w < nw) after(w, j, SEG);
+    }
 }
 
 // Collision check of nw (<= CW <= 32) configurations: B.q, or the waypoints of
@@ -910,53 +959,16 @@ __device__ inline uint32_t cc_chunk(const G& g, const Scene& sc, const CcBufs& B
         for (int i = tid; i < nw * QW; i += T) B.gate[i] = 0u;
     }
     if (J <= 32) {
-        // A+B in registers: a warp segment of SEG lanes per waypoint, lane j
-        // computes joint j's local transform, then pointer jumping composes
-        // the chain -- each round T_j = T_anc(j) o T_j, anc(j) = anc(anc(j)),
-        // ancestors read with shuffles -- in ceil(log2 J) rounds with no
-        // barrier.  Parents precede their children (pack order).
-        const int SEG = J <= 8 ? 8 : (J <= 16 ? 16 : 32);
-        const int per_warp = 32 / SEG, n_warps = T >> 5, warp = tid >> 5, lane = tid & 31;
-        const int sub = lane / SEG, j = lane - sub * SEG;
-        const int rounds = J <= 1 ? 0 : 32 - __clz(J - 1);
-        for (int w0 = warp * per_warp; w0 < nw; w0 += n_warps * per_warp) {
-            const int w = w0 + sub;
-            const bool act = j < J && w < nw;
-            float X[12] = {1.0f, 0.0f, 0.0f, 0.0f, 1.0f, 0.0f, 0.0f, 0.0f, 1.0f, 0.0f, 0.0f, 0.0f};
-            int a = -1;
-            if (act) {
-                const JointRec& jr = sc.joints[j];
-                joint_local(jr, cc_joint_value(jr, B, edge, w), X);
-                const int p = jr.idx.x;
-                a = (p >= 0 && p < j) ? p : -1;
-            }
-            for (int r = 0; r < rounds; ++r) {
-                const int src = lane - j + max(a, 0);
-                float Y[12];
-#pragma unroll
-                for (int i = 0; i < 12; ++i) Y[i] = __shfl_sync(0xffffffffu, X[i], src);
-                const int aa = __shfl_sync(0xffffffffu, a, src);
-                if (a >= 0) {
-                    compose(Y, X, X);
-                    a = aa;
-                }
-            }
-            if (act) {
-                float* P = &B.pose[(w * J + j) * 12];
-#pragma unroll
-                for (int i = 0; i < 12; ++i) P[i] = X[i];
-            }
-            __syncwarp();
-            // C, fused: the segment that composed waypoint w's frames places its
-            // sphere centres (warp-local data, so no CTA barrier in between)
-            if (w < nw) cc_centres(sc, B, w, j, SEG, J, S, S_pad, K, gated, inflate);
-        }
+        // A+B in registers; C, fused: the segment that composed waypoint w's frames
+        // places its sphere centres (warp-local data, so no CTA barrier in between)
+        fk_segments(sc, B.q, B.pose, edge, nw, J, tid, T,
+                    [&](int w, int j, int SEG) { cc_centres(sc, B, w, j, SEG, J, S, S_pad, K, gated, inflate); });
     } else {
         // A: local joint transforms, one (waypoint, joint) per thread
         for (int it = tid; it < nw * J; it += T) {
             const int w = it / J, j = it - w * J;
             const JointRec& jr = sc.joints[j];
-            joint_local(jr, cc_joint_value(jr, B, edge, w), &B.pose[(w * J + j) * 12]);
+            joint_local(jr, cc_joint_value(jr, B.q, edge, w), &B.pose[(w * J + j) * 12]);
         }
         g.sync();
         // B: chain composition in topological order, one waypoint per thread

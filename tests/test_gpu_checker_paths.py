@@ -68,3 +68,94 @@ def test_self_pair_items(cuda, mode, form):
             part["coarse_self_pairs"] = part["self_pair_ranges"] = np.zeros((0, 2), np.int32)
             want = _verdicts(part, robot, 0, q, cuda)
     assert np.array_equal(_verdicts(got, robot, mode, q, cuda), want)
+
+
+def _odd_scene(form, rng):
+    """A scene at the edge of what the culled edge check takes (or past it), and its robot."""
+    robot = scenes.arm(0)
+    ctx = build_collision_context(robot, scenes.uneven_world(rng) if form == "plain" else scenes.tabletop_world(rng))
+    if form == "many":  # more primitives around every link than a link's list holds (256)
+        s = scenes.spheres_world(rng, 700)["world_spheres"]
+        s[:, 3] = 0.01
+        ctx["world_spheres"] = s
+    elif form == "far_sphere":  # a link that reaches past the culled range touches every primitive: full lists
+        ctx["sphere_local"] = ctx["sphere_local"].copy()
+        ctx["sphere_local"][20] = (0.0, 0.0, 40.0)
+    elif form == "uncovered":  # groups that do not cover the first sphere
+        ctx["fine_link_offsets"] = ctx["fine_link_offsets"].copy()
+        ctx["fine_link_offsets"][0] = 1
+    elif form == "mixed_frames":  # a sphere listed in another link's group
+        ctx["sphere_link_idx"] = ctx["sphere_link_idx"].copy()
+        ctx["sphere_link_idx"][17] = 0
+    elif form == "small_coarse":  # coarse spheres that do not enclose their fine spheres (flat checkers ignore them)
+        ctx["coarse_sphere_radius"] = ctx["coarse_sphere_radius"] * 0.1
+    elif form == "long_normal":
+        ctx["world_halfspaces"] = np.array([[0, 0, 3.0, 0, 0, 0.02]], np.float32)
+    elif form == "sheared_boxes":
+        ctx["world_boxes"] = ctx["world_boxes"].copy()
+        ctx["world_boxes"][:, 3:12] *= 1.5
+        ctx["world_boxes"][::2, 3] += 0.4
+    elif form == "negative_radii":
+        ctx["world_spheres"] = ctx["world_spheres"].copy()
+        ctx["world_spheres"][::3, 3] *= -1
+        ctx["world_capsules"] = ctx["world_capsules"].copy()
+        ctx["world_capsules"][0, 6] *= -1
+    elif form == "nan_and_far":
+        ctx["world_spheres"] = np.concatenate([ctx["world_spheres"], np.array(
+            [[np.nan, 0, 0, 0.1], [3e5, -2e5, 1e5, 0.2], [np.inf, 0, 0, 0.1]], np.float32)])
+        ctx["world_capsules"] = np.concatenate([ctx["world_capsules"], ctx["world_capsules"][:1]])
+        ctx["world_capsules"][-1, 3:6] = ctx["world_capsules"][-1, :3] + 1e-25  # no length
+    return robot, ctx
+
+
+FORMS = ["plain", "many", "far_sphere", "uncovered", "mixed_frames", "small_coarse", "long_normal", "sheared_boxes",
+         "negative_radii", "nan_and_far"]
+COARSE = ("coarse_sphere_link_idx", "coarse_sphere_local", "coarse_sphere_radius", "fine_link_offsets",
+          "coarse_self_pairs", "self_pair_ranges")
+
+
+@pytest.mark.parametrize("checker", ["binary", "differentiable"])
+@pytest.mark.parametrize("form", FORMS)
+def test_culled_plans_equal_general_plans(cuda, form, checker):
+    """One explorer per problem: the same scene with its coarse model (culled edge checks) and without it (the
+    general checker) must give the same plans, bit for bit -- wide, ordinary and plain launches."""
+    from prrtc_b200 import prrtc_plan_batch
+
+    robot, ctx = _odd_scene(form, np.random.default_rng(11))
+    bare = {k: v for k, v in ctx.items() if k not in COARSE}
+    B = 6
+    # starts and goals need not be free: a plan that fails has to fail alike
+    q = np.random.default_rng(12).uniform(-1.2, 1.2, (2, B, robot.dim)).astype(np.float32)
+    kw = dict(max_iterations=60, num_new_samples=1, max_nodes=2048, min_vals=robot.lower, max_vals=robot.upper,
+              collision_checker=checker, edge_resolution=0.02, tail_explorers=False)
+
+    def plan(c, launch, threads):
+        return prrtc_plan_batch(q[0], q[1][:, None], collision_context=[c] * B, launch=launch,
+                                threads_per_explorer=threads, waypoint_chunk=16, **kw)
+
+    want = plan(bare, "persistent", 128)
+    for launch, threads in (("persistent", 0), ("per_problem", 64), ("per_problem", 256)):
+        for a, b in zip(plan(ctx, launch, threads), want):
+            assert (a.solved, a.tree_a_size, a.tree_b_size, a.iterations) == (
+                b.solved, b.tree_a_size, b.tree_b_size, b.iterations), (launch, threads)
+            for x, y in ((a.tree_a_configs, b.tree_a_configs), (a.tree_b_configs, b.tree_b_configs)):
+                assert np.array_equal(x.cpu().numpy().view(np.uint32), y.cpu().numpy().view(np.uint32)), (launch, threads)
+
+
+@pytest.mark.parametrize("n_joints", [2, 8, 9, 16])
+def test_culled_plans_across_joint_counts(cuda, n_joints):
+    """Joint counts at the edges of a waypoint's lane segment (8, 16, 32), large trees in a scan's second round."""
+    from prrtc_b200 import prrtc_plan_batch
+
+    robot = scenes.arm(1, n_joints)
+    ctx = build_collision_context(robot, scenes.dense_world(np.random.default_rng(2)))
+    bare = {k: v for k, v in ctx.items() if k not in COARSE}
+    q = np.random.default_rng(3).uniform(-1.0, 1.0, (2, 3, robot.dim)).astype(np.float32)
+    kw = dict(max_iterations=300, num_new_samples=1, max_nodes=1025, min_vals=robot.lower, max_vals=robot.upper,
+              step_size=0.1, edge_resolution=0.013, tail_explorers=False, dynamic_domain=False)
+    a = prrtc_plan_batch(q[0], q[1][:, None], collision_context=ctx, **kw)
+    b = prrtc_plan_batch(q[0], q[1][:, None], collision_context=bare, **kw)
+    for x, y in zip(a, b):
+        assert (x.solved, x.tree_a_size, x.tree_b_size, x.iterations) == (y.solved, y.tree_a_size, y.tree_b_size,
+                                                                          y.iterations)
+        assert np.array_equal(x.tree_a_configs.cpu().numpy().view(np.uint32), y.tree_a_configs.cpu().numpy().view(np.uint32))
