@@ -123,7 +123,7 @@ cudaError_t launch_iteration(float* ta, float* tb, int32_t* pa, int32_t* pb, int
                              int batch, int32_t* sizes, int32_t* completed, const float* step, int32_t* new_cfg,
                              int32_t* new_par, int32_t* valid, int32_t* solved, cudaStream_t st);
 cudaError_t launch_check(const unsigned char* blob, int blob_cap, const int32_t* pairs, int J, int S, int K,
-                         int Q, int dim, const float* configs, int n, int full_sweep, int32_t* verdicts,
+                         int Q, int dim, const float* configs, int n, int full_sweep, bool cull, int32_t* verdicts,
                          cudaStream_t st, const PcView* pc = nullptr);
 
 // pointcloud.cu

@@ -201,7 +201,8 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(PackSrc s, unsigned 
                          fabsf(u[0] * v[0] + u[1] * v[1] + u[2] * v[2]) <= 1e-4f;
                 }
                 note_size(fabsf(c[0]) + fabsf(c[1]) + fabsf(c[2]) + fabsf(c[12]) + fabsf(c[13]) + fabsf(c[14]));
-                o_wb[4 * i + 3] = make_float4(c[12] * kBoxInv, c[13] * kBoxInv, c[14] * kBoxInv, ok ? 0.0f : 1.0f);
+                if (!ok) atomicAnd(&s_cull, 0);
+                o_wb[4 * i + 3] = make_float4(c[12] * kBoxInv, c[13] * kBoxInv, c[14] * kBoxInv, 0.0f);
             }
         } else if (r < e6) {
             const int i = r - e5;
@@ -243,7 +244,7 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(PackSrc s, unsigned 
         for (int off = 4; off > 0; off >>= 1) reach = fmaxf(reach, __shfl_xor_sync(0xffffffffu, reach, off));
         const unsigned all_ok = __ballot_sync(0xffffffffu, ok) >> (tid & 24) & 0xffu;
         if (mine && l8 == 0) {
-            const float pad = kCullPad * (1.0f + __uint_as_float(s_scale));
+            const float pad = kCullPad * (1.0f + reach + __uint_as_float(s_scale));
             const float r = reach * 1.00001f + pad;
             reinterpret_cast<float*>(grp + 2 * k + 1)[3] =
                 all_ok == 0xffu && reach <= kCullReachMax && r < 1e6f ? r : INFINITY;
@@ -591,7 +592,7 @@ static __device__ __noinline__ int culled_edge_collides(const CulledEdges* a, co
         return (general_edge_collides(dsm, a->pairs, &a->pc, dsm + a->blob_cap, a->stats, base, delta, G, a->CW_general)
                     ? 1 : 0) | par << 1;
     }
-    CullBufs B = cull_bufs(dsm + a->blob_cap, a->J, a->K, a->n_obs, a->CW, true);
+    CullBufs B = cull_bufs(dsm + a->blob_cap, a->J, a->K, a->n_obs, a->CW);
     B.stats = a->stats;
     sc.pairs = a->pairs;
     sc.pc = a->pc;
@@ -600,7 +601,7 @@ static __device__ __noinline__ int culled_edge_collides(const CulledEdges* a, co
     for (int c = 0; c < nchunk; ++c) {
         const int nw = (G - c + nchunk - 1) / nchunk;
         const EdgeSrc e{base, delta, G, nchunk, c};
-        if (cull_check<true>(CtaGroup{}, sc, B, nw, a->CW, par, &e) != 0u) return 1 | par << 1;
+        if (cull_check(CtaGroup{}, sc, B, nw, a->CW, par, e) != 0u) return 1 | par << 1;
     }
     return par << 1;
 }
@@ -1099,13 +1100,15 @@ cudaError_t launch_plan(PlanLaunch& L, cudaStream_t st) {
     // per SM (200 tabletop problems, E = 1: 3.97 -> 3.74 ms against 256 threads; 61
     // dual-arm problems: 6.7 -> 5.1 ms; at E = 2 x 512 problems it loses, 4.4
     // -> 4.7 ms).
-    const bool wide = L.persistent && (long long)L.B * L.E <= 2ll * device_sm_count();
+    // So does a plain launch of at most one explorer per SM that asks for no size.
+    const bool wide = L.persistent ? (long long)L.B * L.E <= 2ll * device_sm_count()
+                                   : L.threads == 0 && (long long)L.B * L.E <= device_sm_count();
     bool cull = false;
     if (L.cull) {
         const size_t room = max_smem / (wide ? 1 : 2) - (wide ? 0 : 1024);
         for (int cw = 64; cw >= 8 && !cull; cw /= 2) {
             // the buffers also hold the general checker's, for a scene that is not culled
-            size_t need = (size_t)cull_smem_bytes(L.J, L.K, L.n_obs, cw, true);
+            size_t need = (size_t)cull_smem_bytes(L.J, L.K, L.n_obs, cw);
             need = std::max(need, (size_t)cc_smem_bytes(L.J, L.S, L.K, L.Q, 8));
             if (need + (size_t)L.blob_cap + static_smem > (cw > 8 ? room : max_smem)) continue;
             cull = true;

@@ -9,6 +9,7 @@
 #include <mutex>
 
 #include "kernels.h"
+#include "prrtc_cull.cuh"
 #include "prrtc_device.cuh"
 
 namespace prrtc {
@@ -411,6 +412,149 @@ static void check_go(const CheckLaunch& o, int full_sweep, const unsigned char* 
     kern<<<(unsigned)grid, 128, o.dyn, st>>>(blob, o.blob_cap, pairs, J, S, K, Q, dim, configs, n, verdicts, cloud);
 }
 
+// The culled checker: warps of their own, CW configurations at a time
+// (warp_check), the scene staged per CTA.
+//
+// Bound by instruction issue (65% of the issue slots, 16 to 24 warps per SM),
+// not by memory: of the time of 2^20 random tabletop configurations (79% in
+// collision) link frames take a quarter, self items a third, the links'
+// primitives the rest.  80 registers per thread and 24 warps per SM measured 15%
+// faster than 128 and 16; world links before self items 6% faster here but 20%
+// slower on uneven scenes.  Against the full sweep of the general checker: 2^20
+// tabletop configurations 2117 -> 800 us, uneven scene 2055 -> 870 us, 60,000
+// dual-arm configurations 1332 -> 280 us (gated) and 981 -> 280 us (flat).
+//
+// A scene that is not culled (BlobHeader::cull) takes the general checker, 8
+// configurations at a time by the whole CTA, in the same shared memory.
+static __device__ __noinline__ void check_general(const unsigned char* blob, const int2* pairs, const PcView* pc,
+                                                  unsigned char* smem, const float* configs, int n, int dim,
+                                                  int32_t* verdicts) {
+    constexpr int CW = 8;
+    Scene sc = scene_view(blob);
+    sc.pairs = pairs;
+    sc.pc = *pc;
+    const CcBufs B = cc_bufs(smem, sc.h->J, sc.h->S, sc.h->K, sc.h->Q, CW);
+    if (threadIdx.x == 0) B.hit[0] = B.hit[1] = 0u;
+    int par = 0;
+    __syncthreads();
+    for (int c0 = blockIdx.x * CW; c0 < n; c0 += gridDim.x * CW) {
+        const int nw = min(CW, n - c0);
+        for (int i = threadIdx.x; i < nw * dim; i += blockDim.x) {
+            const int w = i / dim, d = i - w * dim;
+            B.q[w * kDimMax + d] = configs[(size_t)(c0 + w) * dim + d];
+        }
+        __syncthreads();
+        const uint32_t hit = cc_chunk<false>(CtaGroup{}, sc, B, nw, false, par);
+        for (int w = threadIdx.x; w < nw; w += blockDim.x) verdicts[c0 + w] = (hit >> w) & 1u;
+    }
+}
+
+__global__ void __launch_bounds__(256, 3) check_cull_kernel(const unsigned char* __restrict__ gblob, int blob_cap,
+                                                            const int2* pairs, int J, int K, int dim, int CW,
+                                                            const float* __restrict__ configs, int n,
+                                                            int32_t* verdicts, PcView pc) {
+    extern __shared__ __align__(128) unsigned char dsm[];
+    __shared__ __align__(8) uint64_t mbar;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_warps = blockDim.x >> 5;
+    const int bytes = min(reinterpret_cast<const BlobHeader*>(gblob)->used_bytes, blob_cap);
+    if (tid == 0) mbar_init(&mbar);
+    __syncthreads();
+    uint32_t phase = 0;
+    int* err = reinterpret_cast<int*>(const_cast<unsigned char*>(gblob) + offsetof(BlobHeader, error));
+    if (!stage_blob(dsm, gblob, bytes, &mbar, phase, err, kBlobStagingTimeout, kWaitLimit)) {
+        // the bulk copy did not arrive in time: copy the scene with plain loads
+        for (int i = tid; i < bytes / 16; i += blockDim.x)
+            reinterpret_cast<uint4*>(dsm)[i] = reinterpret_cast<const uint4*>(gblob)[i];
+        __syncthreads();
+    }
+    Scene sc = scene_view(dsm);
+    if (!sc.h->cull) {
+        if (sc.h->enabled) {
+            check_general(dsm, pairs, &pc, dsm + blob_cap, configs, n, dim, verdicts);
+        } else {
+            for (int i = blockIdx.x * blockDim.x + tid; i < n; i += gridDim.x * blockDim.x) verdicts[i] = 0;
+        }
+        return;
+    }
+    sc.pairs = pairs;
+    sc.pc = pc;
+    const WarpBufs B = warp_bufs(dsm + blob_cap + warp * warp_check_bytes(J, K, CW), J, K, CW);
+    // chunk index: warps of one CTA take neighbouring chunks
+    for (long long c0 = ((long long)blockIdx.x * n_warps + warp) * CW; c0 < n; c0 += (long long)gridDim.x * n_warps * CW) {
+        const int nw = (int)min((long long)CW, n - c0);
+        for (int i = lane; i < nw * dim; i += 32) {
+            const int w = i / dim, d = i - w * dim;
+            B.q[w * kDimMax + d] = configs[c0 * dim + i];
+        }
+        __syncwarp();
+        const unsigned hit = warp_check(sc, B, nw, CW);
+        if (lane < nw) verdicts[c0 + lane] = (int)(hit >> lane & 1u);
+        __syncwarp();
+    }
+}
+
+// Limits of check_cull_kernel in one device's CUDA context: its largest dynamic
+// shared memory so far and what decides residency, read once.
+struct CullCheckAttrs {
+    unsigned long long ctx = 0ull;
+    int max_dyn = -1, regs = 0, sm_smem = 0, sms = 0;
+};
+static CullCheckAttrs g_cull_check_attr[kCheckAttrDevices];
+
+// Launches the culled checker, or returns cudaErrorInvalidConfiguration when
+// its buffers do not fit (the caller then takes the general one).
+static cudaError_t launch_check_cull(const unsigned char* blob, int blob_cap, const int32_t* pairs, int J, int S, int K,
+                                     int Q, int dim, const float* configs, int n, int32_t* verdicts, cudaStream_t st,
+                                     const PcView& pc) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const unsigned long long ctx = current_context_key();
+    std::lock_guard<std::mutex> lock(g_check_attr_mutex);
+    CullCheckAttrs dflt;
+    CullCheckAttrs& a = dev >= 0 && dev < kCheckAttrDevices ? g_cull_check_attr[dev] : dflt;
+    if (!ctx || a.ctx != ctx) {
+        a = CullCheckAttrs{};
+        cudaFuncAttributes fa;
+        if ((e = cudaFuncGetAttributes(&fa, check_cull_kernel)) != cudaSuccess ||
+            (e = cudaDeviceGetAttribute(&a.sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev)) != cudaSuccess)
+            return e;
+        a.regs = (fa.numRegs + 7) & ~7;
+        a.sms = device_sm_count();
+        a.ctx = ctx;
+    }
+    const int max_dyn = (int)device_max_smem() - 64;
+    const int general = cc_smem_bytes(J, S, K, Q, 8);  // a scene that is not culled
+    int best_cw = 0, best_wpc = 0, best_warps = 0, best_dyn = 0;
+    const int least = pc.n > 0 ? 1 : 4;  // configurations per warp; with a cloud each is 27 cells and their points per sphere
+    for (int cw = 32; cw >= least; cw /= 2) {
+        for (int wpc = 4; wpc <= 8; wpc *= 2) {
+            const int dyn = blob_cap + std::max(wpc * warp_check_bytes(J, K, cw), general);
+            if (dyn > max_dyn) continue;
+            const int per_sm = std::min(a.sm_smem / (dyn + 1024 + 64), 65536 / (a.regs * 32 * wpc));
+            const int warps = std::min(per_sm * wpc, 24);
+            if (warps > best_warps) { best_cw = cw; best_wpc = wpc; best_warps = warps; best_dyn = dyn; }
+        }
+    }
+    if (best_warps == 0) return cudaErrorInvalidConfiguration;
+    int cw = best_cw, wpc = best_wpc;
+    while (cw > least && (long long)cw * a.sms * best_warps > n) cw /= 2;  // fewer per warp before warps go idle
+    const long long chunks = (n + cw - 1) / cw;
+    while (wpc > 1 && chunks < (long long)a.sms * wpc) wpc /= 2;
+    const int dyn = blob_cap + std::max(wpc * warp_check_bytes(J, K, cw), general);
+    if (std::max(dyn, best_dyn) > a.max_dyn) {
+        if ((e = cudaFuncSetAttribute(check_cull_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      std::max(dyn, best_dyn))) != cudaSuccess)
+            return e;
+        a.max_dyn = std::max(dyn, best_dyn);
+    }
+    const long long resident = (long long)a.sms * std::max(1, std::min(a.sm_smem / (dyn + 1024 + 64), 65536 / (a.regs * 32 * wpc)));
+    const long long grid = std::min((chunks + wpc - 1) / wpc, resident);
+    check_cull_kernel<<<(unsigned)grid, wpc * 32, dyn, st>>>(blob, blob_cap, reinterpret_cast<const int2*>(pairs), J, K, dim,
+                                                             cw, configs, n, verdicts, pc);
+    return cudaGetLastError();
+}
+
 // Passes of PRRTC_CHECK_CW configurations, unless their buffers leave fewer
 // than PRRTC_CHECK_MINBLOCKS CTAs per SM (large robots: the sphere centres and
 // link frames of a pass grow with S and J); then half or a quarter as many
@@ -419,12 +563,16 @@ static void check_go(const CheckLaunch& o, int full_sweep, const unsigned char* 
 // per SM at 32 configurations per pass, three at 16 and four at 8: 44.0 M
 // checks/s at 32, 65.4 M at 8.
 cudaError_t launch_check(const unsigned char* blob, int blob_cap, const int32_t* pairs, int J, int S, int K,
-                         int Q, int dim, const float* configs, int n, int full_sweep, int32_t* verdicts,
+                         int Q, int dim, const float* configs, int n, int full_sweep, bool cull, int32_t* verdicts,
                          cudaStream_t st, const PcView* pc) {
     if (n <= 0) return cudaSuccess;
     const PcView cloud = pc ? *pc : PcView{nullptr, nullptr, 0, 0, 0.0f, 0.0f};
     constexpr int CW = PRRTC_CHECK_CW;
     CheckLaunch best, o;
+    if (cull) {
+        const cudaError_t e = launch_check_cull(blob, blob_cap, pairs, J, S, K, Q, dim, configs, n, verdicts, st, cloud);
+        if (e != cudaErrorInvalidConfiguration) return e;
+    }
     cudaError_t e = check_option<CW>(full_sweep, J, S, K, Q, blob_cap, best);
     if (e != cudaSuccess) return e;
     if constexpr (CW / 2 >= 8) {

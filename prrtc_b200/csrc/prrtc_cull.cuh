@@ -29,17 +29,16 @@ namespace prrtc {
 
 constexpr int kCullLinkList = 256;  // primitives listed per link of an edge; more: all of them are tested
 
-// Shared-memory buffers of a culled check of CW waypoints.
+// Shared-memory buffers of a culled edge pass of CW waypoints.
 struct CullBufs {
-    float* q;          // [CW][kDimMax] (configurations; unused for edges)
     float* pose;       // [CW][J][12]
-    float4* cctr;      // [K][CW] coarse sphere centres, .w = radius + inflation
-    float4* swept;     // [K] (edges) bound of the link's cull spheres over the pass
+    float4* cctr;      // [K][CW] coarse sphere centres, .w = radius + inflation (gated) or the cull radius (flat)
+    float4* swept;     // [K] bound of the link's cull spheres over the pass
     uint32_t* dirty;   // [CW][2] links whose coarse sphere touches the world (gated)
     int2* wlist;       // [wcap] (group of 32 << 12 | link << 6 | waypoint, mask of primitives in the group)
     int* slist;        // [scap] self item << 6 | waypoint
-    int4* ncand;       // [K] (edges) primitives listed for a link: ends of the spheres, capsules, boxes, all; .w -1: too many
-    uint16_t* cand;    // [K][ccap] (edges)
+    int4* ncand;       // [K] primitives listed for a link: ends of the spheres, capsules, boxes, all; .w -1: too many
+    uint16_t* cand;    // [K][ccap]
     uint32_t* hit;     // [6]: result words, world and self list lengths, alternating between calls
     int wcap, scap, ccap;
     unsigned long long* stats;
@@ -51,21 +50,18 @@ __host__ __device__ inline int cull_link_list(int n_obs) { return n_obs < kCullL
 __host__ __device__ inline int cull_wcap(int K, int CW) { return (K * CW / 2 + 63) & ~31; }
 __host__ __device__ inline int cull_scap(int CW) { return 12 * CW; }
 
-__host__ __device__ inline int cull_smem_bytes(int J, int K, int n_obs, int CW, bool edge) {
-    int b = edge ? 0 : CW * kDimMax * 4;
-    b += CW * J * 48 + K * CW * 16 + K * 32 + CW * 8;
+__host__ __device__ inline int cull_smem_bytes(int J, int K, int n_obs, int CW) {
+    int b = CW * J * 48 + K * CW * 16 + K * 32 + CW * 8;
     b += cull_wcap(K, CW) * 8 + cull_scap(CW) * 4 + 32;
-    if (edge) b += align16(K * cull_link_list(n_obs) * 2);
-    return b;
+    return b + align16(K * cull_link_list(n_obs) * 2);
 }
 
-__device__ __forceinline__ CullBufs cull_bufs(unsigned char* p, int J, int K, int n_obs, int CW, bool edge) {
+__device__ __forceinline__ CullBufs cull_bufs(unsigned char* p, int J, int K, int n_obs, int CW) {
     CullBufs b;
     b.wcap = cull_wcap(K, CW);
     b.scap = cull_scap(CW);
     b.ccap = cull_link_list(n_obs);
     b.hit = reinterpret_cast<uint32_t*>(p);    p += 32;
-    b.q = reinterpret_cast<float*>(p);         p += edge ? 0 : CW * kDimMax * 4;
     b.pose = reinterpret_cast<float*>(p);      p += CW * J * 48;
     b.cctr = reinterpret_cast<float4*>(p);     p += K * CW * 16;
     b.swept = reinterpret_cast<float4*>(p);    p += K * 16;
@@ -88,30 +84,44 @@ inline bool cull_shape_ok(int J, int K, int n_obs, float inflate) {
 // touch (false for NaN, and for a distance so large that it may be an overflow).
 __device__ __forceinline__ bool cull_far(float d2, float b) { return d2 > b * b && d2 < 1e30f; }
 
-// Whether one primitive of each type may touch the sphere (c, R).
-__device__ __forceinline__ bool cull_sphere(const Scene& sc, int o, float4 c, float R) {
-    const float4 O = sc.ws[2 * o];  // (-2 centre, -2 radius)
-    const float dx = fmaf(0.5f, O.x, c.x), dy = fmaf(0.5f, O.y, c.y), dz = fmaf(0.5f, O.z, c.z);
-    return !cull_far(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), fmaf(0.5f, fabsf(O.w), R));
+// A cull sphere: centre and padded radius, and -(|c|^2 - R^2), the sphere
+// test's threshold.
+struct CullBall {
+    float4 c;
+    float thr;
+};
+
+__device__ __forceinline__ CullBall cull_ball(float4 c, float R) {
+    const float4 b = make_float4(c.x, c.y, c.z, R);
+    return CullBall{b, -sphere_A(b)};
 }
-__device__ __forceinline__ bool cull_capsule(const Scene& sc, int o, float4 c, float R) {
+
+// Whether one primitive of each type may touch the ball: the fine tests' own
+// forms on the cull sphere (four FMAs and a comparison for a sphere; the sign of
+// a radius is dropped, since the fine test squares the sum).
+__device__ __forceinline__ bool cull_sphere(const Scene& sc, int o, const CullBall& b) {
+    const float4 O = sc.ws[2 * o];
+    const float h = fmaf(b.c.x, O.x, fmaf(b.c.y, O.y, fmaf(b.c.z, O.z, fmaf(b.c.w, -fabsf(O.w), sc.ws[2 * o + 1].w))));
+    return !(h > b.thr);
+}
+__device__ __forceinline__ bool cull_capsule(const Scene& sc, int o, const CullBall& b) {
     const float4 p1 = sc.wc[3 * o], dp = sc.wc[3 * o + 1], d = sc.wc[3 * o + 2];
+    const float4 c = b.c;
     const float t = __saturatef(fmaf(dp.x, c.x, fmaf(dp.y, c.y, fmaf(dp.z, c.z, dp.w))));
     const float ex = fmaf(-t, d.x, c.x - p1.x), ey = fmaf(-t, d.y, c.y - p1.y), ez = fmaf(-t, d.z, c.z - p1.z);
-    return !cull_far(fmaf(ex, ex, fmaf(ey, ey, ez * ez)), R + fabsf(p1.w));
+    return !cull_far(fmaf(ex, ex, fmaf(ey, ey, ez * ez)), c.w + fabsf(p1.w));
 }
-__device__ __forceinline__ bool cull_box(const Scene& sc, int o, float4 c, float R) {
-    const float4 cc[1] = {c};
-    const float4 hl = sc.wb[4 * o + 3];
+__device__ __forceinline__ bool cull_box(const Scene& sc, int o, const CullBall& b) {
+    const float4 cc[1] = {b.c};
     float v[1];
-    h_box<1>(v, cc, sc.wb[4 * o], sc.wb[4 * o + 1], sc.wb[4 * o + 2], hl);
-    return !(v[0] > (R * kBoxInv) * (R * kBoxInv)) || hl.w != 0.0f;
+    h_box<1>(v, cc, sc.wb[4 * o], sc.wb[4 * o + 1], sc.wb[4 * o + 2], sc.wb[4 * o + 3]);
+    return !(v[0] > (b.c.w * kBoxInv) * (b.c.w * kBoxInv));
 }
-__device__ __forceinline__ bool cull_halfspace(const Scene& sc, int o, float4 c, float R) {
-    const float4 cc[1] = {c};
+__device__ __forceinline__ bool cull_halfspace(const Scene& sc, int o, const CullBall& b) {
+    const float4 cc[1] = {b.c};
     float v[1];
     h_halfspace<1>(v, cc, sc.wh[o]);
-    return !(v[0] > R);
+    return !(v[0] > b.c.w);
 }
 
 // The exact test of primitive o (combined index) against one sphere: the
@@ -161,7 +171,24 @@ __device__ __forceinline__ float4 fine_centre(const Scene& sc, const float* pose
 // Padded cull radius of a link whose coarse centre is c (grp record .w: reach
 // of its spheres and the scene's share of the pad).
 __device__ __forceinline__ float cull_radius(float reach, float inflate, float4 c) {
-    return reach + inflate + kCullPad * (fabsf(c.x) + fabsf(c.y) + fabsf(c.z));
+    return reach + (1.0f + kCullPad) * inflate + kCullPad * (fabsf(c.x) + fabsf(c.y) + fabsf(c.z));
+}
+
+// Coarse centre of link k at waypoint w with the radius that its checker works
+// with: the coarse sphere's own for a gated one, else the cull radius.
+__device__ __forceinline__ float4 link_centre(const Scene& sc, const float* pose, int J, int w, int k, float inflate,
+                                              bool gated) {
+    float4 l = sc.grp[2 * k];
+    const float4 g = sc.grp[2 * k + 1];
+    l.w += inflate;
+    float4 c = pose_point(pose, J, w, __float_as_int(g.x), l);
+    if (!gated) c.w = cull_radius(g.w, inflate, c);
+    return c;
+}
+
+// The cull radius that belongs to a stored link centre.
+__device__ __forceinline__ float link_radius(const Scene& sc, int k, float inflate, bool gated, float4 c) {
+    return gated ? cull_radius(sc.grp[2 * k + 1].w, inflate, c) : c.w;
 }
 
 // Whether self item ii needs its fine test at waypoint w: the gate of a gated
@@ -179,7 +206,7 @@ __device__ __forceinline__ bool cull_self_touch(const Scene& sc, const CullBufs&
         const float t = a.w + b.w - inflate;
         return d2 <= t * t;
     }
-    return !cull_far(d2, cull_radius(sc.grp[2 * cp.x + 1].w, inflate, a) + cull_radius(sc.grp[2 * cp.y + 1].w, inflate, b));
+    return !cull_far(d2, a.w + b.w);  // a flat checker's block: .w is the cull radius
 }
 
 // Fine test of self item ii at waypoint w by 8 consecutive lanes (l8 = 0..7 of
@@ -194,14 +221,6 @@ __device__ __forceinline__ bool cull_self_item(const Scene& sc, const CullBufs& 
         const int na = item.z >> 16, nb = item.z & 0xffff;
         const float half = 0.5f * inflate;
         float4 a[1] = {l8 < na ? fine_centre(sc, B.pose, J, w, item.x + l8, inflate) : absent_sphere()};
-        // no sphere of the first group near the second link's cull sphere: nothing can touch
-        const int lb = sc.cpair[item.w >= 0 ? item.w : -2 - item.w].y;
-        const float4 cb = B.cctr[lb * CW + w];
-        const float ex = a[0].x - cb.x, ey = a[0].y - cb.y, ez = a[0].z - cb.z;
-        const bool near = l8 < na && !cull_far(fmaf(ex, ex, fmaf(ey, ey, ez * ez)),
-                                               a[0].w + cull_radius(sc.grp[2 * lb + 1].w, inflate, cb) +
-                                                   kCullPad * (fabsf(a[0].x) + fabsf(a[0].y) + fabsf(a[0].z)));
-        if (!__any_sync(mask, near)) return false;
         a[0].w -= half;
         const float thr = -sphere_A(a[0]);
         for (int b0 = 0; b0 < nb; b0 += 8) {
@@ -250,6 +269,101 @@ static __device__ __noinline__ bool cull_link_all(const unsigned char* blob, con
     return hit;
 }
 
+// Up to 32 spheres against the point cloud, one per lane (the whole warp calls
+// it): lane's sphere c (radius + inflation in .w) belongs to configuration w,
+// and `alive` (the same in every lane) says which configurations still matter.
+// Returns the configurations hit, as a mask, the same in every lane.  The
+// verdicts are pc_sphere_hits': every cell of a sphere's bounding box, a box of
+// more than kPcMaxCells cells is a hit.
+//
+// A sphere spans 8 to 27 cells, most of them empty, and an occupied one holds
+// some 20 points.  A lane that walked its own sphere's cells and points made the
+// warp wait for its longest chain of dependent loads, so the cells of all 32
+// spheres are dealt out over the lanes, and the points of an occupied cell over
+// 8 of them: 128 edges of 16 waypoints against 20,000 points take 83 us a call
+// instead of 577, 8000 edges of 33 against 5000 points as long as before.
+__device__ __forceinline__ unsigned cloud_batch(const PcView& pc, float4 c, bool valid, int w, unsigned alive,
+                                                unsigned& flops) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31, l8 = lane & 7, sub = lane >> 3;
+    const float R = c.w + pc.r_env;
+    valid = valid && (alive >> w & 1u) && fabsf(c.x) < kPcExtent && fabsf(c.y) < kPcExtent && fabsf(c.z) < kPcExtent && R >= 0.0f;
+    bool hit = valid && !(R < 1.0e3f);
+    int x0 = 0, y0 = 0, z0 = 0, nx = 0, ny = 0, n = 0;
+    if (valid && !hit) {
+        x0 = (int)floorf((c.x - R) * pc.inv_cell);
+        y0 = (int)floorf((c.y - R) * pc.inv_cell);
+        z0 = (int)floorf((c.z - R) * pc.inv_cell);
+        const int x1 = (int)floorf((c.x + R) * pc.inv_cell), y1 = (int)floorf((c.y + R) * pc.inv_cell);
+        const int z1 = (int)floorf((c.z + R) * pc.inv_cell);
+        const long long cells = ((long long)x1 - x0 + 1) * ((long long)y1 - y0 + 1) * ((long long)z1 - z0 + 1);
+        hit = cells > kPcMaxCells;
+        if (!hit) {
+            nx = x1 - x0 + 1;
+            ny = y1 - y0 + 1;
+            n = (int)cells;
+        }
+    }
+    unsigned hits = __reduce_or_sync(kAll, hit ? 1u << w : 0u);
+    alive &= ~hits;
+    if (!(alive >> w & 1u)) n = 0;
+    int incl = n;  // cells of lanes 0..lane
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int v = __shfl_up_sync(kAll, incl, off);
+        if (lane >= off) incl += v;
+    }
+    const int total = __shfl_sync(kAll, incl, 31);
+    const float R2 = R * R;
+    for (int base = 0; base < total && alive; base += 32) {
+        const int idx = base + lane;
+        int own = 0;  // the first lane whose count passes idx
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1) own += __shfl_sync(kAll, incl, own + step - 1) <= idx ? step : 0;
+        own = min(own, 31);
+        const int r = idx - __shfl_sync(kAll, incl, own) + __shfl_sync(kAll, n, own);
+        const int onx = max(1, __shfl_sync(kAll, nx, own)), ony = max(1, __shfl_sync(kAll, ny, own));
+        const int ow = __shfl_sync(kAll, w, own);
+        const int ryz = r / onx, rx = r - ryz * onx, rz = ryz / ony, ry = ryz - rz * ony;
+        const unsigned b = pc_hash(__shfl_sync(kAll, x0, own) + rx, __shfl_sync(kAll, y0, own) + ry,
+                                   __shfl_sync(kAll, z0, own) + rz, pc.mask);
+        int p0 = 0, p1 = 0;
+        if (idx < total && (alive >> ow & 1u)) {
+            p0 = __ldg(&pc.start[b]);
+            p1 = __ldg(&pc.start[b + 1]);
+        }
+        for (unsigned todo = __ballot_sync(kAll, p1 > p0); todo;) {
+            unsigned t = todo;  // the next four occupied cells, one per group of 8 lanes
+            int src = -1;
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                if (g == sub && t) src = __ffs(t) - 1;
+                t &= t - 1u;
+            }
+            todo = t;
+            const int from = max(src, 0);
+            const int e = __shfl_sync(kAll, own, from), ew = __shfl_sync(kAll, ow, from);
+            const int e0 = __shfl_sync(kAll, p0, from), e1 = __shfl_sync(kAll, p1, from);
+            const float cx = __shfl_sync(kAll, c.x, e), cy = __shfl_sync(kAll, c.y, e), cz = __shfl_sync(kAll, c.z, e);
+            const float cr = __shfl_sync(kAll, R2, e);
+            hit = false;
+            if (src >= 0 && (alive >> ew & 1u)) {
+#pragma unroll 2
+                for (int p = e0 + l8; p < e1; p += 8) {
+                    const float4 q = __ldg(&pc.pts[p]);
+                    const float dx = cx - q.x, dy = cy - q.y, dz = cz - q.z;
+                    hit |= fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= cr;
+                    flops += kFlopPoint;
+                }
+            }
+            const unsigned h = __reduce_or_sync(kAll, hit ? 1u << ew : 0u);
+            hits |= h;
+            alive &= ~h;
+        }
+    }
+    return hits;
+}
+
 // One type's primitives of a link's bound (a warp, a primitive per lane):
 // appends those that touch to the link's list and returns its new length.
 template <class Touch>
@@ -266,15 +380,13 @@ __device__ __forceinline__ int cull_append(int count, int base, int n, int cap, 
     return n;
 }
 
-// Collision check of nw (<= CW <= 64) waypoints of `edge` (EDGE: the answer is
-// whether any collides) or of the configurations in B.q (nw <= 32: bit w of the
-// answer).  Called by every thread of the CTA with the same `par`, which the call
-// flips: the result words and list lengths alternate between calls, so that a
+// Whether any of nw (<= CW <= 64) waypoints of `edge` collides (non-zero).
+// Called by every thread of the CTA with the same `par`, which the call flips: the result words and list lengths alternate between calls, so that a
 // call clears the next call's after its first barrier.  All must be zero and
 // `par` 0 before the first call.  The scene must have BlobHeader::cull set.
-template <bool EDGE, class G>
+template <class G>
 __device__ __forceinline__ uint32_t cull_check(const G& g, const Scene& sc, const CullBufs& B, int nw, int CW, int& par,
-                                               const EdgeSrc* edge) {
+                                               const EdgeSrc& edge) {
     const BlobHeader& h = *sc.h;
     const int tid = g.rank(), T = g.size(), lane = tid & 31, warp = tid >> 5, n_warps = T >> 5;
     const int J = h.J, S = h.S, K = h.K;
@@ -291,11 +403,9 @@ __device__ __forceinline__ uint32_t cull_check(const G& g, const Scene& sc, cons
     // 1. link frames (as cc_chunk) and coarse centres
     if (gated)
         for (int i = tid; i < 2 * nw; i += T) B.dirty[i] = 0u;
-    fk_segments(sc, B.q, B.pose, EDGE ? edge : nullptr, nw, J, tid, T, [&](int w, int j, int SEG) {
+    fk_segments(sc, nullptr, B.pose, &edge, nw, J, tid, T, [&](int w, int j, int SEG) {
         for (int k = j; k < K; k += SEG) {
-            float4 l = sc.grp[2 * k];
-            l.w += inflate;
-            B.cctr[k * CW + w] = pose_point(B.pose, J, w, __float_as_int(sc.grp[2 * k + 1].x), l);
+            B.cctr[k * CW + w] = link_centre(sc, B.pose, J, w, k, inflate, gated);
         }
     });
     g.sync();
@@ -303,32 +413,31 @@ __device__ __forceinline__ uint32_t cull_check(const G& g, const Scene& sc, cons
         B.hit[par] = 0u;
         B.hit[2 + par] = B.hit[4 + par] = 0u;
     }
-    // 2. edges: one bound per link over the pass, and the primitives it touches (a warp per link)
-    if constexpr (EDGE) {
-        for (int k = warp; k < K; k += n_warps) {
-            const float4 m = B.cctr[k * CW + (nw >> 1)];
-            unsigned far2 = 0u;  // bits of the largest squared distance (NaN orders above infinity)
-            for (int w = lane; w < nw; w += 32) {
-                const float4 c = B.cctr[k * CW + w];
-                const float dx = c.x - m.x, dy = c.y - m.y, dz = c.z - m.z;
-                far2 = max(far2, __float_as_uint(fmaf(dx, dx, fmaf(dy, dy, dz * dz))) & 0x7fffffffu);
-            }
-            const float d = __fsqrt_ru(__uint_as_float(__reduce_max_sync(0xffffffffu, far2)));
-            const float R = cull_radius(sc.grp[2 * k + 1].w, inflate, m) + (1.0f + 2.0f * kCullPad) * d;
-            uint16_t* list = B.cand + k * B.ccap;
-            int4 n;
-            n.x = cull_append(Ns, 0, 0, B.ccap, list, lane, [&](int o) { return cull_sphere(sc, o, m, R); });
-            n.y = cull_append(Nc, Ns, n.x, B.ccap, list, lane, [&](int o) { return cull_capsule(sc, o, m, R); });
-            n.z = cull_append(Nb, Ns + Nc, n.y, B.ccap, list, lane, [&](int o) { return cull_box(sc, o, m, R); });
-            n.w = cull_append(Nh, Ns + Nc + Nb, n.z, B.ccap, list, lane, [&](int o) { return cull_halfspace(sc, o, m, R); });
-            if (lane == 0) {
-                B.swept[k] = make_float4(m.x, m.y, m.z, R);
-                B.ncand[k] = n.w <= B.ccap ? n : make_int4(0, 0, 0, -1);
-                if (B.stats) flops += Ns * kFlopSphere + Nc * kFlopCapsule + Nb * kFlopBox + Nh * kFlopHalfspace;
-            }
+    // 2. one bound per link over the pass, and the primitives it touches (a warp per link)
+    for (int k = warp; k < K; k += n_warps) {
+        const float4 m = B.cctr[k * CW + (nw >> 1)];
+        unsigned far2 = 0u;  // bits of the largest squared distance (NaN orders above infinity)
+        for (int w = lane; w < nw; w += 32) {
+            const float4 c = B.cctr[k * CW + w];
+            const float dx = c.x - m.x, dy = c.y - m.y, dz = c.z - m.z;
+            far2 = max(far2, __float_as_uint(fmaf(dx, dx, fmaf(dy, dy, dz * dz))) & 0x7fffffffu);
         }
-        g.sync();
+        const float d = __fsqrt_ru(__uint_as_float(__reduce_max_sync(0xffffffffu, far2)));
+        const float R = cull_radius(sc.grp[2 * k + 1].w, inflate, m) + (1.0f + 2.0f * kCullPad) * d;
+        uint16_t* list = B.cand + k * B.ccap;
+        const CullBall ball = cull_ball(m, R);
+        int4 n;
+        n.x = cull_append(Ns, 0, 0, B.ccap, list, lane, [&](int o) { return cull_sphere(sc, o, ball); });
+        n.y = cull_append(Nc, Ns, n.x, B.ccap, list, lane, [&](int o) { return cull_capsule(sc, o, ball); });
+        n.z = cull_append(Nb, Ns + Nc, n.y, B.ccap, list, lane, [&](int o) { return cull_box(sc, o, ball); });
+        n.w = cull_append(Nh, Ns + Nc + Nb, n.z, B.ccap, list, lane, [&](int o) { return cull_halfspace(sc, o, ball); });
+        if (lane == 0) {
+            B.swept[k] = make_float4(m.x, m.y, m.z, R);
+            B.ncand[k] = n.w <= B.ccap ? n : make_int4(0, 0, 0, -1);
+            if (B.stats) flops += Ns * kFlopSphere + Nc * kFlopCapsule + Nb * kFlopBox + Nh * kFlopHalfspace;
+        }
     }
+    g.sync();
     // 3. touching (link, waypoint) primitives and self items: a warp per link or item, a waypoint per lane
     const int wide = (nw + 31) >> 5;
     for (int u = warp; u < K * wide + h.n_items; u += n_warps) {
@@ -336,30 +445,28 @@ __device__ __forceinline__ uint32_t cull_check(const G& g, const Scene& sc, cons
             const int k = wide == 1 ? u : u >> 1, w = (wide == 1 ? 0 : (u & 1) << 5) + lane;
             int4 n = make_int4(Ns, Ns + Nc, Ns + Nc + Nb, Ns + Nc + Nb + Nh);
             const uint16_t* list = nullptr;  // the link's list, or every primitive
-            if constexpr (EDGE) {
-                const int4 m = B.ncand[k];
-                if (m.w >= 0) {
-                    n = m;
-                    list = B.cand + k * B.ccap;
-                }
+            const int4 m = B.ncand[k];
+            if (m.w >= 0) {
+                n = m;
+                list = B.cand + k * B.ccap;
             }
-            auto at_index = [&](int i) { return EDGE && list ? (int)list[i] : i; };
+            auto at_index = [&](int i) { return list ? (int)list[i] : i; };
             if (w >= nw) continue;
             const float4 c = B.cctr[k * CW + w];
-            const float R = cull_radius(sc.grp[2 * k + 1].w, inflate, c);
+            const CullBall ball = cull_ball(c, link_radius(sc, k, inflate, gated, c));
             bool dirty = false;
             for (int i0 = 0; i0 < n.w; i0 += 32) {
                 const int i1 = min(n.w, i0 + 32);
                 unsigned bits = 0u;
                 int i = i0;
 #pragma unroll 1
-                for (; i < min(n.x, i1); ++i) bits |= (unsigned)cull_sphere(sc, at_index(i), c, R) << (i - i0);
+                for (; i < min(n.x, i1); ++i) bits |= (unsigned)cull_sphere(sc, at_index(i), ball) << (i - i0);
 #pragma unroll 1
-                for (; i < min(n.y, i1); ++i) bits |= (unsigned)cull_capsule(sc, at_index(i) - Ns, c, R) << (i - i0);
+                for (; i < min(n.y, i1); ++i) bits |= (unsigned)cull_capsule(sc, at_index(i) - Ns, ball) << (i - i0);
 #pragma unroll 1
-                for (; i < min(n.z, i1); ++i) bits |= (unsigned)cull_box(sc, at_index(i) - Ns - Nc, c, R) << (i - i0);
+                for (; i < min(n.z, i1); ++i) bits |= (unsigned)cull_box(sc, at_index(i) - Ns - Nc, ball) << (i - i0);
 #pragma unroll 1
-                for (; i < i1; ++i) bits |= (unsigned)cull_halfspace(sc, at_index(i) - Ns - Nc - Nb, c, R) << (i - i0);
+                for (; i < i1; ++i) bits |= (unsigned)cull_halfspace(sc, at_index(i) - Ns - Nc - Nb, ball) << (i - i0);
                 if (!bits) continue;
                 if (gated)
                     for (unsigned rest = bits; rest && !dirty; rest &= rest - 1u)
@@ -373,15 +480,13 @@ __device__ __forceinline__ uint32_t cull_check(const G& g, const Scene& sc, cons
         } else {
             const int ii = u - K * wide;
             const int4 item = sc.item[ii];
-            if constexpr (EDGE) {  // links whose bounds are apart: no waypoint touches
-                const int q = item.w >= 0 ? item.w : -2 - item.w;
-                if (q >= 0) {
-                    const int2 cp = sc.cpair[q];
-                    if (cp.x < 0 || cp.y < 0 || cp.x >= K || cp.y >= K) continue;
-                    const float4 a = B.swept[cp.x], b = B.swept[cp.y];
-                    const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
-                    if (cull_far(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), a.w + b.w)) continue;
-                }
+            const int q = item.w >= 0 ? item.w : -2 - item.w;
+            if (q >= 0) {  // links whose bounds are apart: no waypoint touches
+                const int2 cp = sc.cpair[q];
+                if (cp.x < 0 || cp.y < 0 || cp.x >= K || cp.y >= K) continue;
+                const float4 a = B.swept[cp.x], b = B.swept[cp.y];
+                const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
+                if (cull_far(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), a.w + b.w)) continue;
             }
             for (int w = lane; w < nw; w += 32) {
                 flops += kFlopPairExplicit;
@@ -418,17 +523,15 @@ __device__ __forceinline__ uint32_t cull_check(const G& g, const Scene& sc, cons
                     k = (e.x >> 6) & 63;
                     w = e.x & 63;
                 }
-                if (EDGE ? (seen != 0u) : ((seen >> w) & 1u)) continue;
+                if (seen) continue;
                 if (gated && !(B.dirty[2 * w + (k >> 5)] & (1u << (k & 31)))) continue;
                 if (wfull) {
-                    if (cull_link_all(reinterpret_cast<const unsigned char*>(sc.h), B.pose, k, w, l8))
-                        atomicOr(hw, 1u << (w & 31));
+                    if (cull_link_all(reinterpret_cast<const unsigned char*>(sc.h), B.pose, k, w, l8)) atomicOr(hw, 1u);
                     continue;
                 }
                 const float4 gr = sc.grp[2 * k + 1];
                 const int i0 = (e.x >> 12) << 5;
-                const uint16_t* list = nullptr;
-                if constexpr (EDGE) list = B.ncand[k].w >= 0 ? B.cand + k * B.ccap + i0 : nullptr;
+                const uint16_t* list = B.ncand[k].w >= 0 ? B.cand + k * B.ccap + i0 : nullptr;
                 const int s1 = __float_as_int(gr.z);
 #pragma unroll 1
                 for (int s = __float_as_int(gr.y) + l8; s < s1; s += 8) {
@@ -436,7 +539,7 @@ __device__ __forceinline__ uint32_t cull_check(const G& g, const Scene& sc, cons
 #pragma unroll 1
                     for (unsigned rest = (unsigned)e.y; rest; rest &= rest - 1u) {
                         const int i = __ffs(rest) - 1;
-                        const int o = EDGE && list ? (int)list[i] : i0 + i;
+                        const int o = list ? (int)list[i] : i0 + i;
                         hit |= prim_hits(sc, h, o, c);
                         if (B.stats) flops += prim_flops(h, o);
                     }
@@ -452,20 +555,22 @@ __device__ __forceinline__ uint32_t cull_check(const G& g, const Scene& sc, cons
                     ii = e >> 6;
                     w = e & 63;
                 }
-                if (EDGE ? (seen != 0u) : ((seen >> w) & 1u)) continue;
+                if (seen) continue;
                 if (sfull && !cull_self_touch(sc, B, CW, sc.item[ii], w, inflate)) continue;
                 hit = cull_self_item(sc, B, CW, ii, w, l8, mask, inflate, flops);
             }
-            if (hit) atomicOr(hw, 1u << (w & 31));
+            if (hit) atomicOr(hw, 1u);
         }
         if (cloud) {
-            unsigned long long f = 0;
-            for (int it = tid; it < S * nw; it += T) {
-                const int s = it / nw, w = it - s * nw;
-                if (EDGE ? (*vhit != 0u) : ((*vhit >> w) & 1u)) continue;
-                if (pc_sphere_hits(sc.pc, fine_centre(sc, B.pose, J, w, s, inflate), false, f)) atomicOr(hw, 1u << (w & 31));
+            // every sphere of every waypoint, a batch of 32 per warp (the hit
+            // word is read by one lane for all)
+            for (int it0 = warp << 5; it0 < S * nw; it0 += n_warps << 5) {
+                const uint32_t seen = __shfl_sync(0xffffffffu, (uint32_t)*vhit, 0);
+                if (seen) break;
+                const int it = it0 + lane, s = min(it, S * nw - 1) / nw, w = min(it, S * nw - 1) - s * nw;
+                const float4 c = fine_centre(sc, B.pose, J, w, s, inflate);
+                if (cloud_batch(sc.pc, c, it < S * nw, 0, 1u, flops) && lane == 0) atomicOr(hw, 1u);
             }
-            flops += (unsigned)f;
         }
     }
     if (B.stats) {
@@ -478,6 +583,185 @@ __device__ __forceinline__ uint32_t cull_check(const G& g, const Scene& sc, cons
     if (Lw + Ls == 0 && !cloud) return *vhit;  // no entry, so no write of the word: no barrier
     g.sync();
     return *vhit;
+}
+
+// ----------------------------------------------------------------------------- configurations
+
+// Culled check of up to 32 unrelated configurations by one warp, no CTA barrier:
+// link frames, self items, then the links from the tip to the base, a
+// (configuration, link) per lane.  Each lane marks the primitives that its link's cull sphere touches,
+// and the warp tests the marked links right away, 8 lanes per link.  A
+// configuration leaves at its first hit, and the links still to do are dealt
+// out over the configurations that are left, so the lanes stay full while most
+// configurations of a cluttered scene end after two or three links.
+struct WarpBufs {
+    float* q;        // [CW][kDimMax]; masks of touched primitives after the frames are done
+    float* pose;     // [CW][J][12]
+    float4* cctr;    // [K][CW] as CullBufs
+    int* list;       // [32] configurations left
+};
+
+__host__ __device__ inline int warp_check_bytes(int J, int K, int CW) {
+    return (CW * kDimMax * 4 > 1024 ? CW * kDimMax * 4 : 1024) + CW * J * 48 + K * CW * 16 + 128;
+}
+
+__device__ __forceinline__ WarpBufs warp_bufs(unsigned char* p, int J, int K, int CW) {
+    WarpBufs b;
+    b.list = reinterpret_cast<int*>(p);     p += 128;
+    b.pose = reinterpret_cast<float*>(p);   p += CW * J * 48;
+    b.cctr = reinterpret_cast<float4*>(p);  p += K * CW * 16;
+    b.q = reinterpret_cast<float*>(p);
+    return b;
+}
+
+// Primitives [i0, i0 + 32) that may touch the ball, as a mask.
+__device__ __forceinline__ unsigned cull_mask(const Scene& sc, int Ns, int Nc, int Nb, int Nh, int i0, const CullBall& b) {
+    const int e0 = Ns, e1 = Ns + Nc, e2 = e1 + Nb, e3 = e2 + Nh, i1 = min(e3, i0 + 32);
+    unsigned bits = 0u;
+    int i = i0;
+#pragma unroll 4
+    for (; i < min(e0, i1); ++i) bits |= (unsigned)cull_sphere(sc, i, b) << (i - i0);
+#pragma unroll 1
+    for (; i < min(e1, i1); ++i) bits |= (unsigned)cull_capsule(sc, i - e0, b) << (i - i0);
+#pragma unroll 2
+    for (; i < min(e2, i1); ++i) bits |= (unsigned)cull_box(sc, i - e1, b) << (i - i0);
+#pragma unroll 1
+    for (; i < i1; ++i) bits |= (unsigned)cull_halfspace(sc, i - e2, b) << (i - i0);
+    return bits;
+}
+
+// nw configurations (B.q); returns the mask of those in collision.  The scene
+// must have BlobHeader::cull set.
+__device__ __forceinline__ unsigned warp_check(const Scene& sc, const WarpBufs& B, int nw, int CW) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const BlobHeader& h = *sc.h;
+    const int lane = threadIdx.x & 31, l8 = lane & 7, sub = lane >> 3;
+    const unsigned mask = 0xffu << (lane & 24);
+    const int J = h.J, S = h.S, K = h.K;
+    const int Ns = h.Ns, Nc = h.Nc, Nb = h.Nb, Nh = h.Nh, n_obs = Ns + Nc + Nb + Nh;
+    const bool gated = h.gated != 0;
+    const float inflate = __int_as_float(h.inflate_bits);
+    fk_segments(sc, B.q, B.pose, nullptr, nw, J, lane, 32, [&](int w, int j, int SEG) {
+        for (int k = j; k < K; k += SEG) {
+            B.cctr[k * CW + w] = link_centre(sc, B.pose, J, w, k, inflate, gated);
+        }
+    });
+    __syncwarp();
+    unsigned alive = nw >= 32 ? kAll : (1u << nw) - 1u;  // the same in every lane
+    // self items, an (item, configuration) per lane
+    if (h.n_items > 0) {
+        const int n = nw;
+        CullBufs cb;
+        cb.pose = B.pose;
+        cb.cctr = B.cctr;
+        unsigned flops = 0;
+        for (int it0 = 0; it0 < n * h.n_items; it0 += 32) {
+            const int it = it0 + lane, ii = it / n;
+            bool touch = false;
+            int w = 0;
+            if (it < n * h.n_items) {
+                w = it - ii * n;
+                touch = (alive >> w & 1u) && cull_self_touch(sc, cb, CW, sc.item[ii], w, inflate);
+            }
+            for (unsigned todo = __ballot_sync(kAll, touch); todo;) {
+                unsigned t = todo;
+                int src = -1;
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    if (g == sub && t) src = __ffs(t) - 1;
+                    t &= t - 1u;
+                }
+                todo = t;
+                const int from = max(src, 0);
+                const int ew = __shfl_sync(kAll, w, from), ei = __shfl_sync(kAll, ii, from);
+                bool hit = false;
+                if (src >= 0 && (alive >> ew & 1u)) hit = cull_self_item(sc, cb, CW, ei, ew, l8, mask, inflate, flops);
+                alive &= ~__reduce_or_sync(kAll, hit ? 1u << ew : 0u);
+            }
+        }
+    }
+    uint32_t* marks = reinterpret_cast<uint32_t*>(B.q);  // [8][32] masks of a gated round
+    int k1 = K;  // links [0, k1) are left
+    while (k1 > 0 && alive) {
+        const int n = __popc(alive), per = min(k1, 32 / n);  // `per` links of n configurations at once
+        if (alive >> lane & 1u) B.list[__popc(alive & ((1u << lane) - 1u))] = lane;
+        __syncwarp();
+        const int kk = lane / n;
+        const bool act = kk < per;
+        const int k = act ? k1 - 1 - kk : 0, w = act ? B.list[lane - kk * n] : 0;
+        k1 -= per;
+        __syncwarp();
+        const float4 c = B.cctr[k * CW + w];
+        const CullBall ball = cull_ball(c, link_radius(sc, k, inflate, gated, c));
+        // Tests the links marked in `bits` (primitives i0 + bit) of the lanes.
+        auto fine = [&](unsigned bits, int i0) {
+            for (unsigned todo = __ballot_sync(kAll, bits != 0u && (alive >> w & 1u)); todo;) {
+                // the next four marked lanes, one per group of 8
+                unsigned t = todo;
+                int src = -1;
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    if (g == sub && t) src = __ffs(t) - 1;
+                    t &= t - 1u;
+                }
+                todo = t;
+                const int from = max(src, 0);
+                const int ew = __shfl_sync(kAll, w, from), ek = __shfl_sync(kAll, k, from);
+                unsigned rest = __shfl_sync(kAll, bits, from);
+                bool hit = false;
+                if (src >= 0 && (alive >> ew & 1u)) {
+                    const float4 gr = sc.grp[2 * ek + 1];
+                    const int s1 = __float_as_int(gr.z);
+                    for (int s0 = __float_as_int(gr.y); s0 < s1; s0 += 8) {
+                        const float4 f = s0 + l8 < s1 ? fine_centre(sc, B.pose, J, ew, s0 + l8, inflate) : absent_sphere();
+                        for (unsigned m = rest; m; m &= m - 1u) {
+                            hit = prim_hits(sc, h, i0 + __ffs(m) - 1, f);
+                            hit = __any_sync(mask, hit);
+                            if (hit) break;
+                        }
+                        if (hit) break;
+                    }
+                }
+                alive &= ~__reduce_or_sync(kAll, hit ? 1u << ew : 0u);
+            }
+        };
+        if (!gated) {
+            for (int i0 = 0; i0 < n_obs; i0 += 32) {
+                const unsigned bits = act && (alive >> w & 1u) ? cull_mask(sc, Ns, Nc, Nb, Nh, i0, ball) : 0u;
+                fine(bits, i0);
+            }
+        } else {
+            // the gate first: does the coarse sphere touch any primitive?
+            bool dirty = false;
+            for (int i0 = 0; i0 < n_obs; i0 += 32) {
+                const unsigned bits = act ? cull_mask(sc, Ns, Nc, Nb, Nh, i0, ball) : 0u;
+                for (unsigned m = bits; m && !dirty; m &= m - 1u) dirty = prim_hits(sc, h, i0 + __ffs(m) - 1, c);
+                if (i0 < 256) marks[(i0 >> 5) * 32 + lane] = bits;
+            }
+            if (__any_sync(kAll, dirty)) {
+                for (int i0 = 0; i0 < n_obs; i0 += 32) {
+                    unsigned bits = 0u;
+                    if (dirty && (alive >> w & 1u))
+                        bits = i0 < 256 ? marks[(i0 >> 5) * 32 + lane] : cull_mask(sc, Ns, Nc, Nb, Nh, i0, ball);
+                    fine(bits, i0);
+                }
+            }
+        }
+    }
+    // the point cloud: a (sphere, configuration) per lane
+    if (sc.pc.n > 0 && alive) {
+        const int m = __popc(alive);
+        __syncwarp();
+        if (alive >> lane & 1u) B.list[__popc(alive & ((1u << lane) - 1u))] = lane;
+        __syncwarp();
+        unsigned flops = 0;
+        for (int it0 = 0; it0 < m * S && alive; it0 += 32) {
+            const int it = min(it0 + lane, m * S - 1), s = it / m, w = B.list[it - s * m];
+            const float4 c = fine_centre(sc, B.pose, J, w, s, inflate);
+            alive &= ~cloud_batch(sc.pc, c, it0 + lane < m * S, w, alive, flops);
+        }
+    }
+    return (nw >= 32 ? kAll : (1u << nw) - 1u) & ~alive;
 }
 
 }  // namespace prrtc

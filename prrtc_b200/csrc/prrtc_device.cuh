@@ -66,7 +66,8 @@ struct BlobHeader {
     int32_t o_sch, o_ws, o_wc, o_wb;
     int32_t o_wh, o_item, o_cpair, used_bytes;
     int32_t P, cap_bytes, error;
-    int32_t cull;  // the groups cover every sphere on their own frames: prrtc_cull.cuh applies
+    int32_t cull;  // the groups cover every sphere on their own frames, box axes are orthonormal,
+                   // normals not longer than 1: prrtc_cull.cuh applies
 };
 static_assert(sizeof(BlobHeader) == 128, "header must stay 128 bytes");
 // Bits of BlobHeader::error: the pack kernel's self-pair item list overflowed
@@ -131,7 +132,7 @@ struct Scene {  // typed view of a blob (shared or global memory)
     const int4* sch;
     const float4* ws;    // [Ns][2]: (-2x,-2y,-2z,-2r), (x,y,z, x^2+y^2+z^2-r^2)
     const float4* wc;    // [Nc][3]: (p1, r), (d/|d|^2, -p1.d/|d|^2), (d, 0)   with d = p2 - p1
-    const float4* wb;    // [Nb][4]: (a1, -a1.c), (a2, -a2.c), (a3, -a3.c), (h1, h2, h3, axes not orthonormal)
+    const float4* wb;    // [Nb][4]: (a1, -a1.c), (a2, -a2.c), (a3, -a3.c), (h1, h2, h3, 0)
     const float4* wh;    // [Nh]:    (n, -n.p)
     const int4* item;
     const int2* cpair;

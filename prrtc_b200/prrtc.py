@@ -806,14 +806,16 @@ def _plan_per_problem(lib, bi, res, attrs, tun, contexts, robot_ctx, starts, goa
     main = torch.cuda.current_stream()
     streams = [torch.cuda.Stream(device=dev) for _ in range(min(n_streams, B))]
     ev = torch.cuda.Event()
-    ev.record(main)
     gcs = None if goal_counts is None else np.asarray(goal_counts).reshape(B)
     keep = []
     for i in range(B):
         s = streams[i % len(streams)]
-        s.wait_event(ev)
         ctx = DeviceContext(contexts[i], dev) if contexts[i] is not None else DeviceContext(None, dev)
         keep.append(ctx)
+        # the tables' copies are queued on the caller's stream (a pageable copy may
+        # still be in flight when the call returns)
+        ev.record(main)
+        s.wait_event(ev)
         inp = _lib.Inputs()
         inp.start_config = starts[i].data_ptr()
         ng = G if gcs is None else max(1, min(int(gcs[i]), G))

@@ -159,3 +159,55 @@ def test_culled_plans_across_joint_counts(cuda, n_joints):
         assert (x.solved, x.tree_a_size, x.tree_b_size, x.iterations) == (y.solved, y.tree_a_size, y.tree_b_size,
                                                                           y.iterations)
         assert np.array_equal(x.tree_a_configs.cpu().numpy().view(np.uint32), y.tree_a_configs.cpu().numpy().view(np.uint32))
+
+
+@pytest.mark.parametrize("checker", ["binary", "binary_coarse_coop"])
+@pytest.mark.parametrize("cell,r_env", [(0.1, 0.01), (0.1, 0.0), (0.02, 0.005), (0.013, 0.02), (1.0, 0.05)])
+def test_cloud_batches_equal_general_checker(cuda, cell, r_env, checker):
+    """Point clouds: cells from smaller than the spheres (a box of more than 512 cells is a hit) to larger than the
+    cloud, points on the far side of the coordinate limit, edge counts around a warp; and plans with a cloud."""
+    from prrtc_b200 import PointCloud, PointCloudChecker, prrtc_plan_batch
+
+    robot = scenes.arm(0)
+    world, pts = scenes.pointcloud_world(np.random.default_rng(1), 3000)
+    pts = np.concatenate([pts, np.array([[2e4, 0, 0], [0, 0, np.inf], [np.nan, 0, 0]], np.float32)])
+    ctx = build_collision_context(robot, world)
+    if checker != "binary":
+        # no self pair or world in the gate's way: what is left to compare is the cloud
+        ctx.update({k: v[:0] for k, v in ctx.items() if k.startswith("world_")})
+        for k in ("self_pairs", "coarse_self_pairs", "self_pair_ranges"):
+            ctx[k] = ctx[k][:0]
+    bare = {k: v for k, v in ctx.items() if k not in COARSE}
+    cloud = PointCloud(pts, r_env, cell)
+    rng = np.random.default_rng(2)
+    a = PointCloudChecker(ctx, robot.dim, checker)
+    b = PointCloudChecker(bare, robot.dim, "binary")
+    for n, g in ((1, 1), (31, 1), (33, 2), (700, 3)):
+        e = rng.uniform(robot.lower, robot.upper, (n, g, robot.dim)).astype(np.float32)
+        e[0, 0, 3] = np.nan
+        x = a.check_edges_collision_free(e, None, cloud, r_env).cpu().numpy()
+        assert np.array_equal(x, b.check_edges_collision_free(e, None, cloud, r_env).cpu().numpy()), (n, g)
+    q = rng.uniform(-1.0, 1.0, (2, 3, robot.dim)).astype(np.float32)
+    kw = dict(max_iterations=40, num_new_samples=1, max_nodes=512, min_vals=robot.lower, max_vals=robot.upper,
+              tail_explorers=False, point_cloud=cloud)
+    for x, y in zip(prrtc_plan_batch(q[0], q[1][:, None], collision_context=ctx, collision_checker=checker, **kw),
+                    prrtc_plan_batch(q[0], q[1][:, None], collision_context=bare, **kw)):
+        assert (x.solved, x.tree_a_size, x.tree_b_size, x.iterations) == (y.solved, y.tree_a_size, y.tree_b_size,
+                                                                          y.iterations)
+        assert np.array_equal(x.tree_a_configs.cpu().numpy().view(np.uint32), y.tree_a_configs.cpu().numpy().view(np.uint32))
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2, 3])
+@pytest.mark.parametrize("form", FORMS)
+def test_culled_verdicts_equal_full_sweep(cuda, form, mode):
+    """The default path against the full sweep, over scenes at the edge of what is culled, counts around a warp's
+    share and a configuration that is not a number."""
+    from prrtc_b200.collision import CollisionChecker
+
+    robot, ctx = _odd_scene(form, np.random.default_rng(21))
+    chk = CollisionChecker(ctx, robot.dim, CHECKERS[mode], 0.02, device=cuda)
+    rng = np.random.default_rng(22)
+    for n in (1, 5, 127, 3001):
+        q = rng.uniform(robot.lower, robot.upper, (n, robot.dim)).astype(np.float32)
+        q[n // 2, 2] = (np.nan, np.inf, 1e30, 0.1)[n % 4]
+        assert np.array_equal(chk.check(q).cpu().numpy(), chk.check(q, full_sweep=True).cpu().numpy()), n
