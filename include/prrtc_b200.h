@@ -383,6 +383,14 @@ int prrtc_b200_smooth_cost_grad(const prrtc_robot_t* robot, const prrtc_world_t*
                                 float margin, float beta, float w_len, float* cost, float* grad,
                                 void* workspace, size_t workspace_bytes, void* stream);
 
+/* The same with every sum of the gradient taken in a fixed order (the same bits
+ * in every run), as prrtc_b200_smooth_cost_grad_batch does: for descents, which
+ * follow the rounding of their gradient across the kinks of box distances. */
+int prrtc_b200_smooth_cost_grad_ordered(const prrtc_robot_t* robot, const prrtc_world_t* world, int32_t dim,
+                                        const float* waypoints, int32_t n_paths, int32_t n_waypoints,
+                                        float margin, float beta, float w_len, float* cost, float* grad,
+                                        void* workspace, size_t workspace_bytes, void* stream);
+
 /* The same cost and gradient for the paths of a batch, path p [W,dim] of
  * waypoints [batch,W,dim] against problem p's own world and self pairs, as
  * prrtc_b200_plan_batch reads them from `in` (robot, batch, the per-problem world
@@ -393,6 +401,19 @@ int prrtc_b200_smooth_cost_grad_batch(const prrtc_batch_inputs_t* in, int32_t di
                                       int32_t n_waypoints, float margin, float beta, float w_len,
                                       float* cost, float* grad, void* workspace, size_t workspace_bytes,
                                       void* stream);
+
+/* The two halves of a descent step on a batch of paths.  step_grad_batch: the
+ * gradient alone (as cost_grad_batch's, zero at each path's first and last
+ * waypoint); packed != 0 when the workspace still holds this batch's scenes from
+ * an earlier call with the same inputs.  update: waypoints [n_paths,
+ * n_waypoints, dim] -= lr grad / max(norms[path], 1e-12), held between the joint
+ * limits lower / upper [dim]. */
+int prrtc_b200_smooth_step_grad_batch(const prrtc_batch_inputs_t* in, int32_t dim, const float* waypoints,
+                                      int32_t n_waypoints, float margin, float beta, float w_len, int32_t packed,
+                                      float* grad, void* workspace, size_t workspace_bytes, void* stream);
+int prrtc_b200_smooth_update(float* waypoints, const float* grad, const float* norms, const float* lower,
+                             const float* upper, float lr, int32_t n_paths, int32_t n_waypoints, int32_t dim,
+                             void* stream);
 
 /* Diagnostic: FP32 FFMA throughput probe (blocks x threads, iters x 8 independent
  * FFMA chains per thread); sink receives one value per block so the work is live.

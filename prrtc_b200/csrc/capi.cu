@@ -530,10 +530,10 @@ size_t prrtc_b200_smooth_workspace_size(const prrtc_robot_t* robot, const prrtc_
     return blob_stride(make_pack(*robot, *world, 1, 0, 0.0f));
 }
 
-int prrtc_b200_smooth_cost_grad(const prrtc_robot_t* robot, const prrtc_world_t* world, int32_t dim,
+static int smooth_cost_grad(const prrtc_robot_t* robot, const prrtc_world_t* world, int32_t dim,
                                 const float* waypoints, int32_t n_paths, int32_t n_waypoints, float margin,
                                 float beta, float w_len, float* cost, float* grad, void* ws, size_t ws_bytes,
-                                void* stream) {
+                                void* stream, bool ordered) {
     if (n_paths == 0) return PRRTC_B200_OK;
     if (!robot || !world || !waypoints || !cost || n_paths < 0 || n_waypoints < 1 || !(beta > 0.0f))
         return PRRTC_B200_EARG;
@@ -549,9 +549,25 @@ int prrtc_b200_smooth_cost_grad(const prrtc_robot_t* robot, const prrtc_world_t*
     unsigned char* blob = static_cast<unsigned char*>(ws);
     cudaError_t e = launch_pack(s, 1, blob, stride, st);
     if (e != cudaSuccess) return cuda_fail(e);
-    e = launch_smooth(blob, 0, world->self_pairs, 0, s.J, s.S, dim, waypoints, n_paths, n_waypoints, margin, beta,
-                      w_len, cost, grad, st);
+    e = launch_smooth(blob, 0, (int)stride, world->self_pairs, 0, s.J, s.S, dim, waypoints, n_paths, n_waypoints, margin, beta,
+                      w_len, cost, grad, ordered, st);
     return e == cudaSuccess ? PRRTC_B200_OK : cuda_fail(e);
+}
+
+int prrtc_b200_smooth_cost_grad(const prrtc_robot_t* robot, const prrtc_world_t* world, int32_t dim,
+                                const float* waypoints, int32_t n_paths, int32_t n_waypoints, float margin,
+                                float beta, float w_len, float* cost, float* grad, void* ws, size_t ws_bytes,
+                                void* stream) {
+    return smooth_cost_grad(robot, world, dim, waypoints, n_paths, n_waypoints, margin, beta, w_len, cost, grad, ws,
+                            ws_bytes, stream, false);
+}
+
+int prrtc_b200_smooth_cost_grad_ordered(const prrtc_robot_t* robot, const prrtc_world_t* world, int32_t dim,
+                                        const float* waypoints, int32_t n_paths, int32_t n_waypoints, float margin,
+                                        float beta, float w_len, float* cost, float* grad, void* ws, size_t ws_bytes,
+                                        void* stream) {
+    return smooth_cost_grad(robot, world, dim, waypoints, n_paths, n_waypoints, margin, beta, w_len, cost, grad, ws,
+                            ws_bytes, stream, true);
 }
 
 size_t prrtc_b200_smooth_batch_workspace_size(const prrtc_batch_inputs_t* in) {
@@ -559,12 +575,12 @@ size_t prrtc_b200_smooth_batch_workspace_size(const prrtc_batch_inputs_t* in) {
     return (size_t)in->batch * blob_stride(make_batch_pack(in, 1, 0, 0.0f));
 }
 
-int prrtc_b200_smooth_cost_grad_batch(const prrtc_batch_inputs_t* in, int32_t dim, const float* waypoints,
-                                      int32_t n_waypoints, float margin, float beta, float w_len, float* cost,
-                                      float* grad, void* ws, size_t ws_bytes, void* stream) {
+static int smooth_batch(const prrtc_batch_inputs_t* in, int32_t dim, const float* waypoints,
+                        int32_t n_waypoints, float margin, float beta, float w_len, float* cost,
+                        float* grad, bool packed, void* ws, size_t ws_bytes, void* stream) {
     if (!in) return PRRTC_B200_EARG;
     if (in->batch == 0) return PRRTC_B200_OK;
-    if (in->batch < 0 || !waypoints || !cost || n_waypoints < 1 || !(beta > 0.0f)) return PRRTC_B200_EARG;
+    if (in->batch < 0 || !waypoints || (!cost && !grad) || n_waypoints < 1 || !(beta > 0.0f)) return PRRTC_B200_EARG;
     if (dim < 1 || dim > PRRTC_B200_DIM_MAX) return PRRTC_B200_EUNSUPPORTED;
     if (in->robot.n_joints < 1 || in->robot.n_joints > PRRTC_B200_MAX_JOINTS) return PRRTC_B200_EUNSUPPORTED;
     int rc = check_robot(in->robot);
@@ -574,11 +590,38 @@ int prrtc_b200_smooth_cost_grad_batch(const prrtc_batch_inputs_t* in, int32_t di
     if (!ws || !aligned(ws, 256) || ws_bytes < (size_t)in->batch * stride) return PRRTC_B200_EWORKSPACE;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     unsigned char* blobs = static_cast<unsigned char*>(ws);
-    cudaError_t e = launch_pack(s, in->batch, blobs, stride, st);
+    cudaError_t e = packed ? cudaSuccess : launch_pack(s, in->batch, blobs, stride, st);
     if (e != cudaSuccess) return cuda_fail(e);
     const size_t pstride = in->self_pairs_count ? (size_t)std::max(0, in->max_self_pairs) : 0;
-    e = launch_smooth(blobs, stride, in->self_pairs, pstride, s.J, s.S, dim, waypoints, in->batch, n_waypoints,
-                      margin, beta, w_len, cost, grad, st);
+    e = launch_smooth(blobs, stride, (int)stride, in->self_pairs, pstride, s.J, s.S, dim, waypoints, in->batch, n_waypoints,
+                      margin, beta, w_len, cost, grad, true, st);
+    return e == cudaSuccess ? PRRTC_B200_OK : cuda_fail(e);
+}
+
+int prrtc_b200_smooth_cost_grad_batch(const prrtc_batch_inputs_t* in, int32_t dim, const float* waypoints,
+                                      int32_t n_waypoints, float margin, float beta, float w_len, float* cost,
+                                      float* grad, void* ws, size_t ws_bytes, void* stream) {
+    if (in && in->batch != 0 && !cost) return PRRTC_B200_EARG;
+    return smooth_batch(in, dim, waypoints, n_waypoints, margin, beta, w_len, cost, grad, false, ws, ws_bytes, stream);
+}
+
+int prrtc_b200_smooth_step_grad_batch(const prrtc_batch_inputs_t* in, int32_t dim, const float* waypoints,
+                                      int32_t n_waypoints, float margin, float beta, float w_len, int32_t packed,
+                                      float* grad, void* ws, size_t ws_bytes, void* stream) {
+    if (in && in->batch != 0 && !grad) return PRRTC_B200_EARG;
+    return smooth_batch(in, dim, waypoints, n_waypoints, margin, beta, w_len, nullptr, grad, packed != 0, ws, ws_bytes,
+                        stream);
+}
+
+int prrtc_b200_smooth_update(float* waypoints, const float* grad, const float* norms, const float* lower,
+                             const float* upper, float lr, int32_t n_paths, int32_t n_waypoints, int32_t dim,
+                             void* stream) {
+    if (n_paths == 0) return PRRTC_B200_OK;
+    if (!waypoints || !grad || !norms || !lower || !upper || n_paths < 0 || n_waypoints < 1) return PRRTC_B200_EARG;
+    if (dim < 1 || dim > PRRTC_B200_DIM_MAX) return PRRTC_B200_EUNSUPPORTED;
+    if ((long long)n_waypoints * dim > INT32_MAX) return PRRTC_B200_EUNSUPPORTED;
+    cudaError_t e = launch_smooth_update(waypoints, grad, norms, lower, upper, lr, n_paths, n_waypoints, dim,
+                                         static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? PRRTC_B200_OK : cuda_fail(e);
 }
 

@@ -147,11 +147,17 @@ cudaError_t launch_radius_update(float* radii, const int32_t* idx, const int32_t
                                  float rmin, int sequential, int32_t* err, cudaStream_t st);
 
 // smooth.cu
-// Path p uses the scene at blob + p * blob_stride and the self pairs at
+// blob_cap: capacity of one scene; ordered: every sum in a fixed order (the same
+// bits in every run), as it always is with a scene per path; cost null: the
+// gradient alone, zero at the paths' end points.  Path p uses the scene at blob + p * blob_stride and the self pairs at
 // pairs + 2 * p * pairs_stride (strides 0: one scene for every path).
-cudaError_t launch_smooth(const unsigned char* blob, size_t blob_stride, const int32_t* pairs, size_t pairs_stride,
+cudaError_t launch_smooth(const unsigned char* blob, size_t blob_stride, int blob_cap, const int32_t* pairs,
+                          size_t pairs_stride,
                           int J, int S, int dim, const float* wp, int P, int W, float margin, float beta, float w_len,
-                          float* cost, float* grad, cudaStream_t st);
+                          float* cost, float* grad, bool ordered, cudaStream_t st);
+
+cudaError_t launch_smooth_update(float* x, const float* g, const float* norms, const float* lo, const float* hi,
+                                 float lr, int P, int W, int dim, cudaStream_t st);
 
 cudaError_t launch_fp32_probe(int blocks, int threads, int iters, float* sink, cudaStream_t st);
 cudaError_t launch_fp32x2_probe(int blocks, int threads, int iters, float* sink, cudaStream_t st);

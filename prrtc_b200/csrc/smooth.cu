@@ -18,7 +18,10 @@
 //   5. dC/dq_a = sum over joints driven by a of dv_j/dq_a * dC/dv_j (1 for an
 //      actuated joint, mimic_mul for a mimic joint) plus the length term.
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <math.h>
+
+#include <algorithm>
 
 #include "kernels.h"
 #include "prrtc_device.cuh"
@@ -70,11 +73,12 @@ __host__ __device__ inline int smooth_warp_floats(int J, int S) {
 
 // Accumulate the cost term of a pair at distance d.  sig = sigmoid(beta
 // (margin - d)) is the factor of -dd/dc in the gradient (0 for a skipped pair).
+template <bool COST>
 __device__ __forceinline__ void pair_term(float d, float margin, float beta, float inv_beta, float& cost,
                                           float& sig) {
     const float z = beta * (margin - d);
     const float e = __expf(-fabsf(z));
-    cost = fmaf(fmaxf(z, 0.0f) + log1p_unit(e), inv_beta, cost);
+    if constexpr (COST) cost = fmaf(fmaxf(z, 0.0f) + log1p_unit(e), inv_beta, cost);
     const float r = __fdividef(1.0f, 1.0f + e);
     sig = z >= kTailZ ? (z >= 0.0f ? r : e * r) : 0.0f;
 }
@@ -85,18 +89,94 @@ __device__ __forceinline__ void norm_rnorm(float d2, float& n, float& rn) {
     n = d2 * rn;
 }
 
-template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) smooth_kernel(SmoothArgs a) {
-    extern __shared__ __align__(16) float smf[];
+// v added to the floats at base[0 .. N) of each lane that is `on`; lanes of one
+// key share their base and add one after the other in lane order, so the sums
+// are the same bits in every run (shared-memory float atomics add in that order
+// too, but by compare-and-swap rounds that cost several times as much).
+template <int N>
+__device__ __forceinline__ void add_in_lane_order(bool on, int key, float* base, const float (&v)[N]) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    unsigned rest = __match_any_sync(kAll, on ? key : -1 - lane);
+    const bool leads = on && __ffs(rest) - 1 == lane;
+    if (!on) rest = 0u;
+    float sum[N];
+    if (leads) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) sum[i] = base[i];
+    }
+    while (__any_sync(kAll, leads && rest != 0u)) {
+        const int src = rest ? __ffs(rest) - 1 : lane;
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const float x = __shfl_sync(kAll, v[i], src);
+            if (leads && rest) sum[i] += x;
+        }
+        rest &= rest - 1u;
+    }
+    if (leads) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) base[i] = sum[i];
+    }
+    __syncwarp();
+}
+
+// A warp per waypoint, WARPS waypoints of one path per CTA, the scene staged in
+// shared memory (STAGED) or read from global memory.  Every sum is taken in a
+// fixed order, so a gradient is the same bits in every run and launch: a
+// descent of normalised steps crosses the kinks of box distances, where sums in
+// another order move single paths by 1e-3 within 50 steps.
+//
+// Bound by the latency of its dependent chains (a waypoint's 4,376 pairs in one
+// warp).  32 paths x 64 waypoints in tabletop worlds of their own: 119 -> 76 us
+// for the gradient alone, from ordered warp sums in the place of shared-memory
+// atomics, three lanes in the place of one for the frames' chain, and the scene
+// in shared memory; the bits are those of the atomics.
+// COST false: the gradient alone, zero at a path's end points (a descent step).
+template <int WARPS, bool STAGED, bool COST>
+__global__ void __launch_bounds__(WARPS * 32) smooth_kernel(SmoothArgs a, int blob_cap, int per_path) {
+    extern __shared__ __align__(128) unsigned char dsm[];
+    __shared__ __align__(8) uint64_t mbar;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int c = blockIdx.x * WARPS + warp;
-    if (c >= a.P * a.W) return;
-    const int p = c / a.W, w = c - p * a.W;
-    const Scene sc = scene_view(a.blob + (size_t)p * a.blob_stride);
+    // per_path CTAs for each path, or (one scene for all, per_path 0) all paths'
+    // waypoints one after the other
+    int p, w;
+    bool mine;
+    if (per_path > 0) {
+        p = blockIdx.x / per_path;
+        w = (blockIdx.x - p * per_path) * WARPS + warp;
+        mine = w < a.W;
+    } else {
+        const int c = blockIdx.x * WARPS + warp;
+        p = c / a.W;
+        w = c - p * a.W;
+        mine = c < a.P * a.W;
+    }
+    const unsigned char* gblob = a.blob + (size_t)p * a.blob_stride;  // stride 0 where a CTA spans paths
+    if constexpr (STAGED) {
+        const int bytes = min(reinterpret_cast<const BlobHeader*>(gblob)->used_bytes, blob_cap);
+        if (threadIdx.x == 0) mbar_init(&mbar);
+        __syncthreads();
+        uint32_t phase = 0;
+        if (!stage_blob(dsm, gblob, bytes, &mbar, phase, nullptr, 0, kWaitLimit)) {
+            // the bulk copy did not arrive in time: copy the scene with plain loads
+            for (int i = threadIdx.x; i < bytes / 16; i += WARPS * 32)
+                reinterpret_cast<uint4*>(dsm)[i] = reinterpret_cast<const uint4*>(gblob)[i];
+            __syncthreads();
+        }
+    }
+    if (!mine) return;
+    if constexpr (!COST) {
+        if (w == 0 || w == a.W - 1) {
+            if (lane < a.dim) a.grad[((size_t)p * a.W + w) * a.dim + lane] = 0.0f;
+            return;
+        }
+    }
+    const Scene sc = scene_view(STAGED ? dsm : gblob);
     const int2* pairs = a.pairs + (size_t)p * a.pairs_stride;
     const BlobHeader& h = *sc.h;
     const int J = a.J, S = a.S, dim = a.dim;
-    float* base = smf + (size_t)warp * smooth_warp_floats(J, S);
+    float* base = reinterpret_cast<float*>(dsm + (STAGED ? blob_cap : 0)) + (size_t)warp * smooth_warp_floats(J, S);
     float* pose = base;
     float4* ctr = reinterpret_cast<float4*>(pose + J * 12);
     float4* g = ctr + S;
@@ -112,13 +192,29 @@ __global__ void __launch_bounds__(WARPS * 32) smooth_kernel(SmoothArgs a) {
         joint_local(jr, joint_value(jr, q), &pose[j * 12]);
     }
     __syncwarp();
-    if (lane == 0) {
-        for (int j = 0; j < J; ++j) {
-            const int pj = sc.joints[j].idx.x;
-            if (pj >= 0 && pj < j) compose(&pose[pj * 12], &pose[j * 12], &pose[j * 12]);
+    // the chain in joint order: row r of a frame needs row r of its parent's, so
+    // three lanes take a row each (the operations of `compose`)
+    for (int j = 0; j < J; ++j) {
+        const int pj = sc.joints[j].idx.x;
+        if (pj < 0 || pj >= j) continue;
+        float o[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (lane < 3) {
+            const float* A = &pose[pj * 12];
+            const float* L = &pose[j * 12];
+            const float x = A[3 * lane], y = A[3 * lane + 1], z = A[3 * lane + 2];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) o[c] = fmaf(x, L[c], fmaf(y, L[3 + c], z * L[6 + c]));
+            o[3] = fmaf(x, L[9], fmaf(y, L[10], fmaf(z, L[11], A[9 + lane])));
         }
+        __syncwarp();
+        if (lane < 3) {
+            float* T = &pose[j * 12];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) T[3 * lane + c] = o[c];
+            T[9 + lane] = o[3];
+        }
+        __syncwarp();
     }
-    __syncwarp();
     for (int s = lane; s < S; s += 32) {
         const int f = sc.sfr[s];
         const float4 l = sc.sph[s];
@@ -141,7 +237,7 @@ __global__ void __launch_bounds__(WARPS * 32) smooth_kernel(SmoothArgs a) {
             const float dx = cs.x - ob.x, dy = cs.y - ob.y, dz = cs.z - ob.z;
             float n, rn, sig;
             norm_rnorm(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), n, rn);
-            pair_term(n - r - ob.w, a.margin, a.beta, inv_beta, cost, sig);
+            pair_term<COST>(n - r - ob.w, a.margin, a.beta, inv_beta, cost, sig);
             const float k = -sig * rn;
             gx = fmaf(k, dx, gx); gy = fmaf(k, dy, gy); gz = fmaf(k, dz, gz);
         }
@@ -152,7 +248,7 @@ __global__ void __launch_bounds__(WARPS * 32) smooth_kernel(SmoothArgs a) {
             const float ex = fmaf(-t, dl.x, wx), ey = fmaf(-t, dl.y, wy), ez = fmaf(-t, dl.z, wz);
             float n, rn, sig;
             norm_rnorm(fmaf(ex, ex, fmaf(ey, ey, ez * ez)), n, rn);
-            pair_term(n - r - p1.w, a.margin, a.beta, inv_beta, cost, sig);
+            pair_term<COST>(n - r - p1.w, a.margin, a.beta, inv_beta, cost, sig);
             const float k = -sig * rn;
             gx = fmaf(k, ex, gx); gy = fmaf(k, ey, gy); gz = fmaf(k, ez, gz);
         }
@@ -189,71 +285,73 @@ __global__ void __launch_bounds__(WARPS * 32) smooth_kernel(SmoothArgs a) {
             const float ddy = fmaf(c0, ax[0].y, fmaf(c1, ax[1].y, c2 * ax[2].y));
             const float ddz = fmaf(c0, ax[0].z, fmaf(c1, ax[1].z, c2 * ax[2].z));
             float sig;
-            pair_term(d, a.margin, a.beta, inv_beta, cost, sig);
+            pair_term<COST>(d, a.margin, a.beta, inv_beta, cost, sig);
             gx = fmaf(-sig, ddx, gx); gy = fmaf(-sig, ddy, gy); gz = fmaf(-sig, ddz, gz);
         }
         for (int o = 0; o < h.Nh; ++o) {
             const float4 hs = sc.wh[o];
             const float d = fmaf(hs.x, cs.x, fmaf(hs.y, cs.y, fmaf(hs.z, cs.z, hs.w))) - r;
             float sig;
-            pair_term(d, a.margin, a.beta, inv_beta, cost, sig);
+            pair_term<COST>(d, a.margin, a.beta, inv_beta, cost, sig);
             gx = fmaf(-sig, hs.x, gx); gy = fmaf(-sig, hs.y, gy); gz = fmaf(-sig, hs.z, gz);
         }
         g[s] = make_float4(gx, gy, gz, 0.0f);
     }
     __syncwarp();
-    // 2b. self pairs (explicit list): shared-memory atomics into both spheres
-    for (int k = lane; k < h.P; k += 32) {
-        const int2 pr = __ldg(&pairs[k]);
-        if (pr.x < 0 || pr.y < 0 || pr.x >= S || pr.y >= S) continue;
-        if (sc.sfr[pr.x] < 0 || sc.sfr[pr.y] < 0) continue;
-        const float4 ci = ctr[pr.x], cj = ctr[pr.y];
-        const float dx = ci.x - cj.x, dy = ci.y - cj.y, dz = ci.z - cj.z;
-        float n, rn, sig;
-        norm_rnorm(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), n, rn);
-        pair_term(n - ci.w - cj.w, a.margin, a.beta, inv_beta, cost, sig);
-        if (sig == 0.0f) continue;  // nothing to add
-        const float kk = -sig * rn;
-        atomicAdd(&g[pr.x].x, kk * dx); atomicAdd(&g[pr.x].y, kk * dy); atomicAdd(&g[pr.x].z, kk * dz);
-        atomicAdd(&g[pr.y].x, -kk * dx); atomicAdd(&g[pr.y].y, -kk * dy); atomicAdd(&g[pr.y].z, -kk * dz);
+    // 2b. self pairs (explicit list), 32 at a time, into both spheres
+    for (int k0 = 0; k0 < h.P; k0 += 32) {
+        const int k = k0 + lane;
+        bool on = k < h.P;
+        const int2 pr = on ? __ldg(&pairs[k]) : make_int2(-1, -1);
+        on = on && pr.x >= 0 && pr.y >= 0 && pr.x < S && pr.y < S && sc.sfr[pr.x] >= 0 && sc.sfr[pr.y] >= 0;
+        float v[3] = {0.0f, 0.0f, 0.0f};
+        if (on) {
+            const float4 ci = ctr[pr.x], cj = ctr[pr.y];
+            const float dx = ci.x - cj.x, dy = ci.y - cj.y, dz = ci.z - cj.z;
+            float n, rn, sig;
+            norm_rnorm(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), n, rn);
+            pair_term<COST>(n - ci.w - cj.w, a.margin, a.beta, inv_beta, cost, sig);
+            on = sig != 0.0f;  // else nothing to add
+            const float kk = -sig * rn;
+            v[0] = kk * dx; v[1] = kk * dy; v[2] = kk * dz;
+        }
+        if (!__any_sync(0xffffffffu, on)) continue;
+        add_in_lane_order<3>(on, pr.x, reinterpret_cast<float*>(&g[max(pr.x, 0)]), v);
+        const float m[3] = {-v[0], -v[1], -v[2]};
+        add_in_lane_order<3>(on, pr.y, reinterpret_cast<float*>(&g[max(pr.y, 0)]), m);
     }
     __syncwarp();
     // 3. frame sums
-    for (int s = lane; s < S; s += 32) {
-        const int f = sc.sfr[s];
-        if (f < 0) continue;
+    for (int s0 = 0; s0 < S; s0 += 32) {
+        const int s = min(s0 + lane, S - 1), f = sc.sfr[s];
         const float4 cs = ctr[s], gs = g[s];
-        float* A = &acc[f * 8];
-        atomicAdd(&A[0], gs.x); atomicAdd(&A[1], gs.y); atomicAdd(&A[2], gs.z);
-        atomicAdd(&A[3], cs.y * gs.z - cs.z * gs.y);
-        atomicAdd(&A[4], cs.z * gs.x - cs.x * gs.z);
-        atomicAdd(&A[5], cs.x * gs.y - cs.y * gs.x);
+        const float v[6] = {gs.x, gs.y, gs.z, cs.y * gs.z - cs.z * gs.y, cs.z * gs.x - cs.x * gs.z,
+                            cs.x * gs.y - cs.y * gs.x};
+        add_in_lane_order<6>(s0 + lane < S && f >= 0, f, &acc[max(f, 0) * 8], v);
+    }
+    // 4. reverse sweep: subtree sums a component per lane, then a joint per lane
+    if (lane < 6) {
+        for (int j = J - 1; j >= 0; --j) {
+            const int pj = sc.joints[j].idx.x;
+            if (pj >= 0 && pj < j) acc[pj * 8 + lane] += acc[j * 8 + lane];
+        }
     }
     __syncwarp();
-    // 4. reverse sweep
-    if (lane == 0) {
-        for (int j = J - 1; j >= 0; --j) {
-            const JointRec& jr = sc.joints[j];
-            const float* F = &pose[j * 12];
-            float* A = &acc[j * 8];
-            const float wx = fmaf(F[0], jr.tw.x, fmaf(F[1], jr.tw.y, F[2] * jr.tw.z));
-            const float wy = fmaf(F[3], jr.tw.x, fmaf(F[4], jr.tw.y, F[5] * jr.tw.z));
-            const float wz = fmaf(F[6], jr.tw.x, fmaf(F[7], jr.tw.y, F[8] * jr.tw.z));
-            const float vx = fmaf(F[0], jr.tv.x, fmaf(F[1], jr.tv.y, F[2] * jr.tv.z));
-            const float vy = fmaf(F[3], jr.tv.x, fmaf(F[4], jr.tv.y, F[5] * jr.tv.z));
-            const float vz = fmaf(F[6], jr.tv.x, fmaf(F[7], jr.tv.y, F[8] * jr.tv.z));
-            const float tx = F[9], ty = F[10], tz = F[11];
-            const float mx = A[3] - (ty * A[2] - tz * A[1]);
-            const float my = A[4] - (tz * A[0] - tx * A[2]);
-            const float mz = A[5] - (tx * A[1] - ty * A[0]);
-            dv[j] = wx * mx + wy * my + wz * mz + vx * A[0] + vy * A[1] + vz * A[2];
-            const int pj = jr.idx.x;
-            if (pj >= 0 && pj < j) {
-                float* B = &acc[pj * 8];
-#pragma unroll
-                for (int i = 0; i < 6; ++i) B[i] += A[i];
-            }
-        }
+    for (int j = lane; j < J; j += 32) {
+        const JointRec& jr = sc.joints[j];
+        const float* F = &pose[j * 12];
+        const float* A = &acc[j * 8];
+        const float wx = fmaf(F[0], jr.tw.x, fmaf(F[1], jr.tw.y, F[2] * jr.tw.z));
+        const float wy = fmaf(F[3], jr.tw.x, fmaf(F[4], jr.tw.y, F[5] * jr.tw.z));
+        const float wz = fmaf(F[6], jr.tw.x, fmaf(F[7], jr.tw.y, F[8] * jr.tw.z));
+        const float vx = fmaf(F[0], jr.tv.x, fmaf(F[1], jr.tv.y, F[2] * jr.tv.z));
+        const float vy = fmaf(F[3], jr.tv.x, fmaf(F[4], jr.tv.y, F[5] * jr.tv.z));
+        const float vz = fmaf(F[6], jr.tv.x, fmaf(F[7], jr.tv.y, F[8] * jr.tv.z));
+        const float tx = F[9], ty = F[10], tz = F[11];
+        const float mx = A[3] - (ty * A[2] - tz * A[1]);
+        const float my = A[4] - (tz * A[0] - tx * A[2]);
+        const float mz = A[5] - (tx * A[1] - ty * A[0]);
+        dv[j] = wx * mx + wy * my + wz * mz + vx * A[0] + vy * A[1] + vz * A[2];
     }
     __syncwarp();
     // 5. joint-space gradient + length term
@@ -280,29 +378,531 @@ __global__ void __launch_bounds__(WARPS * 32) smooth_kernel(SmoothArgs a) {
         }
         if (a.grad) a.grad[((size_t)p * a.W + w) * dim + lane] = gq;
     }
-    cost += lenc;
+    if constexpr (COST) {
+        cost += lenc;
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) cost += __shfl_xor_sync(0xffffffffu, cost, off);
-    if (lane == 0) atomicAdd(&a.cost[p], cost);
+        for (int off = 16; off > 0; off >>= 1) cost += __shfl_xor_sync(0xffffffffu, cost, off);
+        if (lane == 0) atomicAdd(&a.cost[p], cost);
+    }
 }
 
-cudaError_t launch_smooth(const unsigned char* blob, size_t blob_stride, const int32_t* pairs, size_t pairs_stride,
-                          int J, int S, int dim, const float* wp, int P, int W, float margin, float beta, float w_len,
-                          float* cost, float* grad, cudaStream_t st) {
-    if (P <= 0 || W <= 0) return cudaSuccess;
-    constexpr int WARPS = 4;
-    cudaError_t e = cudaMemsetAsync(cost, 0, (size_t)P * sizeof(float), st);
-    if (e != cudaSuccess) return e;
-    const size_t smem = (size_t)WARPS * smooth_warp_floats(J, S) * sizeof(float);
-    if (smem > 48 * 1024) {
-        if ((e = cudaFuncSetAttribute(smooth_kernel<WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem)) != cudaSuccess)
-            return e;
+// One step of the descent for every path: x - lr g / max(|g|, 1e-12), held
+// between the joint limits; norms [P] are the gradients' lengths.  The
+// operations and their order are those of the tensor expression (multiply,
+// divide, subtract, then the two bounds, NaN kept).
+__global__ void smooth_update_kernel(float* __restrict__ x, const float* __restrict__ g, const float* __restrict__ norms,
+                                     const float* __restrict__ lo, const float* __restrict__ hi, float lr, int per_path,
+                                     int dim, long long n) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float len = norms[i / per_path], gn = len != len ? len : fmaxf(len, 1e-12f);
+    float v = __fsub_rn(x[i], __fdiv_rn(__fmul_rn(lr, g[i]), gn));
+    const int d = (int)(i % dim);
+    v = v != v || lo[d] != lo[d] ? v + lo[d] : fmaxf(v, lo[d]);
+    v = v != v || hi[d] != hi[d] ? v + hi[d] : fminf(v, hi[d]);
+    x[i] = v;
+}
+
+cudaError_t launch_smooth_update(float* x, const float* g, const float* norms, const float* lo, const float* hi,
+                                 float lr, int P, int W, int dim, cudaStream_t st) {
+    const long long n = (long long)P * W * dim;
+    if (n <= 0) return cudaSuccess;
+    smooth_update_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(x, g, norms, lo, hi, lr, W * dim, dim, n);
+    return cudaGetLastError();
+}
+
+// ----------------------------------------------------------------------------- a warp's lanes are waypoints
+
+// The form for paths of one scene and robots of up to 32 joints, unless the
+// caller wants the sums in a fixed order: a CTA takes 32 waypoints, one per lane, and its warps take (two spheres x every primitive) and (32 self pairs)
+// units from a shared counter.  All lanes of a warp then look at the same
+// primitive, read from shared memory once for the warp, with neighbouring
+// waypoints' distances, which are alike, so the warp as a whole takes the short
+// series for pairs that are far apart (below) instead of the full softplus.
+//
+// Bound by instruction issue and, close behind, the special-function pipe (a
+// reciprocal square root and an exponential per pair, two reciprocals more near
+// contact): 67% of the issue slots, 58 instructions per pair and warp.  Against a
+// warp per waypoint with a sphere per lane (smooth_kernel), 4,376 pairs each:
+// 512 paths x 64 waypoints, tabletop scene, 858 -> 353 us; 40 dual-arm paths x 96
+// waypoints (44,360 pairs) 920 -> 385 us a call.  One sphere at a time instead of
+// two measured 379 us, the library's exponential and reciprocal square root 512 us.
+struct SmoothBufs {
+    float* pose;    // [32][J][12]
+    float* ctr;     // [S][3][32] (the radius is the scene's)
+    float* g;       // [S][3][32]; the joints' local transforms [32][J][12] before
+    float* acc;     // [J][6][32] frame sums G, M
+    float* q;       // [32][kDimMax], then dv [32][J]
+    float* cost;    // [32]
+    uint32_t* sub;  // [J] mask of the joint's subtree (itself included)
+    int* next;      // unit counter
+};
+
+__host__ __device__ inline int smooth_g_bytes(int J, int S) { return S * 384 > J * 1536 ? S * 384 : J * 1536; }
+__host__ __device__ inline int smooth_wide_bytes(int J, int S) {
+    return 32 * J * 48 + S * 3 * 128 + smooth_g_bytes(J, S) + J * 6 * 128 + 32 * (kDimMax > J ? kDimMax : J) * 4 + 128 + 128 + 16;
+}
+
+__device__ __forceinline__ SmoothBufs smooth_bufs(unsigned char* p, int J, int S) {
+    SmoothBufs b;
+    b.pose = reinterpret_cast<float*>(p);   p += 32 * J * 48;
+    b.ctr = reinterpret_cast<float*>(p);    p += S * 3 * 128;
+    b.g = reinterpret_cast<float*>(p);      p += smooth_g_bytes(J, S);
+    b.acc = reinterpret_cast<float*>(p);    p += J * 6 * 128;
+    b.q = reinterpret_cast<float*>(p);      p += 32 * max(kDimMax, J) * 4;
+    b.cost = reinterpret_cast<float*>(p);   p += 128;
+    b.sub = reinterpret_cast<uint32_t*>(p); p += 128;
+    b.next = reinterpret_cast<int*>(p);
+    return b;
+}
+
+// The hardware's exponential and reciprocal square root (2 ulp), without the
+// code for denormal operands: t is finite and d2 at least 1e-36.
+__device__ __forceinline__ float wide_ex2(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float wide_rsqrt(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// Pair terms, all 32 lanes together.  z = beta (margin - d): cost collects
+// softplus(z) in units of 1/beta, sig is the sigmoid, the factor of -dd/dc.
+// With e = exp(-|z|):
+//   some lane nearer than z = -5.6: as pair_term;
+//   all lanes below that (e < 2^-8): log1p(e) = e - e^2/2 + e^3/3 and e/(1+e) = e -
+//     e^2 + e^3, both to e^3 (relative 6e-8, a float's rounding);
+//   all lanes below the tail of pair_term (z = kTailZ): the cost only, as there
+//     (false: no gradient).
+// N terms at once, one vote for all (independent chains, half the branches).
+template <int N>
+__device__ __forceinline__ bool wide_terms(const float (&z)[N], float& cost, float (&sig)[N]) {
+    float e[N], top = z[0];
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        e[k] = wide_ex2(-fabsf(z[k]) * 1.44269504089f);
+        top = fmaxf(top, z[k]);
     }
+    if (__any_sync(0xffffffffu, top > -5.6f)) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            const float r = __fdividef(1.0f, 1.0f + e[k]);
+            cost += fmaxf(z[k], 0.0f) + log1p_unit(e[k]);
+            sig[k] = z[k] >= 0.0f ? r : e[k] * r;
+        }
+        return true;
+    }
+    if (__any_sync(0xffffffffu, top > kTailZ)) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            cost = fmaf(e[k], fmaf(e[k], fmaf(e[k], 1.0f / 3.0f, -0.5f), 1.0f), cost);
+            sig[k] = e[k] * fmaf(e[k], e[k] - 1.0f, 1.0f);
+        }
+        return true;
+    }
+#pragma unroll
+    for (int k = 0; k < N; ++k) cost += e[k];
+    return false;
+}
+
+template <int THREADS, int MINBLOCKS>
+__global__ void __launch_bounds__(THREADS, MINBLOCKS)
+    smooth_wide_kernel(SmoothArgs a, int blob_cap, int parts) {
+    extern __shared__ __align__(128) unsigned char dsm[];
+    __shared__ __align__(8) uint64_t mbar;
+    constexpr unsigned kAll = 0xffffffffu;
+    constexpr int T = THREADS;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int J = a.J, S = a.S, dim = a.dim, W = a.W;
+    // 32 of all paths' waypoints, one path after the other
+    const long long n_all = (long long)a.P * W;
+    const int group = blockIdx.x / parts, part = blockIdx.x - group * parts;
+    const long long first = (long long)group * 32;
+    const int nw = (int)min(32ll, n_all - first);
+    const unsigned char* gblob = a.blob;
+    const int2* pairs = a.pairs;
+    const SmoothBufs B = smooth_bufs(dsm + blob_cap, J, S);
+    if (tid == 0) {
+        mbar_init(&mbar);
+        *B.next = 0;
+    }
+    for (int i = tid; i < 32 * dim; i += T) {
+        const int w = i / dim, d = i - w * dim;
+        B.q[w * kDimMax + d] = w < nw ? a.wp[first * dim + i] : 0.0f;
+    }
+    for (int i = tid; i < J * 192; i += T) B.acc[i] = 0.0f;
+    if (tid < 32) B.cost[tid] = 0.0f;
+    __syncthreads();
+    uint32_t phase = 0;
+    const int bytes = min(reinterpret_cast<const BlobHeader*>(gblob)->used_bytes, blob_cap);
+    if (!stage_blob(dsm, gblob, bytes, &mbar, phase, nullptr, 0, kWaitLimit)) {
+        // the bulk copy did not arrive in time: copy the scene with plain loads
+        for (int i = tid; i < bytes / 16; i += T) reinterpret_cast<uint4*>(dsm)[i] = reinterpret_cast<const uint4*>(gblob)[i];
+        __syncthreads();
+    }
+    const Scene sc = scene_view(dsm);
+    const BlobHeader& h = *sc.h;
+    // 1. frames, subtree masks, sphere centres
+    if (tid < J) {
+        uint32_t m = 0u;
+        for (int k = tid; k < J; ++k) {  // k is in tid's subtree iff tid is on k's way to the root
+            int x = k;
+            while (x > tid) {
+                const int p = sc.joints[x].idx.x;
+                x = p >= 0 && p < x ? p : -1;
+            }
+            m |= x == tid ? 1u << k : 0u;
+        }
+        B.sub[tid] = m;
+    }
+    // local transforms, a (waypoint, joint) per thread, then the chain: row r of a
+    // frame needs row r of its parent's only, so a thread per (waypoint, row)
+    // composes the joints in order, by the same operations as `compose`
+    for (int i = tid; i < 32 * J; i += T) {
+        const int w = i / J, j = i - w * J;
+        const JointRec& jr = sc.joints[j];
+        joint_local(jr, joint_value(jr, B.q + w * kDimMax), B.g + i * 12);
+    }
+    __syncthreads();
+    if (tid < 96) {
+        const int w = tid / 3, r = tid - w * 3;
+        for (int j = 0; j < J; ++j) {
+            const float* b = B.g + (w * J + j) * 12;
+            float* o = B.pose + (w * J + j) * 12;
+            const int p = sc.joints[j].idx.x;
+            if (p >= 0 && p < j) {
+                const float* a_ = B.pose + (w * J + p) * 12;
+                const float x = a_[3 * r], y = a_[3 * r + 1], z = a_[3 * r + 2], t = a_[9 + r];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) o[3 * r + c] = fmaf(x, b[c], fmaf(y, b[3 + c], z * b[6 + c]));
+                o[9 + r] = fmaf(x, b[9], fmaf(y, b[10], fmaf(z, b[11], t)));
+            } else {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) o[3 * r + c] = b[3 * r + c];
+                o[9 + r] = b[9 + r];
+            }
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < S * 96; i += T) B.g[i] = 0.0f;
+    for (int i = tid; i < S * 32; i += T) {
+        const int s = i >> 5, w = i & 31, f = sc.sfr[s];
+        float4 c = make_float4(kFar, kFar, kFar, 0.0f);
+        if (f >= 0) {
+            const float4* p = reinterpret_cast<const float4*>(B.pose + (w * J + f) * 12);
+            const float4 p0 = p[0], p1 = p[1], p2 = p[2];
+            const float F[12] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w, p2.x, p2.y, p2.z, p2.w};
+            c = xform_point(F, sc.sph[s]);
+        }
+        B.ctr[s * 96 + w] = c.x;
+        B.ctr[s * 96 + 32 + w] = c.y;
+        B.ctr[s * 96 + 64 + w] = c.z;
+    }
+    __syncthreads();
+    auto centre = [&](int s, int w) {
+        const float* x = B.ctr + s * 96 + w;
+        return make_float4(x[0], x[32], x[64], sc.sph[s].w);
+    };
+    // 2. units
+    float total = 0.0f;
+    const int n_world = (S + 1) >> 1, n_units = n_world + (h.P + 31) / 32;
+    while (true) {
+        int u = 0;
+        if (lane == 0) u = atomicAdd(B.next, 1);
+        u = part + parts * __shfl_sync(kAll, u, 0);
+        if (u >= n_units) break;
+        float cost = 0.0f;  // of this unit (short sums lose less)
+        if (u < n_world) {
+            // spheres 2u and 2u + 1 against every primitive; an absent one's terms vanish (its radius is far below 0)
+            float4 c[2];
+            float gx[2], gy[2], gz[2];
+            bool on[2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int s = 2 * u + k;
+                on[k] = s < S && sc.sfr[min(s, S - 1)] >= 0;
+                c[k] = centre(min(s, S - 1), lane);
+                if (!on[k]) c[k].w = -1e30f;
+                gx[k] = gy[k] = gz[k] = 0.0f;
+            }
+            for (int o = 0; o < h.Ns; ++o) {
+                const float4 ob = sc.ws[2 * o + 1];
+                const float ro = -0.5f * sc.ws[2 * o].w;
+                float dx[2], dy[2], dz[2], rn[2], z[2], sig[2];
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    dx[k] = c[k].x - ob.x; dy[k] = c[k].y - ob.y; dz[k] = c[k].z - ob.z;
+                    const float d2 = fmaxf(fmaf(dx[k], dx[k], fmaf(dy[k], dy[k], dz[k] * dz[k])), 1e-36f);
+                    rn[k] = wide_rsqrt(d2);
+                    z[k] = a.beta * (a.margin - (d2 * rn[k] - c[k].w - ro));
+                }
+                if (wide_terms<2>(z, cost, sig)) {
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        const float m = -sig[k] * rn[k];
+                        gx[k] = fmaf(m, dx[k], gx[k]); gy[k] = fmaf(m, dy[k], gy[k]); gz[k] = fmaf(m, dz[k], gz[k]);
+                    }
+                }
+            }
+            for (int o = 0; o < h.Nc; ++o) {
+                const float4 p1 = sc.wc[3 * o], dp = sc.wc[3 * o + 1], dl = sc.wc[3 * o + 2];
+                float ex[2], ey[2], ez[2], rn[2], z[2], sig[2];
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const float u_ = __saturatef(fmaf(dp.x, c[k].x, fmaf(dp.y, c[k].y, fmaf(dp.z, c[k].z, dp.w))));
+                    ex[k] = fmaf(-u_, dl.x, c[k].x - p1.x);
+                    ey[k] = fmaf(-u_, dl.y, c[k].y - p1.y);
+                    ez[k] = fmaf(-u_, dl.z, c[k].z - p1.z);
+                    const float d2 = fmaxf(fmaf(ex[k], ex[k], fmaf(ey[k], ey[k], ez[k] * ez[k])), 1e-36f);
+                    rn[k] = wide_rsqrt(d2);
+                    z[k] = a.beta * (a.margin - (d2 * rn[k] - c[k].w - p1.w));
+                }
+                if (wide_terms<2>(z, cost, sig)) {
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        const float m = -sig[k] * rn[k];
+                        gx[k] = fmaf(m, ex[k], gx[k]); gy[k] = fmaf(m, ey[k], gy[k]); gz[k] = fmaf(m, ez[k], gz[k]);
+                    }
+                }
+            }
+            for (int o = 0; o < h.Nb; ++o) {
+                // signed distance as in smooth_kernel, in units of kBoxScale metres (records are stored scaled)
+                const float4 a0 = sc.wb[4 * o], a1 = sc.wb[4 * o + 1], a2 = sc.wb[4 * o + 2], hl = sc.wb[4 * o + 3];
+                float l0[2], l1[2], l2[2], rn[2], z[2], sig[2];
+                bool outside[2];
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    l0[k] = fmaf(a0.x, c[k].x, fmaf(a0.y, c[k].y, fmaf(a0.z, c[k].z, a0.w)));
+                    l1[k] = fmaf(a1.x, c[k].x, fmaf(a1.y, c[k].y, fmaf(a1.z, c[k].z, a1.w)));
+                    l2[k] = fmaf(a2.x, c[k].x, fmaf(a2.y, c[k].y, fmaf(a2.z, c[k].z, a2.w)));
+                    const float q0 = fabsf(l0[k]) - hl.x, q1 = fabsf(l1[k]) - hl.y, q2 = fabsf(l2[k]) - hl.z;
+                    const float p0 = fmaxf(q0, 0.0f), p1 = fmaxf(q1, 0.0f), p2 = fmaxf(q2, 0.0f);
+                    const float out2 = fmaf(p0, p0, fmaf(p1, p1, p2 * p2));
+                    outside[k] = out2 > 0.0f;
+                    rn[k] = outside[k] ? rsqrtf(out2) : 0.0f;
+                    const float d = kBoxScale * (outside[k] ? out2 * rn[k] : fmaxf(q0, fmaxf(q1, q2))) - c[k].w;
+                    z[k] = a.beta * (a.margin - d);
+                }
+                if (wide_terms<2>(z, cost, sig)) {
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        const float q0 = fabsf(l0[k]) - hl.x, q1 = fabsf(l1[k]) - hl.y, q2 = fabsf(l2[k]) - hl.z;
+                        const float qmax = fmaxf(q0, fmaxf(q1, q2)), m = -kBoxScale * sig[k];  // the axes are stored times kBoxInv
+                        const bool k0 = q0 == qmax, k1 = !k0 && q1 == qmax, k2 = !k0 && !k1;
+                        const float c0 = copysignf(outside[k] ? fmaxf(q0, 0.0f) * rn[k] : (k0 ? 1.0f : 0.0f), l0[k]);
+                        const float c1 = copysignf(outside[k] ? fmaxf(q1, 0.0f) * rn[k] : (k1 ? 1.0f : 0.0f), l1[k]);
+                        const float c2 = copysignf(outside[k] ? fmaxf(q2, 0.0f) * rn[k] : (k2 ? 1.0f : 0.0f), l2[k]);
+                        gx[k] = fmaf(m, fmaf(c0, a0.x, fmaf(c1, a1.x, c2 * a2.x)), gx[k]);
+                        gy[k] = fmaf(m, fmaf(c0, a0.y, fmaf(c1, a1.y, c2 * a2.y)), gy[k]);
+                        gz[k] = fmaf(m, fmaf(c0, a0.z, fmaf(c1, a1.z, c2 * a2.z)), gz[k]);
+                    }
+                }
+            }
+            for (int o = 0; o < h.Nh; ++o) {
+                const float4 hs = sc.wh[o];
+                float z[2], sig[2];
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+                    z[k] = a.beta * (a.margin - (fmaf(hs.x, c[k].x, fmaf(hs.y, c[k].y, fmaf(hs.z, c[k].z, hs.w))) - c[k].w));
+                if (wide_terms<2>(z, cost, sig)) {
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        gx[k] = fmaf(-sig[k], hs.x, gx[k]); gy[k] = fmaf(-sig[k], hs.y, gy[k]); gz[k] = fmaf(-sig[k], hs.z, gz[k]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                if (!on[k]) continue;
+                float* G = B.g + (2 * u + k) * 96 + lane;
+                atomicAdd(G, gx[k]); atomicAdd(G + 32, gy[k]); atomicAdd(G + 64, gz[k]);
+            }
+        } else {
+            // 32 self pairs: the first sphere's gradient stays in registers while it stays the same
+            const int k0 = (u - n_world) * 32, n = min(32, h.P - k0);
+            const int2 mine = lane < n ? __ldg(&pairs[k0 + lane]) : make_int2(-1, -1);
+            int cur = -1;
+            float4 ci = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            float gx = 0.0f, gy = 0.0f, gz = 0.0f;
+            auto flush = [&]() {
+                if (cur < 0) return;
+                float* G = B.g + cur * 96 + lane;
+                atomicAdd(G, gx); atomicAdd(G + 32, gy); atomicAdd(G + 64, gz);
+                gx = gy = gz = 0.0f;
+            };
+            for (int k = 0; k < n; ++k) {
+                const int pi = __shfl_sync(kAll, mine.x, k), pj = __shfl_sync(kAll, mine.y, k);
+                if (pi < 0 || pj < 0 || pi >= S || pj >= S || sc.sfr[pi] < 0 || sc.sfr[pj] < 0) continue;
+                if (pi != cur) {
+                    flush();
+                    cur = pi;
+                    ci = centre(pi, lane);
+                }
+                const float4 cj = centre(pj, lane);
+                const float dx = ci.x - cj.x, dy = ci.y - cj.y, dz = ci.z - cj.z;
+                const float d2 = fmaxf(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), 1e-36f), rn = wide_rsqrt(d2);
+                const float z[1] = {a.beta * (a.margin - (d2 * rn - ci.w - cj.w))};
+                float sig[1];
+                if (wide_terms<1>(z, cost, sig)) {
+                    const float m = -sig[0] * rn;
+                    const float x = m * dx, y = m * dy, z = m * dz;
+                    gx += x; gy += y; gz += z;
+                    float* G = B.g + pj * 96 + lane;
+                    atomicAdd(G, -x); atomicAdd(G + 32, -y); atomicAdd(G + 64, -z);
+                }
+            }
+            flush();
+        }
+        total += cost;
+    }
+    atomicAdd(&B.cost[lane], total);
+    __syncthreads();
+    // 3. frame sums
+    for (int i = tid; i < S * 32; i += T) {
+        const int s = i >> 5, w = i & 31, f = sc.sfr[s];
+        if (f < 0) continue;
+        const float4 c = centre(s, w);
+        const float x = B.g[s * 96 + w], y = B.g[s * 96 + 32 + w], z = B.g[s * 96 + 64 + w];
+        float* A = B.acc + f * 192 + w;
+        atomicAdd(A, x); atomicAdd(A + 32, y); atomicAdd(A + 64, z);
+        atomicAdd(A + 96, c.y * z - c.z * y);
+        atomicAdd(A + 128, c.z * x - c.x * z);
+        atomicAdd(A + 160, c.x * y - c.y * x);
+    }
+    __syncthreads();
+    // 4. dC/dv of every joint from its subtree's sums (dv in the place of q)
+    float* dv = B.q;
+    for (int i = tid; i < J * 32; i += T) {
+        const int j = i >> 5, w = i & 31;
+        float A[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        for (uint32_t m = B.sub[j]; m; m &= m - 1u) {
+            const float* x = B.acc + (__ffs(m) - 1) * 192 + w;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) A[k] += x[32 * k];
+        }
+        const JointRec& jr = sc.joints[j];
+        const float* F = B.pose + (w * J + j) * 12;
+        const float wx = fmaf(F[0], jr.tw.x, fmaf(F[1], jr.tw.y, F[2] * jr.tw.z));
+        const float wy = fmaf(F[3], jr.tw.x, fmaf(F[4], jr.tw.y, F[5] * jr.tw.z));
+        const float wz = fmaf(F[6], jr.tw.x, fmaf(F[7], jr.tw.y, F[8] * jr.tw.z));
+        const float vx = fmaf(F[0], jr.tv.x, fmaf(F[1], jr.tv.y, F[2] * jr.tv.z));
+        const float vy = fmaf(F[3], jr.tv.x, fmaf(F[4], jr.tv.y, F[5] * jr.tv.z));
+        const float vz = fmaf(F[6], jr.tv.x, fmaf(F[7], jr.tv.y, F[8] * jr.tv.z));
+        const float tx = F[9], ty = F[10], tz = F[11];
+        const float mx = A[3] - (ty * A[2] - tz * A[1]);
+        const float my = A[4] - (tz * A[0] - tx * A[2]);
+        const float mz = A[5] - (tx * A[1] - ty * A[0]);
+        dv[w * J + j] = wx * mx + wy * my + wz * mz + vx * A[0] + vy * A[1] + vz * A[2];
+    }
+    __syncthreads();
+    // 5. joint-space gradient + length term, coalesced over (waypoint, dimension)
+    const float inv_beta = 1.0f / a.beta;
+    for (int i = tid; i < nw * dim; i += T) {
+        const int w = i / dim, d = i - w * dim;
+        float gq = 0.0f;
+        for (int j = 0; j < J; ++j) {
+            const JointRec& jr = sc.joints[j];
+            if (jr.idx.z >= 0) {
+                if (jr.idx.z == d) gq = fmaf(jr.tv.w, dv[w * J + j], gq);
+            } else if (jr.idx.y == d) {
+                gq += dv[w * J + j];
+            }
+        }
+        const long long at = first * dim + i;
+        const int in_path = (int)((first + w) % W);
+        if (part == 0) {
+            const float qc = a.wp[at];
+            if (in_path + 1 < W) {
+                const float dn = a.wp[at + dim] - qc;
+                gq -= 2.0f * a.w_len * dn;
+                atomicAdd(&B.cost[w], a.beta * a.w_len * dn * dn);  // in units of 1/beta, as the pair terms
+            }
+            if (in_path > 0) gq += 2.0f * a.w_len * (qc - a.wp[at - dim]);
+        }
+        if (a.grad) {
+            if (parts == 1) a.grad[at] = gq;
+            else atomicAdd(&a.grad[at], gq);  // zero before the launch
+        }
+    }
+    __syncthreads();
+    // 6. cost per path: one atomic per CTA when its waypoints are of one path
+    if (warp == 0) {
+        float v = lane < nw ? B.cost[lane] * inv_beta : 0.0f;
+        const long long p0 = first / W, p1 = (first + nw - 1) / W;
+        if (p0 == p1) {
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(kAll, v, off);
+            if (lane == 0) atomicAdd(&a.cost[p0], v);
+        } else if (lane < nw) {
+            atomicAdd(&a.cost[(first + lane) / W], v);
+        }
+    }
+}
+
+cudaError_t launch_smooth(const unsigned char* blob, size_t blob_stride, int blob_cap, const int32_t* pairs,
+                          size_t pairs_stride,
+                          int J, int S, int dim, const float* wp, int P, int W, float margin, float beta, float w_len,
+                          float* cost, float* grad, bool ordered, cudaStream_t st) {
+    if (P <= 0 || W <= 0) return cudaSuccess;
+    cudaError_t e;
+    if (cost && (e = cudaMemsetAsync(cost, 0, (size_t)P * sizeof(float), st)) != cudaSuccess) return e;
     SmoothArgs a{blob, reinterpret_cast<const int2*>(pairs), blob_stride, pairs_stride, J, S, dim, wp, P, W,
                  margin, beta, w_len, cost, grad};
-    const long long n = (long long)P * W;
-    smooth_kernel<WARPS><<<(unsigned)((n + WARPS - 1) / WARPS), WARPS * 32, smem, st>>>(a);
+    const bool shared = blob_stride == 0 && pairs_stride == 0;
+    if (shared && !ordered && cost && J <= 32) {
+        const size_t wide = (size_t)blob_cap + smooth_wide_bytes(J, S);
+        const long long ctas = ((long long)P * W + 31) / 32;
+        if (wide + 64 <= device_max_smem() && ctas * 8 <= INT32_MAX) {
+            // 256 threads and up to three CTAs per SM (registers), or 512 where
+            // shared memory allows only one (large robots)
+            const int by_smem = (int)((device_max_smem() + 1024) / (wide + 1024 + 64));
+            const bool big = by_smem < 2;
+            void (*const kern)(SmoothArgs, int, int) = big ? smooth_wide_kernel<512, 1> : smooth_wide_kernel<256, 3>;
+            // Several CTAs may share 32 waypoints, each with a share of the pairs,
+            // and add up their gradients (which are linear in the pairs' terms):
+            // as many as make the last wave of the launch full, a twelfth of a
+            // CTA's time being its frames and closing sums.
+            const long long room = (long long)device_sm_count() * (big ? 1 : std::min(by_smem, 3));
+            int parts = 1;
+            double best = 1e30;
+            for (int p = 1; p <= 8; ++p) {
+                const double c = (double)((ctas * p + room - 1) / room) * (1.0 / p + 1.0 / 12);
+                if (c < 0.97 * best) { best = c; parts = p; }
+            }
+            if (parts > 1 && grad &&
+                (e = cudaMemsetAsync(grad, 0, (size_t)P * W * dim * sizeof(float), st)) != cudaSuccess)
+                return e;
+            if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wide)) != cudaSuccess)
+                return e;
+            kern<<<(unsigned)(ctas * parts), big ? 512 : 256, wide, st>>>(a, blob_cap, parts);
+            return cudaGetLastError();
+        }
+    }
+    constexpr int WARPS = 8;
+    size_t smem = (size_t)WARPS * smooth_warp_floats(J, S) * sizeof(float);
+    auto per_path = [&](int warps) { return shared ? 0 : (W + warps - 1) / warps; };
+    auto blocks = [&](int warps) {
+        return (unsigned)(shared ? ((long long)P * W + warps - 1) / warps : (long long)P * per_path(warps));
+    };
+    if (smem + blob_cap + 64 <= device_max_smem()) {
+        smem += blob_cap;
+        auto kern = cost ? smooth_kernel<WARPS, true, true> : smooth_kernel<WARPS, true, false>;
+        if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+            return e;
+        kern<<<blocks(WARPS), WARPS * 32, smem, st>>>(a, blob_cap, per_path(WARPS));
+        return cudaGetLastError();
+    }
+    // scene or robot too large to stage: fewer waypoints per CTA, the scene in global memory
+    constexpr int FEW = 4;
+    smem = (size_t)FEW * smooth_warp_floats(J, S) * sizeof(float);
+    auto kern = cost ? smooth_kernel<FEW, false, true> : smooth_kernel<FEW, false, false>;
+    if (smem > 48 * 1024 &&
+        (e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+        return e;
+    kern<<<blocks(FEW), FEW * 32, smem, st>>>(a, 0, per_path(FEW));
     return cudaGetLastError();
 }
 

@@ -40,14 +40,16 @@ class SmoothContext:
         self.ws = workspace(self.lib.prrtc_b200_smooth_workspace_size(C.byref(self.robot), C.byref(self.world)),
                             self.device)
 
-    def cost_grad(self, waypoints: torch.Tensor, need_grad: bool = True):
+    def cost_grad(self, waypoints: torch.Tensor, need_grad: bool = True, ordered: bool = False):
+        """cost [P] and gradient [P, W, dim]; ``ordered``: every sum in a fixed
+        order, so the gradient is the same bits in every run (descents)."""
         wp = waypoints.detach().to(self.device, torch.float32).contiguous()
         P, W, dim = wp.shape
         cost = torch.empty((P,), dtype=torch.float32, device=self.device)
         grad = torch.empty_like(wp) if need_grad else None
-        _lib.check(self.lib.prrtc_b200_smooth_cost_grad(C.byref(self.robot), C.byref(self.world), dim, ptr(wp), P, W,
-                                                        self.margin, self.beta, self.w_len, ptr(cost), ptr(grad),
-                                                        self.ws.data_ptr(), self.ws.numel(), stream_handle()),
+        call = self.lib.prrtc_b200_smooth_cost_grad_ordered if ordered else self.lib.prrtc_b200_smooth_cost_grad
+        _lib.check(call(C.byref(self.robot), C.byref(self.world), dim, ptr(wp), P, W, self.margin, self.beta,
+                        self.w_len, ptr(cost), ptr(grad), self.ws.data_ptr(), self.ws.numel(), stream_handle()),
                    "prrtc_b200_smooth_cost_grad")
         return cost, grad
 
@@ -146,13 +148,13 @@ def smooth_paths(paths: list, collision_context: dict, lower, upper, *, waypoint
     mask = torch.ones_like(x)
     mask[:, 0] = 0.0
     mask[:, -1] = 0.0
-    c0, _ = sctx.cost_grad(init, need_grad=False)
+    c0, _ = sctx.cost_grad(init, need_grad=False, ordered=True)
     for _ in range(steps):
-        _, g = sctx.cost_grad(x)
+        _, g = sctx.cost_grad(x, ordered=True)
         # normalised step per path keeps the update scale independent of the cost scale
         gn = torch.linalg.norm((g * mask).reshape(g.shape[0], -1), dim=1).clamp_min(1e-12)
         x = torch.minimum(torch.maximum(x - lr * (g * mask) / gn[:, None, None], lo), hi)
-    c1, _ = sctx.cost_grad(x, need_grad=False)
+    c1, _ = sctx.cost_grad(x, need_grad=False, ordered=True)
     checker = CollisionChecker(collision_context, dim, "binary", 0.0, dev)
     pts, owner = densify(x, resolution)
     v = checker.check(pts).to(torch.int64)
@@ -193,7 +195,8 @@ class BatchSmoothContext:
         self.bi = bi
         self.ws = workspace(self.lib.prrtc_b200_smooth_batch_workspace_size(C.byref(bi)), self.device)
 
-    def cost_grad(self, waypoints: torch.Tensor, need_grad: bool = True):
+    def cost_grad(self, waypoints: torch.Tensor, need_grad: bool = True, ordered: bool = True):
+        """cost [P] and gradient [P, W, dim], the sums always in a fixed order."""
         wp = waypoints.detach().to(self.device, torch.float32).contiguous()
         P, W, dim = wp.shape
         if P != self.B:
@@ -207,6 +210,25 @@ class BatchSmoothContext:
         return cost, grad
 
 
+    def descend(self, x: torch.Tensor, lo: torch.Tensor, hi: torch.Tensor, steps: int, lr: float) -> None:
+        """`steps` projected gradient steps on x [P, W, dim] in place: per step the
+        gradient (zero at the end points), its length per path, the update.
+        The scenes are packed once."""
+        P, W, dim = x.shape
+        if P != self.B:
+            raise ValueError(f"expected {self.B} paths (one per world), got {P}")
+        g = torch.empty_like(x)
+        lo, hi = (t.reshape(-1).expand(dim).contiguous() for t in (lo, hi))
+        sp = stream_handle()
+        for k in range(steps):
+            _lib.check(self.lib.prrtc_b200_smooth_step_grad_batch(
+                C.byref(self.bi), dim, x.data_ptr(), W, self.margin, self.beta, self.w_len, 1 if k else 0, g.data_ptr(),
+                self.ws.data_ptr(), self.ws.numel(), sp), "prrtc_b200_smooth_step_grad_batch")
+            norms = torch.linalg.norm(g.reshape(P, -1), dim=1)
+            _lib.check(self.lib.prrtc_b200_smooth_update(x.data_ptr(), g.data_ptr(), norms.data_ptr(), lo.data_ptr(),
+                                                         hi.data_ptr(), lr, P, W, dim, sp), "prrtc_b200_smooth_update")
+
+
 def projected_steps(sctx, init: torch.Tensor, lower, upper, steps: int, lr: float) -> torch.Tensor:
     """`steps` projected gradient steps of the adjoint cost from `init` [P, W, dim]:
     endpoints fixed, joint limits enforced, step length lr per path (the
@@ -215,11 +237,14 @@ def projected_steps(sctx, init: torch.Tensor, lower, upper, steps: int, lr: floa
     lo = as_tensor(lower, torch.float32, init.device).reshape(1, 1, dim)
     hi = as_tensor(upper, torch.float32, init.device).reshape(1, 1, dim)
     x = init.clone()
+    if isinstance(sctx, BatchSmoothContext) and x.dtype == torch.float32 and x.is_contiguous() and x.numel():
+        sctx.descend(x, lo, hi, steps, lr)
+        return x
     mask = torch.ones_like(x)
     mask[:, 0] = 0.0
     mask[:, -1] = 0.0
     for _ in range(steps):
-        _, g = sctx.cost_grad(x)
+        _, g = sctx.cost_grad(x, ordered=True)
         gn = torch.linalg.norm((g * mask).reshape(P, -1), dim=1).clamp_min(1e-12)
         x = torch.minimum(torch.maximum(x - lr * (g * mask) / gn[:, None, None], lo), hi)
     return x

@@ -1,0 +1,83 @@
+"""Smoothing cost and gradient at the edges of the kernel's shapes (GPU): waypoints around a warp, odd and absent
+spheres, no self pairs, robots from 2 to 18 joints, one world or one per path, pairs near, far and beyond the tail.
+
+Reference: torch.autograd of a float64 restatement.  A distance is off by at most 1.5e-6 m (float32 frames and a
+reciprocal square root of 2 ulp), so with beta = 50 each pair's term is off by at most 1e-4 of itself.
+"""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+from prrtc_b200 import scenes
+from prrtc_b200.context import build_collision_context
+
+pytestmark = pytest.mark.gpu
+
+
+def _paths(robot, P, W, seed):
+    rng = np.random.default_rng(seed)
+    a, b = rng.uniform(-1.5, 1.5, (2, P, 1, robot.dim))
+    t = np.linspace(0.0, 1.0, W)[None, :, None]
+    return (a + t * (b - a) + rng.normal(0, 0.02, (P, W, robot.dim))).astype(np.float32)
+
+
+def _check(cost, grad, ctxs, w, w_len):
+    from oracle.smooth_autodiff import smooth_grad
+
+    for p, ctx in enumerate(ctxs):
+        c, g = smooth_grad(ctx, w[p].astype(np.float64), 0.02, 50.0, w_len)
+        assert abs(cost[p].item() - c) <= 1e-4 * abs(c), (p, cost[p].item(), c)
+        got = grad[p].cpu().numpy().astype(np.float64)
+        assert np.linalg.norm(got - g) <= 5e-4 * np.linalg.norm(g) + 1e-14, p
+
+
+@pytest.mark.parametrize("P,W", [(1, 1), (3, 2), (2, 31), (3, 33), (1, 65)])
+@pytest.mark.parametrize("joints", [2, 7, 9, 16, 18])
+def test_shapes(cuda, P, W, joints):
+    from prrtc_b200.smoothing import BatchSmoothContext, SmoothContext
+
+    robot = scenes.dual_arm(0) if joints == 18 else scenes.arm(1, joints)
+    worlds = [scenes.tabletop_world(np.random.default_rng(k)) for k in range(P)]
+    ctxs = [build_collision_context(robot, w) for w in worlds]
+    w = _paths(robot, P, W, joints)
+    x = torch.from_numpy(w).to(cuda)
+    cost, grad = SmoothContext(ctxs[0], robot.dim, device=cuda).cost_grad(x)
+    _check(cost, grad, [ctxs[0]] * P, w, 1.0)
+    cost, grad = BatchSmoothContext(ctxs, robot.dim, device=cuda).cost_grad(x)
+    _check(cost, grad, ctxs, w, 1.0)
+
+
+@pytest.mark.parametrize("form", ["odd_spheres", "one_sphere", "no_pairs", "unordered_pairs", "near", "apart", "below_tail"])
+def test_forms(cuda, form):
+    from prrtc_b200.smoothing import SmoothContext
+
+    robot = scenes.arm(2)
+    ctx = build_collision_context(robot, scenes.tabletop_world(np.random.default_rng(4)))
+    w_len = 0.0 if form in ("apart", "below_tail") else 0.5
+    if form in ("odd_spheres", "one_sphere"):
+        n = 1 if form == "one_sphere" else 55
+        for k in ("sphere_link_idx", "sphere_local", "sphere_radius"):
+            ctx[k] = ctx[k][:n]
+        keep = (ctx["self_pairs"] < n).all(1)
+        ctx["self_pairs"] = ctx["self_pairs"][keep][::3]
+    if form in ("no_pairs", "apart", "below_tail"):
+        ctx["self_pairs"] = ctx["self_pairs"][:0]
+    if form == "unordered_pairs":
+        ctx["self_pairs"] = ctx["self_pairs"][np.random.default_rng(5).permutation(len(ctx["self_pairs"]))[:100]]
+    for k in ("coarse_self_pairs", "self_pair_ranges"):
+        ctx[k] = ctx[k][:0]
+    if form == "near":
+        ctx["world_spheres"] = np.concatenate([ctx["world_spheres"], np.array([[0.0, 0.0, 0.5, 0.6]], np.float32)])
+    if form in ("apart", "below_tail"):
+        at = 0.6 if form == "apart" else 1.05  # about 0.4 m and 0.85 m from the nearest link
+        for k in list(ctx):
+            if k.startswith("world_"):
+                ctx[k] = ctx[k][:0]
+        ctx["world_spheres"] = np.array([[at, 0.0, 0.5, 0.1], [at, 0.3, 0.5, 0.1]], np.float32)
+    w = 0.2 * _paths(robot, 2, 40, 9)
+    cost, grad = SmoothContext(ctx, robot.dim, w_len=w_len, device=cuda).cost_grad(torch.from_numpy(w).to(cuda))
+    _check(cost, grad, [ctx] * 2, w, w_len)
+    if form == "below_tail":
+        assert 0.0 < cost.max().item() < 1e-15 and float(grad.abs().max()) < 1e-13
