@@ -298,6 +298,17 @@ int prrtc_b200_check_configs_noalloc(const prrtc_robot_t* robot, const prrtc_wor
                                      float collision_margin, int32_t full_sweep, int32_t* verdicts,
                                      void* stream);
 
+/* Batched collision check with a scene per problem: configurations
+ * [offsets[b], offsets[b+1]) of configs [n, dim] against problem b's world and
+ * self pairs (offsets [batch+1] on the device, ascending from 0 to n); verdicts
+ * as check_configs.  EUNSUPPORTED when the robot has no coarse model or more than
+ * 32 joints, or a scene is too large for shared memory: check the problems one by
+ * one then. */
+size_t prrtc_b200_check_configs_batch_workspace_size(const prrtc_batch_inputs_t* in);
+int prrtc_b200_check_configs_batch(const prrtc_batch_inputs_t* in, int32_t dim, const float* configs,
+                                   const int32_t* offsets, int32_t n, int32_t collision_mode, float collision_margin,
+                                   int32_t* verdicts, void* workspace, size_t workspace_bytes, void* stream);
+
 /* Point cloud [n_points,3] (device) -> hashed grid.  cell >= 1e-3 m (a cell
  * about the largest robot sphere radius + r_env keeps queries to <= 27 cells);
  * n_buckets a power of two <= 2^24, or 0 for the next power of two >= n_points

@@ -104,6 +104,7 @@ EXPORTS = (
     "prrtc_b200_fk", "prrtc_b200_halton", "prrtc_b200_extract_paths", "prrtc_b200_result_block",
     "prrtc_b200_smooth_workspace_size", "prrtc_b200_smooth_cost_grad", "prrtc_b200_smooth_cost_grad_ordered",
     "prrtc_b200_smooth_batch_workspace_size", "prrtc_b200_smooth_cost_grad_batch",
+    "prrtc_b200_check_configs_batch_workspace_size", "prrtc_b200_check_configs_batch",
     "prrtc_b200_smooth_step_grad_batch", "prrtc_b200_smooth_update",
     "prrtc_b200_choose_tree", "prrtc_b200_radius_update",
     "prrtc_b200_fp32_probe", "prrtc_b200_fp32x2_probe",
@@ -133,6 +134,8 @@ _SIGS = {
     "prrtc_b200_smooth_cost_grad": (C.c_int, [P, P, I32, P, I32, I32, F32, F32, F32, P, P, P, C.c_size_t, P]),
     "prrtc_b200_smooth_cost_grad_ordered": (C.c_int, [P, P, I32, P, I32, I32, F32, F32, F32, P, P, P, C.c_size_t, P]),
     "prrtc_b200_smooth_batch_workspace_size": (C.c_size_t, [P]),
+    "prrtc_b200_check_configs_batch_workspace_size": (C.c_size_t, [P]),
+    "prrtc_b200_check_configs_batch": (C.c_int, [P, I32, P, P, I32, I32, F32, P, P, C.c_size_t, P]),
     "prrtc_b200_smooth_step_grad_batch": (C.c_int, [P, I32, P, I32, F32, F32, F32, I32, P, P, C.c_size_t, P]),
     "prrtc_b200_smooth_update": (C.c_int, [P, P, P, P, P, F32, I32, I32, I32, P]),
     "prrtc_b200_smooth_cost_grad_batch": (C.c_int, [P, I32, P, I32, F32, F32, F32, P, P, P, C.c_size_t, P]),

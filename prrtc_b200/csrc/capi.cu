@@ -385,6 +385,35 @@ int prrtc_b200_check_configs(const prrtc_robot_t* robot, const prrtc_world_t* wo
     return e == cudaSuccess ? PRRTC_B200_OK : cuda_fail(e);
 }
 
+size_t prrtc_b200_check_configs_batch_workspace_size(const prrtc_batch_inputs_t* in) {
+    if (!in || in->batch < 1) return 0;
+    return (size_t)in->batch * blob_stride(make_batch_pack(in, 1, 0, 0.0f));
+}
+
+int prrtc_b200_check_configs_batch(const prrtc_batch_inputs_t* in, int32_t dim, const float* configs,
+                                   const int32_t* offsets, int32_t n, int32_t mode, float margin, int32_t* verdicts,
+                                   void* ws, size_t ws_bytes, void* stream) {
+    if (!in) return PRRTC_B200_EARG;
+    if (in->batch == 0 || n == 0) return PRRTC_B200_OK;
+    if (in->batch < 0 || !configs || !offsets || !verdicts || n < 0 || mode < 0 || mode > 3) return PRRTC_B200_EARG;
+    if (dim < 1 || dim > PRRTC_B200_DIM_MAX || in->batch > 65535) return PRRTC_B200_EUNSUPPORTED;
+    int rc = check_robot(in->robot);
+    if (rc) return rc;
+    const PackSrc s = make_batch_pack(in, dim, mode, margin);
+    if (!batch_cull(s, 0)) return PRRTC_B200_EUNSUPPORTED;
+    const size_t stride = blob_stride(s);
+    if (!ws || !aligned(ws, 256) || ws_bytes < (size_t)in->batch * stride) return PRRTC_B200_EWORKSPACE;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    unsigned char* blobs = static_cast<unsigned char*>(ws);
+    cudaError_t e = launch_pack(s, in->batch, blobs, stride, st);
+    if (e != cudaSuccess) return cuda_fail(e);
+    const size_t pstride = in->self_pairs_count ? (size_t)std::max(0, in->max_self_pairs) : 0;
+    e = launch_check_batch(blobs, stride, in->self_pairs, pstride, in->batch, s.J, s.S, s.K, s.Q, dim, configs, offsets,
+                           n, verdicts, st);
+    if (e == cudaErrorInvalidConfiguration) return PRRTC_B200_EUNSUPPORTED;
+    return e == cudaSuccess ? PRRTC_B200_OK : cuda_fail(e);
+}
+
 static int pc_buckets(int32_t n_points, int32_t n_buckets) {
     if (n_buckets > 0) return n_buckets;
     int H = 1024;

@@ -126,6 +126,14 @@ cudaError_t launch_check(const unsigned char* blob, int blob_cap, const int32_t*
                          int Q, int dim, const float* configs, int n, int full_sweep, bool cull, int32_t* verdicts,
                          cudaStream_t st, const PcView* pc = nullptr);
 
+// The culled checker over n_scenes scenes, configurations [offsets[y],
+// offsets[y+1]) against scene y (offsets on the device, ascending, 0 to n);
+// cudaErrorInvalidConfiguration when its buffers do not fit.
+cudaError_t launch_check_batch(const unsigned char* blobs, size_t blob_stride, const int32_t* pairs,
+                               size_t pairs_stride, int n_scenes, int J, int S, int K, int Q, int dim,
+                               const float* configs, const int32_t* offsets, int n, int32_t* verdicts,
+                               cudaStream_t st);
+
 // pointcloud.cu
 size_t pc_workspace_bytes(int n_points, int n_buckets);
 // Hash n_points points [n,3] into n_buckets (power of two) buckets of cells of

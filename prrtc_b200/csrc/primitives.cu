@@ -449,12 +449,28 @@ static __device__ __noinline__ void check_general(const unsigned char* blob, con
     }
 }
 
+// Scenes of one launch: blockIdx.y of them, scene y's configurations being
+// [offsets[y], offsets[y+1]) of n in all; offsets null: one scene.
+struct CheckScenes {
+    const int32_t* offsets;
+    size_t blob_stride, pairs_stride;
+};
+
 __global__ void __launch_bounds__(256, 3) check_cull_kernel(const unsigned char* __restrict__ gblob, int blob_cap,
                                                             const int2* pairs, int J, int K, int dim, int CW,
                                                             const float* __restrict__ configs, int n,
-                                                            int32_t* verdicts, PcView pc) {
+                                                            int32_t* verdicts, PcView pc, CheckScenes scenes) {
     extern __shared__ __align__(128) unsigned char dsm[];
     __shared__ __align__(8) uint64_t mbar;
+    if (scenes.offsets) {
+        const int lo = max(0, min(scenes.offsets[blockIdx.y], n)), hi = max(lo, min(scenes.offsets[blockIdx.y + 1], n));
+        gblob += blockIdx.y * scenes.blob_stride;
+        pairs += blockIdx.y * scenes.pairs_stride;
+        configs += (size_t)lo * dim;
+        verdicts += lo;
+        n = hi - lo;
+        if (n <= 0) return;
+    }
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_warps = blockDim.x >> 5;
     const int bytes = min(reinterpret_cast<const BlobHeader*>(gblob)->used_bytes, blob_cap);
     if (tid == 0) mbar_init(&mbar);
@@ -505,7 +521,7 @@ static CullCheckAttrs g_cull_check_attr[kCheckAttrDevices];
 // its buffers do not fit (the caller then takes the general one).
 static cudaError_t launch_check_cull(const unsigned char* blob, int blob_cap, const int32_t* pairs, int J, int S, int K,
                                      int Q, int dim, const float* configs, int n, int32_t* verdicts, cudaStream_t st,
-                                     const PcView& pc) {
+                                     const PcView& pc, const CheckScenes& scenes, int n_scenes) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -539,7 +555,7 @@ static cudaError_t launch_check_cull(const unsigned char* blob, int blob_cap, co
     if (best_warps == 0) return cudaErrorInvalidConfiguration;
     int cw = best_cw, wpc = best_wpc;
     while (cw > least && (long long)cw * a.sms * best_warps > n) cw /= 2;  // fewer per warp before warps go idle
-    const long long chunks = (n + cw - 1) / cw;
+    const long long chunks = n / cw + n_scenes;  // of all scenes, about
     while (wpc > 1 && chunks < (long long)a.sms * wpc) wpc /= 2;
     const int dyn = blob_cap + std::max(wpc * warp_check_bytes(J, K, cw), general);
     if (std::max(dyn, best_dyn) > a.max_dyn) {
@@ -549,9 +565,12 @@ static cudaError_t launch_check_cull(const unsigned char* blob, int blob_cap, co
         a.max_dyn = std::max(dyn, best_dyn);
     }
     const long long resident = (long long)a.sms * std::max(1, std::min(a.sm_smem / (dyn + 1024 + 64), 65536 / (a.regs * 32 * wpc)));
-    const long long grid = std::min((chunks + wpc - 1) / wpc, resident);
-    check_cull_kernel<<<(unsigned)grid, wpc * 32, dyn, st>>>(blob, blob_cap, reinterpret_cast<const int2*>(pairs), J, K, dim,
-                                                             cw, configs, n, verdicts, pc);
+    // the scenes' configurations may be spread unevenly: each gets the CTAs for
+    // twice its even share, and a CTA strides over what is left
+    const long long each = n_scenes == 1 ? (chunks + wpc - 1) / wpc : (2 * chunks / n_scenes + wpc - 1) / wpc;
+    const long long grid = std::max(1ll, std::min(each, n_scenes == 1 ? resident : (2 * resident + n_scenes - 1) / n_scenes));
+    check_cull_kernel<<<dim3((unsigned)grid, (unsigned)n_scenes), wpc * 32, dyn, st>>>(
+        blob, blob_cap, reinterpret_cast<const int2*>(pairs), J, K, dim, cw, configs, n, verdicts, pc, scenes);
     return cudaGetLastError();
 }
 
@@ -570,7 +589,8 @@ cudaError_t launch_check(const unsigned char* blob, int blob_cap, const int32_t*
     constexpr int CW = PRRTC_CHECK_CW;
     CheckLaunch best, o;
     if (cull) {
-        const cudaError_t e = launch_check_cull(blob, blob_cap, pairs, J, S, K, Q, dim, configs, n, verdicts, st, cloud);
+        const cudaError_t e = launch_check_cull(blob, blob_cap, pairs, J, S, K, Q, dim, configs, n, verdicts, st, cloud,
+                                                 CheckScenes{nullptr, 0, 0}, 1);
         if (e != cudaErrorInvalidConfiguration) return e;
     }
     cudaError_t e = check_option<CW>(full_sweep, J, S, K, Q, blob_cap, best);
@@ -601,6 +621,15 @@ cudaError_t launch_check(const unsigned char* blob, int blob_cap, const int32_t*
     }
     check_go<CW>(best, full_sweep, blob, pairs, J, S, K, Q, dim, configs, n, verdicts, st, cloud);
     return cudaGetLastError();
+}
+
+cudaError_t launch_check_batch(const unsigned char* blobs, size_t blob_stride, const int32_t* pairs,
+                               size_t pairs_stride, int n_scenes, int J, int S, int K, int Q, int dim,
+                               const float* configs, const int32_t* offsets, int n, int32_t* verdicts,
+                               cudaStream_t st) {
+    return launch_check_cull(blobs, (int)blob_stride, pairs, J, S, K, Q, dim, configs, n, verdicts, st,
+                             PcView{nullptr, nullptr, 0, 0, 0.0f, 0.0f}, CheckScenes{offsets, blob_stride, pairs_stride},
+                             n_scenes);
 }
 
 // ============================================================================ FK

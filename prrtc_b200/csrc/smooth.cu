@@ -5,10 +5,11 @@
 // over every (robot sphere, world primitive) pair and every self pair, with
 // softplus_beta(x) = log(1 + exp(beta x)) / beta.
 //
-// Backward pass per waypoint, one warp per waypoint, nothing stored between the
-// forward and backward sweeps except per-sphere centres:
-//   1. recompute FK (joint-local transforms in parallel over lanes, chain
-//      composition on lane 0) and the sphere centres c_s;
+// Backward pass per waypoint, nothing stored between the forward and backward
+// sweeps except per-sphere centres (a warp per waypoint, or a lane per waypoint
+// for paths of one scene):
+//   1. recompute FK (joint-local transforms in parallel, then the chain in joint
+//      order) and the sphere centres c_s;
 //   2. g_s = dC/dc_s from every pair: -sigmoid(beta (m - d)) * dd/dc_s;
 //   3. per frame f: G_f = sum g_s, M_f = sum c_s x g_s over its spheres, then
 //      folded into parents in reverse topological order (subtree sums);

@@ -23,7 +23,7 @@ import torch
 
 from . import _lib
 from .collision import CollisionChecker
-from .device import DeviceContext, as_tensor, cuda_device, ptr, stream_handle, workspace
+from .device import ROBOT_SPEC, DeviceContext, Stager, as_tensor, cuda_device, ptr, stream_handle, workspace
 
 
 class SmoothContext:
@@ -164,6 +164,39 @@ def smooth_paths(paths: list, collision_context: dict, lower, upper, *, waypoint
     return out, accepted, c0, c1
 
 
+class _BatchScenes:
+    """Robot tables plus one world per problem, on the device in one staged
+    copy, as the C struct of the batched entry points."""
+
+    def __init__(self, collision_contexts, device: torch.device):
+        from .prrtc import _pack_worlds
+
+        ctxs = list(collision_contexts)
+        B = self.B = len(ctxs)
+        # whether every context is the first one's robot in another world (the
+        # very same tables), and none has a point cloud
+        self.one_robot = all(c.get("point_cloud") is None and all(c.get(k) is ctxs[0].get(k) for k in ROBOT_SPEC)
+                             for c in ctxs)
+        stage = Stager(device)
+        self.robot_ctx = DeviceContext(ctxs[0], device, world_keys=False, stager=stage)
+        packed, counts = _pack_worlds(ctxs, B)
+        keys = {k: (stage.add(packed[k], torch.int32 if k == "self_pairs" else torch.float32),
+                    stage.add(counts[k], torch.int32)) for k in packed}
+        stage.commit()
+        self.robot_ctx.finish()
+        self.t = {}
+        bi = _lib.BatchInputs()
+        bi.batch = B
+        bi.robot = self.robot_ctx.robot()
+        for key, (k_tab, k_cnt) in keys.items():
+            tab, cnt = stage.get(k_tab), stage.get(k_cnt)
+            self.t[key], self.t[key + "_count"] = tab, cnt
+            setattr(bi, key, ptr(tab))
+            setattr(bi, "max_" + key, int(tab.shape[1]))
+            setattr(bi, key + "_count", cnt.data_ptr())
+        self.bi = bi
+
+
 class BatchSmoothContext:
     """Robot tables plus one world per path, resident on the device, for the
     batched adjoint (prrtc_b200_smooth_cost_grad_batch): path p is costed
@@ -171,29 +204,13 @@ class BatchSmoothContext:
 
     def __init__(self, collision_contexts, dim: int, margin: float = 0.02, beta: float = 50.0, w_len: float = 1.0,
                  device=None):
-        from .prrtc import _pack_worlds
-
         self.lib = _lib.load()
         self.device = cuda_device(device)
         self.dim = int(dim)
         self.margin, self.beta, self.w_len = float(margin), float(beta), float(w_len)
-        ctxs = list(collision_contexts)
-        B = self.B = len(ctxs)
-        self.robot_ctx = DeviceContext(ctxs[0], self.device, world_keys=False)
-        packed, counts = _pack_worlds(ctxs, B)
-        self.t = {}
-        bi = _lib.BatchInputs()
-        bi.batch = B
-        bi.robot = self.robot_ctx.robot()
-        for key in ("world_spheres", "world_capsules", "world_boxes", "world_halfspaces", "self_pairs"):
-            tab = torch.from_numpy(np.ascontiguousarray(packed[key])).to(self.device)
-            cnt = torch.from_numpy(np.ascontiguousarray(counts[key], dtype=np.int32)).to(self.device)
-            self.t[key], self.t[key + "_count"] = tab, cnt
-            setattr(bi, key, tab.data_ptr() if tab.numel() else None)
-            setattr(bi, "max_" + key, int(tab.shape[1]))
-            setattr(bi, key + "_count", cnt.data_ptr())
-        self.bi = bi
-        self.ws = workspace(self.lib.prrtc_b200_smooth_batch_workspace_size(C.byref(bi)), self.device)
+        self.scenes = _BatchScenes(collision_contexts, self.device)
+        self.B, self.bi = self.scenes.B, self.scenes.bi
+        self.ws = workspace(self.lib.prrtc_b200_smooth_batch_workspace_size(C.byref(self.bi)), self.device)
 
     def cost_grad(self, waypoints: torch.Tensor, need_grad: bool = True, ordered: bool = True):
         """cost [P] and gradient [P, W, dim], the sums always in a fixed order."""
@@ -267,15 +284,34 @@ def smooth_paths_batch(paths: list, collision_contexts: list, lower, upper, *, w
     c0, _ = sctx.cost_grad(init, need_grad=False)
     x = projected_steps(sctx, init, lower, upper, steps, lr)
     c1, _ = sctx.cost_grad(x, need_grad=False)
-    accepted = revalidate_batch(x, collision_contexts, resolution, dev)
+    accepted = revalidate_batch(x, collision_contexts, resolution, dev, sctx.scenes)
     out = torch.where(accepted[:, None, None], x, init)
     return out, accepted, c0, c1
 
 
-def revalidate_batch(paths: torch.Tensor, collision_contexts: list, resolution: float, device) -> torch.Tensor:
+def revalidate_batch(paths: torch.Tensor, collision_contexts: list, resolution: float, device,
+                     scenes: _BatchScenes | None = None) -> torch.Tensor:
     """Exact binary re-validation of path p [W, dim] of `paths` at `resolution`
-    against collision_contexts[p]; returns accepted [P] bool."""
+    against collision_contexts[p]; returns accepted [P] bool.  One batched
+    check for all paths where their contexts are one robot in different worlds
+    (``scenes``: their tables, when already on the device)."""
     pts, owner = densify(paths, resolution)
+    P, dim = int(paths.shape[0]), int(paths.shape[2])
+    dev = torch.device(device)
+    lib = _lib.load()
+    if P and pts.dtype == torch.float32 and pts.is_cuda:
+        scenes = scenes if scenes is not None else _BatchScenes(collision_contexts, pts.device)
+        if scenes.one_robot and scenes.B == P:
+            offsets = torch.searchsorted(owner, torch.arange(P + 1, device=owner.device), out_int32=True)
+            pts = pts.contiguous()
+            v = torch.empty((pts.shape[0],), dtype=torch.int32, device=pts.device)
+            ws = workspace(lib.prrtc_b200_check_configs_batch_workspace_size(C.byref(scenes.bi)), pts.device)
+            rc = lib.prrtc_b200_check_configs_batch(C.byref(scenes.bi), dim, ptr(pts), ptr(offsets), int(pts.shape[0]),
+                                                    0, 0.0, ptr(v), ws.data_ptr(), ws.numel(), stream_handle())
+            if rc != _lib.EUNSUPPORTED:
+                _lib.check(rc, "prrtc_b200_check_configs_batch")
+                bad = torch.zeros((P,), dtype=torch.int32, device=pts.device).index_add_(0, owner, v)
+                return (bad == 0).to(dev)
     owner_np = owner.cpu().numpy()
     bounds = np.searchsorted(owner_np, np.arange(paths.shape[0] + 1))
     accepted = torch.ones((paths.shape[0],), dtype=torch.bool, device=device)

@@ -211,3 +211,38 @@ def test_culled_verdicts_equal_full_sweep(cuda, form, mode):
         q = rng.uniform(robot.lower, robot.upper, (n, robot.dim)).astype(np.float32)
         q[n // 2, 2] = (np.nan, np.inf, 1e30, 0.1)[n % 4]
         assert np.array_equal(chk.check(q).cpu().numpy(), chk.check(q, full_sweep=True).cpu().numpy()), n
+
+
+@pytest.mark.parametrize("mode", [0, 1, 3])
+def test_batched_scenes_equal_one_by_one(cuda, mode):
+    """One launch over many scenes (uneven shares, an empty one, one that the culled checker does not take) against
+    a checker per scene."""
+    import ctypes as C
+
+    import torch
+
+    from prrtc_b200 import _lib
+    from prrtc_b200.collision import CollisionChecker
+    from prrtc_b200.smoothing import _BatchScenes
+
+    robot = scenes.arm(0)
+    rng = np.random.default_rng(7)
+    ctxs = [build_collision_context(robot, w) for w in (
+        scenes.tabletop_world(rng), scenes.spheres_world(rng, 16), {}, scenes.uneven_world(rng),
+        {"world_halfspaces": np.array([[0, 0, 3.0, 0, 0, 0.1]], np.float32)}, scenes.tabletop_world(rng))]
+    share = [1, 300, 0, 37, 64, 5]
+    off = np.concatenate([[0], np.cumsum(share)]).astype(np.int32)
+    q = torch.from_numpy(rng.uniform(robot.lower, robot.upper, (off[-1], robot.dim)).astype(np.float32)).to(cuda)
+    sc = _BatchScenes(ctxs, cuda)
+    v = torch.full((int(off[-1]),), -1, dtype=torch.int32, device=cuda)
+    offsets = torch.from_numpy(off).to(cuda)
+    lib = _lib.load()
+    ws = torch.empty(lib.prrtc_b200_check_configs_batch_workspace_size(C.byref(sc.bi)), dtype=torch.uint8, device=cuda)
+    _lib.check(lib.prrtc_b200_check_configs_batch(C.byref(sc.bi), robot.dim, q.data_ptr(), offsets.data_ptr(), int(off[-1]),
+                                                  mode, 0.02, v.data_ptr(), ws.data_ptr(), ws.numel(),
+                                                  torch.cuda.current_stream().cuda_stream), "check_configs_batch")
+    for k, ctx in enumerate(ctxs):
+        if share[k]:
+            seg = slice(int(off[k]), int(off[k + 1]))
+            want = CollisionChecker(ctx, robot.dim, CHECKERS[mode], 0.02, cuda).check(q[seg], full_sweep=True)
+            assert torch.equal(v[seg], want), k
