@@ -242,6 +242,10 @@ int prrtc_b200_nearest_neighbor(const float* tree_configs, int32_t dim, int32_t 
                                 const int32_t* tree_size, const float* queries, int32_t batch,
                                 int32_t* indices, float* dists,
                                 void* workspace, size_t workspace_bytes, void* stream);
+/* The same with the tree's size given by value. */
+int prrtc_b200_nearest_neighbor_sized(const float* tree, int32_t dim, int32_t max_nodes, int32_t tree_size,
+                                      const float* queries, int32_t batch, int32_t* indices, float* dists,
+                                      void* workspace, size_t workspace_bytes, void* stream);
 
 /* Step-limited extend (prrtc_extend.cu:14-73): new = near + (sample-near)*min(1, step/|.|). */
 int prrtc_b200_extend(const float* tree_configs, int32_t dim, int32_t max_nodes,

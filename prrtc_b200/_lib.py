@@ -96,6 +96,7 @@ EXPORTS = (
     "prrtc_b200_plan_workspace_size", "prrtc_b200_plan",
     "prrtc_b200_plan_batch_workspace_size", "prrtc_b200_plan_batch",
     "prrtc_b200_nearest_neighbor_workspace_size", "prrtc_b200_nearest_neighbor",
+    "prrtc_b200_nearest_neighbor_sized",
     "prrtc_b200_extend",
     "prrtc_b200_check_configs_workspace_size", "prrtc_b200_check_configs",
     "prrtc_b200_iteration",
@@ -118,6 +119,7 @@ _SIGS = {
     "prrtc_b200_plan_batch": (C.c_int, [P, P, P, P, P, C.c_size_t, P]),
     "prrtc_b200_nearest_neighbor_workspace_size": (C.c_size_t, [I32]),
     "prrtc_b200_nearest_neighbor": (C.c_int, [P, I32, I32, P, P, I32, P, P, P, C.c_size_t, P]),
+    "prrtc_b200_nearest_neighbor_sized": (C.c_int, [P, I32, I32, I32, P, I32, P, P, P, C.c_size_t, P]),
     "prrtc_b200_extend": (C.c_int, [P, I32, I32, P, P, I32, P, P, P, P, P]),
     "prrtc_b200_check_configs_workspace_size": (C.c_size_t, [P, P]),
     "prrtc_b200_check_configs": (C.c_int, [P, P, I32, P, I32, I32, F32, I32, P, P, C.c_size_t, P]),

@@ -307,7 +307,7 @@ size_t prrtc_b200_nearest_neighbor_workspace_size(int32_t batch) {
     return (((size_t)std::max(batch, 1) * sizeof(unsigned long long)) + 255) & ~(size_t)255;
 }
 
-int prrtc_b200_nearest_neighbor(const float* tree, int32_t dim, int32_t max_nodes, const int32_t* tree_size,
+static int nearest_neighbor(const float* tree, int32_t dim, int32_t max_nodes, const int32_t* tree_size, int32_t size,
                                 const float* queries, int32_t batch, int32_t* indices, float* dists, void* ws,
                                 size_t ws_bytes, void* stream) {
     if (batch == 0) return PRRTC_B200_OK;
@@ -315,9 +315,23 @@ int prrtc_b200_nearest_neighbor(const float* tree, int32_t dim, int32_t max_node
     if (dim < 1 || dim > PRRTC_B200_DIM_MAX) return PRRTC_B200_EUNSUPPORTED;
     if (!ws || !aligned(ws, 256) || ws_bytes < prrtc_b200_nearest_neighbor_workspace_size(batch))
         return PRRTC_B200_EWORKSPACE;
-    cudaError_t e = launch_nearest(tree, dim, max_nodes, tree_size, queries, batch, indices, dists,
+    cudaError_t e = launch_nearest(tree, dim, max_nodes, tree_size, size, queries, batch, indices, dists,
                                    static_cast<unsigned long long*>(ws), static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? PRRTC_B200_OK : cuda_fail(e);
+}
+
+int prrtc_b200_nearest_neighbor(const float* tree, int32_t dim, int32_t max_nodes, const int32_t* tree_size,
+                                const float* queries, int32_t batch, int32_t* indices, float* dists, void* ws,
+                                size_t ws_bytes, void* stream) {
+    return nearest_neighbor(tree, dim, max_nodes, tree_size, max_nodes, queries, batch, indices, dists, ws, ws_bytes,
+                            stream);
+}
+
+int prrtc_b200_nearest_neighbor_sized(const float* tree, int32_t dim, int32_t max_nodes, int32_t tree_size,
+                                      const float* queries, int32_t batch, int32_t* indices, float* dists, void* ws,
+                                      size_t ws_bytes, void* stream) {
+    return nearest_neighbor(tree, dim, max_nodes, nullptr, tree_size, queries, batch, indices, dists, ws, ws_bytes,
+                            stream);
 }
 
 int prrtc_b200_extend(const float* tree, int32_t dim, int32_t max_nodes, const int32_t* nearest,

@@ -114,7 +114,8 @@ cudaError_t launch_result_block(int B, int dim, int max_len, const ResultSrc& R,
                                 const float* paths, float* packed, long long packed_cap, cudaStream_t st);
 
 // primitives.cu
-cudaError_t launch_nearest(const float* tree, int dim, int N, const int32_t* tree_size, const float* q, int batch,
+// The tree's size: *tree_size on the device, or `size` when that is null.
+cudaError_t launch_nearest(const float* tree, int dim, int N, const int32_t* tree_size, int size, const float* q, int batch,
                            int32_t* idx, float* dist, unsigned long long* keys, cudaStream_t st);
 cudaError_t launch_extend(const float* tree, int dim, int N, const int32_t* nearest, const float* samples,
                           int batch, const float* step, float* out, int32_t* parents, int32_t* valid,

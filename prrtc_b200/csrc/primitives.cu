@@ -16,143 +16,123 @@ namespace prrtc {
 
 // ============================================================================ nearest neighbour
 
-// Grid (splits, batch): CTA (s, b) scans its slice of the tree for query b and
-// folds its (dsq, index) minimum into keys[b] with a 64-bit atomicMin on
-// (float bits << 32 | index) -- for non-negative floats the bit pattern orders
-// like the value, so the minimum key is the lexicographic (dsq, lowest index)
-// minimum.  NaN slots never win.
-__global__ void __launch_bounds__(256) nn_kernel(const float* __restrict__ tree, int dim, int N,
-                                                 const int32_t* tree_size, const float* __restrict__ q, int batch,
-                                                 int slice, unsigned long long* keys) {
-    const int b = blockIdx.y, tid = threadIdx.x, T = blockDim.x;
-    int n = tree_size ? tree_size[0] : N;
-    n = max(1, min(n, N));
-    const int lo = blockIdx.x * slice;
-    const int hi = min(n, lo + slice);
-    float qr[kDimMax];
-#pragma unroll
-    for (int d = 0; d < kDimMax; ++d) qr[d] = d < dim ? q[(size_t)b * dim + d] : 0.0f;
-    float best = INFINITY;
-    int bi = INT_MAX;
-    if ((N & 3) == 0 && (lo & 3) == 0 && (reinterpret_cast<uintptr_t>(tree) & 15) == 0) {
-        const float4* t4 = reinterpret_cast<const float4*>(tree);
-        const size_t row4 = (size_t)(N >> 2);
-        const int g0 = lo >> 2, g1 = (hi + 3) >> 2;
-        for (int g = g0 + tid; g < g1; g += T) {
-            float4 v = __ldg(t4 + g);
-            float dx = __fsub_rn(v.x, qr[0]), dy = __fsub_rn(v.y, qr[0]), dz = __fsub_rn(v.z, qr[0]),
-                  dw = __fsub_rn(v.w, qr[0]);
-            float ax = __fmul_rn(dx, dx), ay = __fmul_rn(dy, dy), az = __fmul_rn(dz, dz), aw = __fmul_rn(dw, dw);
-#pragma unroll
-            for (int d = 1; d < kDimMax; ++d) {
-                if (d < dim) {
-                    v = __ldg(t4 + d * row4 + g);
-                    dx = __fsub_rn(v.x, qr[d]); dy = __fsub_rn(v.y, qr[d]);
-                    dz = __fsub_rn(v.z, qr[d]); dw = __fsub_rn(v.w, qr[d]);
-                    ax = __fmaf_rn(dx, dx, ax); ay = __fmaf_rn(dy, dy, ay);
-                    az = __fmaf_rn(dz, dz, az); aw = __fmaf_rn(dw, dw, aw);
-                }
-            }
-            const int i0 = g << 2;
-            if (ax < best && i0 < hi) { best = ax; bi = i0; }
-            if (ay < best && i0 + 1 < hi) { best = ay; bi = i0 + 1; }
-            if (az < best && i0 + 2 < hi) { best = az; bi = i0 + 2; }
-            if (aw < best && i0 + 3 < hi) { best = aw; bi = i0 + 3; }
-        }
-    } else {
-        for (int i = lo + tid; i < hi; i += T) {
-            float dd = __fsub_rn(__ldg(tree + i), qr[0]);
-            float acc = __fmul_rn(dd, dd);
-            for (int d = 1; d < dim; ++d) {
-                dd = __fsub_rn(__ldg(tree + (size_t)d * N + i), qr[d]);
-                acc = __fmaf_rn(dd, dd, acc);
-            }
-            if (acc < best) { best = acc; bi = i; }
-        }
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        const float od = __shfl_xor_sync(0xffffffffu, best, off);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
-        if (od < best || (od == best && oi < bi)) { best = od; bi = oi; }
-    }
-    if ((tid & 31) == 0 && bi != INT_MAX) {
-        const unsigned long long key =
-            ((unsigned long long)__float_as_uint(best) << 32) | (unsigned long long)(unsigned)bi;
-        atomicMin(&keys[b], key);
-    }
+// Every CTA holds up to kNnQueries queries and strides over the tree, a column of
+// 4 nodes per thread, so the tree is read once per 64 queries.  The dimensions go in blocks of 4: after a block, a warp whose 128
+// partial sums all exceed the query's best distance so far leaves the query (a
+// sum of squares only grows, also in rounded arithmetic), which in 7 dimensions
+// is nearly always after the first block.  The best distances are shared: each
+// improvement goes to the CTA's and the global key at once, and every CTA
+// rereads the global keys per column.  Keys order like (squared distance,
+// index), so the result is the nearest node, the lowest index on a tie; NaN and
+// infinite distances never pass.  Per (node, query) x - q (as x + -q, two nodes
+// per instruction), then fma(d, d, sum) from +0 in dimension order, bit-identical
+// to the reference's `dsq += diff*diff` (prrtc_nearest_neighbor.cu).
+//
+// One query is bound by HBM (33.5 M nodes x 7, 90% live: 131 us, 6.45 TB/s, 98%
+// of the measured copy; a CTA per slice with its own minimum took 145 us), 64 by
+// issue: 16 packed instructions, a vote and the loop per query and 128 nodes (4.19
+// M nodes x 7: 505 -> 143 us against 8 queries per pass over the tree and all
+// dimensions; rows that are not 16-byte aligned 3039 -> 148 us, since one load
+// form serves both).  Loops of 1 or 4 queries measured the same.
+constexpr int kNnQueries = 64;
+constexpr unsigned long long kNnNone = 0x7f7fffffffffffffull;  // no node yet: FLT_MAX, above every index
+
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    unsigned long long x, y, r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(a.x), "f"(a.y));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(y) : "f"(b.x), "f"(b.y));
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(r));
+    return a;
+}
+__device__ __forceinline__ float2 square_add2(float2 d, float2 acc) {
+    unsigned long long x, y, r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(d.x), "f"(d.y));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(y) : "f"(acc.x), "f"(acc.y));
+    asm("fma.rn.f32x2 %0, %1, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(acc.x), "=f"(acc.y) : "l"(r));
+    return acc;
 }
 
-// Query-tiled form for batches: CTA (s, t) scans its slice once for QT queries
-// of tile t.  Each thread keeps one 4-node column of every dimension in
-// registers and evaluates all QT queries (held in shared memory) against it, so
-// the tree is read once per QT queries instead of once per query.  Arithmetic
-// per (node, query) is the same sub/mul/fma sequence as nn_kernel.
-template <int QT>
-__global__ void __launch_bounds__(256) nn_tiled_kernel(const float* __restrict__ tree, int dim, int N,
-                                                       const int32_t* tree_size, const float* __restrict__ q,
-                                                       int batch, int slice, unsigned long long* keys) {
-    __shared__ __align__(16) float qs[QT][kDimMax];
-    const int tid = threadIdx.x, T = blockDim.x;
-    const int q0 = blockIdx.y * QT;
-    for (int i = tid; i < QT * kDimMax; i += T) {
-        const int qq = i / kDimMax, d = i - qq * kDimMax;
-        qs[qq][d] = (q0 + qq < batch && d < dim) ? q[(size_t)(q0 + qq) * dim + d] : 0.0f;
+// DB blocks of 4 dimensions; VEC: rows start 16-byte aligned and a thread's 4
+// nodes are neighbours (one 16-byte load per dimension), else they are T apart.
+template <int DB, bool VEC>
+__global__ void __launch_bounds__(256, DB <= 2 ? 3 : 2) nn_scan_kernel(const float* __restrict__ tree, int dim, int N,
+                                                                      const int32_t* tree_size, int size,
+                                                                      const float* __restrict__ q, int batch, int per_cta,
+                                                                      unsigned long long* keys) {
+    __shared__ __align__(16) float2 nq[kNnQueries][DB * 4];  // (-q, -q)
+    __shared__ unsigned long long s_key[kNnQueries];
+    constexpr int T = 256;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int q0 = blockIdx.y * per_cta, nqs = min(per_cta, batch - q0);
+    for (int i = tid; i < nqs * DB * 4; i += T) {
+        const int k = i / (DB * 4), d = i - k * DB * 4;
+        const float x = d < dim ? -q[(size_t)(q0 + k) * dim + d] : 0.0f;
+        nq[k][d] = make_float2(x, x);
     }
+    if (tid < kNnQueries) s_key[tid] = kNnNone;
     __syncthreads();
-    int n = tree_size ? tree_size[0] : N;
+    int n = tree_size ? tree_size[0] : size;
     n = max(1, min(n, N));
-    const int lo = blockIdx.x * slice;
-    const int hi = min(n, lo + slice);
-    float best[QT];
-    int bi[QT];
+    volatile const unsigned* bound = reinterpret_cast<volatile const unsigned*>(s_key);  // high words: odd
+    for (long long base = (long long)blockIdx.x * T * 4; base < n; base += (long long)gridDim.x * T * 4) {
+        const int i0 = (int)base + (VEC ? 4 * tid : tid);
+        constexpr int step = VEC ? 1 : T;
+        unsigned long long seen = ~0ull;
+        if (tid < nqs) seen = __ldcg(&keys[q0 + tid]);
+        // nodes past the end read as far away (never NaN-free near ones)
+        float2 v[DB * 4][2];
 #pragma unroll
-    for (int k = 0; k < QT; ++k) { best[k] = INFINITY; bi[k] = INT_MAX; }
-    const float4* t4 = reinterpret_cast<const float4*>(tree);
-    const size_t row4 = (size_t)(N >> 2);
-    const int g0 = lo >> 2, g1 = (hi + 3) >> 2;
-    for (int g = g0 + tid; g < g1; g += T) {
-        float4 v[kDimMax];
-#pragma unroll
-        for (int d = 0; d < kDimMax; ++d)
-            if (d < dim) v[d] = __ldg(t4 + d * row4 + g);
-        const int i0 = g << 2;
-#pragma unroll
-        for (int k = 0; k < QT; ++k) {
-            float dx = __fsub_rn(v[0].x, qs[k][0]), dy = __fsub_rn(v[0].y, qs[k][0]), dz = __fsub_rn(v[0].z, qs[k][0]),
-                  dw = __fsub_rn(v[0].w, qs[k][0]);
-            float ax = __fmul_rn(dx, dx), ay = __fmul_rn(dy, dy), az = __fmul_rn(dz, dz), aw = __fmul_rn(dw, dw);
-#pragma unroll
-            for (int d = 1; d < kDimMax; ++d) {
-                if (d < dim) {
-                    const float qd = qs[k][d];
-                    dx = __fsub_rn(v[d].x, qd); dy = __fsub_rn(v[d].y, qd);
-                    dz = __fsub_rn(v[d].z, qd); dw = __fsub_rn(v[d].w, qd);
-                    ax = __fmaf_rn(dx, dx, ax); ay = __fmaf_rn(dy, dy, ay);
-                    az = __fmaf_rn(dz, dz, az); aw = __fmaf_rn(dw, dw, aw);
+        for (int d = 0; d < DB * 4; ++d) {
+            float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (d < dim) {
+                const float* row = tree + (size_t)d * N;
+                if (VEC) {
+                    if (i0 < n) x = __ldg(reinterpret_cast<const float4*>(row + i0));  // N % 4 == 0: inside the row
+                } else {
+                    if (i0 < n) x.x = __ldg(row + i0);
+                    if (i0 + T < n) x.y = __ldg(row + i0 + T);
+                    if (i0 + 2 * T < n) x.z = __ldg(row + i0 + 2 * T);
+                    if (i0 + 3 * T < n) x.w = __ldg(row + i0 + 3 * T);
                 }
             }
-            if (ax < best[k] && i0 < hi) { best[k] = ax; bi[k] = i0; }
-            if (ay < best[k] && i0 + 1 < hi) { best[k] = ay; bi[k] = i0 + 1; }
-            if (az < best[k] && i0 + 2 < hi) { best[k] = az; bi[k] = i0 + 2; }
-            if (aw < best[k] && i0 + 3 < hi) { best[k] = aw; bi[k] = i0 + 3; }
+            v[d][0] = make_float2(x.x, x.y);
+            v[d][1] = make_float2(x.z, x.w);
         }
-    }
+        // a node past the end starts from infinity, so that its sum never passes
+        const float2 s0 = make_float2(i0 < n ? 0.0f : INFINITY, i0 + step < n ? 0.0f : INFINITY);
+        const float2 s1 = make_float2(i0 + 2 * step < n ? 0.0f : INFINITY, i0 + 3 * step < n ? 0.0f : INFINITY);
+#pragma unroll 2
+        for (int k = 0; k < nqs; ++k) {
+            const float best = __uint_as_float(bound[2 * k + 1]);
+            float2 a = s0, b = s1;
+            bool in = true;
 #pragma unroll
-    for (int k = 0; k < QT; ++k) {
-        float bk = best[k];
-        int ik = bi[k];
+            for (int blk = 0; blk < DB; ++blk) {
+                if (!in) break;
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const float od = __shfl_xor_sync(0xffffffffu, bk, off);
-            const int oi = __shfl_xor_sync(0xffffffffu, ik, off);
-            if (od < bk || (od == bk && oi < ik)) { bk = od; ik = oi; }
+                for (int d = 4 * blk; d < 4 * blk + 4; ++d) {
+                    const float2 m = nq[k][d];
+                    a = square_add2(add2(v[d][0], m), a);
+                    b = square_add2(add2(v[d][1], m), b);
+                }
+                in = __any_sync(0xffffffffu, fminf(fminf(a.x, a.y), fminf(b.x, b.y)) <= best);
+            }
+            if (!in) continue;
+            // some node of the warp is as near as the best so far
+            float lo = INFINITY;
+            int li = 0x7fffffff;
+            if (a.x < lo) { lo = a.x; li = i0; }
+            if (a.y < lo) { lo = a.y; li = i0 + step; }
+            if (b.x < lo) { lo = b.x; li = i0 + 2 * step; }
+            if (b.y < lo) { lo = b.y; li = i0 + 3 * step; }
+            const unsigned bits = __float_as_uint(lo), wmin = __reduce_min_sync(0xffffffffu, bits);
+            const unsigned idx = __reduce_min_sync(0xffffffffu, bits == wmin ? (unsigned)li : 0x7fffffffu);
+            const unsigned long long key = (unsigned long long)wmin << 32 | idx;
+            if (lane == 0 && key < s_key[k] && atomicMin(&s_key[k], key) > key) atomicMin(&keys[q0 + k], key);
         }
-        if ((tid & 31) == 0 && ik != INT_MAX && q0 + k < batch) {
-            const unsigned long long key =
-                ((unsigned long long)__float_as_uint(bk) << 32) | (unsigned long long)(unsigned)ik;
-            atomicMin(&keys[q0 + k], key);
-        }
+        if (seen < kNnNone && seen < s_key[tid < nqs ? tid : 0] && tid < nqs) atomicMin(&s_key[tid], seen);
     }
 }
 
@@ -169,24 +149,28 @@ __global__ void nn_decode_kernel(const unsigned long long* keys, int batch, int3
     dist[b] = __fsqrt_rn(__uint_as_float((unsigned)(k >> 32)));
 }
 
-cudaError_t launch_nearest(const float* tree, int dim, int N, const int32_t* tree_size, const float* q, int batch,
+cudaError_t launch_nearest(const float* tree, int dim, int N, const int32_t* tree_size, int size, const float* q, int batch,
                            int32_t* idx, float* dist, unsigned long long* keys, cudaStream_t st) {
     if (batch <= 0) return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(keys, 0xFF, (size_t)batch * sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
-    // enough CTAs to cover every SM several times; slices are multiples of 1024 nodes
     const int sms = device_sm_count();
-    constexpr int kQT = 8;
-    const bool tiled = batch >= 4 && (N & 3) == 0 && (reinterpret_cast<uintptr_t>(tree) & 15) == 0;
-    const int tiles = tiled ? (batch + kQT - 1) / kQT : batch;
-    int splits = std::max(1, (4 * sms + tiles - 1) / tiles);
-    int slice = (N + splits - 1) / splits;
-    slice = std::max(1024, (slice + 1023) & ~1023);
-    splits = (N + slice - 1) / slice;
-    if (tiled)
-        nn_tiled_kernel<kQT><<<dim3(splits, tiles), 256, 0, st>>>(tree, dim, N, tree_size, q, batch, slice, keys);
-    else
-        nn_kernel<<<dim3(splits, batch), 256, 0, st>>>(tree, dim, N, tree_size, q, batch, slice, keys);
+    const bool vec = (N & 3) == 0 && (reinterpret_cast<uintptr_t>(tree) & 15) == 0;
+    // columns of 1024 nodes; a small tree is spread by giving each CTA fewer queries
+    const int columns = (int)(((long long)N + 1023) / 1024);
+    const int per_cta = (int)std::min<long long>(kNnQueries, std::max<long long>(4, (long long)batch * columns / (3 * sms)));
+    const int tiles = (batch + per_cta - 1) / per_cta;
+    const dim3 grid((unsigned)std::max(1, std::min(columns, (3 * sms + tiles - 1) / tiles)), (unsigned)tiles);
+    const int db = (dim + 3) / 4;
+    if (tiles > 65535) return cudaErrorInvalidConfiguration;
+#define PRRTC_NN_SCAN(DB)                                                                                            \
+    if (vec) nn_scan_kernel<DB, true><<<grid, 256, 0, st>>>(tree, dim, N, tree_size, size, q, batch, per_cta, keys); \
+    else nn_scan_kernel<DB, false><<<grid, 256, 0, st>>>(tree, dim, N, tree_size, size, q, batch, per_cta, keys)
+    if (db <= 1) { PRRTC_NN_SCAN(1); }
+    else if (db == 2) { PRRTC_NN_SCAN(2); }
+    else if (db == 3) { PRRTC_NN_SCAN(3); }
+    else { PRRTC_NN_SCAN(4); }
+#undef PRRTC_NN_SCAN
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     nn_decode_kernel<<<(batch + 255) / 256, 256, 0, st>>>(keys, batch, idx, dist);
     return cudaGetLastError();

@@ -843,12 +843,12 @@ def prrtc_nearest_neighbor(tree_configs, query_configs, tree_size):
     dim, N = int(tree.shape[0]), int(tree.shape[1])
     q = q.reshape(-1, dim)
     B = int(q.shape[0])
-    ts = as_tensor(np.array([int(tree_size)], dtype=np.int32), torch.int32, dev)
+    size = np.array(int(tree_size), dtype=np.int32).item()
     idx = torch.empty((B,), dtype=torch.int32, device=dev)
     dist = torch.empty((B,), dtype=torch.float32, device=dev)
     ws = workspace(lib.prrtc_b200_nearest_neighbor_workspace_size(B), dev)
-    _lib.check(lib.prrtc_b200_nearest_neighbor(ptr(tree), dim, N, ptr(ts), ptr(q), B, ptr(idx), ptr(dist),
-                                               ws.data_ptr(), ws.numel(), stream_handle()),
+    _lib.check(lib.prrtc_b200_nearest_neighbor_sized(ptr(tree), dim, N, size, ptr(q), B, ptr(idx), ptr(dist),
+                                                     ws.data_ptr(), ws.numel(), stream_handle()),
                "prrtc_b200_nearest_neighbor")
     return dist, idx
 
