@@ -13,7 +13,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .device import DeviceContext, as_tensor, cuda_device, ptr, stream_handle, workspace
+from .device import DeviceContext, Stager, as_tensor, cuda_device, ptr, stream_handle, workspace
 from .prrtc import _resolve_collision_mode
 
 
@@ -77,7 +77,12 @@ def forward_kinematics(configs, collision_context: dict, device=None) -> torch.T
     """Link frames [n, n_joints, 12] (row-major R, then t) in output frame order."""
     lib = _lib.load()
     dev = cuda_device(device)
-    ctx = DeviceContext(collision_context, dev, world_keys=False)
+    # one copy for the robot's tables; this call's kernel alone reads them, on
+    # this stream, so the host does not wait for it
+    stage = Stager(dev)
+    ctx = DeviceContext(collision_context, dev, world_keys=False, stager=stage)
+    stage.commit(wait=dev.index != torch.cuda.current_device())
+    ctx.finish()
     cf = as_tensor(configs, torch.float32, dev)
     dim = int(cf.shape[-1])
     cf = cf.reshape(-1, dim)

@@ -43,7 +43,8 @@ def cuda_device(device=None) -> torch.device:
     d = torch.device(device)
     if d.type != "cuda":
         raise ValueError(f"prrtc_b200 runs on CUDA devices only, got {d}")
-    return d
+    # with its index, as tensors carry it: a tensor already there compares equal
+    return torch.device("cuda", torch.cuda.current_device()) if d.index is None else d
 
 
 # host->device bytes copied by this module (as_tensor of host data, upload);
@@ -79,6 +80,7 @@ def upload(arrays, device: torch.device) -> list[torch.Tensor]:
 _TORCH_DTYPE = {"f4": torch.float32, "i4": torch.int32, "u1": torch.uint8, "i8": torch.int64, "f8": torch.float64}
 _NUMPY_DTYPE = {torch.float32: np.float32, torch.int32: np.int32, torch.uint8: np.uint8, torch.int64: np.int64,
                 torch.float64: np.float64}
+_PAD = bytes(255)
 
 
 class Stager:
@@ -88,27 +90,33 @@ class Stager:
     a tensor already on the device passes through without a copy.
     ``reserve`` sets aside a region that ``on_fill`` callbacks write straight
     into the pinned buffer.  After ``commit`` (one host->device copy),
-    ``get(key)`` is the device tensor."""
+    ``get(key)`` is the device tensor and ``address(key)`` where it lies.
+
+    A call has some 25 small tables, so the cost is per table: their bytes are
+    joined in one go, and a tensor is made only for a key that ``get`` asks for
+    (two views each, 4-5 us)."""
 
     def __init__(self, device: torch.device):
         self.device = device
         self._host: list = []  # np.ndarray, or (nbytes, torch dtype, shape) for a reserved region
         self._fill: list = []
         self._offsets: list[int] = []
-        self._dev: list[torch.Tensor] | None = None
+        self._dev: torch.Tensor | None = None
 
     def add(self, x, dtype: torch.dtype, shape=None):
-        if isinstance(x, torch.Tensor) and x.device == self.device:
-            t = x.to(dtype=dtype)
-            return ("t", (t.reshape(shape) if shape is not None else t).contiguous())
-        a = np.asarray(x.cpu() if isinstance(x, torch.Tensor) else x, dtype=_NUMPY_DTYPE[dtype])
+        if isinstance(x, torch.Tensor):
+            if x.device == self.device:
+                t = x.to(dtype=dtype)
+                return ("t", (t.reshape(shape) if shape is not None else t).contiguous())
+            x = x.detach().to(dtype).cpu().numpy()
+        a = np.asarray(x, dtype=_NUMPY_DTYPE[dtype])
         if shape is not None:
             a = a.reshape(shape)
         self._host.append(np.ascontiguousarray(a))
         return ("h", len(self._host) - 1)
 
     def reserve(self, dtype: torch.dtype, shape):
-        n = int(np.prod(shape)) * torch.empty((), dtype=dtype).element_size()
+        n = int(np.prod(shape)) * dtype.itemsize
         self._host.append((n, dtype, tuple(shape)))
         return ("h", len(self._host) - 1)
 
@@ -116,18 +124,28 @@ class Stager:
         """fn(host_bytes: np.ndarray[uint8], offset_of: callable(key) -> int)."""
         self._fill.append(fn)
 
-    def commit(self) -> None:
-        offs, total = [], 0
+    def commit(self, wait: bool = False) -> None:
+        """Queue the copy on the current stream; ``wait``: until it has run, for
+        tables that a later call may read on any stream."""
+        if not self._host:
+            return
+        offs, total, joined = [], 0, []
         for a in self._host:
             offs.append(total)
             n = a.nbytes if isinstance(a, np.ndarray) else a[0]
-            total += (n + 255) & ~255
+            joined += (a, _PAD[:-n & 255])
+            total += n + (-n & 255)
+        reserved = any(not isinstance(a, np.ndarray) for a in self._host)
         total = max(total, 256)
         host = torch.empty(total, dtype=torch.uint8, pin_memory=True)
         hv = host.numpy()
-        for a, o in zip(self._host, offs):
-            if isinstance(a, np.ndarray):
-                hv[o:o + a.nbytes] = a.reshape(-1).view(np.uint8)
+        if reserved:
+            for a, o in zip(self._host, offs):
+                if isinstance(a, np.ndarray):
+                    hv[o:o + a.nbytes] = a.reshape(-1).view(np.uint8)
+        elif joined:
+            raw = b"".join(joined)
+            hv[:len(raw)] = np.frombuffer(raw, np.uint8)
         self._offsets = offs
         for fn in self._fill:
             fn(hv, lambda key: offs[key[1]])
@@ -136,17 +154,33 @@ class Stager:
         # torch's caching host allocator records the copy on the stream and keeps
         # the pinned block out of reuse until that copy has run
         dev.copy_(host, non_blocking=True)
-        out = []
-        for a, o in zip(self._host, offs):
-            if isinstance(a, np.ndarray):
-                out.append(dev[o:o + a.nbytes].view(_TORCH_DTYPE[a.dtype.str[1:]]).reshape(a.shape))
-            else:
-                out.append(dev[o:o + a[0]].view(a[1]).reshape(a[2]))
-        self._dev = out
+        if wait:
+            torch.cuda.current_stream(self.device).synchronize()
+        self._host = [(a.nbytes, _TORCH_DTYPE[a.dtype.str[1:]], a.shape) if isinstance(a, np.ndarray) else a
+                      for a in self._host]
+        self._dev, self._base = dev, dev.data_ptr()
+
+    def shape(self, key) -> tuple:
+        kind, v = key
+        if kind == "t":
+            return tuple(v.shape)
+        a = self._host[v]
+        return a.shape if isinstance(a, np.ndarray) else a[2]
+
+    def address(self, key) -> int | None:
+        """Device address of a key's data, None when it is empty."""
+        kind, v = key
+        if kind == "t":
+            return ptr(v)
+        return self._base + self._offsets[v] if self._host[v][0] else None
 
     def get(self, key) -> torch.Tensor:
         kind, v = key
-        return v if kind == "t" else self._dev[v]
+        if kind == "t":
+            return v
+        n, dtype, shape = self._host[v]
+        o = self._offsets[v]
+        return self._dev[o:o + n].view(dtype).reshape(shape)
 
 
 def ptr(t: torch.Tensor | None) -> int | None:
@@ -164,41 +198,47 @@ class DeviceContext:
     """collision_context tensors on one CUDA device."""
 
     def __init__(self, ctx: dict | None, device: torch.device, world_keys: bool = True, stager: Stager | None = None):
-        """With a ``stager``, host tables are queued on it and the tensors exist
-        after ``finish()`` (called once the stager has committed)."""
+        """With a ``stager``, host tables are queued on it and exist after
+        ``finish()`` (called once the stager has committed); otherwise they are
+        on the device when this returns, whatever stream reads them."""
         self.device = device
-        self.t: dict[str, torch.Tensor] = {}
+        self._stager = Stager(device) if stager is None else stager
         self._keys: dict = {}
-        spec = dict(ROBOT_SPEC)
+        self._spec = dict(ROBOT_SPEC)
         if world_keys:
-            spec.update(WORLD_SPEC)
-        for k, (dt, cols) in spec.items():
-            if ctx is not None and k in ctx and ctx[k] is not None:
-                if stager is not None:
-                    self._keys[k] = stager.add(ctx[k], dt, (-1, cols) if cols else (-1,))
-                else:
-                    self.t[k] = as_tensor(ctx[k], dt, device, cols)
-            else:
-                self.t[k] = torch.zeros((0, cols) if cols else (0,), dtype=dt, device=device)
-        self._stager = stager
+            self._spec.update(WORLD_SPEC)
+        for k, (dt, cols) in self._spec.items():
+            x = None if ctx is None else ctx.get(k)
+            if x is not None:
+                self._keys[k] = self._stager.add(x, dt, (-1, cols) if cols else (-1,))
+        self._addr: dict = {}
+        self._rows: dict = {}
+        if stager is None:
+            self._stager.commit(wait=True)
+            self.finish()
 
     def finish(self) -> "DeviceContext":
         for k, key in self._keys.items():
-            self.t[k] = self._stager.get(key)
-        self._keys, self._stager = {}, None
+            self._addr[k], self._rows[k] = self._stager.address(key), int(self._stager.shape(key)[0])
         return self
 
+    @property
+    def t(self) -> dict[str, torch.Tensor]:
+        """Every table as a tensor (absent: no rows)."""
+        return {k: self._stager.get(self._keys[k]) if k in self._keys
+                else torch.zeros((0, cols) if cols else (0,), dtype=dt, device=self.device)
+                for k, (dt, cols) in self._spec.items()}
+
     def n(self, key: str) -> int:
-        return int(self.t[key].shape[0])
+        return self._rows.get(key, 0)
 
     def robot(self) -> _lib.Robot:
-        t = self.t
         r = _lib.Robot()
         for k in ("fk_twists", "fk_parent_tf", "fk_parent_idx", "fk_act_idx", "fk_mimic_mul", "fk_mimic_off",
                   "fk_mimic_act_idx", "fk_topo_inv", "sphere_link_idx", "sphere_local", "sphere_radius",
                   "coarse_sphere_link_idx", "coarse_sphere_local", "coarse_sphere_radius", "fine_link_offsets",
                   "coarse_self_pairs", "self_pair_ranges"):
-            setattr(r, k, ptr(t[k]))
+            setattr(r, k, self._addr.get(k))
         r.n_joints = self.n("fk_parent_idx")
         r.n_spheres = self.n("sphere_link_idx")
         nk = self.n("coarse_sphere_link_idx")
@@ -208,10 +248,9 @@ class DeviceContext:
         return r
 
     def world(self) -> _lib.World:
-        t = self.t
         w = _lib.World()
         for k in ("world_spheres", "world_capsules", "world_boxes", "world_halfspaces", "self_pairs"):
-            setattr(w, k, ptr(t[k]))
+            setattr(w, k, self._addr.get(k))
         w.n_world_spheres = self.n("world_spheres")
         w.n_world_capsules = self.n("world_capsules")
         w.n_world_boxes = self.n("world_boxes")

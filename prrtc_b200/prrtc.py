@@ -398,11 +398,10 @@ def prrtc_plan(
     ctx = DeviceContext(collision_context, dev, stager=stage)
     stage.commit()
     ctx.finish()
-    start, goals, lo, hi = (stage.get(k) for k in (k_start, k_goals, k_lo, k_hi))
-
     inp = _lib.Inputs()
-    inp.start_config, inp.goal_configs, inp.num_goals = start.data_ptr(), goals.data_ptr(), goals.shape[0]
-    inp.min_vals, inp.max_vals = lo.data_ptr(), hi.data_ptr()
+    inp.start_config, inp.goal_configs = stage.address(k_start), stage.address(k_goals)
+    inp.num_goals = stage.shape(k_goals)[0]
+    inp.min_vals, inp.max_vals = stage.address(k_lo), stage.address(k_hi)
     inp.robot, inp.world = ctx.robot(), ctx.world()
     attrs = _attrs(max_iterations, step_size, num_new_samples, balance_mode, tree_ratio, dynamic_domain, dd_alpha,
                    dd_radius, dd_min_radius, dim, max_nodes, granularity, collision_mode, collision_margin)
@@ -716,9 +715,9 @@ def prrtc_plan_batch_async(
     bi.robot = robot_ctx.robot()
     if world_keys:
         for key, (k_tab, k_cnt, width) in world_keys.items():
-            setattr(bi, key, ptr(stage.get(k_tab)))
+            setattr(bi, key, stage.address(k_tab))
             setattr(bi, "max_" + key, width)
-            setattr(bi, key + "_count", ptr(stage.get(k_cnt)) if k_cnt is not None else None)
+            setattr(bi, key + "_count", stage.address(k_cnt) if k_cnt is not None else None)
     elif first is not None:
         w = robot_ctx.world()
         bi.world_spheres, bi.max_world_spheres = w.world_spheres, w.n_world_spheres

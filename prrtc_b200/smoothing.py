@@ -107,6 +107,45 @@ def resample_path(path: np.ndarray, W: int) -> np.ndarray:
     return out.astype(np.float32)
 
 
+def _spread(paths: list, W: int) -> np.ndarray:
+    """resample_path of finite float64 paths of 2..W vertices, all at once:
+    [P, W, dim], the same bits (32 paths to 64 points: 2.3 -> 0.3 ms against a
+    path and a segment at a time)."""
+    P, L = len(paths), np.fromiter((p.shape[0] for p in paths), np.int64, len(paths))
+    v = np.concatenate(paths, 0)
+    first = np.cumsum(L) - L                                     # row of each path's first vertex
+    path_of = np.repeat(np.arange(P), L - 1)                     # of each segment
+    a = np.arange(path_of.size) + path_of                        # its first vertex's row
+    d = v[a + 1] - v[a]
+    seg = np.linalg.norm(d, axis=1)
+    total = np.array([seg[f:f + n].sum() for f, n in zip(first - np.arange(P), L - 1)])
+    extra = (W - L)[path_of]
+    with np.errstate(invalid="ignore"):  # 0 / 0 of a path without length
+        share = np.where(total[path_of] > 0, seg / total[path_of] * extra, extra / (L - 1)[path_of])
+    n = np.floor(share).astype(np.int64)
+    # the points left over go to the largest remainders of each path, the first of equal ones first
+    rest = W - L - np.bincount(path_of, weights=n, minlength=P).astype(np.int64)
+    order = np.lexsort((n - share, path_of))
+    rank = np.arange(path_of.size) - (first - np.arange(P))[path_of]
+    n[order[rank < rest[path_of]]] += 1
+    cnt = n + 1
+    at = np.repeat(np.arange(path_of.size), cnt)                 # the segment of each point
+    k = np.arange(at.size) - (np.cumsum(cnt) - cnt)[at]
+    pts = v[a[at]] + (k / cnt[at])[:, None] * d[at]
+    out = np.empty((P, W, v.shape[1]), np.float32)
+    out[:, :-1] = pts.reshape(P, W - 1, -1)
+    out[:, -1] = v[first + L - 1]
+    return out
+
+
+def _resample_paths(paths: list, W: int) -> np.ndarray:
+    """resample_path of every path: [P, W, dim]."""
+    paths = [np.asarray(p, dtype=np.float64) for p in paths]
+    if all(p.ndim == 2 and 1 < p.shape[0] <= W and p.shape[1] == paths[0].shape[1] and np.isfinite(p).all() for p in paths):
+        return _spread(paths, W)
+    return np.stack([resample_path(p, W) for p in paths])
+
+
 def densify(paths: torch.Tensor, resolution: float) -> tuple[torch.Tensor, torch.Tensor]:
     """Points every <= `resolution` (joint-space L2) along each polyline [P, W, dim];
     returns configs [M, dim] and the path index of each point."""
@@ -140,7 +179,7 @@ def smooth_paths(paths: list, collision_context: dict, lower, upper, *, waypoint
     cost before [P], cost after [P])."""
     dev = cuda_device(device)
     dim = int(np.asarray(paths[0]).shape[1])
-    init = torch.from_numpy(np.stack([resample_path(p, waypoints) for p in paths])).to(dev)
+    init = torch.from_numpy(_resample_paths(paths, waypoints)).to(dev)
     lo = as_tensor(lower, torch.float32, dev).reshape(1, 1, dim)
     hi = as_tensor(upper, torch.float32, dev).reshape(1, 1, dim)
     sctx = SmoothContext(collision_context, dim, margin, beta, w_len, dev)
@@ -169,7 +208,7 @@ class _BatchScenes:
     copy, as the C struct of the batched entry points."""
 
     def __init__(self, collision_contexts, device: torch.device):
-        from .prrtc import _pack_worlds
+        from .prrtc import _native_pack, _pack_worlds
 
         ctxs = list(collision_contexts)
         B = self.B = len(ctxs)
@@ -179,21 +218,23 @@ class _BatchScenes:
                              for c in ctxs)
         stage = Stager(device)
         self.robot_ctx = DeviceContext(ctxs[0], device, world_keys=False, stager=stage)
-        packed, counts = _pack_worlds(ctxs, B)
-        keys = {k: (stage.add(packed[k], torch.int32 if k == "self_pairs" else torch.float32),
-                    stage.add(counts[k], torch.int32)) for k in packed}
+        native = _native_pack(ctxs, stage)
+        if native is not None:
+            keys = native[0]
+        else:
+            packed, counts = _pack_worlds(ctxs, B)
+            keys = {k: (stage.add(packed[k], torch.int32 if k == "self_pairs" else torch.float32),
+                        stage.add(counts[k], torch.int32), int(packed[k].shape[1])) for k in packed}
         stage.commit()
         self.robot_ctx.finish()
-        self.t = {}
+        self.stage = stage  # holds the tables
         bi = _lib.BatchInputs()
         bi.batch = B
         bi.robot = self.robot_ctx.robot()
-        for key, (k_tab, k_cnt) in keys.items():
-            tab, cnt = stage.get(k_tab), stage.get(k_cnt)
-            self.t[key], self.t[key + "_count"] = tab, cnt
-            setattr(bi, key, ptr(tab))
-            setattr(bi, "max_" + key, int(tab.shape[1]))
-            setattr(bi, key + "_count", cnt.data_ptr())
+        for key, (k_tab, k_cnt, width) in keys.items():
+            setattr(bi, key, stage.address(k_tab))
+            setattr(bi, "max_" + key, width)
+            setattr(bi, key + "_count", stage.address(k_cnt) if k_cnt is not None else None)
         self.bi = bi
 
 
@@ -279,7 +320,7 @@ def smooth_paths_batch(paths: list, collision_contexts: list, lower, upper, *, w
     cost after [P])."""
     dev = cuda_device(device)
     dim = int(np.asarray(paths[0]).shape[1])
-    init = torch.from_numpy(np.stack([resample_path(p, waypoints) for p in paths])).to(dev)
+    init = torch.from_numpy(_resample_paths(paths, waypoints)).to(dev)
     sctx = BatchSmoothContext(collision_contexts, dim, margin, beta, w_len, dev)
     c0, _ = sctx.cost_grad(init, need_grad=False)
     x = projected_steps(sctx, init, lower, upper, steps, lr)
