@@ -626,9 +626,10 @@ cudaError_t launch_check_batch(const unsigned char* blobs, size_t blob_stride, c
 // k = sorted joint topo_inv[k]).  Shared-memory rows are one 16-byte vector longer
 // than J frames, which spreads a warp's configurations over the banks.
 //
-// Bound by memory: 48 B written per frame.  65,537 configurations x 18 joints
-// (56.6 MB): 130 -> 31 us (1.8 TB/s: shared-memory traffic and the chain of joints hold it there) against a configuration per thread with its
-// frames in local memory and 48 B stores 864 B apart.
+// Bound by shared-memory traffic and the chain of joints (48 B written per frame
+// leave at 1.8 TB/s).  65,537 configurations x 18 joints (56.6 MB): 130 -> 31 us
+// against a configuration per thread with its frames in local memory and 48 B
+// stores 864 B apart; tiles of 20, or 256 threads, measured 33 and 37 us.
 constexpr int kFkTile = 40, kFkThreads = 128;  // 10 configurations x 3 rows per warp
 
 __host__ __device__ inline int fk_smem_bytes(int J) { return J * (int)sizeof(JointRec) + kFkTile * (J * 12 + 4) * 4 + J * 4; }

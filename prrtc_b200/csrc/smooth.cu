@@ -67,9 +67,12 @@ struct SmoothArgs {
     float* grad;
 };
 
-// per-warp shared memory: pose J*12, ctr S*4, g S*4, acc J*8, dv J, q dim (padded)
+constexpr int kStageRow = 36;  // a value per lane and a 16-byte step, for the banks
+constexpr int kStage = 6 * kStageRow + 32;
+
+// per-warp shared memory: pose J*12, ctr S*4, g S*4, acc J*8, stage, dv J, q dim (padded)
 __host__ __device__ inline int smooth_warp_floats(int J, int S) {
-    return (J * 12 + S * 4 + S * 4 + J * 8 + J + kDimMax + 3) & ~3;  // keep every warp slice 16-byte aligned
+    return (J * 12 + S * 4 + S * 4 + J * 8 + kStage + J + kDimMax + 3) & ~3;  // keep every warp slice 16-byte aligned
 }
 
 // Accumulate the cost term of a pair at distance d.  sig = sigmoid(beta
@@ -90,36 +93,55 @@ __device__ __forceinline__ void norm_rnorm(float d2, float& n, float& rn) {
     n = d2 * rn;
 }
 
-// v added to the floats at base[0 .. N) of each lane that is `on`; lanes of one
-// key share their base and add one after the other in lane order, so the sums
-// are the same bits in every run (shared-memory float atomics add in that order
-// too, but by compare-and-swap rounds that cost several times as much).
+// v of each lane of `on` added to the floats at base[key * stride + 0 .. N), lanes
+// of one key in lane order, so the sums are the same bits in every run and launch.
+// `heads` starts the runs of lanes of one key (lane 0 is one); `apart`: no two
+// runs have the same key, so a lane per run and component may add its run's values,
+// else the runs follow one another.  `stage`: N rows of kStageRow floats and a row
+// of 32 masks.  A chain of some 8 cycles per value from shared memory; shared-memory
+// float atomics take the same order, but by compare-and-swap rounds, and a search
+// for equal keys by __match_any_sync costs a pass per key.
 template <int N>
-__device__ __forceinline__ void add_in_lane_order(bool on, int key, float* base, const float (&v)[N]) {
+__device__ __forceinline__ void add_runs(unsigned on, unsigned heads, bool apart, int key, float* base, int stride,
+                                         const float (&v)[N], float* stage) {
     constexpr unsigned kAll = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    unsigned rest = __match_any_sync(kAll, on ? key : -1 - lane);
-    const bool leads = on && __ffs(rest) - 1 == lane;
-    if (!on) rest = 0u;
-    float sum[N];
-    if (leads) {
+    constexpr int kRuns = 32 / N;
+    const int lane = threadIdx.x & 31, runs = __popc(heads), nth = lane / N, c = lane - nth * N;
+    unsigned* masks = reinterpret_cast<unsigned*>(stage + N * kStageRow);
 #pragma unroll
-        for (int i = 0; i < N; ++i) sum[i] = base[i];
-    }
-    while (__any_sync(kAll, leads && rest != 0u)) {
-        const int src = rest ? __ffs(rest) - 1 : lane;
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-            const float x = __shfl_sync(kAll, v[i], src);
-            if (leads && rest) sum[i] += x;
-        }
-        rest &= rest - 1u;
-    }
-    if (leads) {
-#pragma unroll
-        for (int i = 0; i < N; ++i) base[i] = sum[i];
+    for (int i = 0; i < N; ++i) stage[i * kStageRow + lane] = v[i];
+    if (heads >> lane & 1u) {  // the lanes of the run that starts here
+        const unsigned above = heads & (kAll - 1u << lane), next = above & (0u - above);
+        masks[__popc(heads & ((1u << lane) - 1u))] = (next - 1u) & (kAll << lane) & on;
     }
     __syncwarp();
+    const int step = apart ? kRuns : 1;
+    for (int r0 = 0; r0 < runs; r0 += step) {
+        const int r = r0 + nth;
+        const unsigned mine = nth < step && r < runs ? masks[r] : 0u;
+        float* b = base + __shfl_sync(kAll, key, mine ? __ffs(mine) - 1 : 0) * stride + c;
+        if (mine) {
+            const float* row = stage + c * kStageRow;
+            int i = (__ffs(mine) - 1) & ~3;
+            const int end = 32 - __clz(mine);
+            float sum = *b;
+            do {  // 8 lanes of the run at a time
+                const float4 t = *reinterpret_cast<const float4*>(row + i), u = *reinterpret_cast<const float4*>(row + i + 4);
+                const unsigned m = mine >> i;
+                if (m & 1u) sum += t.x;
+                if (m & 2u) sum += t.y;
+                if (m & 4u) sum += t.z;
+                if (m & 8u) sum += t.w;
+                if (m & 16u) sum += u.x;
+                if (m & 32u) sum += u.y;
+                if (m & 64u) sum += u.z;
+                if (m & 128u) sum += u.w;
+                i += 8;
+            } while (i < end);
+            *b = sum;
+        }
+        __syncwarp();
+    }
 }
 
 // A warp per waypoint, WARPS waypoints of one path per CTA, the scene staged in
@@ -129,10 +151,13 @@ __device__ __forceinline__ void add_in_lane_order(bool on, int key, float* base,
 // another order move single paths by 1e-3 within 50 steps.
 //
 // Bound by the latency of its dependent chains (a waypoint's 4,376 pairs in one
-// warp).  32 paths x 64 waypoints in tabletop worlds of their own: 119 -> 76 us
-// for the gradient alone, from ordered warp sums in the place of shared-memory
-// atomics, three lanes in the place of one for the frames' chain, and the scene
-// in shared memory; the bits are those of the atomics.
+// warp; at 32 paths 3.5 warps per scheduler issue 55% of the time).  32 paths x 64
+// waypoints in tabletop worlds of their own: 119 -> 57 us for the gradient alone,
+// from ordered sums over runs of pairs in the place of shared-memory atomics, the
+// next pairs fetched ahead of the sums, three lanes in the place of one for the
+// frames' chain, and the scene in shared memory; the bits are those of the
+// atomics.  Two spheres per lane for each primitive, in the place of two passes
+// over them, measured the same at 32 paths and 4% slower at 128.
 // COST false: the gradient alone, zero at a path's end points (a descent step).
 template <int WARPS, bool STAGED, bool COST>
 __global__ void __launch_bounds__(WARPS * 32) smooth_kernel(SmoothArgs a, int blob_cap, int per_path) {
@@ -182,7 +207,8 @@ __global__ void __launch_bounds__(WARPS * 32) smooth_kernel(SmoothArgs a, int bl
     float4* ctr = reinterpret_cast<float4*>(pose + J * 12);
     float4* g = ctr + S;
     float* acc = reinterpret_cast<float*>(g + S);  // [J][8]: G xyz, M xyz
-    float* dv = acc + J * 8;
+    float* stage = acc + J * 8;  // add_runs' rows
+    float* dv = stage + kStage;
     float* q = dv + J;
     const float* qw = a.wp + ((size_t)p * a.W + w) * dim;
     if (lane < dim) q[lane] = qw[lane];
@@ -299,27 +325,49 @@ __global__ void __launch_bounds__(WARPS * 32) smooth_kernel(SmoothArgs a, int bl
         g[s] = make_float4(gx, gy, gz, 0.0f);
     }
     __syncwarp();
-    // 2b. self pairs (explicit list), 32 at a time, into both spheres
-    for (int k0 = 0; k0 < h.P; k0 += 32) {
-        const int k = k0 + lane;
-        bool on = k < h.P;
-        const int2 pr = on ? __ldg(&pairs[k]) : make_int2(-1, -1);
-        on = on && pr.x >= 0 && pr.y >= 0 && pr.x < S && pr.y < S && sc.sfr[pr.x] >= 0 && sc.sfr[pr.y] >= 0;
-        float v[3] = {0.0f, 0.0f, 0.0f};
-        if (on) {
-            const float4 ci = ctr[pr.x], cj = ctr[pr.y];
-            const float dx = ci.x - cj.x, dy = ci.y - cj.y, dz = ci.z - cj.z;
-            float n, rn, sig;
-            norm_rnorm(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), n, rn);
-            pair_term<COST>(n - ci.w - cj.w, a.margin, a.beta, inv_beta, cost, sig);
-            on = sig != 0.0f;  // else nothing to add
-            const float kk = -sig * rn;
-            v[0] = kk * dx; v[1] = kk * dy; v[2] = kk * dz;
+    // 2b. self pairs (explicit list), 32 at a time, into both spheres; the terms of
+    // two lots and the pairs of the next two are on their way while sums are taken
+    auto pair_at = [&](int k) { return k < h.P ? __ldg(&pairs[k]) : make_int2(-1, -1); };
+    auto self_term = [&](int2 pr, float (&v)[3]) {
+        v[0] = v[1] = v[2] = 0.0f;
+        if (!(pr.x >= 0 && pr.y >= 0 && pr.x < S && pr.y < S && sc.sfr[pr.x] >= 0 && sc.sfr[pr.y] >= 0)) return false;
+        const float4 ci = ctr[pr.x], cj = ctr[pr.y];
+        const float dx = ci.x - cj.x, dy = ci.y - cj.y, dz = ci.z - cj.z;
+        float n, rn, sig;
+        norm_rnorm(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), n, rn);
+        pair_term<COST>(n - ci.w - cj.w, a.margin, a.beta, inv_beta, cost, sig);
+        const float kk = -sig * rn;
+        v[0] = kk * dx; v[1] = kk * dy; v[2] = kk * dz;
+        return sig != 0.0f;  // else nothing to add
+    };
+    auto self_sum = [&](int k, int2 pr, bool on, const float (&v)[3]) {
+        const unsigned live = __ballot_sync(0xffffffffu, on);
+        if (!live) return;
+        // runs of pairs with one first sphere and rising second ones: in a run the
+        // second spheres are all different
+        const int px = __shfl_up_sync(0xffffffffu, pr.x, 1), py = __shfl_up_sync(0xffffffffu, pr.y, 1);
+        const bool head = lane == 0 || pr.x != px || pr.y <= py;
+        const unsigned heads = __ballot_sync(0xffffffffu, head);
+        const bool apart = __all_sync(0xffffffffu, lane == 0 || !head || pr.x > px || k >= h.P);
+        add_runs<3>(live, heads, apart, pr.x, reinterpret_cast<float*>(g), 4, v, stage);
+        const int run = __popc(heads & (0xffffffffu >> (31 - lane)));
+        for (int r = 1; r <= __popc(heads); ++r) {
+            if (on && run == r) {
+                float4* t = &g[pr.y];
+                t->x -= v[0]; t->y -= v[1]; t->z -= v[2];
+            }
+            __syncwarp();
         }
-        if (!__any_sync(0xffffffffu, on)) continue;
-        add_in_lane_order<3>(on, pr.x, reinterpret_cast<float*>(&g[max(pr.x, 0)]), v);
-        const float m[3] = {-v[0], -v[1], -v[2]};
-        add_in_lane_order<3>(on, pr.y, reinterpret_cast<float*>(&g[max(pr.y, 0)]), m);
+    };
+    int2 pr0 = pair_at(lane), pr1 = pair_at(32 + lane);
+    for (int k0 = 0; k0 < h.P; k0 += 64) {
+        const int2 next0 = pair_at(k0 + 64 + lane), next1 = pair_at(k0 + 96 + lane);
+        float v0[3], v1[3];
+        const bool on0 = self_term(pr0, v0), on1 = self_term(pr1, v1);
+        self_sum(k0 + lane, pr0, on0, v0);
+        self_sum(k0 + 32 + lane, pr1, on1, v1);
+        pr0 = next0;
+        pr1 = next1;
     }
     __syncwarp();
     // 3. frame sums
@@ -328,7 +376,10 @@ __global__ void __launch_bounds__(WARPS * 32) smooth_kernel(SmoothArgs a, int bl
         const float4 cs = ctr[s], gs = g[s];
         const float v[6] = {gs.x, gs.y, gs.z, cs.y * gs.z - cs.z * gs.y, cs.z * gs.x - cs.x * gs.z,
                             cs.x * gs.y - cs.y * gs.x};
-        add_in_lane_order<6>(s0 + lane < S && f >= 0, f, &acc[max(f, 0) * 8], v);
+const int fp = __shfl_up_sync(0xffffffffu, f, 1);
+        const bool head = lane == 0 || f != fp;
+        add_runs<6>(__ballot_sync(0xffffffffu, s0 + lane < S && f >= 0), __ballot_sync(0xffffffffu, head),
+                    __all_sync(0xffffffffu, !head || lane == 0 || f > fp), f, acc, 8, v, stage);
     }
     // 4. reverse sweep: subtree sums a component per lane, then a joint per lane
     if (lane < 6) {
