@@ -59,8 +59,8 @@ __device__ __forceinline__ float2 square_add2(float2 d, float2 acc) {
 template <int DB, bool VEC>
 __global__ void __launch_bounds__(256, DB <= 2 ? 3 : 2) nn_scan_kernel(const float* __restrict__ tree, int dim, int N,
                                                                       const int32_t* tree_size, int size,
-                                                                      const float* __restrict__ q, int batch, int per_cta,
-                                                                      unsigned long long* keys) {
+                                                                      int limit, const float* __restrict__ q, int batch,
+                                                                      int per_cta, unsigned long long* keys) {
     __shared__ __align__(16) float2 nq[kNnQueries][DB * 4];  // (-q, -q)
     __shared__ unsigned long long s_key[kNnQueries];
     constexpr int T = 256;
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(256, DB <= 2 ? 3 : 2) nn_scan_kernel(const flo
     if (tid < kNnQueries) s_key[tid] = kNnNone;
     __syncthreads();
     int n = tree_size ? tree_size[0] : size;
-    n = max(1, min(n, N));
+    n = min(max(1, min(n, N)), limit);
     volatile const unsigned* bound = reinterpret_cast<volatile const unsigned*>(s_key);  // high words: odd
     for (long long base = (long long)blockIdx.x * T * 4; base < n; base += (long long)gridDim.x * T * 4) {
         const int i0 = (int)base + (VEC ? 4 * tid : tid);
@@ -136,6 +136,238 @@ __global__ void __launch_bounds__(256, DB <= 2 ? 3 : 2) nn_scan_kernel(const flo
     }
 }
 
+// Batches on large trees: the tensor cores rule nodes out, the rest is computed as
+// above.  A dot product in tf32 gives (1 - c)|x|^2 - 2 x.q for 16 nodes and 8
+// queries per instruction (the norm from the squares against 1 - c); above
+// best (1 + 2^-16) - (1 - c)|q|^2, the node is farther than the best so far.  Rounding both factors to tf32 moves 2 x.q by at most 2^-10 (|x|^2 +
+// |q|^2) and the norm by 2^-11 |x|^2; sums in float32 (of at most 17 terms, in any
+// order and rounding) add 2^-17 (|x|^2 + |q|^2) + 2^-18 best; c = 2^-9 covers them, and 2^-16
+// the rounding of the exact sum.  Squares from 1e37 on, infinities and NaN count
+// as near.  So every node that could be nearest is computed exactly,
+// and the result is that of nn_scan_kernel bit for bit.
+//
+// A warp takes 32 nodes at a time, 4 neighbours per lane (one 16-byte load per
+// dimension and 128 bytes in a row per warp): the fragments' rows may be nodes in
+// any order.  The best distances start from a scan of the first kNnFirst nodes,
+// and are shared as above.
+//
+// Bound by the latency of its own chain (16 warps per SM issue half the time; the
+// tensor pipe is 25% busy, and the tree's 117 MB would take 18 us): 64 queries, 4.19
+// M nodes x 7: 146 -> 58 us for the call's kernels, 14 dimensions 244 -> 98. A step
+// of 32 nodes per warp took 65 us, the norm as one more dimension summed by
+// shuffles 65 us, sums started from the best distance 73 us.
+constexpr int kNnFirst = 8192;
+// The filter from 16 queries and 2^23 pairs on: 64 queries x 131,072 nodes 18.4
+// against 19.6 us by scan, 16 x 1 M 21.3 against 27.2, but 16 x 262,144 17.4 against
+// 15.4 (the first scan and one more launch), and below 16 queries the scan waits
+// for memory as the filter does.
+constexpr int kNnFilterBatch = 16;
+constexpr long long kNnFilterPairs = 1ll << 23;
+constexpr int kNnGroups = 2;  // groups of 32 nodes per warp and step, up to 8 dimensions
+constexpr float kNnSlack = 1.0f / 512;
+
+__device__ __forceinline__ float min_nan(float a, float b, float c) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ uint32_t to_tf32(float x) {
+    uint32_t r;
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+    return r;
+}
+// d = c + a (16 nodes x 8 KS) times b (8 KS x 8 queries).  volatile: the rare second
+// pass must compute its products again, not keep the first pass's in registers
+template <int KS>
+__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[KS][4], const uint32_t (&b)[KS][2],
+                                         const float (&c)[4]) {
+#pragma unroll
+    for (int k = 0; k < KS; ++k) {
+        const float* from = k ? d : c;
+        asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+                     "{%10, %11, %12, %13};"
+                     : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+                     : "r"(a[k][0]), "r"(a[k][1]), "r"(a[k][2]), "r"(a[k][3]), "r"(b[k][0]), "r"(b[k][1]), "f"(from[0]),
+                       "f"(from[1]), "f"(from[2]), "f"(from[3]));
+    }
+}
+
+struct NnShared {
+    float q[kNnQueries][17];            // the queries
+    float start[kNnQueries];            // (1 - c)|q|^2 - best (1 + 2^-16) - 1e-36
+    float qn[kNnQueries];               // (1 - c)|q|^2
+    unsigned long long key[kNnQueries]; // best so far
+};
+
+// The pairs of `bits` (4 i + 2 e + r: query + r, node + 32 (i / 2) + 2 (i % 2) + e) that
+// are not ruled out, exactly.
+static __device__ __noinline__ void nn_exact(NnShared& s, unsigned bits, const float* __restrict__ tree, int dim, int N, int n,
+                                             int node, int query, int nqs, unsigned long long* keys) {
+    for (; bits; bits &= bits - 1u) {
+        const int i = __ffs(bits) - 1, k = query + (i & 1), x = node + 32 * (i >> 3) + ((i >> 1) & 3);
+        if (k >= nqs || x >= n) continue;
+        float d2 = 0.0f;
+        for (int d0 = 0; d0 < dim; d0 += 8) {  // eight loads on their way together
+            float r[8];
+#pragma unroll
+            for (int d = 0; d < 8; ++d) r[d] = __ldg(tree + (size_t)min(d0 + d, dim - 1) * N + x);
+#pragma unroll
+            for (int d = 0; d < 8; ++d) {
+                const float d1 = __fadd_rn(r[d], -s.q[k][min(d0 + d, dim - 1)]);
+                if (d0 + d < dim) d2 = __fmaf_rn(d1, d1, d2);
+            }
+        }
+        const unsigned long long key = (unsigned long long)__float_as_uint(d2) << 32 | (unsigned)x;
+        if (d2 <= FLT_MAX && key < s.key[k] && atomicMin(&s.key[k], key) > key) {
+            atomicMin(&keys[k], key);
+            s.start[k] = s.qn[k] - __fmaf_ru(d2, 1.0f + 1.0f / 65536, 1e-36f);  // an older, larger best only rules out less
+        }
+    }
+}
+
+// KS steps of 8 dimensions, NT tiles of 8 queries, G groups of 32 nodes per warp and step.
+template <int KS, int NT, int G, bool VEC>
+__global__ void __launch_bounds__(256, 2) nn_filter_kernel(const float* __restrict__ tree, int dim, int N,
+                                                           const int32_t* tree_size, int size, const float* __restrict__ q,
+                                                           int batch, unsigned long long* keys) {
+    __shared__ __align__(16) NnShared s;
+    constexpr int T = 256, kCta = NT * 8;
+    const int tid = threadIdx.x, lane = tid & 31, c = lane & 3, g = lane >> 2;
+    const int q0 = blockIdx.y * kCta, nqs = min(kCta, batch - q0);
+    keys += q0;
+    if (tid < kCta) {
+        float norm = 0.0f;
+        for (int d = 0; d < dim; ++d) {
+            const float x = tid < nqs ? q[(size_t)(q0 + tid) * dim + d] : 0.0f;
+            s.q[tid][d] = x;
+            norm = fmaf(x, x, norm);
+        }
+        s.qn[tid] = tid >= nqs ? INFINITY : (norm < 1e37f ? (1.0f - kNnSlack) * norm : NAN);
+        s.key[tid] = tid < nqs ? min(kNnNone, __ldcg(&keys[tid])) : 0ull;
+        s.start[tid] = s.qn[tid] - __fmaf_ru(__uint_as_float((unsigned)(s.key[tid] >> 32)), 1.0f + 1.0f / 65536, 1e-36f);
+    }
+    __syncthreads();
+    uint32_t b[NT][KS][2];
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int slot = 8 * ks + 4 * h + c;
+                b[j][ks][h] = to_tf32(slot < dim ? -2.0f * s.q[8 * j + g][slot] : 0.0f);
+            }
+    int n = tree_size ? tree_size[0] : size;
+    n = max(1, min(n, N));
+    uint32_t ones[KS][2];  // the norm: the squares against 1 - c, for every query
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) ones[ks][0] = ones[ks][1] = to_tf32(1.0f - kNnSlack);
+    const long long stride = (long long)gridDim.x * T * G;
+    long long base = kNnFirst + ((long long)blockIdx.x * T + (tid & ~31)) * G;
+    float4 v[G][KS][2];
+    auto fetch = [&](long long from) {
+#pragma unroll
+        for (int f = 0; f < G; ++f)
+#pragma unroll
+            for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int d = 8 * ks + 4 * h + c;
+                    const long long i = from + 32 * f + 4 * g;
+                    float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (d < dim) {
+                        const float* row = tree + (size_t)d * N;
+                        if (VEC) {
+                            if (i < n) x = __ldg(reinterpret_cast<const float4*>(row + i));  // N % 4 == 0: inside the row
+                        } else {
+                            if (i < n) x.x = __ldg(row + i);
+                            if (i + 1 < n) x.y = __ldg(row + i + 1);
+                            if (i + 2 < n) x.z = __ldg(row + i + 2);
+                            if (i + 3 < n) x.w = __ldg(row + i + 3);
+                        }
+                    }
+                    v[f][ks][h] = x;
+                }
+    };
+    auto start = [&](int j) { return *reinterpret_cast<const volatile unsigned long long*>(&s.start[8 * j + 2 * c]); };
+    fetch(base);
+    for (; base < n; base += stride) {
+        unsigned long long seen = ~0ull;
+        if (tid < nqs) seen = __ldcg(&keys[tid]);
+        // tile 2 f + t: nodes 2 t, 2 t + 1 of each lane's four in group f
+        uint32_t a[2 * G][KS][4];
+        float norm[2 * G][4], top = 0.0f;
+#pragma unroll
+        for (int f = 0; f < G; ++f)
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                uint32_t sq[KS][4];
+#pragma unroll
+                for (int ks = 0; ks < KS; ++ks) {
+                    const float4 lo = v[f][ks][0], hi = v[f][ks][1];
+                    const float x[4] = {t ? lo.z : lo.x, t ? lo.w : lo.y, t ? hi.z : hi.x, t ? hi.w : hi.y};
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const float x2 = x[r] * x[r];
+                        top = fmaxf(top, x2);
+                        a[2 * f + t][ks][r] = to_tf32(x[r]);
+                        sq[ks][r] = to_tf32(x2);
+                    }
+                }
+                const float zero[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                mma_tf32<KS>(norm[2 * f + t], sq, ones, zero);
+            }
+        fetch(base + stride);
+        float m = top < 1e37f ? INFINITY : NAN;
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+            const unsigned long long w = start(j);
+            float lo0 = INFINITY, lo1 = INFINITY;
+#pragma unroll
+            for (int i = 0; i < 2 * G; ++i) {
+                float d[4];
+                mma_tf32<KS>(d, a[i], b[j], norm[i]);
+                lo0 = min_nan(lo0, d[0], d[2]);
+                lo1 = min_nan(lo1, d[1], d[3]);
+            }
+            const float2 x = add2(make_float2(lo0, lo1), make_float2(__uint_as_float((unsigned)w), __uint_as_float((unsigned)(w >> 32))));
+            m = min_nan(m, x.x, x.y);
+        }
+        if (__any_sync(0xffffffffu, !(m > 0.0f))) {
+            const bool wide = __any_sync(0xffffffffu, !(top < 1e37f));
+#pragma unroll 1
+            for (int j = 0; j < NT; ++j) {
+                uint32_t bj[KS][2];
+#pragma unroll
+                for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int slot = 8 * ks + 4 * h + c;
+                        bj[ks][h] = to_tf32(slot < dim ? -2.0f * s.q[8 * j + g][slot] : 0.0f);
+                    }
+                const unsigned long long w = start(j);
+                const float s0 = __uint_as_float((unsigned)w), s1 = __uint_as_float((unsigned)(w >> 32));
+                unsigned bits = 0u;
+#pragma unroll
+                for (int i = 0; i < 2 * G; ++i) {
+                    float d[4];
+                    mma_tf32<KS>(d, a[i], bj, norm[i]);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r)
+                        bits |= (unsigned)(wide || !(d[r] + (r & 1 ? s1 : s0) > 0.0f)) << (4 * i + r);
+                }
+                if (bits) nn_exact(s, bits, tree, dim, N, n, (int)base + 4 * g, 8 * j + 2 * c, nqs, keys);
+                __syncwarp();
+            }
+        }
+        if (tid < nqs && seen < s.key[tid]) {  // what other CTAs found
+            atomicMin(&s.key[tid], seen);
+            s.start[tid] = s.qn[tid] - __fmaf_ru(__uint_as_float((unsigned)(seen >> 32)), 1.0f + 1.0f / 65536, 1e-36f);
+        }
+        __syncwarp();
+    }
+}
+
 __global__ void nn_decode_kernel(const unsigned long long* keys, int batch, int32_t* idx, float* dist) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= batch) return;
@@ -160,17 +392,41 @@ cudaError_t launch_nearest(const float* tree, int dim, int N, const int32_t* tre
     const int columns = (int)(((long long)N + 1023) / 1024);
     const int per_cta = (int)std::min<long long>(kNnQueries, std::max<long long>(4, (long long)batch * columns / (3 * sms)));
     const int tiles = (batch + per_cta - 1) / per_cta;
-    const dim3 grid((unsigned)std::max(1, std::min(columns, (3 * sms + tiles - 1) / tiles)), (unsigned)tiles);
     const int db = (dim + 3) / 4;
     if (tiles > 65535) return cudaErrorInvalidConfiguration;
-#define PRRTC_NN_SCAN(DB)                                                                                            \
-    if (vec) nn_scan_kernel<DB, true><<<grid, 256, 0, st>>>(tree, dim, N, tree_size, size, q, batch, per_cta, keys); \
-    else nn_scan_kernel<DB, false><<<grid, 256, 0, st>>>(tree, dim, N, tree_size, size, q, batch, per_cta, keys)
+    const bool filter = batch >= kNnFilterBatch && (long long)batch * N >= kNnFilterPairs;
+    const int limit = filter ? kNnFirst : INT_MAX;
+    dim3 grid((unsigned)std::max(1, std::min(columns, (3 * sms + tiles - 1) / tiles)), (unsigned)tiles);
+    int share = per_cta;
+    if (filter) {  // the first nodes only: a CTA per column and few queries
+        const int first = kNnFirst / 1024;
+        share = std::max(4, (int)((long long)batch * first / (2 * sms)));
+        share = std::min(share, kNnQueries);
+        if ((batch + share - 1) / share > 65535) return cudaErrorInvalidConfiguration;
+        grid = dim3((unsigned)first, (unsigned)((batch + share - 1) / share));
+    }
+#define PRRTC_NN_SCAN(DB)                                                                                              \
+    if (vec) nn_scan_kernel<DB, true><<<grid, 256, 0, st>>>(tree, dim, N, tree_size, size, limit, q, batch, share, keys); \
+    else nn_scan_kernel<DB, false><<<grid, 256, 0, st>>>(tree, dim, N, tree_size, size, limit, q, batch, share, keys)
     if (db <= 1) { PRRTC_NN_SCAN(1); }
     else if (db == 2) { PRRTC_NN_SCAN(2); }
     else if (db == 3) { PRRTC_NN_SCAN(3); }
     else { PRRTC_NN_SCAN(4); }
 #undef PRRTC_NN_SCAN
+    if (filter) {
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        const int nt = batch <= 32 ? 4 : 8, y = (batch + 8 * nt - 1) / (8 * nt);
+        const int step = 256 * (dim <= 8 ? kNnGroups : 1), cols = (N - kNnFirst + step - 1) / step;
+        const dim3 fgrid((unsigned)std::max(1, std::min(cols, (2 * sms + y - 1) / y)), (unsigned)y);
+#define PRRTC_NN_FILTER(KS, NT, G)                                                                                    \
+    if (vec) nn_filter_kernel<KS, NT, G, true><<<fgrid, 256, 0, st>>>(tree, dim, N, tree_size, size, q, batch, keys); \
+    else nn_filter_kernel<KS, NT, G, false><<<fgrid, 256, 0, st>>>(tree, dim, N, tree_size, size, q, batch, keys)
+        if (dim <= 8 && nt == 4) { PRRTC_NN_FILTER(1, 4, kNnGroups); }
+        else if (dim <= 8) { PRRTC_NN_FILTER(1, 8, kNnGroups); }
+        else if (nt == 4) { PRRTC_NN_FILTER(2, 4, 1); }
+        else { PRRTC_NN_FILTER(2, 8, 1); }
+#undef PRRTC_NN_FILTER
+    }
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     nn_decode_kernel<<<(batch + 255) / 256, 256, 0, st>>>(keys, batch, idx, dist);
     return cudaGetLastError();
