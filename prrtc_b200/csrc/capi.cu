@@ -489,8 +489,14 @@ int prrtc_b200_check_edges(const prrtc_robot_t* robot, const prrtc_world_t* worl
     int32_t* verdicts = reinterpret_cast<int32_t*>(blob + stride);
     cudaError_t e = launch_pack(s, 1, blob, stride, st);
     if (e != cudaSuccess) return cuda_fail(e);
+    EdgeHits hits;
+    if (G > 1) {  // the output serves as the edges' flags until the reduction writes it
+        hits.hit = free_flags;
+        hits.G = G;
+        if ((e = cudaMemsetAsync(free_flags, 0, (size_t)n_edges * sizeof(int32_t), st)) != cudaSuccess) return cuda_fail(e);
+    }
     e = launch_check(blob, (int)stride, world->self_pairs, s.J, s.S, s.K, s.Q, dim, edges, n_edges * G,
-                     batch_sweep(mode, 0), batch_cull(s, 0), verdicts, st, &pc);
+                     batch_sweep(mode, 0), batch_cull(s, 0), verdicts, st, &pc, hits);
     if (e != cudaSuccess) return cuda_fail(e);
     e = launch_edge_reduce(verdicts, n_edges, G, free_flags, st);
     return e == cudaSuccess ? PRRTC_B200_OK : cuda_fail(e);

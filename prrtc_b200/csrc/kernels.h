@@ -123,9 +123,18 @@ cudaError_t launch_extend(const float* tree, int dim, int N, const int32_t* near
 cudaError_t launch_iteration(float* ta, float* tb, int32_t* pa, int32_t* pb, int dim, int N, const float* samples,
                              int batch, int32_t* sizes, int32_t* completed, const float* step, int32_t* new_cfg,
                              int32_t* new_par, int32_t* valid, int32_t* solved, cudaStream_t st);
+// Configurations that are the waypoints of edges, G after G: hit[e] (0 before the
+// launch) becomes 1 with the first waypoint of edge e found in collision, and
+// waypoints of such an edge may then be left out (their verdict is 1).  hit null:
+// every configuration stands for itself.
+struct EdgeHits {
+    int32_t* hit = nullptr;
+    int G = 0;
+};
+
 cudaError_t launch_check(const unsigned char* blob, int blob_cap, const int32_t* pairs, int J, int S, int K,
                          int Q, int dim, const float* configs, int n, int full_sweep, bool cull, int32_t* verdicts,
-                         cudaStream_t st, const PcView* pc = nullptr);
+                         cudaStream_t st, const PcView* pc = nullptr, const EdgeHits& edges = {});
 
 // The culled checker over n_scenes scenes, configurations [offsets[y],
 // offsets[y+1]) against scene y (offsets on the device, ascending, 0 to n);

@@ -696,10 +696,14 @@ struct CheckScenes {
     size_t blob_stride, pairs_stride;
 };
 
+// EDGES: the configurations are waypoints and `edges` their edges' flags (a form of
+// its own: the tests of the flags cost bulk checks 1.6%).
+template <bool EDGES>
 __global__ void __launch_bounds__(256, 3) check_cull_kernel(const unsigned char* __restrict__ gblob, int blob_cap,
                                                             const int2* pairs, int J, int K, int dim, int CW,
                                                             const float* __restrict__ configs, int n,
-                                                            int32_t* verdicts, PcView pc, CheckScenes scenes) {
+                                                            int32_t* verdicts, PcView pc, CheckScenes scenes,
+                                                            EdgeHits edges) {
     extern __shared__ __align__(128) unsigned char dsm[];
     __shared__ __align__(8) uint64_t mbar;
     if (scenes.offsets) {
@@ -738,6 +742,12 @@ __global__ void __launch_bounds__(256, 3) check_cull_kernel(const unsigned char*
     // chunk index: warps of one CTA take neighbouring chunks
     for (long long c0 = ((long long)blockIdx.x * n_warps + warp) * CW; c0 < n; c0 += (long long)gridDim.x * n_warps * CW) {
         const int nw = (int)min((long long)CW, n - c0);
+        if constexpr (EDGES) {
+            if (__all_sync(0xffffffffu, lane >= nw || __ldcg(&edges.hit[(c0 + lane) / edges.G]) != 0)) {
+                if (lane < nw) verdicts[c0 + lane] = 1;  // another waypoint has answered for the edge
+                continue;
+            }
+        }
         for (int i = lane; i < nw * dim; i += 32) {
             const int w = i / dim, d = i - w * dim;
             B.q[w * kDimMax + d] = configs[c0 * dim + i];
@@ -745,6 +755,9 @@ __global__ void __launch_bounds__(256, 3) check_cull_kernel(const unsigned char*
         __syncwarp();
         const unsigned hit = warp_check(sc, B, nw, CW);
         if (lane < nw) verdicts[c0 + lane] = (int)(hit >> lane & 1u);
+        if constexpr (EDGES) {
+            if (lane < nw && hit >> lane & 1u) edges.hit[(c0 + lane) / edges.G] = 1;
+        }
         __syncwarp();
     }
 }
@@ -755,24 +768,25 @@ struct CullCheckAttrs {
     unsigned long long ctx = 0ull;
     int max_dyn = -1, regs = 0, sm_smem = 0, sms = 0;
 };
-static CullCheckAttrs g_cull_check_attr[kCheckAttrDevices];
+static CullCheckAttrs g_cull_check_attr[2][kCheckAttrDevices];
 
 // Launches the culled checker, or returns cudaErrorInvalidConfiguration when
 // its buffers do not fit (the caller then takes the general one).
 static cudaError_t launch_check_cull(const unsigned char* blob, int blob_cap, const int32_t* pairs, int J, int S, int K,
                                      int Q, int dim, const float* configs, int n, int32_t* verdicts, cudaStream_t st,
-                                     const PcView& pc, const CheckScenes& scenes, int n_scenes) {
+                                     const PcView& pc, const CheckScenes& scenes, int n_scenes, const EdgeHits& edges) {
+    auto kern = edges.hit ? check_cull_kernel<true> : check_cull_kernel<false>;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     const unsigned long long ctx = current_context_key();
     std::lock_guard<std::mutex> lock(g_check_attr_mutex);
     CullCheckAttrs dflt;
-    CullCheckAttrs& a = dev >= 0 && dev < kCheckAttrDevices ? g_cull_check_attr[dev] : dflt;
+    CullCheckAttrs& a = dev >= 0 && dev < kCheckAttrDevices ? g_cull_check_attr[edges.hit ? 1 : 0][dev] : dflt;
     if (!ctx || a.ctx != ctx) {
         a = CullCheckAttrs{};
         cudaFuncAttributes fa;
-        if ((e = cudaFuncGetAttributes(&fa, check_cull_kernel)) != cudaSuccess ||
+        if ((e = cudaFuncGetAttributes(&fa, kern)) != cudaSuccess ||
             (e = cudaDeviceGetAttribute(&a.sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev)) != cudaSuccess)
             return e;
         a.regs = (fa.numRegs + 7) & ~7;
@@ -782,7 +796,7 @@ static cudaError_t launch_check_cull(const unsigned char* blob, int blob_cap, co
     const int max_dyn = (int)device_max_smem() - 64;
     const int general = cc_smem_bytes(J, S, K, Q, 8);  // a scene that is not culled
     int best_cw = 0, best_wpc = 0, best_warps = 0, best_dyn = 0;
-    const int least = pc.n > 0 ? 1 : 4;  // configurations per warp; with a cloud each is 27 cells and their points per sphere
+    const int least = pc.n > 0 ? 1 : 4;  // configurations per warp
     for (int cw = 32; cw >= least; cw /= 2) {
         for (int wpc = 4; wpc <= 8; wpc *= 2) {
             const int dyn = blob_cap + std::max(wpc * warp_check_bytes(J, K, cw), general);
@@ -793,13 +807,18 @@ static cudaError_t launch_check_cull(const unsigned char* blob, int blob_cap, co
         }
     }
     if (best_warps == 0) return cudaErrorInvalidConfiguration;
-    int cw = best_cw, wpc = best_wpc;
+    // With a cloud a configuration is 27 cells and their points per sphere until one
+    // hits: one per warp, so that an edge's other waypoints find its flag set and
+    // uneven configurations spread (3384 edges x 33 waypoints against 41,277 points:
+    // 708 us; with 2 per warp 750, 4 1160, 16 2870, and 3070 without flags; 4000 x 8
+    // against 1000 points: 283 us, with 8 per warp 530).
+    int cw = pc.n > 0 ? 1 : best_cw, wpc = best_wpc;
     while (cw > least && (long long)cw * a.sms * best_warps > n) cw /= 2;  // fewer per warp before warps go idle
     const long long chunks = n / cw + n_scenes;  // of all scenes, about
     while (wpc > 1 && chunks < (long long)a.sms * wpc) wpc /= 2;
     const int dyn = blob_cap + std::max(wpc * warp_check_bytes(J, K, cw), general);
     if (std::max(dyn, best_dyn) > a.max_dyn) {
-        if ((e = cudaFuncSetAttribute(check_cull_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       std::max(dyn, best_dyn))) != cudaSuccess)
             return e;
         a.max_dyn = std::max(dyn, best_dyn);
@@ -809,8 +828,8 @@ static cudaError_t launch_check_cull(const unsigned char* blob, int blob_cap, co
     // twice its even share, and a CTA strides over what is left
     const long long each = n_scenes == 1 ? (chunks + wpc - 1) / wpc : (2 * chunks / n_scenes + wpc - 1) / wpc;
     const long long grid = std::max(1ll, std::min(each, n_scenes == 1 ? resident : (2 * resident + n_scenes - 1) / n_scenes));
-    check_cull_kernel<<<dim3((unsigned)grid, (unsigned)n_scenes), wpc * 32, dyn, st>>>(
-        blob, blob_cap, reinterpret_cast<const int2*>(pairs), J, K, dim, cw, configs, n, verdicts, pc, scenes);
+    kern<<<dim3((unsigned)grid, (unsigned)n_scenes), wpc * 32, dyn, st>>>(
+        blob, blob_cap, reinterpret_cast<const int2*>(pairs), J, K, dim, cw, configs, n, verdicts, pc, scenes, edges);
     return cudaGetLastError();
 }
 
@@ -823,14 +842,14 @@ static cudaError_t launch_check_cull(const unsigned char* blob, int blob_cap, co
 // checks/s at 32, 65.4 M at 8.
 cudaError_t launch_check(const unsigned char* blob, int blob_cap, const int32_t* pairs, int J, int S, int K,
                          int Q, int dim, const float* configs, int n, int full_sweep, bool cull, int32_t* verdicts,
-                         cudaStream_t st, const PcView* pc) {
+                         cudaStream_t st, const PcView* pc, const EdgeHits& edges) {
     if (n <= 0) return cudaSuccess;
     const PcView cloud = pc ? *pc : PcView{nullptr, nullptr, 0, 0, 0.0f, 0.0f};
     constexpr int CW = PRRTC_CHECK_CW;
     CheckLaunch best, o;
     if (cull) {
         const cudaError_t e = launch_check_cull(blob, blob_cap, pairs, J, S, K, Q, dim, configs, n, verdicts, st, cloud,
-                                                 CheckScenes{nullptr, 0, 0}, 1);
+                                                 CheckScenes{nullptr, 0, 0}, 1, edges);
         if (e != cudaErrorInvalidConfiguration) return e;
     }
     cudaError_t e = check_option<CW>(full_sweep, J, S, K, Q, blob_cap, best);
@@ -869,7 +888,7 @@ cudaError_t launch_check_batch(const unsigned char* blobs, size_t blob_stride, c
                                cudaStream_t st) {
     return launch_check_cull(blobs, (int)blob_stride, pairs, J, S, K, Q, dim, configs, n, verdicts, st,
                              PcView{nullptr, nullptr, 0, 0, 0.0f, 0.0f}, CheckScenes{offsets, blob_stride, pairs_stride},
-                             n_scenes);
+                             n_scenes, EdgeHits{});
 }
 
 // ============================================================================ FK
