@@ -205,9 +205,10 @@ def smooth_paths(paths: list, collision_context: dict, lower, upper, *, waypoint
 
 class _BatchScenes:
     """Robot tables plus one world per problem, on the device in one staged
-    copy, as the C struct of the batched entry points."""
+    copy, as the C struct of the batched entry points.  ``wait``: until that copy
+    has run, for tables that are read on other streams than the current one."""
 
-    def __init__(self, collision_contexts, device: torch.device):
+    def __init__(self, collision_contexts, device: torch.device, wait: bool = False):
         from .prrtc import _native_pack, _pack_worlds
 
         ctxs = list(collision_contexts)
@@ -225,7 +226,7 @@ class _BatchScenes:
             packed, counts = _pack_worlds(ctxs, B)
             keys = {k: (stage.add(packed[k], torch.int32 if k == "self_pairs" else torch.float32),
                         stage.add(counts[k], torch.int32), int(packed[k].shape[1])) for k in packed}
-        stage.commit()
+        stage.commit(wait=wait)
         self.robot_ctx.finish()
         self.stage = stage  # holds the tables
         bi = _lib.BatchInputs()
@@ -241,15 +242,17 @@ class _BatchScenes:
 class BatchSmoothContext:
     """Robot tables plus one world per path, resident on the device, for the
     batched adjoint (prrtc_b200_smooth_cost_grad_batch): path p is costed
-    against collision_contexts[p]'s world and self pairs."""
+    against collision_contexts[p]'s world and self pairs.  The tables are on the
+    device when the constructor returns, whatever stream reads them; with
+    ``wait=False`` their copy is only queued, for use on the current stream."""
 
     def __init__(self, collision_contexts, dim: int, margin: float = 0.02, beta: float = 50.0, w_len: float = 1.0,
-                 device=None):
+                 device=None, *, wait: bool = True):
         self.lib = _lib.load()
         self.device = cuda_device(device)
         self.dim = int(dim)
         self.margin, self.beta, self.w_len = float(margin), float(beta), float(w_len)
-        self.scenes = _BatchScenes(collision_contexts, self.device)
+        self.scenes = _BatchScenes(collision_contexts, self.device, wait)
         self.B, self.bi = self.scenes.B, self.scenes.bi
         self.ws = workspace(self.lib.prrtc_b200_smooth_batch_workspace_size(C.byref(self.bi)), self.device)
 
@@ -321,7 +324,8 @@ def smooth_paths_batch(paths: list, collision_contexts: list, lower, upper, *, w
     dev = cuda_device(device)
     dim = int(np.asarray(paths[0]).shape[1])
     init = torch.from_numpy(_resample_paths(paths, waypoints)).to(dev)
-    sctx = BatchSmoothContext(collision_contexts, dim, margin, beta, w_len, dev)
+    # used on this stream alone, and gone with the call
+    sctx = BatchSmoothContext(collision_contexts, dim, margin, beta, w_len, dev, wait=False)
     c0, _ = sctx.cost_grad(init, need_grad=False)
     x = projected_steps(sctx, init, lower, upper, steps, lr)
     c1, _ = sctx.cost_grad(x, need_grad=False)
