@@ -298,14 +298,20 @@ def projected_steps(sctx, init: torch.Tensor, lower, upper, steps: int, lr: floa
     lo = as_tensor(lower, torch.float32, init.device).reshape(1, 1, dim)
     hi = as_tensor(upper, torch.float32, init.device).reshape(1, 1, dim)
     x = init.clone()
-    if isinstance(sctx, BatchSmoothContext) and x.dtype == torch.float32 and x.is_contiguous() and x.numel():
+    # the kernels take plain memory of the scenes' device and one number for lr;
+    # anything else (paths elsewhere, recorded by autograd, without an inner
+    # waypoint, another object's gradient) goes by the tensor expression
+    if (isinstance(sctx, BatchSmoothContext) and type(sctx).cost_grad is BatchSmoothContext.cost_grad
+            and type(x) is torch.Tensor and x.device == sctx.device and x.dtype == torch.float32 and x.is_contiguous()
+            and P > 0 and W > 2 and isinstance(lr, (int, float)) and not (x.requires_grad or lo.requires_grad or hi.requires_grad)):
         sctx.descend(x, lo, hi, steps, lr)
         return x
+    order = {"ordered": True} if type(sctx) is SmoothContext else {}
     mask = torch.ones_like(x)
     mask[:, 0] = 0.0
     mask[:, -1] = 0.0
     for _ in range(steps):
-        _, g = sctx.cost_grad(x, ordered=True)
+        _, g = sctx.cost_grad(x, **order)
         gn = torch.linalg.norm((g * mask).reshape(P, -1), dim=1).clamp_min(1e-12)
         x = torch.minimum(torch.maximum(x - lr * (g * mask) / gn[:, None, None], lo), hi)
     return x
