@@ -214,9 +214,10 @@ class _BatchScenes:
         ctxs = list(collision_contexts)
         B = self.B = len(ctxs)
         # whether every context is the first one's robot in another world (the
-        # very same tables), and none has a point cloud
-        self.one_robot = all(c.get("point_cloud") is None and all(c.get(k) is ctxs[0].get(k) for k in ROBOT_SPEC)
-                             for c in ctxs)
+        # very same tables), and none has a point cloud; a context of None is a
+        # path without a world, which only the per-path check takes
+        self.one_robot = all(c is not None and c.get("point_cloud") is None
+                             and all(c.get(k) is ctxs[0].get(k) for k in ROBOT_SPEC) for c in ctxs)
         stage = Stager(device)
         self.robot_ctx = DeviceContext(ctxs[0], device, world_keys=False, stager=stage)
         native = _native_pack(ctxs, stage)
@@ -348,7 +349,7 @@ def revalidate_batch(paths: torch.Tensor, collision_contexts: list, resolution: 
     (``scenes``: their tables, when already on the device)."""
     pts, owner = densify(paths, resolution)
     P, dim = int(paths.shape[0]), int(paths.shape[2])
-    dev = torch.device(device)
+    dev = torch.empty(0, device=device).device  # None: torch's default
     lib = _lib.load()
     if P and pts.dtype == torch.float32 and pts.is_cuda:
         scenes = scenes if scenes is not None else _BatchScenes(collision_contexts, pts.device)

@@ -81,3 +81,26 @@ def test_forms(cuda, form):
     _check(cost, grad, [ctx] * 2, w, w_len)
     if form == "below_tail":
         assert 0.0 < cost.max().item() < 1e-15 and float(grad.abs().max()) < 1e-13
+
+
+def test_paths_without_a_world(cuda):
+    """A context of None is a path without world or self pairs; re-validation with no device named answers on torch's
+    default one."""
+    from prrtc_b200.smoothing import BatchSmoothContext, SmoothContext, revalidate_batch
+
+    robot = scenes.arm(0)
+    ctx = build_collision_context(robot, scenes.tabletop_world(np.random.default_rng(4)))
+    empty = {k: v[:0] if k.startswith("world_") or k == "self_pairs" else v for k, v in ctx.items()}
+    for k in ("coarse_self_pairs", "self_pair_ranges"):
+        empty[k] = empty[k][:0]
+    x = torch.from_numpy(_paths(robot, 3, 9, 2)).to(cuda)
+    ctxs = [ctx, None, ctx]
+    cost, grad = BatchSmoothContext(ctxs, robot.dim, device=cuda).cost_grad(x)
+    for p, c in enumerate((ctx, empty, ctx)):
+        c1, g1 = SmoothContext(c, robot.dim, device=cuda).cost_grad(x[p:p + 1], ordered=True)
+        assert torch.equal(grad[p], g1[0])
+        assert abs(cost[p].item() - c1.item()) <= 2e-6 * abs(c1.item())  # 9 waypoints' costs in any order
+    want = revalidate_batch(x, ctxs, 0.02, cuda)
+    got = revalidate_batch(x, ctxs, 0.02, None)
+    assert got.device == torch.empty(0).device and torch.equal(got, want.cpu()) and bool(want[1])
+    assert torch.equal(revalidate_batch(x, [ctx] * 3, 0.02, None), revalidate_batch(x, [ctx] * 3, 0.02, cuda).cpu())
