@@ -113,6 +113,19 @@ struct ResultSrc {
 cudaError_t launch_result_block(int B, int dim, int max_len, const ResultSrc& R, int32_t* block,
                                 const float* paths, float* packed, long long packed_cap, cudaStream_t st);
 
+// The largest dynamic shared-memory limit set on a kernel, per device and CUDA
+// context.  The limit is only raised, never lowered, so a call on another host
+// thread cannot shrink it between this call's check and its launch, and a call
+// that needs no more than before sets nothing (setting an attribute while an
+// earlier launch runs can make the host wait for that launch).
+struct DynLimit {
+    unsigned long long ctx = 0ull;  // context key (current_context_key)
+    int max_dyn = -1;
+};
+constexpr int kDynLimitDevices = 256;
+// limits: one per device, of this kernel alone.
+cudaError_t raise_dyn_limit(const void* kern, DynLimit (&limits)[kDynLimitDevices], size_t dyn);
+
 // primitives.cu
 // The tree's size: *tree_size on the device, or `size` when that is null.
 cudaError_t launch_nearest(const float* tree, int dim, int N, const int32_t* tree_size, int size, const float* q, int batch,

@@ -1287,11 +1287,10 @@ cudaError_t launch_extract_paths(int B, int dim, int N, const float* ta, const f
                                  float* paths, int32_t* lengths, float* costs, cudaStream_t st) {
     const size_t smem = (size_t)max_len * sizeof(int);
     cudaError_t e;
-    if (smem > 48 * 1024) {
-        if ((e = cudaFuncSetAttribute(extract_paths_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem)) != cudaSuccess)
-            return e;
-    }
+    static DynLimit limit[kDynLimitDevices];
+    if (smem > 48 * 1024 &&
+        (e = raise_dyn_limit(reinterpret_cast<const void*>(extract_paths_kernel), limit, smem)) != cudaSuccess)
+        return e;
     extract_paths_kernel<<<B, 32, smem, st>>>(B, dim, N, ta, tb, pa, pb, conn, solved, max_len, paths, lengths,
                                               costs);
     return cudaGetLastError();

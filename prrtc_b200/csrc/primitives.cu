@@ -586,31 +586,18 @@ struct CheckLaunch {
     size_t dyn = 0;
 };
 
-// The largest dynamic shared-memory limit set on each check_kernel
-// instantiation, per device and CUDA context.  The limit is only raised, never
-// lowered, so a call on another host thread cannot shrink it between this
-// call's check and its launch, and a call that needs no more than before sets
-// nothing (setting an attribute while an earlier launch runs can make the host
-// wait for that launch).
-struct CheckAttrs {
-    unsigned long long ctx = 0ull;  // context key (current_context_key)
-    int max_dyn = -1;
-};
-constexpr int kCheckAttrDevices = 256;
-static CheckAttrs g_check_attr[kCheckAttrDevices][6];  // [device][2 * (pass size: CW, CW/2, CW/4) + full]
 static std::mutex g_check_attr_mutex;
 
-template <class Kern>
-static cudaError_t check_raise_dyn(Kern kern, int slot, size_t dyn) {
+cudaError_t raise_dyn_limit(const void* kern, DynLimit (&limits)[kDynLimitDevices], size_t dyn) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     const unsigned long long ctx = current_context_key();
     std::lock_guard<std::mutex> lock(g_check_attr_mutex);
-    CheckAttrs dflt;
-    CheckAttrs& c = (dev >= 0 && dev < kCheckAttrDevices && slot >= 0 && slot < 6) ? g_check_attr[dev][slot] : dflt;
+    DynLimit dflt;
+    DynLimit& c = (dev >= 0 && dev < kDynLimitDevices) ? limits[dev] : dflt;
     if (!ctx || c.ctx != ctx) {
-        c = CheckAttrs{};
+        c = DynLimit{};
         c.ctx = ctx;
     }
     if ((int)dyn > c.max_dyn) {
@@ -620,6 +607,8 @@ static cudaError_t check_raise_dyn(Kern kern, int slot, size_t dyn) {
     }
     return cudaSuccess;
 }
+
+static DynLimit g_check_limit[6][kDynLimitDevices];  // 2 * (pass size: CW, CW/2, CW/4) + full
 
 template <int CW>
 static cudaError_t check_option(int full_sweep, int J, int S, int K, int Q, int blob_cap, CheckLaunch& o) {
@@ -631,7 +620,7 @@ static cudaError_t check_option(int full_sweep, int J, int S, int K, int Q, int 
     }
     auto kern = full_sweep ? check_kernel<CW, true> : check_kernel<CW, false>;
     constexpr int size_idx = CW == PRRTC_CHECK_CW ? 0 : (2 * CW == PRRTC_CHECK_CW ? 1 : 2);
-    cudaError_t e = check_raise_dyn(kern, 2 * size_idx + (full_sweep ? 1 : 0), dyn);
+    cudaError_t e = raise_dyn_limit(reinterpret_cast<const void*>(kern), g_check_limit[2 * size_idx + (full_sweep ? 1 : 0)], dyn);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, dyn)) != cudaSuccess) return e;
@@ -768,7 +757,7 @@ struct CullCheckAttrs {
     unsigned long long ctx = 0ull;
     int max_dyn = -1, regs = 0, sm_smem = 0, sms = 0;
 };
-static CullCheckAttrs g_cull_check_attr[2][kCheckAttrDevices];
+static CullCheckAttrs g_cull_check_attr[2][kDynLimitDevices];
 
 // Launches the culled checker, or returns cudaErrorInvalidConfiguration when
 // its buffers do not fit (the caller then takes the general one).
@@ -782,7 +771,7 @@ static cudaError_t launch_check_cull(const unsigned char* blob, int blob_cap, co
     const unsigned long long ctx = current_context_key();
     std::lock_guard<std::mutex> lock(g_check_attr_mutex);
     CullCheckAttrs dflt;
-    CullCheckAttrs& a = dev >= 0 && dev < kCheckAttrDevices ? g_cull_check_attr[edges.hit ? 1 : 0][dev] : dflt;
+    CullCheckAttrs& a = dev >= 0 && dev < kDynLimitDevices ? g_cull_check_attr[edges.hit ? 1 : 0][dev] : dflt;
     if (!ctx || a.ctx != ctx) {
         a = CullCheckAttrs{};
         cudaFuncAttributes fa;
@@ -981,8 +970,9 @@ cudaError_t launch_fk(const FkTables& t, int dim, const float* configs, int n, f
     if (n <= 0 || t.J <= 0) return cudaSuccess;
     const int smem = fk_smem_bytes(t.J);
     cudaError_t e;
+    static DynLimit limit[kDynLimitDevices];
     if (smem > 48 * 1024 &&
-        (e = cudaFuncSetAttribute(fk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess)
+        (e = raise_dyn_limit(reinterpret_cast<const void*>(fk_kernel), limit, (size_t)smem)) != cudaSuccess)
         return e;
     const long long tiles = ((long long)n + kFkTile - 1) / kFkTile;
     fk_kernel<<<(unsigned)std::min<long long>(tiles, 8ll * device_sm_count()), kFkThreads, smem, st>>>(

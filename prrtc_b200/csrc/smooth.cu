@@ -927,7 +927,8 @@ cudaError_t launch_smooth(const unsigned char* blob, size_t blob_stride, int blo
             if (parts > 1 && grad &&
                 (e = cudaMemsetAsync(grad, 0, (size_t)P * W * dim * sizeof(float), st)) != cudaSuccess)
                 return e;
-            if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wide)) != cudaSuccess)
+            static DynLimit limit[2][kDynLimitDevices];
+            if ((e = raise_dyn_limit(reinterpret_cast<const void*>(kern), limit[big ? 1 : 0], wide)) != cudaSuccess)
                 return e;
             kern<<<(unsigned)(ctas * parts), big ? 512 : 256, wide, st>>>(a, blob_cap, parts);
             return cudaGetLastError();
@@ -942,8 +943,8 @@ cudaError_t launch_smooth(const unsigned char* blob, size_t blob_stride, int blo
     if (smem + blob_cap + 64 <= device_max_smem()) {
         smem += blob_cap;
         auto kern = cost ? smooth_kernel<WARPS, true, true> : smooth_kernel<WARPS, true, false>;
-        if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
-            return e;
+        static DynLimit limit[2][kDynLimitDevices];
+        if ((e = raise_dyn_limit(reinterpret_cast<const void*>(kern), limit[cost ? 1 : 0], smem)) != cudaSuccess) return e;
         kern<<<blocks(WARPS), WARPS * 32, smem, st>>>(a, blob_cap, per_path(WARPS));
         return cudaGetLastError();
     }
@@ -951,8 +952,9 @@ cudaError_t launch_smooth(const unsigned char* blob, size_t blob_stride, int blo
     constexpr int FEW = 4;
     smem = (size_t)FEW * smooth_warp_floats(J, S) * sizeof(float);
     auto kern = cost ? smooth_kernel<FEW, false, true> : smooth_kernel<FEW, false, false>;
+    static DynLimit limit[2][kDynLimitDevices];
     if (smem > 48 * 1024 &&
-        (e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+        (e = raise_dyn_limit(reinterpret_cast<const void*>(kern), limit[cost ? 1 : 0], smem)) != cudaSuccess)
         return e;
     kern<<<blocks(FEW), FEW * 32, smem, st>>>(a, 0, per_path(FEW));
     return cudaGetLastError();
