@@ -521,10 +521,18 @@ __device__ __forceinline__ float wide_rsqrt(float x) {
     return r;
 }
 
+// The larger operand, NaN where one is (fmaxf would give the other): a distance
+// that is not a number stays one.
+__device__ __forceinline__ float wide_max(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 // Pair terms, all 32 lanes together.  z = beta (margin - d): cost collects
 // softplus(z) in units of 1/beta, sig is the sigmoid, the factor of -dd/dc.
 // With e = exp(-|z|):
-//   some lane nearer than z = -5.6: as pair_term;
+//   some lane nearer than z = -5.6, or not a number: as pair_term;
 //   all lanes below that (e < 2^-8): log1p(e) = e - e^2/2 + e^3/3 and e/(1+e) = e -
 //     e^2 + e^3, both to e^3 (relative 6e-8, a float's rounding);
 //   all lanes below the tail of pair_term (z = kTailZ): the cost only, as there
@@ -536,9 +544,9 @@ __device__ __forceinline__ bool wide_terms(const float (&z)[N], float& cost, flo
 #pragma unroll
     for (int k = 0; k < N; ++k) {
         e[k] = wide_ex2(-fabsf(z[k]) * 1.44269504089f);
-        top = fmaxf(top, z[k]);
+        top = wide_max(top, z[k]);
     }
-    if (__any_sync(0xffffffffu, top > -5.6f)) {
+    if (__any_sync(0xffffffffu, !(top <= -5.6f))) {
 #pragma unroll
         for (int k = 0; k < N; ++k) {
             const float r = __fdividef(1.0f, 1.0f + e[k]);
@@ -687,7 +695,7 @@ __global__ void __launch_bounds__(THREADS, MINBLOCKS)
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
                     dx[k] = c[k].x - ob.x; dy[k] = c[k].y - ob.y; dz[k] = c[k].z - ob.z;
-                    const float d2 = fmaxf(fmaf(dx[k], dx[k], fmaf(dy[k], dy[k], dz[k] * dz[k])), 1e-36f);
+                    const float d2 = wide_max(fmaf(dx[k], dx[k], fmaf(dy[k], dy[k], dz[k] * dz[k])), 1e-36f);
                     rn[k] = wide_rsqrt(d2);
                     z[k] = a.beta * (a.margin - (d2 * rn[k] - c[k].w - ro));
                 }
@@ -708,7 +716,7 @@ __global__ void __launch_bounds__(THREADS, MINBLOCKS)
                     ex[k] = fmaf(-u_, dl.x, c[k].x - p1.x);
                     ey[k] = fmaf(-u_, dl.y, c[k].y - p1.y);
                     ez[k] = fmaf(-u_, dl.z, c[k].z - p1.z);
-                    const float d2 = fmaxf(fmaf(ex[k], ex[k], fmaf(ey[k], ey[k], ez[k] * ez[k])), 1e-36f);
+                    const float d2 = wide_max(fmaf(ex[k], ex[k], fmaf(ey[k], ey[k], ez[k] * ez[k])), 1e-36f);
                     rn[k] = wide_rsqrt(d2);
                     z[k] = a.beta * (a.margin - (d2 * rn[k] - c[k].w - p1.w));
                 }
@@ -795,7 +803,7 @@ __global__ void __launch_bounds__(THREADS, MINBLOCKS)
                 }
                 const float4 cj = centre(pj, lane);
                 const float dx = ci.x - cj.x, dy = ci.y - cj.y, dz = ci.z - cj.z;
-                const float d2 = fmaxf(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), 1e-36f), rn = wide_rsqrt(d2);
+                const float d2 = wide_max(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), 1e-36f), rn = wide_rsqrt(d2);
                 const float z[1] = {a.beta * (a.margin - (d2 * rn - ci.w - cj.w))};
                 float sig[1];
                 if (wide_terms<1>(z, cost, sig)) {

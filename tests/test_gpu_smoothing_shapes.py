@@ -104,3 +104,29 @@ def test_paths_without_a_world(cuda):
     got = revalidate_batch(x, ctxs, 0.02, None)
     assert got.device == torch.empty(0).device and torch.equal(got, want.cpu()) and bool(want[1])
     assert torch.equal(revalidate_batch(x, [ctx] * 3, 0.02, None), revalidate_batch(x, [ctx] * 3, 0.02, cuda).cpu())
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("scene", ["spheres", "capsules", "boxes", "halfspaces", "self_pairs", "all"])
+def test_a_waypoint_that_is_not_a_number(cuda, scene, bad):
+    """A path of one waypoint with a coordinate that is not a number (no length term carries it): its cost and every
+    gradient entry that depends on it are not numbers either, and the paths beside it keep their values."""
+    from prrtc_b200.smoothing import SmoothContext
+
+    robot = scenes.arm(2)
+    ctx = build_collision_context(robot, scenes.tabletop_world(np.random.default_rng(4)))
+    for k in ("world_spheres", "world_capsules", "world_boxes", "world_halfspaces", "self_pairs"):
+        if scene != "all" and not k.endswith(scene):
+            ctx[k] = ctx[k][:0]
+    for k in ("coarse_self_pairs", "self_pair_ranges"):
+        ctx[k] = ctx[k][:0]
+    sctx = SmoothContext(ctx, robot.dim, device=cuda)
+    x = torch.from_numpy(_paths(robot, 3, 1, 6)).to(cuda)
+    want_cost, want_grad = sctx.cost_grad(x)
+    x[1, 0, 1] = bad
+    cost, grad = sctx.cost_grad(x)
+    assert torch.isnan(cost).tolist() == [False, True, False]
+    assert torch.equal(torch.isnan(grad), torch.isnan(sctx.cost_grad(x, ordered=True)[1])) and bool(torch.isnan(grad[1]).any())
+    for p in (0, 2):  # neighbouring lanes may take the full softplus with it: a term's rounding, at most 1e-6 of it
+        assert torch.allclose(cost[p], want_cost[p], rtol=1e-5, atol=0.0)
+        assert torch.allclose(grad[p], want_grad[p], rtol=1e-5, atol=1e-5 * float(want_grad[p].abs().max()))
