@@ -391,16 +391,18 @@ int prrtc_b200_result_block(int32_t batch, int32_t dim, int32_t max_len,
 /* Smooth collision + length cost of P paths of W waypoints [P,W,dim] and its
  * gradient (hand-written adjoint through FK, link transforms recomputed):
  *   cost_p = sum_w sum_pairs softplus_beta(margin - d) + w_len * sum_w |q_{w+1}-q_w|^2
- * grad may be NULL (cost only). */
+ * grad may be NULL (cost only).  The gradient is the same bits in every run of the
+ * same call on the same device; the cost is added up in any order. */
 size_t prrtc_b200_smooth_workspace_size(const prrtc_robot_t* robot, const prrtc_world_t* world);
 int prrtc_b200_smooth_cost_grad(const prrtc_robot_t* robot, const prrtc_world_t* world, int32_t dim,
                                 const float* waypoints, int32_t n_paths, int32_t n_waypoints,
                                 float margin, float beta, float w_len, float* cost, float* grad,
                                 void* workspace, size_t workspace_bytes, void* stream);
 
-/* The same with every sum of the gradient taken in a fixed order (the same bits
- * in every run), as prrtc_b200_smooth_cost_grad_batch does: for descents, which
- * follow the rounding of their gradient across the kinks of box distances. */
+/* The same with the sums of the gradient in the order of
+ * prrtc_b200_smooth_cost_grad_batch: a path's gradient is then the same bits
+ * whatever paths are beside it, and those of the batched entry.  For descents,
+ * which follow the rounding of their gradient across the kinks of box distances. */
 int prrtc_b200_smooth_cost_grad_ordered(const prrtc_robot_t* robot, const prrtc_world_t* world, int32_t dim,
                                         const float* waypoints, int32_t n_paths, int32_t n_waypoints,
                                         float margin, float beta, float w_len, float* cost, float* grad,

@@ -178,8 +178,8 @@ cudaError_t launch_radius_update(float* radii, const int32_t* idx, const int32_t
                                  float rmin, int sequential, int32_t* err, cudaStream_t st);
 
 // smooth.cu
-// blob_cap: capacity of one scene; ordered: every sum in a fixed order (the same
-// bits in every run), as it always is with a scene per path; cost null: the
+// blob_cap: capacity of one scene; ordered: a path's gradient is the same bits
+// whatever paths are beside it, as it always is with a scene per path; cost null: the
 // gradient alone, zero at the paths' end points.  Path p uses the scene at blob + p * blob_stride and the self pairs at
 // pairs + 2 * p * pairs_stride (strides 0: one scene for every path).
 cudaError_t launch_smooth(const unsigned char* blob, size_t blob_stride, int blob_cap, const int32_t* pairs,

@@ -466,11 +466,22 @@ cudaError_t launch_smooth_update(float* x, const float* g, const float* norms, c
 // ----------------------------------------------------------------------------- a warp's lanes are waypoints
 
 // The form for paths of one scene and robots of up to 32 joints, unless the
-// caller wants the sums in a fixed order: a CTA takes 32 waypoints, one per lane, and its warps take (two spheres x every primitive) and (32 self pairs)
-// units from a shared counter.  All lanes of a warp then look at the same
-// primitive, read from shared memory once for the warp, with neighbouring
-// waypoints' distances, which are alike, so the warp as a whole takes the short
-// series for pairs that are far apart (below) instead of the full softplus.
+// caller wants the sums in smooth_kernel's order: a CTA takes 32 waypoints, one
+// per lane.  All lanes of a warp then look at the same primitive, read from
+// shared memory once for the warp, with neighbouring waypoints' distances, which
+// are alike, so the warp as a whole takes the short series for pairs that are far
+// apart (below) instead of the full softplus.
+//
+// The gradient is the same bits in every run of the same call: every one of its
+// sums has one order.  The warps draw units from a counter, a unit being two
+// spheres against every primitive or against every sphere that they make a self
+// pair with.  A sphere's sums stay in registers and meet in shared memory as two
+// terms, so their order does not matter, and frame sums go over the spheres in
+// order.  A self pair is computed twice for that, once for each of its spheres:
+// adding its terms to the other one by atomics has another order in every run (369 us
+// a call for 512 paths x 64 waypoints in the tabletop scene, 344 with this), and terms
+// left in shared memory for each sphere's warp to add after a barrier took 571 us.
+// (The cost is added up by atomics.)
 //
 // Bound by instruction issue and, close behind, the special-function pipe (a
 // reciprocal square root and an exponential per pair, two reciprocals more near
@@ -487,12 +498,14 @@ struct SmoothBufs {
     float* q;       // [32][kDimMax], then dv [32][J]
     float* cost;    // [32]
     uint32_t* sub;  // [J] mask of the joint's subtree (itself included)
-    int* next;      // unit counter
+    uint32_t* adj;  // [S][words of S bits] the spheres that a sphere makes a self pair with
+    int* next;      // unit counter, then whether the list repeats a pair
 };
 
 __host__ __device__ inline int smooth_g_bytes(int J, int S) { return S * 384 > J * 1536 ? S * 384 : J * 1536; }
 __host__ __device__ inline int smooth_wide_bytes(int J, int S) {
-    return 32 * J * 48 + S * 3 * 128 + smooth_g_bytes(J, S) + J * 6 * 128 + 32 * (kDimMax > J ? kDimMax : J) * 4 + 128 + 128 + 16;
+    return 32 * J * 48 + S * 3 * 128 + smooth_g_bytes(J, S) + J * 6 * 128 + 32 * (kDimMax > J ? kDimMax : J) * 4 + 128 + 128 +
+           align16(S * cdiv(S, 32) * 4) + 16;
 }
 
 __device__ __forceinline__ SmoothBufs smooth_bufs(unsigned char* p, int J, int S) {
@@ -504,6 +517,7 @@ __device__ __forceinline__ SmoothBufs smooth_bufs(unsigned char* p, int J, int S
     b.q = reinterpret_cast<float*>(p);      p += 32 * max(kDimMax, J) * 4;
     b.cost = reinterpret_cast<float*>(p);   p += 128;
     b.sub = reinterpret_cast<uint32_t*>(p); p += 128;
+    b.adj = reinterpret_cast<uint32_t*>(p); p += align16(S * cdiv(S, 32) * 4);
     b.next = reinterpret_cast<int*>(p);
     return b;
 }
@@ -568,13 +582,27 @@ __device__ __forceinline__ bool wide_terms(const float (&z)[N], float& cost, flo
     return false;
 }
 
+// The CTAs of a cluster meet: writes before it, of every thread of them, are seen after it.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The value at `p` (in this CTA's shared memory) in the cluster's CTA `rank`.
+__device__ __forceinline__ float cluster_load(const float* p, int rank) {
+    unsigned at;
+    float v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at));
+    return v;
+}
+
 template <int THREADS, int MINBLOCKS>
 __global__ void __launch_bounds__(THREADS, MINBLOCKS)
     smooth_wide_kernel(SmoothArgs a, int blob_cap, int parts) {
     extern __shared__ __align__(128) unsigned char dsm[];
     __shared__ __align__(8) uint64_t mbar;
     constexpr unsigned kAll = 0xffffffffu;
-    constexpr int T = THREADS;
+    constexpr int T = THREADS, WARPS = THREADS / 32;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int J = a.J, S = a.S, dim = a.dim, W = a.W;
     // 32 of all paths' waypoints, one path after the other
@@ -587,13 +615,14 @@ __global__ void __launch_bounds__(THREADS, MINBLOCKS)
     const SmoothBufs B = smooth_bufs(dsm + blob_cap, J, S);
     if (tid == 0) {
         mbar_init(&mbar);
-        *B.next = 0;
+        B.next[0] = B.next[1] = 0;
     }
+    const int adj_words = cdiv(S, 32);
+    for (int i = tid; i < S * adj_words; i += T) B.adj[i] = 0u;
     for (int i = tid; i < 32 * dim; i += T) {
         const int w = i / dim, d = i - w * dim;
         B.q[w * kDimMax + d] = w < nw ? a.wp[first * dim + i] : 0.0f;
     }
-    for (int i = tid; i < J * 192; i += T) B.acc[i] = 0.0f;
     if (tid < 32) B.cost[tid] = 0.0f;
     __syncthreads();
     uint32_t phase = 0;
@@ -617,6 +646,21 @@ __global__ void __launch_bounds__(THREADS, MINBLOCKS)
             m |= x == tid ? 1u << k : 0u;
         }
         B.sub[tid] = m;
+    }
+    // both directions of every self pair; a bit that was set already is a pair (or its reverse) that the list repeats
+    // (four loads on their way together)
+    for (int k0 = tid; k0 < h.P; k0 += 4 * T) {
+        int2 pr[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) pr[i] = k0 + i * T < h.P ? __ldg(&pairs[k0 + i * T]) : make_int2(-1, -1);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int x = pr[i].x, y = pr[i].y;
+            if (x < 0 || y < 0 || x >= S || y >= S || sc.sfr[x] < 0 || sc.sfr[y] < 0) continue;
+            const uint32_t b0 = atomicOr(&B.adj[x * adj_words + (y >> 5)], 1u << (y & 31)) >> (y & 31);
+            const uint32_t b1 = atomicOr(&B.adj[y * adj_words + (x >> 5)], 1u << (x & 31)) >> (x & 31);
+            if ((b0 | b1) & 1u) B.next[1] = 1;
+        }
     }
     // local transforms, a (waypoint, joint) per thread, then the chain: row r of a
     // frame needs row r of its parent's only, so a thread per (waypoint, row)
@@ -666,171 +710,188 @@ __global__ void __launch_bounds__(THREADS, MINBLOCKS)
         const float* x = B.ctr + s * 96 + w;
         return make_float4(x[0], x[32], x[64], sc.sph[s].w);
     };
-    // 2. units
     float total = 0.0f;
-    const int n_world = (S + 1) >> 1, n_units = n_world + (h.P + 31) / 32;
+    // 2. units
+    const int n_world = (S + 1) >> 1, n_units = 2 * n_world;
+    const bool repeats = B.next[1] != 0;
+    // how often the list has the pair of spheres i and j (both ways; twice for a sphere with itself), once unless it repeats pairs
+    auto times = [&](int i, int j) {
+        int n = 0;
+        for (int k0 = 0; k0 < h.P; k0 += 32) {
+            const int2 pr = k0 + lane < h.P ? __ldg(&pairs[k0 + lane]) : make_int2(-1, -1);
+            n += __popc(__ballot_sync(kAll, pr.x == i && pr.y == j)) + __popc(__ballot_sync(kAll, pr.x == j && pr.y == i));
+        }
+        return n;
+    };
     while (true) {
         int u = 0;
         if (lane == 0) u = atomicAdd(B.next, 1);
         u = part + parts * __shfl_sync(kAll, u, 0);
         if (u >= n_units) break;
+        // spheres 2u and 2u + 1 against every primitive, or against their self-pair partners; an absent one's terms
+        // vanish (its radius is far below 0)
+        const bool world = u < n_world;
+        if (!world) u -= n_world;
+        const int Ns = world ? h.Ns : 0, Nc = world ? h.Nc : 0, Nb = world ? h.Nb : 0, Nh = world ? h.Nh : 0;
+        const int words = world ? 0 : adj_words;
         float cost = 0.0f;  // of this unit (short sums lose less)
-        if (u < n_world) {
-            // spheres 2u and 2u + 1 against every primitive; an absent one's terms vanish (its radius is far below 0)
-            float4 c[2];
-            float gx[2], gy[2], gz[2];
-            bool on[2];
+        float4 c[2];
+        float gx[2], gy[2], gz[2];
+        bool on[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int s = 2 * u + k;
+            on[k] = s < S && sc.sfr[min(s, S - 1)] >= 0;
+            c[k] = centre(min(s, S - 1), lane);
+            if (!on[k]) c[k].w = -1e30f;
+            gx[k] = gy[k] = gz[k] = 0.0f;
+        }
+        for (int o = 0; o < Ns; ++o) {
+            const float4 ob = sc.ws[2 * o + 1];
+            const float ro = -0.5f * sc.ws[2 * o].w;
+            float dx[2], dy[2], dz[2], rn[2], z[2], sig[2];
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
-                const int s = 2 * u + k;
-                on[k] = s < S && sc.sfr[min(s, S - 1)] >= 0;
-                c[k] = centre(min(s, S - 1), lane);
-                if (!on[k]) c[k].w = -1e30f;
-                gx[k] = gy[k] = gz[k] = 0.0f;
+                dx[k] = c[k].x - ob.x; dy[k] = c[k].y - ob.y; dz[k] = c[k].z - ob.z;
+                const float d2 = wide_max(fmaf(dx[k], dx[k], fmaf(dy[k], dy[k], dz[k] * dz[k])), 1e-36f);
+                rn[k] = wide_rsqrt(d2);
+                z[k] = a.beta * (a.margin - (d2 * rn[k] - c[k].w - ro));
             }
-            for (int o = 0; o < h.Ns; ++o) {
-                const float4 ob = sc.ws[2 * o + 1];
-                const float ro = -0.5f * sc.ws[2 * o].w;
+            if (wide_terms<2>(z, cost, sig)) {
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const float m = -sig[k] * rn[k];
+                    gx[k] = fmaf(m, dx[k], gx[k]); gy[k] = fmaf(m, dy[k], gy[k]); gz[k] = fmaf(m, dz[k], gz[k]);
+                }
+            }
+        }
+        for (int o = 0; o < Nc; ++o) {
+            const float4 p1 = sc.wc[3 * o], dp = sc.wc[3 * o + 1], dl = sc.wc[3 * o + 2];
+            float ex[2], ey[2], ez[2], rn[2], z[2], sig[2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const float u_ = __saturatef(fmaf(dp.x, c[k].x, fmaf(dp.y, c[k].y, fmaf(dp.z, c[k].z, dp.w))));
+                ex[k] = fmaf(-u_, dl.x, c[k].x - p1.x);
+                ey[k] = fmaf(-u_, dl.y, c[k].y - p1.y);
+                ez[k] = fmaf(-u_, dl.z, c[k].z - p1.z);
+                const float d2 = wide_max(fmaf(ex[k], ex[k], fmaf(ey[k], ey[k], ez[k] * ez[k])), 1e-36f);
+                rn[k] = wide_rsqrt(d2);
+                z[k] = a.beta * (a.margin - (d2 * rn[k] - c[k].w - p1.w));
+            }
+            if (wide_terms<2>(z, cost, sig)) {
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const float m = -sig[k] * rn[k];
+                    gx[k] = fmaf(m, ex[k], gx[k]); gy[k] = fmaf(m, ey[k], gy[k]); gz[k] = fmaf(m, ez[k], gz[k]);
+                }
+            }
+        }
+        for (int o = 0; o < Nb; ++o) {
+            // signed distance as in smooth_kernel, in units of kBoxScale metres (records are stored scaled)
+            const float4 a0 = sc.wb[4 * o], a1 = sc.wb[4 * o + 1], a2 = sc.wb[4 * o + 2], hl = sc.wb[4 * o + 3];
+            float l0[2], l1[2], l2[2], rn[2], z[2], sig[2];
+            bool outside[2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                l0[k] = fmaf(a0.x, c[k].x, fmaf(a0.y, c[k].y, fmaf(a0.z, c[k].z, a0.w)));
+                l1[k] = fmaf(a1.x, c[k].x, fmaf(a1.y, c[k].y, fmaf(a1.z, c[k].z, a1.w)));
+                l2[k] = fmaf(a2.x, c[k].x, fmaf(a2.y, c[k].y, fmaf(a2.z, c[k].z, a2.w)));
+                const float q0 = fabsf(l0[k]) - hl.x, q1 = fabsf(l1[k]) - hl.y, q2 = fabsf(l2[k]) - hl.z;
+                const float p0 = fmaxf(q0, 0.0f), p1 = fmaxf(q1, 0.0f), p2 = fmaxf(q2, 0.0f);
+                const float out2 = fmaf(p0, p0, fmaf(p1, p1, p2 * p2));
+                outside[k] = out2 > 0.0f;
+                rn[k] = outside[k] ? rsqrtf(out2) : 0.0f;
+                const float d = kBoxScale * (outside[k] ? out2 * rn[k] : fmaxf(q0, fmaxf(q1, q2))) - c[k].w;
+                z[k] = a.beta * (a.margin - d);
+            }
+            if (wide_terms<2>(z, cost, sig)) {
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const float q0 = fabsf(l0[k]) - hl.x, q1 = fabsf(l1[k]) - hl.y, q2 = fabsf(l2[k]) - hl.z;
+                    const float qmax = fmaxf(q0, fmaxf(q1, q2)), m = -kBoxScale * sig[k];  // the axes are stored times kBoxInv
+                    const bool k0 = q0 == qmax, k1 = !k0 && q1 == qmax, k2 = !k0 && !k1;
+                    const float c0 = copysignf(outside[k] ? fmaxf(q0, 0.0f) * rn[k] : (k0 ? 1.0f : 0.0f), l0[k]);
+                    const float c1 = copysignf(outside[k] ? fmaxf(q1, 0.0f) * rn[k] : (k1 ? 1.0f : 0.0f), l1[k]);
+                    const float c2 = copysignf(outside[k] ? fmaxf(q2, 0.0f) * rn[k] : (k2 ? 1.0f : 0.0f), l2[k]);
+                    gx[k] = fmaf(m, fmaf(c0, a0.x, fmaf(c1, a1.x, c2 * a2.x)), gx[k]);
+                    gy[k] = fmaf(m, fmaf(c0, a0.y, fmaf(c1, a1.y, c2 * a2.y)), gy[k]);
+                    gz[k] = fmaf(m, fmaf(c0, a0.z, fmaf(c1, a1.z, c2 * a2.z)), gz[k]);
+                }
+            }
+        }
+        for (int o = 0; o < Nh; ++o) {
+            const float4 hs = sc.wh[o];
+            float z[2], sig[2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+                z[k] = a.beta * (a.margin - (fmaf(hs.x, c[k].x, fmaf(hs.y, c[k].y, fmaf(hs.z, c[k].z, hs.w))) - c[k].w));
+            if (wide_terms<2>(z, cost, sig)) {
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    gx[k] = fmaf(-sig[k], hs.x, gx[k]); gy[k] = fmaf(-sig[k], hs.y, gy[k]); gz[k] = fmaf(-sig[k], hs.z, gz[k]);
+                }
+            }
+        }
+        const bool odd = 2 * u + 1 < S;
+        for (int word = 0; word < words; ++word) {
+            const uint32_t w0 = B.adj[2 * u * adj_words + word], w1 = odd ? B.adj[(2 * u + 1) * adj_words + word] : 0u;
+            for (uint32_t rest = w0 | w1; rest; rest &= rest - 1u) {
+                const int bit = __ffs(rest) - 1, j = 32 * word + bit;
+                int n[2] = {(int)(w0 >> bit & 1u), (int)(w1 >> bit & 1u)};
+                if (repeats) {
+                    n[0] = n[0] ? times(2 * u, j) : 0;
+                    n[1] = n[1] ? times(2 * u + 1, j) : 0;
+                }
+                const float4 cj = centre(j, lane);
                 float dx[2], dy[2], dz[2], rn[2], z[2], sig[2];
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
-                    dx[k] = c[k].x - ob.x; dy[k] = c[k].y - ob.y; dz[k] = c[k].z - ob.z;
+                    dx[k] = c[k].x - cj.x; dy[k] = c[k].y - cj.y; dz[k] = c[k].z - cj.z;
                     const float d2 = wide_max(fmaf(dx[k], dx[k], fmaf(dy[k], dy[k], dz[k] * dz[k])), 1e-36f);
                     rn[k] = wide_rsqrt(d2);
-                    z[k] = a.beta * (a.margin - (d2 * rn[k] - c[k].w - ro));
+                    z[k] = a.beta * (a.margin - (d2 * rn[k] - c[k].w - cj.w));
                 }
-                if (wide_terms<2>(z, cost, sig)) {
+                for (; n[0] > 0 || n[1] > 0; --n[0], --n[1]) {
+                    if (n[0] <= 0) z[0] = -1e30f;  // not a pair: no term
+                    if (n[1] <= 0) z[1] = -1e30f;
+                    if (wide_terms<2>(z, cost, sig)) {
 #pragma unroll
-                    for (int k = 0; k < 2; ++k) {
-                        const float m = -sig[k] * rn[k];
-                        gx[k] = fmaf(m, dx[k], gx[k]); gy[k] = fmaf(m, dy[k], gy[k]); gz[k] = fmaf(m, dz[k], gz[k]);
+                        for (int k = 0; k < 2; ++k) {
+                            if (n[k] <= 0) continue;
+                            const float m = -sig[k] * rn[k];
+                            gx[k] = fmaf(m, dx[k], gx[k]); gy[k] = fmaf(m, dy[k], gy[k]); gz[k] = fmaf(m, dz[k], gz[k]);
+                        }
                     }
                 }
             }
-            for (int o = 0; o < h.Nc; ++o) {
-                const float4 p1 = sc.wc[3 * o], dp = sc.wc[3 * o + 1], dl = sc.wc[3 * o + 2];
-                float ex[2], ey[2], ez[2], rn[2], z[2], sig[2];
-#pragma unroll
-                for (int k = 0; k < 2; ++k) {
-                    const float u_ = __saturatef(fmaf(dp.x, c[k].x, fmaf(dp.y, c[k].y, fmaf(dp.z, c[k].z, dp.w))));
-                    ex[k] = fmaf(-u_, dl.x, c[k].x - p1.x);
-                    ey[k] = fmaf(-u_, dl.y, c[k].y - p1.y);
-                    ez[k] = fmaf(-u_, dl.z, c[k].z - p1.z);
-                    const float d2 = wide_max(fmaf(ex[k], ex[k], fmaf(ey[k], ey[k], ez[k] * ez[k])), 1e-36f);
-                    rn[k] = wide_rsqrt(d2);
-                    z[k] = a.beta * (a.margin - (d2 * rn[k] - c[k].w - p1.w));
-                }
-                if (wide_terms<2>(z, cost, sig)) {
-#pragma unroll
-                    for (int k = 0; k < 2; ++k) {
-                        const float m = -sig[k] * rn[k];
-                        gx[k] = fmaf(m, ex[k], gx[k]); gy[k] = fmaf(m, ey[k], gy[k]); gz[k] = fmaf(m, ez[k], gz[k]);
-                    }
-                }
-            }
-            for (int o = 0; o < h.Nb; ++o) {
-                // signed distance as in smooth_kernel, in units of kBoxScale metres (records are stored scaled)
-                const float4 a0 = sc.wb[4 * o], a1 = sc.wb[4 * o + 1], a2 = sc.wb[4 * o + 2], hl = sc.wb[4 * o + 3];
-                float l0[2], l1[2], l2[2], rn[2], z[2], sig[2];
-                bool outside[2];
-#pragma unroll
-                for (int k = 0; k < 2; ++k) {
-                    l0[k] = fmaf(a0.x, c[k].x, fmaf(a0.y, c[k].y, fmaf(a0.z, c[k].z, a0.w)));
-                    l1[k] = fmaf(a1.x, c[k].x, fmaf(a1.y, c[k].y, fmaf(a1.z, c[k].z, a1.w)));
-                    l2[k] = fmaf(a2.x, c[k].x, fmaf(a2.y, c[k].y, fmaf(a2.z, c[k].z, a2.w)));
-                    const float q0 = fabsf(l0[k]) - hl.x, q1 = fabsf(l1[k]) - hl.y, q2 = fabsf(l2[k]) - hl.z;
-                    const float p0 = fmaxf(q0, 0.0f), p1 = fmaxf(q1, 0.0f), p2 = fmaxf(q2, 0.0f);
-                    const float out2 = fmaf(p0, p0, fmaf(p1, p1, p2 * p2));
-                    outside[k] = out2 > 0.0f;
-                    rn[k] = outside[k] ? rsqrtf(out2) : 0.0f;
-                    const float d = kBoxScale * (outside[k] ? out2 * rn[k] : fmaxf(q0, fmaxf(q1, q2))) - c[k].w;
-                    z[k] = a.beta * (a.margin - d);
-                }
-                if (wide_terms<2>(z, cost, sig)) {
-#pragma unroll
-                    for (int k = 0; k < 2; ++k) {
-                        const float q0 = fabsf(l0[k]) - hl.x, q1 = fabsf(l1[k]) - hl.y, q2 = fabsf(l2[k]) - hl.z;
-                        const float qmax = fmaxf(q0, fmaxf(q1, q2)), m = -kBoxScale * sig[k];  // the axes are stored times kBoxInv
-                        const bool k0 = q0 == qmax, k1 = !k0 && q1 == qmax, k2 = !k0 && !k1;
-                        const float c0 = copysignf(outside[k] ? fmaxf(q0, 0.0f) * rn[k] : (k0 ? 1.0f : 0.0f), l0[k]);
-                        const float c1 = copysignf(outside[k] ? fmaxf(q1, 0.0f) * rn[k] : (k1 ? 1.0f : 0.0f), l1[k]);
-                        const float c2 = copysignf(outside[k] ? fmaxf(q2, 0.0f) * rn[k] : (k2 ? 1.0f : 0.0f), l2[k]);
-                        gx[k] = fmaf(m, fmaf(c0, a0.x, fmaf(c1, a1.x, c2 * a2.x)), gx[k]);
-                        gy[k] = fmaf(m, fmaf(c0, a0.y, fmaf(c1, a1.y, c2 * a2.y)), gy[k]);
-                        gz[k] = fmaf(m, fmaf(c0, a0.z, fmaf(c1, a1.z, c2 * a2.z)), gz[k]);
-                    }
-                }
-            }
-            for (int o = 0; o < h.Nh; ++o) {
-                const float4 hs = sc.wh[o];
-                float z[2], sig[2];
-#pragma unroll
-                for (int k = 0; k < 2; ++k)
-                    z[k] = a.beta * (a.margin - (fmaf(hs.x, c[k].x, fmaf(hs.y, c[k].y, fmaf(hs.z, c[k].z, hs.w))) - c[k].w));
-                if (wide_terms<2>(z, cost, sig)) {
-#pragma unroll
-                    for (int k = 0; k < 2; ++k) {
-                        gx[k] = fmaf(-sig[k], hs.x, gx[k]); gy[k] = fmaf(-sig[k], hs.y, gy[k]); gz[k] = fmaf(-sig[k], hs.z, gz[k]);
-                    }
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                if (!on[k]) continue;
-                float* G = B.g + (2 * u + k) * 96 + lane;
-                atomicAdd(G, gx[k]); atomicAdd(G + 32, gy[k]); atomicAdd(G + 64, gz[k]);
-            }
-        } else {
-            // 32 self pairs: the first sphere's gradient stays in registers while it stays the same
-            const int k0 = (u - n_world) * 32, n = min(32, h.P - k0);
-            const int2 mine = lane < n ? __ldg(&pairs[k0 + lane]) : make_int2(-1, -1);
-            int cur = -1;
-            float4 ci = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            float gx = 0.0f, gy = 0.0f, gz = 0.0f;
-            auto flush = [&]() {
-                if (cur < 0) return;
-                float* G = B.g + cur * 96 + lane;
-                atomicAdd(G, gx); atomicAdd(G + 32, gy); atomicAdd(G + 64, gz);
-                gx = gy = gz = 0.0f;
-            };
-            for (int k = 0; k < n; ++k) {
-                const int pi = __shfl_sync(kAll, mine.x, k), pj = __shfl_sync(kAll, mine.y, k);
-                if (pi < 0 || pj < 0 || pi >= S || pj >= S || sc.sfr[pi] < 0 || sc.sfr[pj] < 0) continue;
-                if (pi != cur) {
-                    flush();
-                    cur = pi;
-                    ci = centre(pi, lane);
-                }
-                const float4 cj = centre(pj, lane);
-                const float dx = ci.x - cj.x, dy = ci.y - cj.y, dz = ci.z - cj.z;
-                const float d2 = wide_max(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), 1e-36f), rn = wide_rsqrt(d2);
-                const float z[1] = {a.beta * (a.margin - (d2 * rn - ci.w - cj.w))};
-                float sig[1];
-                if (wide_terms<1>(z, cost, sig)) {
-                    const float m = -sig[0] * rn;
-                    const float x = m * dx, y = m * dy, z = m * dz;
-                    gx += x; gy += y; gz += z;
-                    float* G = B.g + pj * 96 + lane;
-                    atomicAdd(G, -x); atomicAdd(G + 32, -y); atomicAdd(G + 64, -z);
-                }
-            }
-            flush();
         }
-        total += cost;
+        // the two units of a sphere add to zero: of two terms the order does not matter
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            if (!on[k]) continue;
+            float* G = B.g + (2 * u + k) * 96 + lane;
+            atomicAdd(G, gx[k]); atomicAdd(G + 32, gy[k]); atomicAdd(G + 64, gz[k]);
+        }
+        total = fmaf(world ? 1.0f : 0.5f, cost, total);  // a self pair is in the units of both its spheres
     }
     atomicAdd(&B.cost[lane], total);
     __syncthreads();
-    // 3. frame sums
-    for (int i = tid; i < S * 32; i += T) {
-        const int s = i >> 5, w = i & 31, f = sc.sfr[s];
-        if (f < 0) continue;
-        const float4 c = centre(s, w);
-        const float x = B.g[s * 96 + w], y = B.g[s * 96 + 32 + w], z = B.g[s * 96 + 64 + w];
-        float* A = B.acc + f * 192 + w;
-        atomicAdd(A, x); atomicAdd(A + 32, y); atomicAdd(A + 64, z);
-        atomicAdd(A + 96, c.y * z - c.z * y);
-        atomicAdd(A + 128, c.z * x - c.x * z);
-        atomicAdd(A + 160, c.x * y - c.y * x);
+    // 3. frame sums, a joint per warp over the spheres in order
+    for (int j = warp; j < J; j += WARPS) {
+        float A[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        for (int s0 = 0; s0 < S; s0 += 32) {
+            for (unsigned on = __ballot_sync(kAll, s0 + lane < S && sc.sfr[min(s0 + lane, S - 1)] == j); on; on &= on - 1u) {
+                const int s = s0 + __ffs(on) - 1;
+                const float4 c = centre(s, lane);
+                const float x = B.g[s * 96 + lane], y = B.g[s * 96 + 32 + lane], z = B.g[s * 96 + 64 + lane];
+                A[0] += x; A[1] += y; A[2] += z;
+                A[3] += c.y * z - c.z * y;
+                A[4] += c.z * x - c.x * z;
+                A[5] += c.x * y - c.y * x;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 6; ++k) B.acc[j * 192 + 32 * k + lane] = A[k];
     }
     __syncthreads();
     // 4. dC/dv of every joint from its subtree's sums (dv in the place of q)
@@ -860,6 +921,7 @@ __global__ void __launch_bounds__(THREADS, MINBLOCKS)
     __syncthreads();
     // 5. joint-space gradient + length term, coalesced over (waypoint, dimension)
     const float inv_beta = 1.0f / a.beta;
+    float* share = B.g;  // [nw][dim], in the place of the sphere gradients
     for (int i = tid; i < nw * dim; i += T) {
         const int w = i / dim, d = i - w * dim;
         float gq = 0.0f;
@@ -884,8 +946,18 @@ __global__ void __launch_bounds__(THREADS, MINBLOCKS)
         }
         if (a.grad) {
             if (parts == 1) a.grad[at] = gq;
-            else atomicAdd(&a.grad[at], gq);  // zero before the launch
+            else if (parts == 2) atomicAdd(&a.grad[at], gq);  // zero before the launch; of two terms the order does not matter
+            else share[i] = gq;
         }
+    }
+    if (parts > 2 && a.grad) {  // the parts are the CTAs of a cluster: their shares are added in their order
+        cluster_sync();
+        for (int i = part * T + tid; i < nw * dim; i += parts * T) {
+            float sum = 0.0f;
+            for (int k = 0; k < parts; ++k) sum += cluster_load(share + i, k);
+            a.grad[first * dim + i] = sum;
+        }
+        cluster_sync();  // the shares are read before a CTA ends
     }
     __syncthreads();
     // 6. cost per path: one atomic per CTA when its waypoints are of one path
@@ -913,32 +985,43 @@ cudaError_t launch_smooth(const unsigned char* blob, size_t blob_stride, int blo
                  margin, beta, w_len, cost, grad};
     const bool shared = blob_stride == 0 && pairs_stride == 0;
     if (shared && !ordered && cost && J <= 32) {
+        // 256 threads and up to three CTAs per SM (registers), or 512 where
+        // shared memory allows only one (large robots)
         const size_t wide = (size_t)blob_cap + smooth_wide_bytes(J, S);
+        const int by_smem = (int)((device_max_smem() + 1024) / (wide + 1024 + 64));
+        const bool big = by_smem < 2;
         const long long ctas = ((long long)P * W + 31) / 32;
         if (wide + 64 <= device_max_smem() && ctas * 8 <= INT32_MAX) {
-            // 256 threads and up to three CTAs per SM (registers), or 512 where
-            // shared memory allows only one (large robots)
-            const int by_smem = (int)((device_max_smem() + 1024) / (wide + 1024 + 64));
-            const bool big = by_smem < 2;
             void (*const kern)(SmoothArgs, int, int) = big ? smooth_wide_kernel<512, 1> : smooth_wide_kernel<256, 3>;
             // Several CTAs may share 32 waypoints, each with a share of the pairs,
             // and add up their gradients (which are linear in the pairs' terms):
             // as many as make the last wave of the launch full, a twelfth of a
-            // CTA's time being its frames and closing sums.
+            // CTA's time being its frames and closing sums.  Two add into zeroed
+            // memory; four or eight are a cluster, which adds in their order.
             const long long room = (long long)device_sm_count() * (big ? 1 : std::min(by_smem, 3));
             int parts = 1;
             double best = 1e30;
-            for (int p = 1; p <= 8; ++p) {
+            for (int p = 1; p <= 8; p *= 2) {
                 const double c = (double)((ctas * p + room - 1) / room) * (1.0 / p + 1.0 / 12);
                 if (c < 0.97 * best) { best = c; parts = p; }
             }
-            if (parts > 1 && grad &&
+            if (parts == 2 && grad &&
                 (e = cudaMemsetAsync(grad, 0, (size_t)P * W * dim * sizeof(float), st)) != cudaSuccess)
                 return e;
             static DynLimit limit[2][kDynLimitDevices];
             if ((e = raise_dyn_limit(reinterpret_cast<const void*>(kern), limit[big ? 1 : 0], wide)) != cudaSuccess)
                 return e;
-            kern<<<(unsigned)(ctas * parts), big ? 512 : 256, wide, st>>>(a, blob_cap, parts);
+            cudaLaunchAttribute cluster;
+            cluster.id = cudaLaunchAttributeClusterDimension;
+            cluster.val.clusterDim = {(unsigned)parts, 1u, 1u};
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)(ctas * parts));
+            cfg.blockDim = dim3(big ? 512 : 256);
+            cfg.dynamicSmemBytes = wide;
+            cfg.stream = st;
+            cfg.attrs = &cluster;
+            cfg.numAttrs = parts > 2 ? 1 : 0;
+            if ((e = cudaLaunchKernelEx(&cfg, kern, a, blob_cap, parts)) != cudaSuccess) return e;
             return cudaGetLastError();
         }
     }

@@ -41,8 +41,9 @@ class SmoothContext:
                             self.device)
 
     def cost_grad(self, waypoints: torch.Tensor, need_grad: bool = True, ordered: bool = False):
-        """cost [P] and gradient [P, W, dim]; ``ordered``: every sum in a fixed
-        order, so the gradient is the same bits in every run (descents)."""
+        """cost [P] and gradient [P, W, dim], the gradient the same bits in every run
+        of the same call; ``ordered``: also whatever paths are beside it, as
+        BatchSmoothContext's (descents)."""
         wp = waypoints.detach().to(self.device, torch.float32).contiguous()
         P, W, dim = wp.shape
         cost = torch.empty((P,), dtype=torch.float32, device=self.device)

@@ -72,3 +72,44 @@ def test_pair_lists(cuda, form):
         c, g = smooth_grad({**ctx, "self_pairs": base["self_pairs"][ok]}, x[p].astype(np.float64), 0.02, 50.0, 1.0)
         assert abs(cost[p].item() - c) <= 1e-4 * abs(c)
         assert np.linalg.norm(grad[p].cpu().numpy().astype(np.float64) - g) <= 5e-4 * np.linalg.norm(g)
+
+
+@pytest.mark.parametrize("form", ["by_link", "reversed", "shuffled", "swapped", "repeated", "both_ways", "itself", "invalid", "first_1",
+                                  "unsorted_spheres"])
+def test_pair_lists_of_one_scene(cuda, form):
+    """The same lists with one scene for all paths (a lane per waypoint, a pair computed once for each of its spheres):
+    lists that repeat a pair, name it both ways or pair a sphere with itself are added up as often as they say."""
+    from oracle.smooth_autodiff import smooth_grad
+    from prrtc_b200.smoothing import SmoothContext
+
+    robot = scenes.arm(2)
+    ctx = build_collision_context(robot, scenes.tabletop_world(np.random.default_rng(3)))
+    for k in ("coarse_self_pairs", "self_pair_ranges"):
+        ctx[k] = ctx[k][:0]
+    if form == "unsorted_spheres":
+        perm = np.random.default_rng(3).permutation(len(ctx["sphere_link_idx"]))
+        for k in ("sphere_link_idx", "sphere_local", "sphere_radius"):
+            ctx[k] = ctx[k][perm]
+        ctx["self_pairs"] = np.argsort(perm).astype(np.int32)[ctx["self_pairs"]]
+    pairs = ctx["self_pairs"]
+    if form == "both_ways":
+        pairs = np.concatenate([pairs[:40], pairs[20:60, ::-1], pairs[:3]])
+    elif form == "itself":
+        pairs = np.insert(pairs, np.arange(0, 100, 9), np.arange(0, 100, 9)[:, None] % 50, axis=0)
+    else:
+        pairs = _pairs(form, pairs)
+    ctx["self_pairs"] = np.ascontiguousarray(pairs)
+    rng = np.random.default_rng(11)
+    x = (rng.uniform(-0.4, 0.4, (3, 1, robot.dim)) + rng.normal(0, 0.05, (3, 9, robot.dim))).astype(np.float32)
+    sctx = SmoothContext(ctx, robot.dim, device=cuda)
+    xd = torch.from_numpy(x).to(cuda)
+    cost, grad = sctx.cost_grad(xd)
+    assert torch.equal(grad, sctx.cost_grad(xd)[1])
+    ok = ((pairs >= 0) & (pairs < len(ctx["sphere_link_idx"]))).all(1) & (pairs[:, 0] != pairs[:, 1])
+    # a sphere paired with itself: no gradient, and a cost that is added by hand (distance -2 r)
+    r = ctx["sphere_radius"][pairs[(pairs[:, 0] == pairs[:, 1]) & (pairs[:, 0] >= 0), 0]].astype(np.float64)
+    alone = 9 * float(np.logaddexp(0.0, 50.0 * (0.02 + 2 * r)).sum()) / 50.0
+    for p in range(3):
+        c, g = smooth_grad({**ctx, "self_pairs": pairs[ok]}, x[p].astype(np.float64), 0.02, 50.0, 1.0)
+        assert abs(cost[p].item() - c - alone) <= 1e-4 * abs(c + alone)
+        assert np.linalg.norm(grad[p].cpu().numpy().astype(np.float64) - g) <= 5e-4 * np.linalg.norm(g)

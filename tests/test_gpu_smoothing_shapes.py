@@ -130,3 +130,20 @@ def test_a_waypoint_that_is_not_a_number(cuda, scene, bad):
     for p in (0, 2):  # neighbouring lanes may take the full softplus with it: a term's rounding, at most 1e-6 of it
         assert torch.allclose(cost[p], want_cost[p], rtol=1e-5, atol=0.0)
         assert torch.allclose(grad[p], want_grad[p], rtol=1e-5, atol=1e-5 * float(want_grad[p].abs().max()))
+
+
+@pytest.mark.parametrize("joints,P,W", [(7, 1, 64), (7, 14, 33), (7, 97, 33), (7, 194, 33), (7, 427, 33), (18, 3, 40), (18, 90, 40)])
+def test_gradients_are_the_same_bits_in_every_run(cuda, joints, P, W):
+    """From a few waypoints, shared by eight CTAs, to more than the GPU holds at once: five calls, the same gradient,
+    and the one of the kernel with a warp per waypoint within the two kernels' bounds (each 5e-4 of the path's)."""
+    from prrtc_b200.smoothing import SmoothContext
+
+    robot = scenes.dual_arm(0) if joints == 18 else scenes.arm(1, joints)
+    world = scenes.large_world(np.random.default_rng(3)) if joints == 18 else scenes.tabletop_world(np.random.default_rng(3))
+    sctx = SmoothContext(build_collision_context(robot, world), robot.dim, device=cuda)
+    x = torch.from_numpy(_paths(robot, P, W, 5)).to(cuda)
+    grads = [sctx.cost_grad(x)[1].clone() for _ in range(5)]
+    assert all(torch.equal(g, grads[0]) for g in grads[1:])
+    want = sctx.cost_grad(x, ordered=True)[1]
+    off = torch.linalg.norm((grads[0] - want).reshape(P, -1), dim=1)
+    assert bool((off <= 1e-3 * torch.linalg.norm(want.reshape(P, -1), dim=1)).all())
