@@ -23,6 +23,7 @@
 #include <math.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "kernels.h"
 #include "prrtc_device.cuh"
@@ -1039,16 +1040,21 @@ cudaError_t launch_smooth(const unsigned char* blob, size_t blob_stride, int blo
         kern<<<blocks(WARPS), WARPS * 32, smem, st>>>(a, blob_cap, per_path(WARPS));
         return cudaGetLastError();
     }
-    // scene or robot too large to stage: fewer waypoints per CTA, the scene in global memory
-    constexpr int FEW = 4;
-    smem = (size_t)FEW * smooth_warp_floats(J, S) * sizeof(float);
-    auto kern = cost ? smooth_kernel<FEW, false, true> : smooth_kernel<FEW, false, false>;
-    static DynLimit limit[2][kDynLimitDevices];
-    if (smem > 48 * 1024 &&
-        (e = raise_dyn_limit(reinterpret_cast<const void*>(kern), limit[cost ? 1 : 0], smem)) != cudaSuccess)
-        return e;
-    kern<<<blocks(FEW), FEW * 32, smem, st>>>(a, 0, per_path(FEW));
-    return cudaGetLastError();
+    // scene or robot too large to stage: fewer waypoints per CTA, the scene in
+    // global memory (four take robots of about 1,760 spheres, two twice that)
+    auto few = [&](auto count) {
+        constexpr int FEW = decltype(count)::value;
+        const size_t bytes = (size_t)FEW * smooth_warp_floats(J, S) * sizeof(float);
+        auto kern = cost ? smooth_kernel<FEW, false, true> : smooth_kernel<FEW, false, false>;
+        static DynLimit limit[2][kDynLimitDevices];
+        if (bytes > 48 * 1024 &&
+            (e = raise_dyn_limit(reinterpret_cast<const void*>(kern), limit[cost ? 1 : 0], bytes)) != cudaSuccess)
+            return e;
+        kern<<<blocks(FEW), FEW * 32, bytes, st>>>(a, 0, per_path(FEW));
+        return cudaGetLastError();
+    };
+    if ((size_t)4 * smooth_warp_floats(J, S) * sizeof(float) + 64 <= device_max_smem()) return few(std::integral_constant<int, 4>());
+    return few(std::integral_constant<int, 2>());
 }
 
 }  // namespace prrtc

@@ -147,3 +147,25 @@ def test_gradients_are_the_same_bits_in_every_run(cuda, joints, P, W):
     want = sctx.cost_grad(x, ordered=True)[1]
     off = torch.linalg.norm((grads[0] - want).reshape(P, -1), dim=1)
     assert bool((off <= 1e-3 * torch.linalg.norm(want.reshape(P, -1), dim=1)).all())
+
+
+@pytest.mark.parametrize("spheres", [1200, 1764, 1790, 1795])
+def test_robots_of_many_spheres(cuda, spheres):
+    """Robots whose sphere tables fill shared memory: scenes that are not staged, up to the largest robot that four
+    waypoints per CTA took before their sums had a row of their own (1,795 spheres with 7 joints)."""
+    from prrtc_b200.smoothing import BatchSmoothContext, SmoothContext
+
+    robot = scenes.arm(2)
+    ctx = build_collision_context(robot, scenes.spheres_world(np.random.default_rng(4), 3))
+    rng = np.random.default_rng(8)
+    pick = rng.integers(0, len(ctx["sphere_link_idx"]), spheres)
+    for k in ("sphere_link_idx", "sphere_local", "sphere_radius"):
+        ctx[k] = ctx[k][pick]
+    ctx["sphere_local"] = (ctx["sphere_local"] + rng.uniform(-0.01, 0.01, (spheres, 3))).astype(np.float32)
+    ctx["self_pairs"] = ctx["self_pairs"][:7]
+    for k in ("coarse_self_pairs", "self_pair_ranges"):
+        ctx[k] = ctx[k][:0]
+    w = _paths(robot, 2, 3, 9)
+    x = torch.from_numpy(w).to(cuda)
+    for got in (SmoothContext(ctx, robot.dim, device=cuda).cost_grad(x), BatchSmoothContext([ctx] * 2, robot.dim, device=cuda).cost_grad(x)):
+        _check(*got, [ctx] * 2, w, 1.0)
