@@ -665,6 +665,7 @@ __device__ __forceinline__ void run_explorer(const Grp& grp, const PlanLaunch& L
                 sv = X.pre_solved;
                 sa = X.pre_a;
                 sb = X.pre_b;
+                X.pre = 0;  // for this iteration only: one without a nearest node reads none ahead
             } else {
                 // the three loads go out together: one round trip, not three
                 sv = ld_volatile(P.solved);
