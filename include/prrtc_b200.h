@@ -158,8 +158,8 @@ typedef struct {
 typedef struct {
     float edge_resolution;       /* >0: an edge gets max(granularity, ceil(len/res)) waypoints */
     int32_t threads_per_explorer;/* threads of one explorer (one explorer per CTA): 32, 64, 128
-                                    or 256; default: chosen by the launch (128 or 256).  A batch
-                                    of at most two explorers per SM is given 512. */
+                                    or 256; default: chosen by the launch (128 or 256, or 512
+                                    for a batch of at most two explorers per SM) */
     int32_t waypoint_chunk;      /* waypoints of an edge checked per CTA pass: 8, 16, 32 or 64
                                     (default 16).  The culled edge check (robots of up to 32
                                     joints with a coarse model) chooses its own pass size. */

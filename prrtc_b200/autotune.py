@@ -2,7 +2,8 @@
 
 For one capacity bucket, times a plan of the bucket's problems for each
 candidate (explorers per problem = samples per iteration, threads per explorer
-(one explorer per CTA), waypoints per shared-memory chunk, CTAs per SM) by solved plans per second: the median of three launches
+(one explorer per CTA), CTAs per SM, and waypoints per chunk where the edge
+check takes the caller's) by solved plans per second: the median of three launches
 per candidate, then a second round between the three best (six more launches
 each, taken in turn) decides; L2 is flushed before every timed launch.  Results
 are cached per (device, bucket, problem count, shape) in
@@ -20,8 +21,24 @@ SAMPLES = (1, 2, 4, 8, 16)
 THREADS = (64, 128, 256)  # 32 stays available (a one-warp CTA) but is slower on every bucket measured
 CHUNKS = (8, 16, 32, 64)  # 64: one pass for most edges of a 0.5 rad step at 0.01 rad resolution
 CTAS_PER_SM = (0, 2)  # 0: as many as fit; 2: two, with the rest of shared memory given to L1
-CANDIDATES = tuple((e, t, c, r) for r in CTAS_PER_SM for t in THREADS for c in CHUNKS for e in SAMPLES)
 CACHE = Path(os.environ.get("PRRTC_B200_CACHE", Path.home() / ".cache" / "prrtc_b200")) / "autotune.json"
+
+
+def _culled(ctx: dict) -> bool:
+    return all(ctx.get(k) is not None and len(ctx[k]) > 0 for k in ("fine_link_offsets", "coarse_sphere_radius")) \
+        and len(ctx["fk_parent_idx"]) <= 32
+
+
+def _candidates(problems, settings, sms: int) -> list[tuple]:
+    """(explorers, threads, chunk, CTAs per SM) to time, no launch twice: the culled
+    edge check (robots of up to 32 joints with a coarse model) chooses its own pass
+    size, so the chunk is an axis for other robots only; threads of 0 are the
+    launch's own choice, another one than 256 where there are at most two explorers
+    per SM."""
+    culled = _culled(problems[0].context)
+    chunks = (settings.waypoint_chunk,) if culled else CHUNKS
+    return [(e, t, c, r) for r in CTAS_PER_SM for t in (0,) + THREADS for c in chunks for e in SAMPLES
+            if t or (culled and e * len(problems) <= 2 * sms)]
 
 
 def _key(dev, N, problems, settings) -> str:
@@ -31,7 +48,8 @@ def _key(dev, N, problems, settings) -> str:
         caps = [int(c) for c in N]
         N = f"caps{max(caps)}x{len(caps)}h{hash(tuple(caps)) & 0xffffff:06x}"
     return (f"{name}|N{N}|B{len(problems)}|dim{p.dim}|S{p.context['sphere_radius'].shape[0]}|"
-            f"{settings.collision_checker}|res{settings.edge_resolution}|T{settings.threads_per_explorer}")
+            f"{settings.collision_checker}|res{settings.edge_resolution}|T{settings.threads_per_explorer}|"
+            f"{'culled' if _culled(p.context) else 'general'}")
 
 
 def _load() -> dict:
@@ -53,10 +71,11 @@ def _rate(pl, flush=None) -> float:
     return solved / (e0.elapsed_time(e1) * 1e-3)
 
 
-def choose(problems, N, settings, dev, candidates=CANDIDATES, use_cache: bool = True, finalists: int = 3,
+def choose(problems, N, settings, dev, candidates=None, use_cache: bool = True, finalists: int = 3,
            final_reps: int = 6) -> dict:
     """Best {num_new_samples, threads_per_explorer, waypoint_chunk, ctas_per_sm} for this bucket
-    (N: one tree capacity, or a per-problem list of them).
+    (N: one tree capacity, or a per-problem list of them; ``candidates``: what to
+    time, by default what differs for these problems).
 
     Two rounds: every candidate is timed by the median of three launches (the
     explorers race, so one launch is noisy); the best ``finalists`` are then
@@ -65,10 +84,12 @@ def choose(problems, N, settings, dev, candidates=CANDIDATES, use_cache: bool = 
     launches wins."""
     from .batch import BatchPlanner, PlanSettings
 
-    key = "v10|" + _key(dev, N, problems, settings)
+    key = "v11|" + _key(dev, N, problems, settings)
     cache = _load() if use_cache else {}
     if key in cache:
         return dict(cache[key])
+    if candidates is None:
+        candidates = _candidates(problems, settings, torch.cuda.get_device_properties(dev).multi_processor_count)
 
     def planner(c):
         E, T, CW, R = c

@@ -37,7 +37,7 @@ class PlanSettings:
     collision_checker: str = "binary_coarse_coop"
     collision_margin: float = 0.02
     edge_resolution: float = 0.01
-    threads_per_explorer: int = 128
+    threads_per_explorer: int = 0  # chosen by the launch
     waypoint_chunk: int = 16
     resident_ctas: int = 0
     tail_explorers: bool = True

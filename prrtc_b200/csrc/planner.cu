@@ -1096,17 +1096,18 @@ cudaError_t launch_plan(PlanLaunch& L, cudaStream_t st) {
     // leave room for its CTAs: a pass costs mostly the latency of its phases,
     // so fewer passes win (batches of 300 tabletop problems, E = 2: 2.49 -> 2.20
     // ms against 16 per pass; 61 dual-arm problems, E = 1: 7.3 -> 5.2 ms).
-    // Wide form: a batch of at most two explorers per SM leaves most of the GPU
-    // idle at the sizes it asks for, so each explorer gets 512 threads, one CTA
-    // per SM (200 tabletop problems, E = 1: 3.97 -> 3.74 ms against 256 threads; 61
-    // dual-arm problems: 6.7 -> 5.1 ms; at E = 2 x 512 problems it loses, 4.4
-    // -> 4.7 ms).
-    // So does a plain launch of at most one explorer per SM that asks for no size.
-    const bool wide = L.persistent ? (long long)L.B * L.E <= 2ll * device_sm_count()
-                                   : L.threads == 0 && (long long)L.B * L.E <= device_sm_count();
+    // Wide form, where the caller names no size: a batch of at most two explorers
+    // per SM leaves most of the GPU idle at 256 threads, so each explorer gets 512,
+    // one CTA per SM.  E = 1, a call in ms with 256 -> 512 threads: tabletop, 100
+    // problems 2.15 -> 1.96, 200 3.89 -> 3.72, 296 3.99 -> 3.86; dual arm, 61 7.03 ->
+    // 5.61, 149 9.92 -> 7.19, 296 11.04 -> 8.82; at E = 2 x 512 problems it loses,
+    // 4.4 -> 4.7.  So does a plain launch of at most one explorer per SM.
+    const long long explorers = (long long)L.B * L.E;
+    const bool wide = L.threads == 0 && explorers <= (L.persistent ? 2ll : 1ll) * device_sm_count();
+    const bool one_per_sm = wide || explorers <= device_sm_count();
     bool cull = false;
     if (L.cull) {
-        const size_t room = max_smem / (wide ? 1 : 2) - (wide ? 0 : 1024);
+        const size_t room = one_per_sm ? max_smem : max_smem / 2 - 1024;
         for (int cw = 64; cw >= 8 && !cull; cw /= 2) {
             // the buffers also hold the general checker's, for a scene that is not culled
             size_t need = (size_t)cull_smem_bytes(L.J, L.K, L.n_obs, cw);
