@@ -423,7 +423,7 @@ int prrtc_b200_check_configs_batch(const prrtc_batch_inputs_t* in, int32_t dim, 
     if (e != cudaSuccess) return cuda_fail(e);
     const size_t pstride = in->self_pairs_count ? (size_t)std::max(0, in->max_self_pairs) : 0;
     e = launch_check_batch(blobs, stride, in->self_pairs, pstride, in->batch, s.J, s.S, s.K, s.Q, dim, configs, offsets,
-                           n, verdicts, st);
+                           n, batch_sweep(mode, 0), verdicts, st);
     if (e == cudaErrorInvalidConfiguration) return PRRTC_B200_EUNSUPPORTED;
     return e == cudaSuccess ? PRRTC_B200_OK : cuda_fail(e);
 }

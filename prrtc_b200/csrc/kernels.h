@@ -154,7 +154,7 @@ cudaError_t launch_check(const unsigned char* blob, int blob_cap, const int32_t*
 // cudaErrorInvalidConfiguration when its buffers do not fit.
 cudaError_t launch_check_batch(const unsigned char* blobs, size_t blob_stride, const int32_t* pairs,
                                size_t pairs_stride, int n_scenes, int J, int S, int K, int Q, int dim,
-                               const float* configs, const int32_t* offsets, int n, int32_t* verdicts,
+                               const float* configs, const int32_t* offsets, int n, int full_sweep, int32_t* verdicts,
                                cudaStream_t st);
 
 // pointcloud.cu

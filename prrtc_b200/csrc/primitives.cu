@@ -653,27 +653,30 @@ static void check_go(const CheckLaunch& o, int full_sweep, const unsigned char* 
 // tabletop configurations 2117 -> 800 us, uneven scene 2055 -> 870 us, 60,000
 // dual-arm configurations 1332 -> 280 us (gated) and 981 -> 280 us (flat).
 //
-// A scene that is not culled (BlobHeader::cull) takes the general checker, 8
-// configurations at a time by the whole CTA, in the same shared memory.
+// A scene that is not culled (BlobHeader::cull: groups that do not cover the
+// spheres, ...) takes the general checker in the same shared memory, by the whole
+// CTA: up to CW configurations at a time, as many as the launch found room for, and
+// fewer where there are CTAs to share them; FULL as the general launch would sweep.
+template <bool FULL>
 static __device__ __noinline__ void check_general(const unsigned char* blob, const int2* pairs, const PcView* pc,
-                                                  unsigned char* smem, const float* configs, int n, int dim,
+                                                  unsigned char* smem, int CW, const float* configs, int n, int dim,
                                                   int32_t* verdicts) {
-    constexpr int CW = 8;
     Scene sc = scene_view(blob);
     sc.pairs = pairs;
     sc.pc = *pc;
+    CW = min(CW, max(1, (int)((n + (long long)gridDim.x - 1) / gridDim.x)));
     const CcBufs B = cc_bufs(smem, sc.h->J, sc.h->S, sc.h->K, sc.h->Q, CW);
     if (threadIdx.x == 0) B.hit[0] = B.hit[1] = 0u;
     int par = 0;
     __syncthreads();
-    for (int c0 = blockIdx.x * CW; c0 < n; c0 += gridDim.x * CW) {
-        const int nw = min(CW, n - c0);
+    for (long long c0 = (long long)blockIdx.x * CW; c0 < n; c0 += (long long)gridDim.x * CW) {
+        const int nw = (int)min((long long)CW, n - c0);
         for (int i = threadIdx.x; i < nw * dim; i += blockDim.x) {
             const int w = i / dim, d = i - w * dim;
             B.q[w * kDimMax + d] = configs[(size_t)(c0 + w) * dim + d];
         }
         __syncthreads();
-        const uint32_t hit = cc_chunk<false>(CtaGroup{}, sc, B, nw, false, par);
+        const uint32_t hit = cc_chunk<FULL>(CtaGroup{}, sc, B, nw, false, par);
         for (int w = threadIdx.x; w < nw; w += blockDim.x) verdicts[c0 + w] = (hit >> w) & 1u;
     }
 }
@@ -692,7 +695,7 @@ __global__ void __launch_bounds__(256, 3) check_cull_kernel(const unsigned char*
                                                             const int2* pairs, int J, int K, int dim, int CW,
                                                             const float* __restrict__ configs, int n,
                                                             int32_t* verdicts, PcView pc, CheckScenes scenes,
-                                                            EdgeHits edges) {
+                                                            EdgeHits edges, int general_cw, int full_sweep) {
     extern __shared__ __align__(128) unsigned char dsm[];
     __shared__ __align__(8) uint64_t mbar;
     if (scenes.offsets) {
@@ -719,7 +722,8 @@ __global__ void __launch_bounds__(256, 3) check_cull_kernel(const unsigned char*
     Scene sc = scene_view(dsm);
     if (!sc.h->cull) {
         if (sc.h->enabled) {
-            check_general(dsm, pairs, &pc, dsm + blob_cap, configs, n, dim, verdicts);
+            if (full_sweep) check_general<true>(dsm, pairs, &pc, dsm + blob_cap, general_cw, configs, n, dim, verdicts);
+            else check_general<false>(dsm, pairs, &pc, dsm + blob_cap, general_cw, configs, n, dim, verdicts);
         } else {
             for (int i = blockIdx.x * blockDim.x + tid; i < n; i += gridDim.x * blockDim.x) verdicts[i] = 0;
         }
@@ -762,8 +766,9 @@ static CullCheckAttrs g_cull_check_attr[2][kDynLimitDevices];
 // Launches the culled checker, or returns cudaErrorInvalidConfiguration when
 // its buffers do not fit (the caller then takes the general one).
 static cudaError_t launch_check_cull(const unsigned char* blob, int blob_cap, const int32_t* pairs, int J, int S, int K,
-                                     int Q, int dim, const float* configs, int n, int32_t* verdicts, cudaStream_t st,
-                                     const PcView& pc, const CheckScenes& scenes, int n_scenes, const EdgeHits& edges) {
+                                     int Q, int dim, const float* configs, int n, int full_sweep, int32_t* verdicts,
+                                     cudaStream_t st, const PcView& pc, const CheckScenes& scenes, int n_scenes,
+                                     const EdgeHits& edges) {
     auto kern = edges.hit ? check_cull_kernel<true> : check_cull_kernel<false>;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -805,20 +810,28 @@ static cudaError_t launch_check_cull(const unsigned char* blob, int blob_cap, co
     while (cw > least && (long long)cw * a.sms * best_warps > n) cw /= 2;  // fewer per warp before warps go idle
     const long long chunks = n / cw + n_scenes;  // of all scenes, about
     while (wpc > 1 && chunks < (long long)a.sms * wpc) wpc /= 2;
-    const int dyn = blob_cap + std::max(wpc * warp_check_bytes(J, K, cw), general);
+    int dyn = blob_cap + std::max(wpc * warp_check_bytes(J, K, cw), general);
+    const int per_sm = std::max(1, std::min(a.sm_smem / (dyn + 1024 + 64), 65536 / (a.regs * 32 * wpc)));
+    // the general checker's pass: as large as the shared memory of that many CTAs takes
+    int general_cw = 8;
+    while (general_cw < 32 &&
+           blob_cap + cc_smem_bytes(J, S, K, Q, 2 * general_cw) <= std::min(max_dyn, a.sm_smem / per_sm - 1024 - 64))
+        general_cw *= 2;
+    dyn = std::max(dyn, blob_cap + cc_smem_bytes(J, S, K, Q, general_cw));
     if (std::max(dyn, best_dyn) > a.max_dyn) {
         if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       std::max(dyn, best_dyn))) != cudaSuccess)
             return e;
         a.max_dyn = std::max(dyn, best_dyn);
     }
-    const long long resident = (long long)a.sms * std::max(1, std::min(a.sm_smem / (dyn + 1024 + 64), 65536 / (a.regs * 32 * wpc)));
+    const long long resident = (long long)a.sms * per_sm;
     // the scenes' configurations may be spread unevenly: each gets the CTAs for
     // twice its even share, and a CTA strides over what is left
     const long long each = n_scenes == 1 ? (chunks + wpc - 1) / wpc : (2 * chunks / n_scenes + wpc - 1) / wpc;
     const long long grid = std::max(1ll, std::min(each, n_scenes == 1 ? resident : (2 * resident + n_scenes - 1) / n_scenes));
     kern<<<dim3((unsigned)grid, (unsigned)n_scenes), wpc * 32, dyn, st>>>(
-        blob, blob_cap, reinterpret_cast<const int2*>(pairs), J, K, dim, cw, configs, n, verdicts, pc, scenes, edges);
+        blob, blob_cap, reinterpret_cast<const int2*>(pairs), J, K, dim, cw, configs, n, verdicts, pc, scenes, edges,
+        general_cw, full_sweep);
     return cudaGetLastError();
 }
 
@@ -837,8 +850,8 @@ cudaError_t launch_check(const unsigned char* blob, int blob_cap, const int32_t*
     constexpr int CW = PRRTC_CHECK_CW;
     CheckLaunch best, o;
     if (cull) {
-        const cudaError_t e = launch_check_cull(blob, blob_cap, pairs, J, S, K, Q, dim, configs, n, verdicts, st, cloud,
-                                                 CheckScenes{nullptr, 0, 0}, 1, edges);
+        const cudaError_t e = launch_check_cull(blob, blob_cap, pairs, J, S, K, Q, dim, configs, n, full_sweep, verdicts, st,
+                                                 cloud, CheckScenes{nullptr, 0, 0}, 1, edges);
         if (e != cudaErrorInvalidConfiguration) return e;
     }
     cudaError_t e = check_option<CW>(full_sweep, J, S, K, Q, blob_cap, best);
@@ -873,9 +886,9 @@ cudaError_t launch_check(const unsigned char* blob, int blob_cap, const int32_t*
 
 cudaError_t launch_check_batch(const unsigned char* blobs, size_t blob_stride, const int32_t* pairs,
                                size_t pairs_stride, int n_scenes, int J, int S, int K, int Q, int dim,
-                               const float* configs, const int32_t* offsets, int n, int32_t* verdicts,
+                               const float* configs, const int32_t* offsets, int n, int full_sweep, int32_t* verdicts,
                                cudaStream_t st) {
-    return launch_check_cull(blobs, (int)blob_stride, pairs, J, S, K, Q, dim, configs, n, verdicts, st,
+    return launch_check_cull(blobs, (int)blob_stride, pairs, J, S, K, Q, dim, configs, n, full_sweep, verdicts, st,
                              PcView{nullptr, nullptr, 0, 0, 0.0f, 0.0f}, CheckScenes{offsets, blob_stride, pairs_stride},
                              n_scenes, EdgeHits{});
 }
