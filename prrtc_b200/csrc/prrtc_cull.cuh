@@ -46,7 +46,7 @@ struct CullBufs {
 
 __host__ __device__ inline int cull_link_list(int n_obs) { return n_obs < kCullLinkList ? (n_obs + 7) & ~7 : kCullLinkList; }
 // List capacities: room for every second link of every waypoint; a pass that
-// needs more tests without lists.
+// needs more goes over all (link, waypoint) pairs.
 __host__ __device__ inline int cull_wcap(int K, int CW) { return (K * CW / 2 + 63) & ~31; }
 __host__ __device__ inline int cull_scap(int CW) { return 12 * CW; }
 
@@ -253,18 +253,42 @@ __device__ __forceinline__ bool cull_self_item(const Scene& sc, const CullBufs& 
     return hit;
 }
 
-// Fine test of link k at waypoint w against every primitive, sphere lane l8 of 8
-// (a pass whose world list ran over).  Out of line: the code is rarely needed.
-static __device__ __noinline__ bool cull_link_all(const unsigned char* blob, const float* pose, int k, int w, int l8) {
+// Fine test of link k at waypoint w in a pass whose world list ran over, by 8
+// consecutive lanes (l8 = 0..7 of `mask`): they find the touching primitives of the
+// link's list again, four of 32 each, and test them with a sphere per lane.  Out of
+// line: the code is rarely needed.  (A floor box of 500 m touches every link at
+// every waypoint; with all primitives tested then, a plan of 40 dual-arm problems
+// took 17 ms in the place of 2.4.)
+static __device__ __noinline__ bool cull_link_again(const unsigned char* blob, const CullBufs* Bp, int CW, int k, int w, int l8,
+                                                    unsigned mask) {
     const Scene sc = scene_view(blob);
     const BlobHeader& h = *sc.h;
-    const float4 gr = sc.grp[2 * k + 1];
+    const CullBufs& B = *Bp;
+    const float inflate = __int_as_float(h.inflate_bits);
+    const int e0 = h.Ns, e1 = e0 + h.Nc, e2 = e1 + h.Nb;
+    const int listed = B.ncand[k].w, n = listed >= 0 ? listed : e2 + h.Nh;
+    const uint16_t* list = listed >= 0 ? B.cand + k * B.ccap : nullptr;
+    const float4 c = B.cctr[k * CW + w], gr = sc.grp[2 * k + 1];
+    const CullBall ball = cull_ball(c, link_radius(sc, k, inflate, h.gated != 0, c));
     const int s1 = __float_as_int(gr.z);
     bool hit = false;
-    for (int s = __float_as_int(gr.y) + l8; s < s1; s += 8) {
-        const float4 c = fine_centre(sc, pose, h.J, w, s, __int_as_float(h.inflate_bits));
+    for (int i0 = 0; i0 < n; i0 += 32) {
+        unsigned bits = 0u;
+        for (int i = i0 + l8; i < min(n, i0 + 32); i += 8) {
+            const int o = list ? (int)list[i] : i;
+            const bool t = o < e0 ? cull_sphere(sc, o, ball)
+                           : o < e1 ? cull_capsule(sc, o - e0, ball) : o < e2 ? cull_box(sc, o - e1, ball) : cull_halfspace(sc, o - e2, ball);
+            bits |= (unsigned)t << (i - i0);
+        }
+        bits = __reduce_or_sync(mask, bits);
+        for (int s = __float_as_int(gr.y) + l8; s < s1 && bits; s += 8) {
+            const float4 f = fine_centre(sc, B.pose, h.J, w, s, inflate);
 #pragma unroll 1
-        for (int o = 0; o < h.Ns + h.Nc + h.Nb + h.Nh; ++o) hit |= prim_hits(sc, h, o, c);
+            for (unsigned rest = bits; rest; rest &= rest - 1u) {
+                const int i = i0 + __ffs(rest) - 1;
+                hit |= prim_hits(sc, h, list ? (int)list[i] : i, f);
+            }
+        }
     }
     return hit;
 }
@@ -498,8 +522,7 @@ __device__ __forceinline__ uint32_t cull_check(const G& g, const Scene& sc, cons
     }
     g.sync();
     // 4. fine tests, 8 lanes per entry.  A list that ran over is not used: every
-    // (link, waypoint) with every primitive, or every (item, waypoint), is an
-    // entry then.  Nothing here may depend on *vhit without a vote of the 8
+    // (link, waypoint), or every (item, waypoint), is an entry then.  Nothing here may depend on *vhit without a vote of the 8
     // lanes: it changes under other warps, and lanes that disagreed would wait
     // for one another.
     const bool wfull = *nwl > B.wcap, sfull = *nsl > B.scap;
@@ -526,7 +549,7 @@ __device__ __forceinline__ uint32_t cull_check(const G& g, const Scene& sc, cons
                 if (seen) continue;
                 if (gated && !(B.dirty[2 * w + (k >> 5)] & (1u << (k & 31)))) continue;
                 if (wfull) {
-                    if (cull_link_all(reinterpret_cast<const unsigned char*>(sc.h), B.pose, k, w, l8)) atomicOr(hw, 1u);
+                    if (cull_link_again(reinterpret_cast<const unsigned char*>(sc.h), &B, CW, k, w, l8, mask)) atomicOr(hw, 1u);
                     continue;
                 }
                 const float4 gr = sc.grp[2 * k + 1];
