@@ -53,6 +53,7 @@ __device__ __forceinline__ int clampi(int x, int lo, int hi) { return x < lo ? l
 // Exclusive prefix of one value per thread over a CTA of kPackThreads, plus the
 // CTA total.
 constexpr int kPackThreads = 512;
+constexpr float kCullStretchMax = 1e8f;  // box axes and normals of a length of up to 10,000 (squared) are culled
 
 __device__ __forceinline__ int pack_exclusive_scan(int v, int* warp_sums, int& total) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -191,18 +192,20 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(PackSrc s, unsigned 
                     const float off = -(ax * c[0] + ay * c[1] + az * c[2]);
                     o_wb[4 * i + k] = make_float4(ax * kBoxInv, ay * kBoxInv, az * kBoxInv, off * kBoxInv);
                 }
-                // distances along the axes bound distances only for orthonormal axes (or shorter ones)
-                bool ok = true;
+                // how much longer than its argument a vector along the axes can be (their largest singular
+                // value, bounded by the row sums of A A^T; sheared and long axes cull by a larger sphere)
+                float rows[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    const float* u = c + 3 + 3 * k;
-                    const float* v = c + 3 + 3 * ((k + 1) % 3);
-                    ok = ok && u[0] * u[0] + u[1] * u[1] + u[2] * u[2] <= 1.0002f &&
-                         fabsf(u[0] * v[0] + u[1] * v[1] + u[2] * v[2]) <= 1e-4f;
+                for (int k = 0; k < 9; ++k) {
+                    const float* u = c + 3 + 3 * (k / 3);
+                    const float* v = c + 3 + 3 * (k % 3);
+                    rows[k / 3] += fabsf(u[0] * v[0] + u[1] * v[1] + u[2] * v[2]);
                 }
+                const float stretch = fmaxf(1.0f, 1.00001f * sqrtf(fmaxf(rows[0], fmaxf(rows[1], rows[2]))));
+                const bool ok = rows[0] <= kCullStretchMax && rows[1] <= kCullStretchMax && rows[2] <= kCullStretchMax;
                 note_size(fabsf(c[0]) + fabsf(c[1]) + fabsf(c[2]) + fabsf(c[12]) + fabsf(c[13]) + fabsf(c[14]));
                 if (!ok) atomicAnd(&s_cull, 0);
-                o_wb[4 * i + 3] = make_float4(c[12] * kBoxInv, c[13] * kBoxInv, c[14] * kBoxInv, 0.0f);
+                o_wb[4 * i + 3] = make_float4(c[12] * kBoxInv, c[13] * kBoxInv, c[14] * kBoxInv, stretch);
             }
         } else if (r < e6) {
             const int i = r - e5;
@@ -210,7 +213,7 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(PackSrc s, unsigned 
                 const float* c = &wh[i * 6];
                 o_wh[i] = make_float4(c[0], c[1], c[2], -(c[0] * c[3] + c[1] * c[4] + c[2] * c[5]));
                 note_size(fabsf(c[3]) + fabsf(c[4]) + fabsf(c[5]));
-                if (!(c[0] * c[0] + c[1] * c[1] + c[2] * c[2] <= 1.0002f)) atomicAnd(&s_cull, 0);
+                if (!(c[0] * c[0] + c[1] * c[1] + c[2] * c[2] <= kCullStretchMax)) atomicAnd(&s_cull, 0);
             }
         } else {
             const int q = r - e6;
@@ -219,7 +222,7 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(PackSrc s, unsigned 
     }
     // cull spheres (prrtc_cull.cuh): a link's reach about its coarse centre plus
     // the scene's share of the pad, 8 lanes per link; infinite when the reach is
-    // not finite, too large or a radius is negative, so that nothing is culled
+    // not finite, too large for its squares or a radius is negative, so that nothing is culled
     __syncthreads();  // s_scale
     if (coarse_ok) {
         const int k = tid >> 3, l8 = tid & 7;
@@ -234,7 +237,7 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(PackSrc s, unsigned 
             for (int i = clampi(f0, 0, S) + l8; i < clampi(f1, 0, S); i += 8) {
                 const float dx = s.sloc[3 * i] - cx, dy = s.sloc[3 * i + 1] - cy, dz = s.sloc[3 * i + 2] - cz;
                 const float x = sqrtf(dx * dx + dy * dy + dz * dz) + s.srad[i];
-                ok = ok && s.srad[i] >= 0.0f && x <= kCullReachMax;
+                ok = ok && s.srad[i] >= 0.0f && x < 1e6f;
                 own = own && s.sli[i] == s.cli[k];
                 reach = fmaxf(reach, x);
             }
@@ -244,10 +247,9 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(PackSrc s, unsigned 
         for (int off = 4; off > 0; off >>= 1) reach = fmaxf(reach, __shfl_xor_sync(0xffffffffu, reach, off));
         const unsigned all_ok = __ballot_sync(0xffffffffu, ok) >> (tid & 24) & 0xffu;
         if (mine && l8 == 0) {
-            const float pad = kCullPad * (1.0f + reach + __uint_as_float(s_scale));
-            const float r = reach * 1.00001f + pad;
-            reinterpret_cast<float*>(grp + 2 * k + 1)[3] =
-                all_ok == 0xffu && reach <= kCullReachMax && r < 1e6f ? r : INFINITY;
+            const float local = fabsf(s.cloc[3 * k]) + fabsf(s.cloc[3 * k + 1]) + fabsf(s.cloc[3 * k + 2]);
+            const float r = (1.0f + kCullPad) * reach + kCullScenePad * (local + __uint_as_float(s_scale));
+            reinterpret_cast<float*>(grp + 2 * k + 1)[3] = all_ok == 0xffu && r < 1e6f ? r : INFINITY;
         }
         if (mine && !own) atomicAnd(&s_cull, 0);
     }

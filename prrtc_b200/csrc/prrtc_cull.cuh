@@ -5,13 +5,20 @@
 // and a radius that encloses its fine spheres and the coarse sphere with a pad.
 // A primitive whose distance from the cull sphere is positive cannot pass any
 // fine test of that link, so only the links, waypoints and primitives that
-// touch are tested, with the same arithmetic as cc_chunk's.  The pad covers the
-// rounding of the fine tests: the largest error of the expanded sphere test,
-// |c|^2 - r^2 + |o|^2 - r_o^2 - 2 (c.o + r r_o), is below 1.1e-6 M^2 for
-// M = |c| + |o| + radii, and a gap of d metres beyond the cull sphere leaves
-// |c_f - o|^2 - (r_f + r_o)^2 >= d^2, so d = 2e-3 M (4e-6 M^2) suffices; the
-// other tests are first order in the distance and need 1e-6 M.  Comparisons are
-// written so that NaN and infinities count as touching.
+// touch are tested, with the same arithmetic as cc_chunk's.
+//
+// The pad covers rounding.  The expanded sphere test, |c|^2 - r^2 + |o|^2 - r_o^2 -
+// 2 (c.o + r r_o), is off by at most e M^2, e = 1.1e-6, M = |c| + |o| + radii, on a fine
+// sphere and on the cull sphere.  With m = |c| + R (R without the pad, c the cull
+// sphere's centre; a link's fine spheres lie within m of the origin) and a gap of g
+// between the unpadded sphere and the primitive, M <= 2 (m + r_o) + g, so a fine test
+// can only pass for g^2 + 2 g r_o < e M^2, hence only for e M^2 < B = 4.5e-6 (m + r_o)^2.
+// A pad of d = 3.2e-3 m + 4.6e-6 r_o keeps it from that: a cull sphere found apart has
+// g^2 + 2 g (R + r_o) > d^2 + 2 d (R + r_o) - B, which gives g > 2.2e-3 m + 2.3e-6 r_o, and
+// then g^2 + 2 g r_o > B.  So the pad grows with the robot's own coordinates and
+// hardly with the primitives' (a floor of 500 m pads by 1 cm).  The other tests are
+// first order in the distance and need 1e-6 (m + size of the primitive).  Comparisons
+// are written so that NaN and infinities count as touching.
 //
 // For the waypoints of an edge a first level bounds each link's cull spheres
 // over the whole pass by one sphere (centre of the middle waypoint) and lists
@@ -113,15 +120,19 @@ __device__ __forceinline__ bool cull_capsule(const Scene& sc, int o, const CullB
 }
 __device__ __forceinline__ bool cull_box(const Scene& sc, int o, const CullBall& b) {
     const float4 cc[1] = {b.c};
+    const float4 hl = sc.wb[4 * o + 3];
     float v[1];
-    h_box<1>(v, cc, sc.wb[4 * o], sc.wb[4 * o + 1], sc.wb[4 * o + 2], sc.wb[4 * o + 3]);
-    return !(v[0] > (b.c.w * kBoxInv) * (b.c.w * kBoxInv));
+    h_box<1>(v, cc, sc.wb[4 * o], sc.wb[4 * o + 1], sc.wb[4 * o + 2], hl);
+    const float r = b.c.w * hl.w * kBoxInv;  // hl.w: the axes' stretch, at least 1
+    return !(v[0] > r * r);
 }
 __device__ __forceinline__ bool cull_halfspace(const Scene& sc, int o, const CullBall& b) {
     const float4 cc[1] = {b.c};
+    const float4 n = sc.wh[o];
     float v[1];
-    h_halfspace<1>(v, cc, sc.wh[o]);
-    return !(v[0] > b.c.w);
+    h_halfspace<1>(v, cc, n);
+    const float n2 = fmaxf(1.0f, fmaf(n.x, n.x, fmaf(n.y, n.y, n.z * n.z)));  // the normal's length may exceed 1
+    return !(v[0] > 0.0f && v[0] * v[0] > b.c.w * b.c.w * (1.000001f * n2));
 }
 
 // The exact test of primitive o (combined index) against one sphere: the
@@ -168,8 +179,8 @@ __device__ __forceinline__ float4 fine_centre(const Scene& sc, const float* pose
     return pose_point(pose, J, w, f, l);
 }
 
-// Padded cull radius of a link whose coarse centre is c (grp record .w: reach
-// of its spheres and the scene's share of the pad).
+// Padded cull radius of a link whose coarse centre is c (grp record .w: the padded
+// reach of its spheres and the scene's share of the pad).
 __device__ __forceinline__ float cull_radius(float reach, float inflate, float4 c) {
     return reach + (1.0f + kCullPad) * inflate + kCullPad * (fabsf(c.x) + fabsf(c.y) + fabsf(c.z));
 }

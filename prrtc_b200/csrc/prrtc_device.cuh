@@ -34,8 +34,10 @@ constexpr int kObsChunk = 32;    // world primitives per work item
 #endif
 constexpr int kSphChunk = PRRTC_SPH_CHUNK;  // fine spheres held in registers per work item
 constexpr int kPairChunk = 32;   // explicit self pairs per work item
-constexpr float kCullPad = 2.0e-3f;  // pad of the cull spheres per metre of coordinate size (prrtc_cull.cuh)
-constexpr float kCullReachMax = 4.0f;  // a link reaching further (or not finite) is never culled
+// Pads of the cull spheres (prrtc_cull.cuh): per unit of the robot's own coordinate
+// size, and per unit of the scene's largest primitive.
+constexpr float kCullPad = 3.5e-3f;
+constexpr float kCullScenePad = 5.0e-6f;
 constexpr float kFar = 1.0e18f;  // centre of a sphere that can never collide
 // Box records are stored scaled by 1/kBoxScale (a power of two, so the scaling
 // is exact): the checker's relu(|l| - h) becomes a saturating add, exact for
@@ -66,8 +68,8 @@ struct BlobHeader {
     int32_t o_sch, o_ws, o_wc, o_wb;
     int32_t o_wh, o_item, o_cpair, used_bytes;
     int32_t P, cap_bytes, error;
-    int32_t cull;  // the groups cover every sphere on their own frames, box axes are orthonormal,
-                   // normals not longer than 1: prrtc_cull.cuh applies
+    int32_t cull;  // the groups cover every sphere on their own frames, box axes and normals
+                   // are finite: prrtc_cull.cuh applies
 };
 static_assert(sizeof(BlobHeader) == 128, "header must stay 128 bytes");
 // Bits of BlobHeader::error: the pack kernel's self-pair item list overflowed
