@@ -20,6 +20,7 @@ import ctypes as C
 
 import numpy as np
 import torch
+from torch.autograd import forward_ad
 
 from . import _lib
 from .collision import CollisionChecker
@@ -292,6 +293,10 @@ class BatchSmoothContext:
                                                          hi.data_ptr(), lr, P, W, dim, sp), "prrtc_b200_smooth_update")
 
 
+def _differentiated(t: torch.Tensor) -> bool:
+    return t.requires_grad or forward_ad.unpack_dual(t).tangent is not None
+
+
 def projected_steps(sctx, init: torch.Tensor, lower, upper, steps: int, lr: float) -> torch.Tensor:
     """`steps` projected gradient steps of the adjoint cost from `init` [P, W, dim]:
     endpoints fixed, joint limits enforced, step length lr per path (the
@@ -301,11 +306,11 @@ def projected_steps(sctx, init: torch.Tensor, lower, upper, steps: int, lr: floa
     hi = as_tensor(upper, torch.float32, init.device).reshape(1, 1, dim)
     x = init.clone()
     # the kernels take plain memory of the scenes' device and one number for lr;
-    # anything else (paths elsewhere, recorded by autograd, without an inner
-    # waypoint, another object's gradient) goes by the tensor expression
+    # anything else (paths elsewhere, recorded by autograd or with tangents, without
+    # an inner waypoint, another object's gradient) goes by the tensor expression
     if (isinstance(sctx, BatchSmoothContext) and type(sctx).cost_grad is BatchSmoothContext.cost_grad
             and type(x) is torch.Tensor and x.device == sctx.device and x.dtype == torch.float32 and x.is_contiguous()
-            and P > 0 and W > 2 and isinstance(lr, (int, float)) and not (x.requires_grad or lo.requires_grad or hi.requires_grad)):
+            and P > 0 and W > 2 and isinstance(lr, (int, float)) and not any(map(_differentiated, (x, lo, hi)))):
         sctx.descend(x, lo, hi, steps, lr)
         return x
     order = {"ordered": True} if type(sctx) is SmoothContext else {}

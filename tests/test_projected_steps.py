@@ -54,6 +54,18 @@ def test_kernels_take_plain_paths_only(form, monkeypatch):
         assert torch.equal(torch.autograd.grad(x.sum(), init)[0], torch.autograd.grad(want.sum(), init)[0])
 
 
+def test_tangents_are_kept(monkeypatch):
+    """Paths in forward mode, inside the limits: the tangents come back with them (after no steps, as they went in)."""
+    from torch.autograd import forward_ad
+
+    monkeypatch.setattr(BatchSmoothContext, "cost_grad", lambda self, x, need_grad=True: (None, 2.0 * x.detach()))
+    s = _batch_context("cpu")
+    init, t = (torch.from_numpy(np.random.default_rng(k).uniform(-1, 1, (2, 6, 3)).astype(np.float32)) for k in (0, 1))
+    with forward_ad.dual_level():
+        x = projected_steps(s, forward_ad.make_dual(init, t), [-2.0] * 3, [2.0] * 3, 0, 0.1)
+        assert not s.calls and torch.equal(forward_ad.unpack_dual(x).tangent, t)
+
+
 def test_kernels_take_plain_paths(monkeypatch):
     monkeypatch.setattr(BatchSmoothContext, "cost_grad", lambda self, x, need_grad=True: (None, 2.0 * x))
     s = _batch_context("cpu")
