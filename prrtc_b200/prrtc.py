@@ -806,15 +806,17 @@ def _plan_per_problem(lib, bi, res, attrs, tun, contexts, robot_ctx, starts, goa
     streams = [torch.cuda.Stream(device=dev) for _ in range(min(n_streams, B))]
     ev = torch.cuda.Event()
     gcs = None if goal_counts is None else np.asarray(goal_counts).reshape(B)
+    # all tables in one copy on the caller's stream, which every launch waits for
+    stage = Stager(dev)
+    ctxs = [DeviceContext(contexts[i], dev, stager=stage) for i in range(B)]
+    stage.commit()
+    ev.record(main)
+    for s in streams:
+        s.wait_event(ev)
     keep = []
     for i in range(B):
         s = streams[i % len(streams)]
-        ctx = DeviceContext(contexts[i], dev) if contexts[i] is not None else DeviceContext(None, dev)
-        keep.append(ctx)
-        # the tables' copies are queued on the caller's stream (a pageable copy may
-        # still be in flight when the call returns)
-        ev.record(main)
-        s.wait_event(ev)
+        ctx = ctxs[i].finish()
         inp = _lib.Inputs()
         inp.start_config = starts[i].data_ptr()
         ng = G if gcs is None else max(1, min(int(gcs[i]), G))
