@@ -123,6 +123,9 @@ struct DynLimit {
     int max_dyn = -1;
 };
 constexpr int kDynLimitDevices = 256;
+// Static shared memory of the checkers and the smoothing kernels: a barrier, padded
+// to the alignment of the dynamic part.
+constexpr size_t kStaticSmem = 128;
 // limits: one per device, of this kernel alone.
 cudaError_t raise_dyn_limit(const void* kern, DynLimit (&limits)[kDynLimitDevices], size_t dyn);
 

@@ -614,7 +614,7 @@ template <int CW>
 static cudaError_t check_option(int full_sweep, int J, int S, int K, int Q, int blob_cap, CheckLaunch& o) {
     const size_t cc = (size_t)cc_smem_bytes(J, S, K, Q, CW);
     size_t dyn = cc + (size_t)blob_cap;
-    if (dyn + 64 > device_max_smem()) {
+    if (dyn + kStaticSmem > device_max_smem()) {
         blob_cap = 0;
         dyn = cc;
     }
@@ -787,7 +787,7 @@ static cudaError_t launch_check_cull(const unsigned char* blob, int blob_cap, co
         a.sms = device_sm_count();
         a.ctx = ctx;
     }
-    const int max_dyn = (int)device_max_smem() - 64;
+    const int max_dyn = (int)(device_max_smem() - kStaticSmem);
     const int general = cc_smem_bytes(J, S, K, Q, 8);  // a scene that is not culled
     int best_cw = 0, best_wpc = 0, best_warps = 0, best_dyn = 0;
     const int least = pc.n > 0 ? 1 : 4;  // configurations per warp
@@ -795,7 +795,7 @@ static cudaError_t launch_check_cull(const unsigned char* blob, int blob_cap, co
         for (int wpc = 4; wpc <= 8; wpc *= 2) {
             const int dyn = blob_cap + std::max(wpc * warp_check_bytes(J, K, cw), general);
             if (dyn > max_dyn) continue;
-            const int per_sm = std::min(a.sm_smem / (dyn + 1024 + 64), 65536 / (a.regs * 32 * wpc));
+            const int per_sm = std::min(a.sm_smem / (dyn + 1024 + (int)kStaticSmem), 65536 / (a.regs * 32 * wpc));
             const int warps = std::min(per_sm * wpc, 24);
             if (warps > best_warps) { best_cw = cw; best_wpc = wpc; best_warps = warps; best_dyn = dyn; }
         }
@@ -811,13 +811,13 @@ static cudaError_t launch_check_cull(const unsigned char* blob, int blob_cap, co
     const long long chunks = n / cw + n_scenes;  // of all scenes, about
     while (wpc > 1 && chunks < (long long)a.sms * wpc) wpc /= 2;
     int dyn = blob_cap + std::max(wpc * warp_check_bytes(J, K, cw), general);
-    const int per_sm = std::max(1, std::min(a.sm_smem / (dyn + 1024 + 64), 65536 / (a.regs * 32 * wpc)));
+    const int per_sm = std::max(1, std::min(a.sm_smem / (dyn + 1024 + (int)kStaticSmem), 65536 / (a.regs * 32 * wpc)));
     // the general checker's pass: as large as the shared memory of that many CTAs takes, but
     // not where a cloud is read through what is left of it as L1 (4000 configurations
     // against 200,000 points 683 us, 840 with the larger pass)
     int general_cw = 8;
     while (pc.n == 0 && general_cw < 32 &&
-           blob_cap + cc_smem_bytes(J, S, K, Q, 2 * general_cw) <= std::min(max_dyn, a.sm_smem / per_sm - 1024 - 64))
+           blob_cap + cc_smem_bytes(J, S, K, Q, 2 * general_cw) <= std::min(max_dyn, a.sm_smem / per_sm - 1024 - (int)kStaticSmem))
         general_cw *= 2;
     dyn = std::max(dyn, blob_cap + cc_smem_bytes(J, S, K, Q, general_cw));
     if (std::max(dyn, best_dyn) > a.max_dyn) {

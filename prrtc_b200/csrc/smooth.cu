@@ -989,10 +989,10 @@ cudaError_t launch_smooth(const unsigned char* blob, size_t blob_stride, int blo
         // 256 threads and up to three CTAs per SM (registers), or 512 where
         // shared memory allows only one (large robots)
         const size_t wide = (size_t)blob_cap + smooth_wide_bytes(J, S);
-        const int by_smem = (int)((device_max_smem() + 1024) / (wide + 1024 + 64));
+        const int by_smem = (int)((device_max_smem() + 1024) / (wide + 1024 + kStaticSmem));
         const bool big = by_smem < 2;
         const long long ctas = ((long long)P * W + 31) / 32;
-        if (wide + 64 <= device_max_smem() && ctas * 8 <= INT32_MAX) {
+        if (wide + kStaticSmem <= device_max_smem() && ctas * 8 <= INT32_MAX) {
             void (*const kern)(SmoothArgs, int, int) = big ? smooth_wide_kernel<512, 1> : smooth_wide_kernel<256, 3>;
             // Several CTAs may share 32 waypoints, each with a share of the pairs,
             // and add up their gradients (which are linear in the pairs' terms):
@@ -1032,7 +1032,7 @@ cudaError_t launch_smooth(const unsigned char* blob, size_t blob_stride, int blo
     auto blocks = [&](int warps) {
         return (unsigned)(shared ? ((long long)P * W + warps - 1) / warps : (long long)P * per_path(warps));
     };
-    if (smem + blob_cap + 64 <= device_max_smem()) {
+    if (smem + blob_cap + kStaticSmem <= device_max_smem()) {
         smem += blob_cap;
         auto kern = cost ? smooth_kernel<WARPS, true, true> : smooth_kernel<WARPS, true, false>;
         static DynLimit limit[2][kDynLimitDevices];
