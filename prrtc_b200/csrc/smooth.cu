@@ -23,6 +23,7 @@
 #include <math.h>
 
 #include <algorithm>
+#include <mutex>
 #include <type_traits>
 
 #include "kernels.h"
@@ -377,7 +378,7 @@ __global__ void __launch_bounds__(WARPS * 32) smooth_kernel(SmoothArgs a, int bl
         const float4 cs = ctr[s], gs = g[s];
         const float v[6] = {gs.x, gs.y, gs.z, cs.y * gs.z - cs.z * gs.y, cs.z * gs.x - cs.x * gs.z,
                             cs.x * gs.y - cs.y * gs.x};
-const int fp = __shfl_up_sync(0xffffffffu, f, 1);
+        const int fp = __shfl_up_sync(0xffffffffu, f, 1);
         const bool head = lane == 0 || f != fp;
         add_runs<6>(__ballot_sync(0xffffffffu, s0 + lane < S && f >= 0), __ballot_sync(0xffffffffu, head),
                     __all_sync(0xffffffffu, !head || lane == 0 || f > fp), f, acc, 8, v, stage);
@@ -975,6 +976,46 @@ __global__ void __launch_bounds__(THREADS, MINBLOCKS)
     }
 }
 
+// Launch of `parts` CTAs per cluster (up to 2: none).
+static cudaLaunchConfig_t cluster_config(cudaLaunchAttribute& cluster, int threads, size_t smem, int parts) {
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim = {(unsigned)parts, 1u, 1u};
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)parts);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = &cluster;
+    cfg.numAttrs = parts > 2 ? 1 : 0;
+    return cfg;
+}
+
+// How many clusters of 3 to 8 CTAs the device holds at once, 0 if none, for a kernel
+// of which `per_sm` CTAs (up to 3) fit an SM: asked once per device and CUDA context.
+static int cluster_room(void (*kern)(SmoothArgs, int, int), int per_sm, int threads, size_t smem, int parts) {
+    struct Room {
+        unsigned long long ctx = 0ull;
+        int n = 0;
+    };
+    static Room rooms[4][9][kDynLimitDevices];
+    static std::mutex mutex;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    const unsigned long long ctx = current_context_key();
+    std::lock_guard<std::mutex> lock(mutex);
+    Room none;
+    Room& r = dev >= 0 && dev < kDynLimitDevices ? rooms[per_sm][parts][dev] : none;
+    if (!ctx || r.ctx != ctx) {
+        cudaLaunchAttribute cluster;
+        const cudaLaunchConfig_t cfg = cluster_config(cluster, threads, smem, parts);
+        r = Room{ctx, 0};
+        if (cudaOccupancyMaxActiveClusters(&r.n, kern, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            r.n = 0;
+        }
+    }
+    return r.n;
+}
+
 cudaError_t launch_smooth(const unsigned char* blob, size_t blob_stride, int blob_cap, const int32_t* pairs,
                           size_t pairs_stride,
                           int J, int S, int dim, const float* wp, int P, int W, float margin, float beta, float w_len,
@@ -998,30 +1039,34 @@ cudaError_t launch_smooth(const unsigned char* blob, size_t blob_stride, int blo
             // and add up their gradients (which are linear in the pairs' terms):
             // as many as make the last wave of the launch full, a twelfth of a
             // CTA's time being its frames and closing sums.  Two add into zeroed
-            // memory; four or eight are a cluster, which adds in their order.
-            const long long room = (long long)device_sm_count() * (big ? 1 : std::min(by_smem, 3));
+            // memory; more are a cluster, which adds in their order.
+            // A cluster lies within one GPC, so fewer of them fit than the SMs would
+            // hold CTAs (8 dual-arm paths of 64 waypoints: 16 clusters of 8 took two
+            // waves, 171 us a call; as clusters of 7 they take one, 111).
+            // How many is the same for every scene of as many CTAs per SM, so that a call's
+            // gradient does not depend on the calls before it.
+            const int per_sm = big ? 1 : std::min(by_smem, 3);
+            const size_t most = (device_max_smem() + 1024) / per_sm - 1024 - kStaticSmem;  // what so many CTAs have each, at least `wide`
+            static DynLimit limit[2][kDynLimitDevices];
+            if ((e = raise_dyn_limit(reinterpret_cast<const void*>(kern), limit[big ? 1 : 0], most)) != cudaSuccess)
+                return e;
+            const long long room = (long long)device_sm_count() * per_sm;
+            const int threads = big ? 512 : 256;
             int parts = 1;
             double best = 1e30;
-            for (int p = 1; p <= 8; p *= 2) {
-                const double c = (double)((ctas * p + room - 1) / room) * (1.0 / p + 1.0 / 12);
+            for (int p = 1; p <= 8; ++p) {
+                const long long fit = p > 2 ? cluster_room(kern, per_sm, threads, most, p) : room / p;
+                if (fit < 1) continue;
+                const double c = (double)((ctas + fit - 1) / fit) * (1.0 / p + 1.0 / 12);
                 if (c < 0.97 * best) { best = c; parts = p; }
             }
             if (parts == 2 && grad &&
                 (e = cudaMemsetAsync(grad, 0, (size_t)P * W * dim * sizeof(float), st)) != cudaSuccess)
                 return e;
-            static DynLimit limit[2][kDynLimitDevices];
-            if ((e = raise_dyn_limit(reinterpret_cast<const void*>(kern), limit[big ? 1 : 0], wide)) != cudaSuccess)
-                return e;
             cudaLaunchAttribute cluster;
-            cluster.id = cudaLaunchAttributeClusterDimension;
-            cluster.val.clusterDim = {(unsigned)parts, 1u, 1u};
-            cudaLaunchConfig_t cfg = {};
+            cudaLaunchConfig_t cfg = cluster_config(cluster, threads, wide, parts);
             cfg.gridDim = dim3((unsigned)(ctas * parts));
-            cfg.blockDim = dim3(big ? 512 : 256);
-            cfg.dynamicSmemBytes = wide;
             cfg.stream = st;
-            cfg.attrs = &cluster;
-            cfg.numAttrs = parts > 2 ? 1 : 0;
             if ((e = cudaLaunchKernelEx(&cfg, kern, a, blob_cap, parts)) != cudaSuccess) return e;
             return cudaGetLastError();
         }
