@@ -265,21 +265,20 @@ __device__ __forceinline__ bool cull_self_item(const Scene& sc, const CullBufs& 
 }
 
 // Fine test of link k at waypoint w in a pass whose world list ran over, by 8
-// consecutive lanes (l8 = 0..7 of `mask`): they find the touching primitives of the
-// link's list again, four of 32 each, and test them with a sphere per lane.  Out of
-// line: the code is rarely needed.  (A floor box of 500 m touches every link at
-// every waypoint; with all primitives tested then, a plan of 40 dual-arm problems
-// took 17 ms in the place of 2.4.)
-static __device__ __noinline__ bool cull_link_again(const unsigned char* blob, const CullBufs* Bp, int CW, int k, int w, int l8,
-                                                    unsigned mask) {
+// consecutive lanes (l8 = 0..7 of `mask`): they find the touching primitives again,
+// four of 32 each, and test them with a sphere per lane.  c: the link's centre;
+// list: its `listed` primitives, or every one for listed < 0.  Out of line: the code
+// is rarely needed.  It takes values, not the buffers: with their address taken
+// every access to them is through local memory, 8% of a plan (explore_kernel of 16
+// spheres, 128 explorers: 82 -> 89 us).
+static __device__ __noinline__ bool cull_link_again(const unsigned char* blob, const float* pose, int k, int w, int l8,
+                                                    unsigned mask, const uint16_t* list, int listed, float4 c) {
     const Scene sc = scene_view(blob);
     const BlobHeader& h = *sc.h;
-    const CullBufs& B = *Bp;
     const float inflate = __int_as_float(h.inflate_bits);
-    const int e0 = h.Ns, e1 = e0 + h.Nc, e2 = e1 + h.Nb;
-    const int listed = B.ncand[k].w, n = listed >= 0 ? listed : e2 + h.Nh;
-    const uint16_t* list = listed >= 0 ? B.cand + k * B.ccap : nullptr;
-    const float4 c = B.cctr[k * CW + w], gr = sc.grp[2 * k + 1];
+    const int e0 = h.Ns, e1 = e0 + h.Nc, e2 = e1 + h.Nb, n = listed >= 0 ? listed : e2 + h.Nh;
+    if (listed < 0) list = nullptr;
+    const float4 gr = sc.grp[2 * k + 1];
     const CullBall ball = cull_ball(c, link_radius(sc, k, inflate, h.gated != 0, c));
     const int s1 = __float_as_int(gr.z);
     bool hit = false;
@@ -288,12 +287,13 @@ static __device__ __noinline__ bool cull_link_again(const unsigned char* blob, c
         for (int i = i0 + l8; i < min(n, i0 + 32); i += 8) {
             const int o = list ? (int)list[i] : i;
             const bool t = o < e0 ? cull_sphere(sc, o, ball)
-                           : o < e1 ? cull_capsule(sc, o - e0, ball) : o < e2 ? cull_box(sc, o - e1, ball) : cull_halfspace(sc, o - e2, ball);
+                           : o < e1 ? cull_capsule(sc, o - e0, ball)
+                           : o < e2 ? cull_box(sc, o - e1, ball) : cull_halfspace(sc, o - e2, ball);
             bits |= (unsigned)t << (i - i0);
         }
         bits = __reduce_or_sync(mask, bits);
         for (int s = __float_as_int(gr.y) + l8; s < s1 && bits; s += 8) {
-            const float4 f = fine_centre(sc, B.pose, h.J, w, s, inflate);
+            const float4 f = fine_centre(sc, pose, h.J, w, s, inflate);
 #pragma unroll 1
             for (unsigned rest = bits; rest; rest &= rest - 1u) {
                 const int i = i0 + __ffs(rest) - 1;
@@ -315,8 +315,8 @@ static __device__ __noinline__ bool cull_link_again(const unsigned char* blob, c
 // some 20 points.  A lane that walked its own sphere's cells and points made the
 // warp wait for its longest chain of dependent loads, so the cells of all 32
 // spheres are dealt out over the lanes, and the points of an occupied cell over
-// 8 of them: 128 edges of 16 waypoints against 20,000 points take 83 us a call
-// instead of 577, 8000 edges of 33 against 5000 points as long as before.
+// 8 of them: 128 edges of 16 waypoints against 20,000 points take 80 us a call
+// instead of 464, 4000 edges of 33 against 500 points 567 us instead of 684.
 __device__ __forceinline__ unsigned cloud_batch(const PcView& pc, float4 c, bool valid, int w, unsigned alive,
                                                 unsigned& flops) {
     constexpr unsigned kAll = 0xffffffffu;
@@ -416,9 +416,10 @@ __device__ __forceinline__ int cull_append(int count, int base, int n, int cap, 
 }
 
 // Whether any of nw (<= CW <= 64) waypoints of `edge` collides (non-zero).
-// Called by every thread of the CTA with the same `par`, which the call flips: the result words and list lengths alternate between calls, so that a
-// call clears the next call's after its first barrier.  All must be zero and
-// `par` 0 before the first call.  The scene must have BlobHeader::cull set.
+// Called by every thread of the CTA with the same `par`, which the call flips: the
+// result words and list lengths alternate between calls, so that a call clears the
+// next call's after its first barrier.  All must be zero and `par` 0 before the
+// first call.  The scene must have BlobHeader::cull set.
 template <class G>
 __device__ __forceinline__ uint32_t cull_check(const G& g, const Scene& sc, const CullBufs& B, int nw, int CW, int& par,
                                                const EdgeSrc& edge) {
@@ -533,9 +534,9 @@ __device__ __forceinline__ uint32_t cull_check(const G& g, const Scene& sc, cons
     }
     g.sync();
     // 4. fine tests, 8 lanes per entry.  A list that ran over is not used: every
-    // (link, waypoint), or every (item, waypoint), is an entry then.  Nothing here may depend on *vhit without a vote of the 8
-    // lanes: it changes under other warps, and lanes that disagreed would wait
-    // for one another.
+    // (link, waypoint), or every (item, waypoint), is an entry then.  Nothing here
+    // may depend on *vhit without a vote of the 8 lanes: it changes under other
+    // warps, and lanes that disagreed would wait for one another.
     const bool wfull = *nwl > B.wcap, sfull = *nsl > B.scap;
     const int Lw = wfull ? K * nw : *nwl, Ls = sfull ? h.n_items * nw : *nsl;
     const bool cloud = sc.pc.n > 0;
@@ -560,7 +561,9 @@ __device__ __forceinline__ uint32_t cull_check(const G& g, const Scene& sc, cons
                 if (seen) continue;
                 if (gated && !(B.dirty[2 * w + (k >> 5)] & (1u << (k & 31)))) continue;
                 if (wfull) {
-                    if (cull_link_again(reinterpret_cast<const unsigned char*>(sc.h), &B, CW, k, w, l8, mask)) atomicOr(hw, 1u);
+                    if (cull_link_again(reinterpret_cast<const unsigned char*>(sc.h), B.pose, k, w, l8, mask, B.cand + k * B.ccap,
+                                        B.ncand[k].w, B.cctr[k * CW + w]))
+                        atomicOr(hw, 1u);
                     continue;
                 }
                 const float4 gr = sc.grp[2 * k + 1];
