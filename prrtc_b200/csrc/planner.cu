@@ -9,13 +9,14 @@
 // sub-edges; the first explorer whose connect completes solves the problem.
 //
 // B200 design:
-//  * an explorer is a CTA of 64-256 threads; nearest neighbour is a CTA scan of
-//    the SoA tree with 128-bit L2-coherent loads and a lexicographic (dsq, idx)
-//    warp-shuffle argmin (ties to the lowest index);
-//  * an edge's waypoints are checked cooperatively by the whole CTA (FK per
-//    waypoint, sphere centres, then (waypoint x sphere-chunk x obstacle-chunk)
-//    and (waypoint x self-block) work items) against the scene staged in shared
-//    memory by one bulk TMA copy;
+//  * an explorer is a CTA of 32-512 threads; nearest neighbour is a CTA scan of
+//    the SoA tree with 128-bit L2-coherent loads and an argmin by integer minima
+//    (ties to the lowest index);
+//  * an edge's waypoints are checked by the whole CTA against the scene staged in
+//    shared memory by one bulk TMA copy: link frames, a bound per link over the
+//    pass, then only the links, waypoints and primitives that touch
+//    (prrtc_cull.cuh); robots without a coarse model or of more than 32 joints
+//    take the general check of every pair (prrtc_device.cuh);
 //  * tree slots are pre-filled with NaN, so a reader scanning [0, tree_size)
 //    never uses a half-written node (its squared distance is NaN and loses every
 //    comparison); this replaces the reference's `completed` counter as the scan
@@ -222,7 +223,7 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(PackSrc s, unsigned 
     }
     // cull spheres (prrtc_cull.cuh): a link's reach about its coarse centre plus
     // the scene's share of the pad, 8 lanes per link; infinite when the reach is
-    // not finite, too large for its squares or a radius is negative, so that nothing is culled
+    // not finite or too large for its squares, so that nothing is culled
     __syncthreads();  // s_scale
     if (coarse_ok) {
         const int k = tid >> 3, l8 = tid & 7;
@@ -236,8 +237,8 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(PackSrc s, unsigned 
             reach = fabsf(s.crad[k]);
             for (int i = clampi(f0, 0, S) + l8; i < clampi(f1, 0, S); i += 8) {
                 const float dx = s.sloc[3 * i] - cx, dy = s.sloc[3 * i + 1] - cy, dz = s.sloc[3 * i + 2] - cz;
-                const float x = sqrtf(dx * dx + dy * dy + dz * dz) + s.srad[i];
-                ok = ok && s.srad[i] >= 0.0f && x < 1e6f;
+                const float x = sqrtf(dx * dx + dy * dy + dz * dz) + fabsf(s.srad[i]);  // no fine test passes beyond |r|
+                ok = ok && x < 1e6f;
                 own = own && s.sli[i] == s.cli[k];
                 reach = fmaxf(reach, x);
             }
@@ -371,8 +372,6 @@ cudaError_t launch_pack(const PackSrc& s, int batch, unsigned char* blobs, size_
     pack_kernel<<<batch, kPackThreads, 0, st>>>(s, blobs, stride, (int)stride);
     return cudaGetLastError();
 }
-
-// ============================================================================ helpers
 
 // ============================================================================ nearest neighbour
 

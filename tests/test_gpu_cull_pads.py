@@ -131,6 +131,9 @@ def _odd(form, rng):
         b[1, 7] = np.inf
         ctx["world_boxes"] = b
         ctx["world_halfspaces"] = np.array([[0, 0, np.inf, 0, 0, -3], [0, np.nan, 1, 0, 0, -3], [0, 0, 1, 0, 0, -0.05]], np.float32)
+    elif form == "negative_radii":
+        ctx["sphere_radius"] = ctx["sphere_radius"] * np.where(np.arange(len(ctx["sphere_radius"])) % 5 == 2, -1, 1).astype(np.float32)
+        ctx["coarse_sphere_radius"] = ctx["coarse_sphere_radius"] * np.where(np.arange(len(ctx["coarse_sphere_radius"])) == 3, -1, 1).astype(np.float32)
     elif form == "centimetres":
         s = 100.0
         ctx = _scaled(ctx, s)
@@ -147,7 +150,7 @@ def _odd(form, rng):
 
 
 ODD = ["plain", "floor_500", "first_sphere_left_out", "last_spheres_left_out", "all_but_one_link", "another_frame", "no_ranges",
-       "nan_axis", "centimetres", "stretched"]
+       "nan_axis", "negative_radii", "centimetres", "stretched"]
 
 
 @pytest.mark.parametrize("mode", [0, 1, 2, 3])
