@@ -17,10 +17,11 @@ namespace prrtc {
 // ============================================================================ nearest neighbour
 
 // Every CTA holds up to kNnQueries queries and strides over the tree, a column of
-// 4 nodes per thread, so the tree is read once per 64 queries.  The dimensions go in blocks of 4: after a block, a warp whose 128
-// partial sums all exceed the query's best distance so far leaves the query (a
-// sum of squares only grows, also in rounded arithmetic), which in 7 dimensions
-// is nearly always after the first block.  The best distances are shared: each
+// 4 nodes per thread, so the tree is read once per 64 queries.  The dimensions go
+// in blocks of 4: after a block, a warp whose 128 partial sums all exceed the
+// query's best distance so far leaves the query (a sum of squares only grows, also
+// in rounded arithmetic), which in 7 dimensions is nearly always after the first
+// block.  The best distances are shared: each
 // improvement goes to the CTA's and the global key at once, and every CTA
 // rereads the global keys per column.  Keys order like (squared distance,
 // index), so the result is the nearest node, the lowest index on a tie; NaN and
@@ -139,12 +140,13 @@ __global__ void __launch_bounds__(256, DB <= 2 ? 3 : 2) nn_scan_kernel(const flo
 // Batches on large trees: the tensor cores rule nodes out, the rest is computed as
 // above.  A dot product in tf32 gives (1 - c)|x|^2 - 2 x.q for 16 nodes and 8
 // queries per instruction (the norm from the squares against 1 - c); above
-// best (1 + 2^-16) - (1 - c)|q|^2, the node is farther than the best so far.  Rounding both factors to tf32 moves 2 x.q by at most 2^-10 (|x|^2 +
-// |q|^2) and the norm by 2^-11 |x|^2; sums in float32 (of at most 17 terms, in any
-// order and rounding) add 2^-17 (|x|^2 + |q|^2) + 2^-18 best; c = 2^-9 covers them, and 2^-16
-// the rounding of the exact sum.  Squares from 1e37 on, infinities and NaN count
-// as near.  So every node that could be nearest is computed exactly,
-// and the result is that of nn_scan_kernel bit for bit.
+// best (1 + 2^-16) - (1 - c)|q|^2, the node is farther than the best so far.
+// Rounding both factors to tf32 moves 2 x.q by at most 2^-10 (|x|^2 + |q|^2) and the
+// norm by 2^-11 |x|^2; sums in float32 (of at most 17 terms, in any order and
+// rounding) add 2^-17 (|x|^2 + |q|^2) + 2^-18 best; c = 2^-9 covers them, and 2^-16 the
+// rounding of the exact sum.  Squares from 1e37 on, infinities and NaN count as
+// near.  So every node that could be nearest is computed exactly, and the result
+// is that of nn_scan_kernel bit for bit.
 //
 // A warp takes 32 nodes at a time, 4 neighbours per lane (one 16-byte load per
 // dimension and 128 bytes in a row per warp): the fragments' rows may be nodes in
