@@ -560,7 +560,7 @@ def planner_roofline(torch, lib, dev, planners, settings, tuned, cap_of):
                        # DRAM bytes of one planner launch of this workload from one ncu capture
                        # (dram__bytes.sum.per_second x gpu__time_duration, profiles/explore_kernel_uneven512_eager.md):
                        # the trees, radii and scenes live in L1/L2, so the planner hardly touches HBM
-                       "traffic": 7.4e6, "traffic_unit": "bytes per launch (ncu)",
+                       "traffic": 7.3e6, "traffic_unit": "bytes per launch (ncu)",
                        "peak_source": "measured in bench.py, the faster of the scalar FFMA and packed fma.rn.f32x2 "
                                       "probes (no FP32 entry in MEASURED_PEAKS.json)",
                        "launch_ms": ms, "launches_timed": n_time, "launches_counted": n_stat,
@@ -988,13 +988,13 @@ def measure_nn(torch, dev, peaks, reps: int = 3, launches: int = 20):
     return {"nn_kernel": {"workload": "1 query x 33554432 nodes x 7 dims (940 MB tree, HBM-streamed)",
                           "ms": ms_h, "achieved_gbs": gbs_h, "hbm_peak_gbs": hbm,
                           "frac": gbs_h / hbm if hbm else None,
-                          # one ncu capture (profiles/nn_kernel_1q_32M_hbm.md): 6.34 TB/s x 148.9 us
+                          # one ncu capture (profiles/nn_scan_kernel_1q_32M_hbm.md): 6.79 TB/s x 139.1 us
                           "traffic_bytes_ncu": 944e6,
                           "note": "algorithmic bytes = nodes x dim x 4 per query; per-launch time of 20 "
                                   "back-to-back launches (init of the 64-bit argmin keys, scan, decode)"},
             "nn_kernel_l2": {"workload": "64 queries x 4194304 nodes x 7 dims (117 MB tree, L2-resident)",
                              "ms": ms_l, "achieved_gbs": by_l / (ms_l * 1e-3) / 1e9,
-                             "note": "each query re-reads the tree from L2, so the rate exceeds HBM peak"}}
+                             "note": "64 queries share a pass over the tree; the rate counts its bytes for each"}}
 
 
 # ----------------------------------------------------------------------------- the other configurations

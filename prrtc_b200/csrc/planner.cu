@@ -852,10 +852,10 @@ __device__ __forceinline__ void run_explorer(const Grp& grp, const PlanLaunch& L
 // cycle and scheduler, its warps waiting for fixed-latency results and shared
 // memory.  So an explorer gets 128 registers per thread (80 and three CTAs per
 // SM measured 8-12% slower per plan, no faster per batch), and more threads
-// where SMs are idle (launch_plan).  Against the general
-// checker, kernel times: 152 -> 95 us (16 spheres, 128 explorers), 2.50 -> 1.60
-// ms (512 uneven problems, E = 2), 4.74 -> 2.57 ms (200 tabletop problems, E =
-// 1), 34.1 -> 5.6 ms (61 dual-arm problems, E = 1).
+// where SMs are idle (launch_plan).  Kernel times, medians of 20, against the general
+// checker: 136 -> 82 us (16 spheres, 128 explorers), 2.38 -> 1.42 ms (512 uneven
+// problems, E = 2), 4.71 ms -> 2.83 with 256 threads and 2.57 with 512 (200 tabletop
+// problems, E = 1), 34.2 -> 6.78 and 5.59 ms (61 dual-arm problems, E = 1).
 template <bool CULL, int THREADS, int MINBLOCKS>
 __global__ void __launch_bounds__(THREADS, MINBLOCKS) explore_kernel(PlanLaunch L) {
     extern __shared__ __align__(128) unsigned char dsm[];
@@ -1107,7 +1107,7 @@ cudaError_t launch_plan(PlanLaunch& L, cudaStream_t st) {
     // one CTA per SM.  E = 1, a call in ms with 256 -> 512 threads: tabletop, 100
     // problems 2.15 -> 1.96, 200 3.89 -> 3.72, 296 3.99 -> 3.86; dual arm, 61 7.03 ->
     // 5.61, 149 9.92 -> 7.19, 296 11.04 -> 8.82; at E = 2 x 512 problems it loses,
-    // 4.4 -> 4.7.  So does a plain launch of at most one explorer per SM.
+    // 4.4 -> 4.7.  A plain launch of at most one explorer per SM gets 512 as well.
     const long long explorers = (long long)L.B * L.E;
     const bool wide = L.threads == 0 && explorers <= (L.persistent ? 2ll : 1ll) * device_sm_count();
     const bool one_per_sm = wide || explorers <= device_sm_count();

@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(256, DB <= 2 ? 3 : 2) nn_scan_kernel(const flo
 // and are shared as above.
 //
 // Bound by the latency of its own chain (16 warps per SM issue half the time; the
-// tensor pipe is 25% busy, and the tree's 117 MB would take 18 us): 64 queries, 4.19
+// tensor pipe is 35% busy, and the tree's 117 MB would take 18 us): 64 queries, 4.19
 // M nodes x 7: 146 -> 58 us for the call's kernels, 14 dimensions 244 -> 98. A step
 // of 32 nodes per warp took 65 us, the norm as one more dimension summed by
 // shuffles 65 us, sums started from the best distance 73 us.
@@ -646,14 +646,14 @@ static void check_go(const CheckLaunch& o, int full_sweep, const unsigned char* 
 // The culled checker: warps of their own, CW configurations at a time
 // (warp_check), the scene staged per CTA.
 //
-// Bound by instruction issue (65% of the issue slots, 16 to 24 warps per SM),
+// Bound by instruction issue (75% of the issue slots, 22 warps per SM),
 // not by memory: of the time of 2^20 random tabletop configurations (79% in
 // collision) link frames take a quarter, self items a third, the links'
 // primitives the rest.  80 registers per thread and 24 warps per SM measured 15%
 // faster than 128 and 16; world links before self items 6% faster here but 20%
-// slower on uneven scenes.  Against the full sweep of the general checker: 2^20
-// tabletop configurations 2117 -> 800 us, uneven scene 2055 -> 870 us, 60,000
-// dual-arm configurations 1332 -> 280 us (gated) and 981 -> 280 us (flat).
+// slower on uneven scenes.  Against the general checker: 2^20 tabletop
+// configurations 2112 -> 773 us (gated 2321 -> 830), uneven scene 2052 -> 805 us
+// (gated 1301 -> 825), 60,000 dual-arm configurations 976 -> 253 us (gated 1333).
 //
 // A scene that is not culled (BlobHeader::cull: groups that do not cover the
 // spheres, ...) takes the general checker in the same shared memory, by the whole

@@ -485,13 +485,13 @@ cudaError_t launch_smooth_update(float* x, const float* g, const float* norms, c
 // left in shared memory for each sphere's warp to add after a barrier took 571 us.
 // (The cost is added up by atomics.)
 //
-// Bound by instruction issue and, close behind, the special-function pipe (a
-// reciprocal square root and an exponential per pair, two reciprocals more near
-// contact): 67% of the issue slots, 58 instructions per pair and warp.  Against a
-// warp per waypoint with a sphere per lane (smooth_kernel), 4,376 pairs each:
-// 512 paths x 64 waypoints, tabletop scene, 858 -> 353 us; 40 dual-arm paths x 96
-// waypoints (44,360 pairs) 920 -> 385 us a call.  One sphere at a time instead of
-// two measured 379 us, the library's exponential and reciprocal square root 512 us.
+// Bound by instruction issue: 77% of the issue slots, 51 instructions per computed
+// pair and warp (a reciprocal square root and an exponential each, two reciprocals
+// more near contact: the special-function pipe is 31% busy).  Against a warp per
+// waypoint with a sphere per lane (smooth_kernel), 4,376 pairs each: 512 paths x 64
+// waypoints, tabletop scene, 858 -> 322 us of kernel time; 40 dual-arm paths x 96
+// waypoints (44,360 pairs) 920 -> 346 us a call.  One sphere at a time instead of
+// two was 7% slower, the library's exponential and reciprocal square root 45%.
 struct SmoothBufs {
     float* pose;    // [32][J][12]
     float* ctr;     // [S][3][32] (the radius is the scene's)
