@@ -727,7 +727,8 @@ __global__ void __launch_bounds__(256, 3) check_cull_kernel(const unsigned char*
             if (full_sweep) check_general<true>(dsm, pairs, &pc, dsm + blob_cap, general_cw, configs, n, dim, verdicts);
             else check_general<false>(dsm, pairs, &pc, dsm + blob_cap, general_cw, configs, n, dim, verdicts);
         } else {
-            for (int i = blockIdx.x * blockDim.x + tid; i < n; i += gridDim.x * blockDim.x) verdicts[i] = 0;
+            for (long long i = (long long)blockIdx.x * blockDim.x + tid; i < n; i += (long long)gridDim.x * blockDim.x)
+                verdicts[i] = 0;
         }
         return;
     }
