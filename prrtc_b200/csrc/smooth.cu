@@ -175,10 +175,10 @@ __global__ void __launch_bounds__(WARPS * 32) smooth_kernel(SmoothArgs a, int bl
         w = (blockIdx.x - p * per_path) * WARPS + warp;
         mine = w < a.W;
     } else {
-        const int c = blockIdx.x * WARPS + warp;
-        p = c / a.W;
-        w = c - p * a.W;
-        mine = c < a.P * a.W;
+        const long long c = (long long)blockIdx.x * WARPS + warp;
+        p = (int)(c / a.W);
+        w = (int)(c - (long long)p * a.W);
+        mine = c < (long long)a.P * a.W;
     }
     const unsigned char* gblob = a.blob + (size_t)p * a.blob_stride;  // stride 0 where a CTA spans paths
     if constexpr (STAGED) {
