@@ -51,11 +51,11 @@ size_t blob_stride(const PackSrc& s) {
 
 __device__ __forceinline__ int clampi(int x, int lo, int hi) { return x < lo ? lo : (x > hi ? hi : x); }
 
+constexpr float kCullStretchMax = 1e8f;  // box axes and normals of a length of up to 10,000 (squared) are culled
+constexpr int kPackThreads = 512;
+
 // Exclusive prefix of one value per thread over a CTA of kPackThreads, plus the
 // CTA total.
-constexpr int kPackThreads = 512;
-constexpr float kCullStretchMax = 1e8f;  // box axes and normals of a length of up to 10,000 (squared) are culled
-
 __device__ __forceinline__ int pack_exclusive_scan(int v, int* warp_sums, int& total) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int inc = v;
